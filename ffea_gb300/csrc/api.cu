@@ -115,6 +115,7 @@ void set_last_error(const char *msg) { g_last_error = msg; }
 struct ffea_gpu {
     HostBatch host;
     DeviceBatch dev;
+    GroupBatch group;                            // when dev.group points to it
     DeviceArena arena;
     cudaStream_t stream = nullptr;
     cudaGraphExec_t step_exec = nullptr;
@@ -344,6 +345,100 @@ std::vector<int32_t> deal_segments(const HostBatch &H, int G)
     }
     return order;
 }
+
+// The groups of k_cg_group: which CTA solves which segments, in which order,
+// and the rows of other segments each segment couples to.
+struct GroupPlan {
+    std::vector<int32_t> ptr, task;   // per CTA: its segments
+    std::vector<int32_t> hptr, halo;  // per segment: its halo rows, ascending
+    int max_rows = 0, max_halo = 0, max_segs = 0;
+};
+
+// One CTA per segment; false when a blob has more segments than CTAs.
+// Longest solve first (iterations grow with the radius, an iteration with
+// the rows of a CTA), each blob on the CTAs that are free first.  Every CTA
+// runs its segments in this order, so waiting for a group's CTAs cannot form
+// a cycle.  Sets g.grid.
+bool plan_groups(const HostBatch &H, int ctas, GroupBatch &g, GroupPlan &plan)
+{
+    const int nb = H.num_blobs, ns = (int)H.seg_row0.size();
+    std::vector<int32_t> blobs(nb);
+    std::vector<double> cost(nb);
+    for (int b = 0; b < nb; b++) {
+        const BlobParams &bp = H.bp[b];
+        if (bp.seg_cnt > ctas) return false;
+        blobs[b] = b;
+        int rows = 0;
+        for (int s = bp.seg_off; s < bp.seg_off + bp.seg_cnt; s++) rows = std::max(rows, H.seg_rows[s]);
+        plan.max_rows = std::max(plan.max_rows, rows);
+        plan.max_segs = std::max(plan.max_segs, bp.seg_cnt);
+        cost[b] = std::cbrt((double)bp.node_cnt) * (500.0 + rows);
+    }
+    if (plan.max_rows > CG_SEG_MAX_ROWS) return false;
+    // halos
+    std::vector<int32_t> seen(H.nl_pad, -1);
+    plan.hptr.assign(1, 0);
+    for (int s = 0; s < ns; s++) {
+        const int r0 = H.seg_row0[s], r1 = r0 + H.seg_rows[s];
+        const size_t h0 = plan.halo.size();
+        for (int r = r0; r < r1; r++)
+            for (int j = 0; j < H.slice_len[r >> 5]; j++) {
+                const int q = H.sell_col[H.slice_ptr[r >> 5] + 32 * j + (r & 31)];
+                if ((q < r0 || q >= r1) && seen[q] != s) {
+                    seen[q] = s;
+                    plan.halo.push_back(q);
+                }
+            }
+        std::sort(plan.halo.begin() + h0, plan.halo.end());
+        plan.hptr.push_back((int32_t)plan.halo.size());
+        plan.max_halo = std::max(plan.max_halo, (int)(plan.halo.size() - h0));
+    }
+    if (plan.max_halo > 32768) return false;  // (16-bit places)
+    // the schedule
+    g.grid = std::min(ctas, ns);
+    std::stable_sort(blobs.begin(), blobs.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+    const int G = g.grid;
+    std::vector<double> busy(G, 0.0);
+    std::vector<int> order(G);
+    std::vector<std::vector<int32_t>> per(G);
+    for (int b : blobs) {
+        const BlobParams &bp = H.bp[b];
+        for (int c = 0; c < G; c++) order[c] = c;
+        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return busy[x] < busy[y]; });
+        const double end = busy[order[bp.seg_cnt - 1]] + cost[b];
+        // segments to CTAs in CTA order: neighbours in the blob on neighbouring CTAs
+        std::sort(order.begin(), order.begin() + bp.seg_cnt);
+        for (int k = 0; k < bp.seg_cnt; k++) {
+            per[order[k]].push_back(bp.seg_off + k);
+            busy[order[k]] = end;
+        }
+    }
+    plan.ptr.assign(1, 0);
+    for (const auto &v : per) {
+        plan.task.insert(plan.task.end(), v.begin(), v.end());
+        plan.ptr.push_back((int32_t)plan.task.size());
+    }
+    return true;
+}
+
+// Per matrix entry its column's place in the CTA's copy of u: the local row,
+// or `rows` + its place in the segment's halo.
+std::vector<uint16_t> group_columns(const HostBatch &H, const GroupPlan &plan, int rows)
+{
+    std::vector<uint16_t> out(H.sell_col.size(), 0);
+    std::vector<int32_t> place(H.nl_pad, 0);
+    for (size_t s = 0; s + 1 < plan.hptr.size(); s++) {
+        const int r0 = H.seg_row0[s], r1 = r0 + H.seg_rows[s];
+        for (int k = plan.hptr[s]; k < plan.hptr[s + 1]; k++) place[plan.halo[k]] = rows + (k - plan.hptr[s]);
+        for (int r = r0; r < r1; r++)
+            for (int j = 0; j < H.slice_len[r >> 5]; j++) {
+                const size_t e = (size_t)H.slice_ptr[r >> 5] + 32 * j + (r & 31);
+                const int q = H.sell_col[e];
+                out[e] = (uint16_t)(q >= r0 && q < r1 ? q - r0 : place[q]);
+            }
+    }
+    return out;
+}
 }  // namespace
 
 int ffea_gpu_create_batch(int32_t num_blobs, const ffea_gpu_mesh *meshes, const ffea_gpu_params *params,
@@ -354,21 +449,21 @@ int ffea_gpu_create_batch(int32_t num_blobs, const ffea_gpu_mesh *meshes, const 
     if (rng_mode != FFEA_GPU_RNG_PER_BLOB && rng_mode != FFEA_GPU_RNG_SHARED) return fail("unknown rng_mode");
     std::unique_ptr<ffea_gpu> h(new ffea_gpu());
     std::string err;
-    // persistent CG kernel: all CTAs co-resident (cooperative launch); the
-    // register-resident variant when every CG segment gets a CTA of its own.
+    // persistent CG kernel: all CTAs co-resident (cooperative launch);
+    // k_cg_group when every blob's CG segments fit the grid.
     // FFEA_GPU_CG_MAX_CTAS caps the grid, FFEA_GPU_CG_MEMORY_STATE=1 keeps the
-    // segments but runs the memory-resident variant (both for tests).
+    // segments but runs the memory-resident kernel, FFEA_GPU_CG_LAST_ARRIVER=1
+    // runs it with its last-arriver reduction (all three for tests).
     if (num_blobs <= 0) return fail("num_blobs must be >= 1");
     const int prec = params[0].precision;
-    const int reg_grid0 = cg_max_grid(prec, 1, 0);
-    const int max_grid = cg_max_grid(prec, 0, cg_mem_defer_bytes(prec));
-    const bool sized = reg_grid0 > 0 && max_grid > 0;
+    const int max_grid = cg_max_grid(prec, cg_mem_defer_bytes(prec));
+    const bool sized = max_grid > 0;
     int cap = std::numeric_limits<int>::max();
     if (const char *e = std::getenv("FFEA_GPU_CG_MAX_CTAS")) cap = std::max(1, std::atoi(e));
     const int mem_cap = std::min(max_grid, cap);
     // the input is validated first, so that its errors are reported even
     // where no device is usable
-    if (!build_batch(num_blobs, meshes, params, rng_mode, sized ? std::min(reg_grid0, cap) : 1, h->host, err))
+    if (!build_batch(num_blobs, meshes, params, rng_mode, sized ? mem_cap : 1, h->host, err))
         return fail("%s", err.c_str());
     if (!sized) return fail("cannot size the persistent CG kernel on this device");
     HostBatch &H = h->host;
@@ -380,10 +475,7 @@ int ffea_gpu_create_batch(int32_t num_blobs, const ffea_gpu_mesh *meshes, const 
     int max_cols = 0;
     for (int32_t L : H.slice_len) max_cols = std::max(max_cols, (int)L);
     const int32_t n_segs = plan_cg_segments(H);
-    // two-level preconditioner: NoMass blobs, mixed precision.  The
-    // register-resident kernel carries it with one segment per CTA, local
-    // reductions and at most CG_THREADS coarse dofs per blob; every other
-    // batch runs it in the memory-resident kernel
+    // two-level preconditioner: NoMass blobs, mixed precision
     const int want = params[0].preconditioner;
     for (int b = 1; b < num_blobs; b++)
         if (params[b].preconditioner != want) return fail("all blobs of a batch must use the same preconditioner");
@@ -395,36 +487,37 @@ int ffea_gpu_create_batch(int32_t num_blobs, const ffea_gpu_mesh *meshes, const 
     bool coarse_ok = want != FFEA_GPU_PRECOND_JACOBI && H.precision == PREC_MIXED && !H.any_mass && !H.any_lumped &&
                      coarse_total <= INT32_MAX && H.coarse_htotal <= INT32_MAX;
     for (const BlobParams &bp : H.bp) coarse_nmax = std::max(coarse_nmax, (int)bp.coarse_n);
-    const bool coarse_reg_ok = coarse_ok && coarse_nmax <= CG_THREADS;
-    // phi per row, the CTA's six rows of X, c, 6 x 32 reduction floats and
-    // the carried P^T s per coarse dof
-    const size_t coarse_bytes =
-        coarse_reg_ok ? 16 + 16 * (size_t)CG_THREADS +
-                        sizeof(float) * (6 * (size_t)coarse_nmax + 8 + 6 * 32 + (size_t)CG_THREADS)
-                  : 0;
-    size_t dyn_bytes = 0;
-    int cache_slots = 0, cache_cols = 0;
-    if (cg_smem_plan(H.precision, max_slots, max_cols, coarse_bytes, &cache_slots, &cache_cols, &dyn_bytes) != 0)
-        return fail("cannot size the shared memory of the CG kernel");
-    const int reg_grid = cg_max_grid(H.precision, 1, dyn_bytes);
-    if (reg_grid <= 0) return fail("cannot size the persistent CG kernel on this device");
-    const int reg_cap = std::min(reg_grid, cap);
-    const char *force_mem = std::getenv("FFEA_GPU_CG_MEMORY_STATE");
+    d.num_blobs = H.num_blobs;
     d.n_segs = n_segs;
-    d.cg_reg = n_segs <= reg_cap && !(force_mem && force_mem[0] == '1');
-    d.cg_grid = n_segs <= reg_cap ? n_segs : std::min(mem_cap, n_segs);
-    d.cg_cache_slots = d.cg_reg ? cache_slots : 0;
-    d.cg_cache_cols = d.cg_reg ? cache_cols : 0;
-    d.cg_dyn_smem = d.cg_reg ? (int32_t)dyn_bytes : (int32_t)cg_mem_defer_bytes(H.precision);
-    if ((int64_t)d.cg_grid * CG_MAX_SEGS < n_segs)
-        return fail("batch too large: %d CG segments need more than %d co-resident CTAs", n_segs, mem_cap);
-    // local reduction (every CTA sums all partials, no serial last-arriver
-    // step) while that read stays small
+    d.precision = H.precision;
+    d.any_mass = H.any_mass;
+    d.any_nomass = H.any_nomass;
+    d.any_lumped = H.any_lumped;
+    const char *force_mem = std::getenv("FFEA_GPU_CG_MEMORY_STATE");
     const char *force_last = std::getenv("FFEA_GPU_CG_LAST_ARRIVER");
-    d.cg_local = H.num_blobs <= CG_LOCAL_MAX_BLOBS && n_segs <= CG_LOCAL_MAX_SEGS &&
-                 !(force_last && force_last[0] == '1');
-    d.coarse = coarse_reg_ok && d.cg_reg && d.cg_local;
-    if (coarse_ok && !d.coarse) {
+    const bool last_arriver = force_last && force_last[0] == '1';
+    if ((int64_t)std::min(mem_cap, n_segs) * CG_MAX_SEGS < n_segs)
+        return fail("batch too large: %d CG segments need more than %d co-resident CTAs", n_segs, mem_cap);
+    GroupPlan groups;
+    if (!(force_mem && force_mem[0] == '1') && !last_arriver) {
+        d.coarse = coarse_ok;
+        d.coarse_nmax = coarse_ok ? coarse_nmax : 0;
+        GroupBatch &g = h->group;
+        if (plan_groups(H, mem_cap, g, groups) &&
+            cg_group_plan(d, g, max_slots, max_cols, groups.max_rows, groups.max_halo, groups.max_segs) == 0 &&
+            cg_group_max_grid(d, g) >= g.grid)
+            d.group = &g;
+        else
+            d.coarse = 0;
+    }
+    if (!d.group) {
+        d.cg_grid = std::min(mem_cap, n_segs);
+        d.cg_dyn_smem = (int32_t)cg_mem_defer_bytes(H.precision);
+    }
+    // memory-resident kernel: local reduction (every CTA sums all partials, no
+    // serial last-arriver step) while that read stays small
+    d.cg_local = H.num_blobs <= CG_LOCAL_MAX_BLOBS && n_segs <= CG_LOCAL_MAX_SEGS && !last_arriver;
+    if (coarse_ok && !d.group) {
         // the memory-resident kernel with the coarse space: its shared memory
         // holds g of one blob and P^T s of every blob a CTA touches
         const int G = std::min(mem_cap, n_segs);
@@ -444,11 +537,9 @@ int ffea_gpu_create_batch(int32_t num_blobs, const ffea_gpu_mesh *meshes, const 
         }
         const size_t mem_bytes = cg_mem_defer_bytes(H.precision) + cg_mem_coarse_bytes(hmax);
         if ((int64_t)G * CG_MAX_SEGS >= n_segs && cg_mem_smem_allow(H.precision, mem_bytes) == 0 &&
-            cg_max_grid(H.precision, 0, mem_bytes) >= G) {
+            cg_max_grid(H.precision, mem_bytes) >= G) {
             d.coarse = 1;
-            d.cg_reg = 0;
             d.cg_grid = G;
-            d.cg_cache_slots = d.cg_cache_cols = 0;
             d.cg_dyn_smem = (int32_t)mem_bytes;
             d.coarse_hmax = hmax;
         }
@@ -456,17 +547,12 @@ int ffea_gpu_create_batch(int32_t num_blobs, const ffea_gpu_mesh *meshes, const 
     d.coarse_nmax = d.coarse ? coarse_nmax : 0;
     d.part_stride = d.coarse ? 20 : 8;  // floats: DF dot terms 0..5; coarse P^T r 8..13, P^T w 14..19
     h->precond = d.coarse ? want : FFEA_GPU_PRECOND_JACOBI;
-    d.num_blobs = H.num_blobs;
     d.nl_pad = H.nl_pad;
     d.ne_pad = H.ne_pad;
     d.n_edges = H.n_edges;
     d.n_tiles = H.n_tiles;
     d.n_etiles = H.n_etiles;
     d.num_streams = H.num_streams;
-    d.precision = H.precision;
-    d.any_mass = H.any_mass;
-    d.any_nomass = H.any_nomass;
-    d.any_lumped = H.any_lumped;
     const size_t ts = H.precision == PREC_FP64 ? sizeof(double) : sizeof(float);
     h->tsize = ts;
     CK(upload(A, d.bp, H.bp));
@@ -475,7 +561,16 @@ int ffea_gpu_create_batch(int32_t num_blobs, const ffea_gpu_mesh *meshes, const 
     CK(upload(A, d.seg_row0, H.seg_row0));
     CK(upload(A, d.seg_rows, H.seg_rows));
     CK(upload(A, d.seg_blob, H.seg_blob));
-    if (!d.cg_reg) {
+    if (d.group) {
+        GroupBatch &g = h->group;
+        CK(upload(A, g.ptr, groups.ptr));
+        CK(upload(A, g.task, groups.task));
+        CK(upload(A, g.hptr, groups.hptr));
+        CK(upload(A, g.halo, groups.halo));
+        CK(upload(A, g.lcol, group_columns(H, groups, g.rows)));
+        CK(A.alloc(g.words, 2 * (size_t)GRP_WORDS * n_segs));
+        CK(A.alloc(g.pub, (size_t)(H.precision == PREC_FP64 ? 3 : 1) * H.nl_pad));
+    } else {
         const std::vector<int32_t> order = deal_segments(H, d.cg_grid);
         if (!order.empty()) CK(upload(A, d.seg_order, order));
     }
@@ -561,7 +656,7 @@ int ffea_gpu_create_batch(int32_t num_blobs, const ffea_gpu_mesh *meshes, const 
         CK(cudaMemcpy(d.phi, H.phi.data(), H.phi.size() * sizeof(float), cudaMemcpyHostToDevice));
         CK(A.alloc(d.coarse_A, (size_t)coarse_total));
         CK(A.alloc(d.coarse_X, (size_t)coarse_total));
-        if (!d.cg_reg) {
+        if (!d.group) {
             // the memory-resident kernel reads X every iteration from global
             // memory: an FP16 copy, scaled to unit diagonal, halves that read
             size_t dofs = 0;
@@ -582,7 +677,7 @@ int ffea_gpu_create_batch(int32_t num_blobs, const ffea_gpu_mesh *meshes, const 
     CK(A.alloc(d.status, (size_t)H.num_blobs));
     CK(A.alloc(d.inverted, (size_t)H.num_blobs));
     CK(A.alloc(d.energy, 2 * (size_t)H.num_blobs));
-    CK(A.alloc(d.bar, 8));
+    CK(A.alloc(d.bar, 16));
     CK(A.alloc(d.loop_count, 1));
     // a blocking stream: the zero fills (cudaMemset) and host-to-device
     // copies (cudaMemcpy) that set up and update the handle's buffers run on

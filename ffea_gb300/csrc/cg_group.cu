@@ -1,0 +1,994 @@
+// cg_group.cu -- the CG solve of blobs that fit on chip.
+//
+// One persistent cooperative launch solves every blob of a batch to
+// convergence.  A blob's CG segments (at most CG_SEG_MAX_ROWS rows each) are
+// its group of CTAs, one segment per CTA.  Groups are independent: each
+// exchanges only among its own CTAs and stops when its own blob has
+// converged, and a CTA then goes on to the next segment of its list.  Every
+// CTA's list follows one order of the blobs, so a group's CTAs wait for each
+// other without a cycle.
+//
+// The recurrences, the stopping rule and the order of every FP32 sum are
+// those of the memory-resident solve (k_cg in kernels.cu): Jacobi- or
+// two-level-PCG in the Chronopoulos-Gear form, one product and one group of
+// sums per iteration.
+//
+// What bounds an iteration is the latency of its two exchanges and of the
+// instructions between them and, for full segments, the L2 reads of the
+// matrix.  So nothing waits on a barrier word:
+//   - u is published row by row as one 128-bit store (x, y, z, tag); a CTA
+//     reads the rows its segment couples to (its halo, each row once) until
+//     their tags are the iteration's, into shared memory beside its own rows,
+//     and the product's inner loop reads shared memory alone;
+//   - a segment's partial sums are published the same way, and every CTA of
+//     the group reads all of them: a few warps wait for the dot terms, and the
+//     coarse restrictions are read once those are in, while the CG transition
+//     runs.
+// Two things decide the time of an exchange (152 CTAs, alone, in thousand
+// cycles): words of one CTA leave in whole 32-byte sectors (2.0; stored 16
+// bytes at a time into sectors that others are reading, 7 to 9), and few
+// threads wait (with one in every thread 4.5: their reads hold up the stores
+// they wait for).  A counter that all CTAs add to took 3.6.
+// The tag travels in the same single-copy-atomic word as the value, so no
+// fence, no counter and no second round trip is needed.  A row of u is
+// rewritten only after its CTA has read the group's sums of the iteration,
+// which every CTA publishes after its last read of u; the sums alternate
+// between two buffers for the same reason.  Tags never repeat from one launch
+// to the next (the base in bar[6] grows by the tags a launch used).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "cg_common.cuh"
+#include "kernels.h"
+#include "mrg32k3a.cuh"
+
+namespace ffea {
+
+namespace {
+
+extern __shared__ __align__(16) unsigned char grp_dyn[];
+
+template <typename X>
+__device__ __forceinline__ X *dyn(int32_t off)
+{
+    return reinterpret_cast<X *>(grp_dyn + off);
+}
+
+// ---------------------------------------------------------------- tagged words
+__device__ __forceinline__ void st_b128(void *p, uint64_t lo, uint64_t hi)
+{
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+                 "l"(lo), "l"(hi)
+                 : "memory");
+}
+__device__ __forceinline__ void ld_b128(const void *p, uint64_t &lo, uint64_t &hi)
+{
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(lo), "=l"(hi)
+                 : "l"(p));
+}
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) { return (uint64_t)hi << 32 | lo; }
+
+// A published row: x, y, z and the tag, in one 128-bit word (FP32), or each
+// component with the tag in its own plane of n words (FP64: neighbouring rows
+// then store whole sectors).
+template <typename T> struct PubRow;
+template <> struct PubRow<float> {
+    float x, y, z;
+    uint32_t tag;
+    static __device__ __forceinline__ void put(uint4 *base, int, int row, const float v[3], uint32_t tag)
+    {
+        st_b128(base + row, pack2(__float_as_uint(v[0]), __float_as_uint(v[1])), pack2(__float_as_uint(v[2]), tag));
+    }
+    __device__ __forceinline__ void get(const uint4 *base, int, int row)
+    {
+        uint64_t lo, hi;
+        ld_b128(base + row, lo, hi);
+        x = __uint_as_float((uint32_t)lo);
+        y = __uint_as_float((uint32_t)(lo >> 32));
+        z = __uint_as_float((uint32_t)hi);
+        tag = (uint32_t)(hi >> 32);
+    }
+    __device__ __forceinline__ bool is(uint32_t t) const { return tag == t; }
+};
+template <> struct PubRow<double> {
+    double x, y, z;
+    uint32_t tag, tag1, tag2;
+    static __device__ __forceinline__ void put(uint4 *base, int n, int row, const double v[3], uint32_t tag)
+    {
+#pragma unroll
+        for (int k = 0; k < 3; k++) st_b128(base + (size_t)k * n + row, (uint64_t)__double_as_longlong(v[k]), tag);
+    }
+    __device__ __forceinline__ void get(const uint4 *base, int n, int row)
+    {
+        uint64_t a, b, c, ta, tb, tc;
+        ld_b128(base + row, a, ta);
+        ld_b128(base + (size_t)n + row, b, tb);
+        ld_b128(base + 2 * (size_t)n + row, c, tc);
+        x = __longlong_as_double((long long)a);
+        y = __longlong_as_double((long long)b);
+        z = __longlong_as_double((long long)c);
+        tag = (uint32_t)ta;
+        tag1 = (uint32_t)tb;
+        tag2 = (uint32_t)tc;
+    }
+    __device__ __forceinline__ bool is(uint32_t t) const { return tag == t && tag1 == t && tag2 == t; }
+};
+
+constexpr unsigned int kGroupSpins = 1u << 22;  // reads of one word, a few seconds, then give up
+
+// Whether a wait goes on: bounded, and given up when another wait of the CTA
+// or of the grid has run out (bar[4]).  A wait that runs out raises both.
+__device__ __noinline__ bool keep_waiting(unsigned int &spins, volatile int *s_err, unsigned int *bar)
+{
+    if ((++spins & 63u) == 0 && (spins > kGroupSpins || *s_err || ((volatile unsigned int *)bar)[4])) {
+        *s_err = 1;
+        atomicExch(&bar[4], 1u);
+        return false;
+    }
+    return true;
+}
+
+// Words a thread waits for at once when it reads the restrictions.
+constexpr int kBulk = 3;
+
+// The first n of N words, `stride` words apart, once each carries the tag: a
+// round reads every word still missing, so that it takes one trip to L2
+// however many are late.
+template <int N>
+__device__ __forceinline__ void wait_words(const uint4 *p, int stride, int n, uint32_t tag, uint64_t (&lo)[N],
+                                           uint64_t (&hi)[N], volatile int *s_err, unsigned int *bar)
+{
+    unsigned int spins = 0;
+    bool missing[N], any;
+#pragma unroll
+    for (int g = 0; g < N; g++) missing[g] = g < n;
+    do {
+#pragma unroll
+        for (int g = 0; g < N; g++)
+            if (missing[g]) ld_b128(p + (size_t)g * stride, lo[g], hi[g]);
+        any = false;
+#pragma unroll
+        for (int g = 0; g < N; g++) {
+            if (missing[g]) missing[g] = (uint32_t)(hi[g] >> 32) != tag;
+            any |= missing[g];
+        }
+    } while (any && keep_waiting(spins, s_err, bar));
+}
+
+// The row again until it carries the tag (the slow path of a neighbour read).
+template <typename T>
+__device__ __noinline__ PubRow<T> wait_row(const uint4 *base, int n, int row, uint32_t tag, volatile int *s_err,
+                                           unsigned int *bar)
+{
+    PubRow<T> y;
+    unsigned int spins = 0;
+    do y.get(base, n, row);
+    while (!y.is(tag) && keep_waiting(spins, s_err, bar));
+    return y;
+}
+
+// transition_core out of line: its FP64 arithmetic (64 issue slots an
+// instruction on GB300) stays out of the iteration's code.
+__device__ __noinline__ bool transition_any(CgScalars *cg, const BlobParams *bp, const DF *sums, int *bits, bool fast)
+{
+    return transition_core(*cg, *bp, sums, bits, fast);
+}
+
+// An RNG stream's state one step's draws on.
+__device__ __noinline__ void advance_stream(uint32_t *state, const mrg::JumpMat *step)
+{
+    uint32_t st[6];
+#pragma unroll 1
+    for (int i = 0; i < 6; i++) st[i] = state[i];
+    mrg::apply(*step, st);
+#pragma unroll 1
+    for (int i = 0; i < 6; i++) state[i] = st[i];
+}
+
+// A sum in three FP32 parts (about 70 bits): FP32 runs at 64 times the FP64
+// rate on GB300.
+struct Sum3 {
+    float s0, s1, s2;
+};
+__device__ __forceinline__ float two_sum(float a, float b, float &err)
+{
+    const float s = a + b, bb = s - a;
+    err = (a - (s - bb)) + (b - bb);
+    return s;
+}
+// S += K (dh + dl), the products exact (two FMAs each)
+__device__ __forceinline__ void add_product(Sum3 &S, float K, float dh, float dl)
+{
+    const float p = __fmul_rn(K, dh), e = fmaf(K, dh, -p);
+    const float q = __fmul_rn(K, dl), f = fmaf(K, dl, -q);
+    float t0, t1, t2, t3;
+    S.s0 = two_sum(S.s0, p, t0);
+    t0 = two_sum(t0, e, t1);
+    t0 = two_sum(t0, q, t2);
+    S.s1 = two_sum(S.s1, t0, t3);
+    S.s2 += (t1 + t2) + (t3 + f);
+}
+
+// Slots j0 .. j1 - 1 of a row's product A x added to a, with at least FP64
+// precision: entry e + 32 j, column places lcol into su, the row's own x in
+// xr (NoMass: difference form).  FP32 data: exact products and differences in
+// three-part sums on the FP32 pipes.  One FP64 instruction takes 64 issue
+// slots on GB300; in FP64 the 24 of a slot made the check of a 1,000-row CTA
+// take 80 us, the 330 FP32 ones take a fifth of that.
+__device__ __noinline__ void add_residual_slots(double (&a)[3], const float *val, const uint16_t *lcol, const float *su,
+                                                const float *xr, int e, int j0, int j1, bool nomass)
+{
+    const float x[3] = {nomass ? xr[0] : 0.f, nomass ? xr[1] : 0.f, nomass ? xr[2] : 0.f};
+    Sum3 S[3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+#pragma unroll 1
+    for (int j = j0; j < j1; j++) {
+        const float *y = su + 4 * (size_t)__ldg(&lcol[e + 32 * j]);
+        float dh[3], dl[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) dh[k] = two_sum(y[k], -x[k], dl[k]);
+        if (nomass) {
+            const float *v = val + sell_vidx(e + 32 * j, 0);
+            float K[9];
+#pragma unroll
+            for (int k = 0; k < 9; k++) K[k] = __ldg(&v[32 * k]);
+#pragma unroll
+            for (int i = 0; i < 3; i++)
+#pragma unroll
+                for (int k = 0; k < 3; k++) add_product(S[i], K[3 * i + k], dh[k], dl[k]);
+        } else {
+            const float m = __ldg(&val[e + 32 * j]);
+#pragma unroll
+            for (int k = 0; k < 3; k++) add_product(S[k], m, dh[k], dl[k]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) a[k] += (double)S[k].s0 + ((double)S[k].s1 + (double)S[k].s2);
+}
+
+// The same for FP64 data.
+__device__ __noinline__ void add_residual_slots(double (&a)[3], const double *val, const uint16_t *lcol,
+                                                const double *su, const double *xr, int e, int j0, int j1, bool nomass)
+{
+#pragma unroll 1
+    for (int j = j0; j < j1; j++) {
+        const double *y = su + 4 * (size_t)__ldg(&lcol[e + 32 * j]);
+        if (nomass) {
+            const double *K = val + sell_vidx(e + 32 * j, 0);
+#pragma unroll
+            for (int i = 0; i < 3; i++)
+#pragma unroll
+                for (int k = 0; k < 3; k++) a[i] += __ldg(&K[32 * (3 * i + k)]) * (y[k] - xr[k]);
+        } else {
+            const double m = __ldg(&val[e + 32 * j]);
+#pragma unroll
+            for (int k = 0; k < 3; k++) a[k] += m * y[k];
+        }
+    }
+}
+
+// The transition of an iteration that goes on, in FP32: transition_core's
+// arithmetic.  False, with nothing changed, where the solve may stop or fail.
+__device__ __forceinline__ bool transition_on(CgScalars &cg, int limit, const DF sums[3])
+{
+    const float g = sums[0].hi + sums[0].lo, dl = sums[1].hi + sums[1].lo, rr = sums[2].hi + sums[2].lo;
+    const int iters = cg.iters;
+    if (cg.state != CG_ACTIVE || (iters > 0 && rr < cg.stop_f) || !(rr == rr) || !(dl == dl) || iters >= limit)
+        return false;
+    const float beta = iters == 0 ? 0.f : g / cg.gamma_f;
+    const float pap = iters == 0 ? dl : fmaf(-beta * beta, cg.pap_f, dl);
+    if (!(pap > 0.f) || !(g > 0.f)) return false;
+    cg.beta_f = beta;
+    cg.pap_f = pap;
+    cg.alpha_f = g / pap;
+    cg.gamma_f = g;
+    cg.iters = iters + 1;
+    return true;
+}
+
+// Matrix slots per step of the product: values on chip, and values from L2 (9
+// registers in flight each).
+template <typename T, int MAXT> struct SlotDepth { static constexpr int kOn = 4, kOff = 4; };
+template <> struct SlotDepth<float, 1024> { static constexpr int kOn = 2, kOff = 2; };
+template <> struct SlotDepth<double, 512> { static constexpr int kOn = 2, kOff = 2; };
+template <> struct SlotDepth<double, 1024> { static constexpr int kOn = 1, kOff = 1; };
+
+// ---------------------------------------------------------------- the kernel
+// T: arithmetic type of the vectors and the matrix.  COARSE: the two-level
+// preconditioner (FP32).  MAXT: threads per CTA at most, which sets the
+// registers a thread may use and the strides of the shared-memory arrays.
+//
+// A thread has one row.  The values of a row's first cache_slots matrix
+// slots are in shared memory, the others come from L2.
+template <typename T, bool COARSE, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch gb)
+{
+    constexpr bool fast = sizeof(T) == 4;
+    constexpr bool kRegs = MAXT <= 512;      // x, D^-1, p and s in registers, else in shared memory
+    using Row = PubRow<T>;
+    using T2 = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
+    __shared__ double s_dot[3 * 32];         // per slice: r.u, w.u, r.r (T, or FP64 for the true residual)
+    __shared__ float s_res[12 * 32];         // per slice: P^T r, P^T w
+    __shared__ float s_red6[6 * 32];
+    __shared__ float s_cvec[8];
+    __shared__ CgScalars s_cg;
+    __shared__ float s_out[18];              // the segment's sums: r.u, w.u, r.r (hi, lo), P^T r, P^T w
+    __shared__ DF s_part[3 * 32];            // the dot terms summed over 32 segments of the group each
+    __shared__ DF s_last[3];                 // the sums of the last transition
+    __shared__ BlobParams s_bp;
+    __shared__ int s_err, s_stop;
+    const int tid = threadIdx.x, NT = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = NT >> 5;
+    const uint32_t base = __ldcg(&d.bar[6]);  // the tags of this launch start above it
+    T *const sx = dyn<T>(gb.o_state);         // x | D^-1 | p | s, 3 MAXT each (unless kRegs)
+    T *const su = dyn<T>(gb.o_u);             // u of the CTA's rows, then of its halo, (x, y, z, 0) each
+    uint4 *const pub = gb.pub;
+    uint32_t maxseq = 0;
+    int maxloops = 0;
+    if (tid == 0) s_err = s_stop = 0;
+
+#pragma unroll 1
+    for (int ti = gb.ptr[blockIdx.x]; ti < gb.ptr[blockIdx.x + 1]; ti++) {
+        const int seg = gb.task[ti], b = d.seg_blob[seg];
+        __syncthreads();  // the previous task is done with shared memory
+#pragma unroll 1
+        for (int k = tid; k < (int)(sizeof(BlobParams) / 4); k += NT)
+            reinterpret_cast<int *>(&s_bp)[k] = reinterpret_cast<const int *>(d.bp + b)[k];
+#pragma unroll 1
+        for (int k = tid; k < (int)(sizeof(CgScalars) / 4); k += NT)
+            reinterpret_cast<int *>(&s_cg)[k] = __ldcg(reinterpret_cast<const int *>(d.cg + b) + k);
+        const int row0 = d.seg_row0[seg], nrows = d.seg_rows[seg], nsl = (nrows + 31) >> 5;
+        __syncthreads();
+        const int cnt = s_bp.seg_cnt;          // segments of the group
+        const bool solo = cnt == 1;
+        const bool leader = seg == s_bp.seg_off;
+        const bool nomass = s_bp.solver == SOLVER_NOMASS;
+        const int cn = COARSE ? s_bp.coarse_n : 0;
+        const int limit = s_bp.solver == SOLVER_MASS ? s_bp.max_iter - 1 : s_bp.max_iter;
+        const bool run = s_cg.state == CG_ACTIVE;
+        const int h0 = gb.hptr[seg], nh = gb.hptr[seg + 1] - h0;  // halo rows
+        const int row = row0 + tid;
+        const bool in = tid < nrows;
+        const bool valid = in && !(d.flags[row] & NODE_PINNED);  // a free row of the segment
+        T diag = (T)0;
+        int L = 0, ebase = 0;  // slots of the row, its first entry
+        T r[3] = {0, 0, 0}, u[3] = {0, 0, 0}, w[3] = {0, 0, 0};
+        T st[4][kRegs ? 3 : 1];  // x, D^-1, p, s
+        auto state_of = [&](int f, int k) -> T & {
+            if constexpr (kRegs) return st[f][k];
+            else return sx[(3 * f + k) * MAXT + tid];
+        };
+#pragma unroll
+        for (int f = 0; f < 4; f++)
+#pragma unroll
+            for (int k = 0; k < 3; k++) state_of(f, k) = (T)0;
+        if (run) {
+            if (in) {
+                const size_t o = 3 * (size_t)row;
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    r[k] = static_cast<const T *>(d.r)[o + k];
+                    state_of(1, k) = static_cast<const T *>(d.dinv)[o + k];
+                }
+            }
+            if (valid) {
+                diag = nomass ? (T)(s_bp.calc_stokes == 1 ? d.drag[row] : 0.0)
+                                  : static_cast<const T *>(d.mass_diag)[row];
+                L = d.slice_len[row >> 5];
+                ebase = d.slice_ptr[row >> 5] + (row & 31);
+            }
+        }
+        // the row's neighbours (places in su) and matrix values on chip:
+        // constant during the solve
+        if (run && valid) {
+            uint16_t *col = dyn<uint16_t>(gb.o_col) + tid;
+#pragma unroll 1
+            for (int j = 0; j < min(gb.cache_cols, L); j++) col[j * MAXT] = gb.lcol[ebase + 32 * j];
+            T *kv1 = dyn<T>(gb.o_kv1) + tid;
+            T2 *kv2 = dyn<T2>(gb.o_kv2) + tid;
+#pragma unroll 1
+            for (int i = 0; i < min(gb.cache_slots, L); i++) {
+                const int e = ebase + 32 * i;
+                if (nomass) {
+                    const T *val = static_cast<const T *>(d.sell_val) + sell_vidx(e, 0);
+#pragma unroll
+                    for (int m = 0; m < 4; m++) {
+                        T2 kp;
+                        kp.x = val[32 * (2 * m)];
+                        kp.y = val[32 * (2 * m + 1)];
+                        kv2[(4 * i + m) * MAXT] = kp;
+                    }
+                    kv1[i * MAXT] = val[32 * 8];
+                } else {
+                    kv1[i * MAXT] = static_cast<const T *>(d.sell_mval)[e];
+                }
+            }
+        }
+        if (COARSE && run && in)
+            dyn<float4>(gb.o_phi)[tid] = valid ? d.phi[row] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (run) {
+            int *halo = dyn<int>(gb.o_halo);
+#pragma unroll 1
+            for (int k = tid; k < nh; k += NT) halo[k] = gb.halo[h0 + k];
+            if (COARSE) {
+                const float *Xg = d.coarse_X + s_bp.coarse_xoff + (size_t)(6 * (seg - s_bp.seg_off)) * cn;
+                float *xr = dyn<float>(gb.o_xrow), *h = dyn<float>(gb.o_h);
+#pragma unroll 1
+                for (int k = tid; k < 6 * cn; k += NT) xr[k] = Xg[k];
+#pragma unroll 1
+                for (int k = tid; k < cn; k += NT) h[k] = 0.f;
+            }
+#pragma unroll 1
+            for (int k = tid; k < 3 * 32; k += NT) s_dot[k] = 0.0;
+#pragma unroll 1
+            for (int k = tid; k < 12 * 32; k += NT) s_res[k] = 0.f;
+        }
+        __syncthreads();
+
+        uint32_t seq = 0;  // exchanges of this solve
+        int parity = 0, loops = -1;
+        // fresh: the vectors restart (the first trip, and after a failed true
+        // residual): no update.  first_coarse: the restriction of r_0, which
+        // the first u needs
+        bool fresh = true, first_coarse = COARSE;
+        bool going = run;
+        while (going) {
+            const int state = s_cg.state;
+            const uint32_t tag = base + ++seq;
+            const bool verify = state == CG_VERIFY;
+            const bool product = !verify && !first_coarse;
+            if (product) {
+                // phase A: p = u + beta p; s = w + beta s; x += alpha p;
+                // r -= alpha s; u = M r; publish u
+                T a, be;
+                cg_coefs<T>(s_cg, a, be);
+                if (valid) {
+                    if (!fresh) {
+                        const bool first = be == (T)0;
+#pragma unroll
+                        for (int k = 0; k < 3; k++) {
+                            T &p = state_of(2, k), &s = state_of(3, k);
+                            const T pn = first ? u[k] : u[k] + be * p;
+                            const T sn = first ? w[k] : w[k] + be * s;
+                            p = pn;
+                            s = sn;
+                            state_of(0, k) += a * pn;
+                            r[k] -= a * sn;
+                        }
+                    }
+                    T dinv[3];
+#pragma unroll
+                    for (int k = 0; k < 3; k++) dinv[k] = state_of(1, k);
+                    if (COARSE) {
+                        coarse_u_of<T>(dyn<float4>(gb.o_phi)[tid], s_cvec, dinv, r, u);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 3; k++) u[k] = dinv[k] * r[k];
+                    }
+                }
+                if (in) {
+                    if (!solo) Row::put(pub, d.nl_pad, row, u, tag);
+#pragma unroll
+                    for (int k = 0; k < 3; k++) su[4 * tid + k] = u[k];
+                }
+            } else if (verify) {
+                // publish x for the true residual
+                if (in) {
+                    const T xv[3] = {state_of(0, 0), state_of(0, 1), state_of(0, 2)};
+                    if (!solo) Row::put(pub, d.nl_pad, row, xv, tag);
+#pragma unroll
+                    for (int k = 0; k < 3; k++) su[4 * tid + k] = xv[k];
+                }
+            }
+            // the row's terms of r.u and r.r and its restriction of r, and
+            // their slice sums (a slice is a warp)
+            T pg = (T)0, pr = (T)0;
+            float ex[6] = {0, 0, 0, 0, 0, 0};
+            if (valid && product)
+#pragma unroll
+                for (int k = 0; k < 3; k++) {
+                    pg += r[k] * u[k];
+                    pr += r[k] * r[k];
+                }
+            if (COARSE && valid && !verify) restrict6_of<T>(dyn<float4>(gb.o_phi)[tid], r, ex);
+            if constexpr (fast) {
+                if (product) {
+                    constexpr int NV = COARSE ? 8 : 2;
+                    float v[NV];
+                    v[0] = (float)pg;
+                    v[1] = (float)pr;
+                    if (COARSE)
+#pragma unroll
+                        for (int k = 0; k < 6; k++) v[2 + k] = ex[k];
+                    int idx;
+                    const float t = warp_sum_multi<NV>(v, idx);
+                                        if ((lane & (32 / NV - 1)) == 0) {
+                        if (idx < 2) reinterpret_cast<float *>(s_dot)[(idx == 0 ? 0 : 2) * 32 + warp] = t;
+                        else s_res[(idx - 2) * 32 + warp] = t;
+                    }
+                }
+            }
+            // the halo's rows of u (or x), when their CTAs have published them
+            if (!solo && !first_coarse)
+#pragma unroll 1
+                for (int k = tid; k < nh; k += NT) {
+                    const int q = dyn<int>(gb.o_halo)[k];
+                    Row y;
+                    y.get(pub, d.nl_pad, q);
+                    if (!y.is(tag)) y = wait_row<T>(pub, d.nl_pad, q, tag, &s_err, d.bar);
+                    T *o = su + 4 * (size_t)(MAXT + k);
+                    o[0] = y.x;
+                    o[1] = y.y;
+                    o[2] = y.z;
+                }
+            __syncthreads();  // su
+            auto load3 = [&](int q, T y[3]) {
+                const T *s = su + 4 * (size_t)q;
+                if constexpr (fast) {
+                    const float4 f = *reinterpret_cast<const float4 *>(s);
+                    y[0] = f.x;
+                    y[1] = f.y;
+                    y[2] = f.z;
+                } else {
+                    const double2 f = *reinterpret_cast<const double2 *>(s);
+                    y[0] = f.x;
+                    y[1] = f.y;
+                    y[2] = s[2];
+                }
+            };
+            if (product) {
+                // phase B: w = A u
+                T acc[3] = {diag * u[0], diag * u[1], diag * u[2]};
+                // slots on chip, then the others.  Past the last of them a
+                // step takes the row itself with zero values
+                const int JC = gb.cache_cols, J1 = min(gb.cache_slots, L);
+                const uint16_t *col = dyn<uint16_t>(gb.o_col) + tid;
+                const T *kv1 = dyn<T>(gb.o_kv1) + tid;
+                if (nomass) {
+                    const T2 *kv2 = dyn<T2>(gb.o_kv2) + tid;
+                    constexpr int G1 = SlotDepth<T, MAXT>::kOn, G2 = SlotDepth<T, MAXT>::kOff;
+#pragma unroll 1
+                    for (int j0 = 0; j0 < J1; j0 += G1) {
+                        T y[G1][3];
+#pragma unroll
+                        for (int g = 0; g < G1; g++) load3(j0 + g < J1 ? col[(j0 + g) * MAXT] : tid, y[g]);
+#pragma unroll
+                        for (int g = 0; g < G1; g++) {
+                            const int j = j0 + g < J1 ? j0 + g : j0;
+                            T Kj[9];
+#pragma unroll
+                            for (int m = 0; m < 4; m++) {
+                                const T2 kp = kv2[(4 * j + m) * MAXT];
+                                Kj[2 * m] = kp.x;
+                                Kj[2 * m + 1] = kp.y;
+                            }
+                            Kj[8] = kv1[j * MAXT];
+                            // (past the last slot y is u: the products are zeros)
+                            block_fma(Kj, y[g][0] - u[0], y[g][1] - u[1], y[g][2] - u[2], acc[0], acc[1], acc[2]);
+                        }
+                    }
+                    const T *vp = static_cast<const T *>(d.sell_val) + sell_vidx(ebase + 32 * J1, 0);
+#pragma unroll 1
+                    for (int j0 = J1; j0 < L; j0 += G2, vp += 288 * G2) {
+                        T Kj[G2][9];
+#pragma unroll
+                        for (int g = 0; g < G2; g++)
+#pragma unroll
+                            for (int k = 0; k < 9; k++)
+                                Kj[g][k] = j0 + g < L ? __ldg(vp + 288 * g + 32 * k) : (T)0;
+#pragma unroll
+                        for (int g = 0; g < G2; g++) {
+                            const int j = j0 + g;
+                            T y[3];
+                            load3(j >= L ? tid : j < JC ? col[j * MAXT] : __ldg(&gb.lcol[ebase + 32 * j]), y);
+                            block_fma(Kj[g], y[0] - u[0], y[1] - u[1], y[2] - u[2], acc[0], acc[1], acc[2]);
+                        }
+                    }
+                } else {
+                    const T *mv = static_cast<const T *>(d.sell_mval);
+#pragma unroll 2
+                    for (int j = 0; j < L; j++) {
+                        T y[3];
+                        load3(j < JC ? col[j * MAXT] : __ldg(&gb.lcol[ebase + 32 * j]), y);
+                        const T m = j < J1 ? kv1[j * MAXT] : __ldg(&mv[ebase + 32 * j]);
+#pragma unroll
+                        for (int k = 0; k < 3; k++) acc[k] = fma(m, y[k], acc[k]);
+                    }
+                }
+                T pd = (T)0;
+                if (valid)
+#pragma unroll
+                    for (int k = 0; k < 3; k++) {
+                        w[k] = acc[k];
+                        pd += w[k] * u[k];
+                    }
+                                if constexpr (fast) {
+                    float ew[6] = {0, 0, 0, 0, 0, 0};
+                    if (COARSE && valid) restrict6_of<T>(dyn<float4>(gb.o_phi)[tid], w, ew);
+                    constexpr int NV = COARSE ? 8 : 2;
+                    float v[NV];
+                    v[0] = (float)pd;
+                    v[1] = 0.f;
+                    if (COARSE)
+#pragma unroll
+                        for (int k = 0; k < 6; k++) v[2 + k] = ew[k];
+                    int idx;
+                    const float t = warp_sum_multi<NV>(v, idx);
+                    if ((lane & (32 / NV - 1)) == 0) {
+                        if (idx == 0) reinterpret_cast<float *>(s_dot)[1 * 32 + warp] = t;
+                        else if (idx >= 2) s_res[(6 + idx - 2) * 32 + warp] = t;
+                    }
+                } else {
+                    T v[4] = {pg, pd, pr, (T)0}, t = (T)0;
+                    int idx = lane >> 3;
+                    if (warp < nsl) t = warp_sum_multi<4>(v, idx);
+                    if ((lane & 7) == 0 && idx < 3) reinterpret_cast<T *>(s_dot)[idx * 32 + warp] = t;
+                }
+            } else {
+                // the FP64 true residual b - A x of the published x becomes r
+                // (VERIFY), or the restriction of r_0 alone.
+                double vr = 0.0, vg = 0.0;
+                if (verify) {
+                    double a[3] = {0.0, 0.0, 0.0};
+                    if (valid) {
+                        const T *xr = su + 4 * (size_t)tid;
+#pragma unroll
+                        for (int k = 0; k < 3; k++) a[k] = (double)diag * (double)xr[k];
+                        add_residual_slots(a, static_cast<const T *>(nomass ? d.sell_val : d.sell_mval), gb.lcol,
+                                              su, xr, ebase, 0, L, nomass);
+                    }
+                    if (valid) {
+                        const size_t o = 3 * (size_t)(row);
+#pragma unroll
+                        for (int k = 0; k < 3; k++) {
+                            const double rt = d.rhs[o + k] - a[k];
+                            r[k] = (T)rt;
+                            const T uk = state_of(1, k) * r[k];
+                            vr += rt * rt;
+                            vg += (double)r[k] * (double)uk;
+                        }
+                        if (COARSE) restrict6_of<T>(dyn<float4>(gb.o_phi)[tid], r, ex);
+                    }
+                    vg = warp_sum<double>(vg);
+                    vr = warp_sum<double>(vr);
+                }
+                                if (lane == 0) {
+                    s_dot[0 * 32 + warp] = vg;
+                    s_dot[1 * 32 + warp] = 0.0;
+                    s_dot[2 * 32 + warp] = vr;
+                }
+                if (COARSE) {
+#pragma unroll
+                    for (int k = 0; k < 6; k++) {
+                        const float t = warp_sum<float>(ex[k]);
+                        if (lane == 0) {
+                            s_res[k * 32 + warp] = t;
+                            s_res[(6 + k) * 32 + warp] = 0.f;
+                        }
+                    }
+                }
+            }
+            __syncthreads();  // the slices' sums
+            // butterflies as wide as the slices need
+            const int half = nsl > 1 ? 1 << (31 - __clz(nsl - 1)) : 0;
+            // The segment's sums over its slices into s_out: warp q < 3 dot
+            // term q (hi, lo), warps 3..6 three values each of P^T r, P^T w
+            if (warp < 3) {
+                float hi, lo;
+                if (sizeof(T) == 8 || !product) {
+                    double a = lane < nsl ? s_dot[warp * 32 + lane] : 0.0;
+#pragma unroll
+                    for (int k = 16; k > 0; k >>= 1)
+                        if (k <= half) a += __shfl_xor_sync(0xffffffffu, a, k);
+                    hi = (float)a;
+                    lo = (float)(a - (double)hi);
+                } else {
+                    DF v{lane < nsl ? reinterpret_cast<const float *>(s_dot)[warp * 32 + lane] : 0.f, 0.f};
+#pragma unroll
+                    for (int k = 16; k > 0; k >>= 1)
+                        if (k <= half)
+                            v = df_add(v, DF{__shfl_xor_sync(0xffffffffu, v.hi, k), __shfl_xor_sync(0xffffffffu, v.lo, k)});
+                    hi = v.hi;
+                    lo = v.lo;
+                }
+                if (lane == 0) {
+                    s_out[2 * warp] = hi;
+                    s_out[2 * warp + 1] = lo;
+                }
+            } else if (COARSE && warp < 7) {
+                const int k0 = 3 * (warp - 3);
+                float v[3];
+#pragma unroll
+                for (int q = 0; q < 3; q++) v[q] = lane < nsl ? s_res[(k0 + q) * 32 + lane] : 0.f;
+#pragma unroll
+                for (int k = 16; k > 0; k >>= 1)
+                    if (k <= half)
+#pragma unroll
+                        for (int q = 0; q < 3; q++) v[q] += __shfl_xor_sync(0xffffffffu, v[q], k);
+                if (lane == 0)
+#pragma unroll
+                    for (int q = 0; q < 3; q++) s_out[6 + k0 + q] = v[q];
+            }
+            __syncthreads();  // s_out
+            // published in whole 32-byte sectors by one store: words 0, 1 the
+            // dot terms, 2..5 P^T r and P^T w, three values each
+            uint4 *const dots = gb.words + (size_t)parity * 2 * d.n_segs;
+            uint4 *const rest = gb.words + (size_t)4 * d.n_segs + (size_t)parity * 4 * d.n_segs;
+            float *const swr = dyn<float>(gb.o_words), *const sww = swr + 6 * cnt;  // the group's P^T r and P^T w
+            if (warp == 0 && lane < (COARSE ? 6 : 2)) {
+                const float a = s_out[3 * lane], b2 = s_out[3 * lane + 1], c = s_out[3 * lane + 2];
+                if (!solo) {
+                    uint4 *o = lane < 2 ? dots + 2 * (size_t)seg + lane : rest + 4 * (size_t)seg + lane - 2;
+                    st_b128(o, pack2(__float_as_uint(a), __float_as_uint(b2)), pack2(__float_as_uint(c), tag));
+                } else if (lane >= 2) {
+                    float *o = swr + 3 * (lane - 2);  // (sww follows: one segment)
+                    o[0] = a;
+                    o[1] = b2;
+                    o[2] = c;
+                }
+            }
+            // the dot terms of every segment of the group, a segment per lane
+            // of the first warps, summed per warp
+            if (32 * warp < cnt) {
+                DF sum[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+                const int sg = 32 * warp + lane;
+                if (solo) {
+                    if (lane == 0)
+#pragma unroll
+                        for (int q = 0; q < 3; q++) sum[q] = DF{s_out[2 * q], s_out[2 * q + 1]};
+                } else if (sg < cnt) {
+                    uint64_t lo[2], hi[2];
+                    wait_words<2>(dots + 2 * (size_t)(s_bp.seg_off + sg), 1, 2, tag, lo, hi, &s_err, d.bar);
+                    sum[0] = DF{__uint_as_float((uint32_t)lo[0]), __uint_as_float((uint32_t)(lo[0] >> 32))};
+                    sum[1] = DF{__uint_as_float((uint32_t)hi[0]), __uint_as_float((uint32_t)lo[1])};
+                    sum[2] = DF{__uint_as_float((uint32_t)(lo[1] >> 32)), __uint_as_float((uint32_t)hi[1])};
+                }
+                __syncwarp();
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+                    if (o < cnt)  // (lanes past cnt hold zeros)
+#pragma unroll
+                        for (int q = 0; q < 3; q++)
+                            sum[q] = df_add(sum[q], DF{__shfl_xor_sync(0xffffffffu, sum[q].hi, o),
+                                                       __shfl_xor_sync(0xffffffffu, sum[q].lo, o)});
+                if (lane == 0)
+#pragma unroll
+                    for (int q = 0; q < 3; q++) s_part[3 * warp + q] = sum[q];
+            }
+            __syncthreads();  // sw
+            if (warp == 0) {
+                if (lane == 0) {
+                    if (!first_coarse) {
+                        DF sums[3];
+#pragma unroll
+                        for (int q = 0; q < 3; q++) {
+                            sums[q] = s_part[q];
+                            for (int k = 1; 32 * k < cnt; k++) sums[q] = df_add(sums[q], s_part[3 * k + q]);
+                            s_last[q] = sums[q];
+                        }
+                        int bits;
+                        if (!(fast && transition_on(s_cg, limit, sums)) &&
+                            transition_any(&s_cg, &s_bp, s_last, &bits, fast) && bits && leader)
+                            atomicOr(&d.status[b], bits);
+                    }
+                    s_stop = s_err;
+                }
+            } else if (COARSE && !solo) {
+                // meanwhile every segment's restrictions, kBulk words in flight
+                const uint4 *gr = rest + 4 * (size_t)s_bp.seg_off;
+                const int n = 4 * cnt, step = NT - 32;
+#pragma unroll 1
+                for (int i0 = tid - 32; i0 < n; i0 += kBulk * step) {
+                    uint64_t lo[kBulk], hi[kBulk];
+                    wait_words<kBulk>(gr + i0, step, (n - i0 + step - 1) / step, tag, lo, hi, &s_err, d.bar);
+#pragma unroll
+                    for (int g = 0; g < kBulk; g++) {
+                        const int i = i0 + g * step;
+                        if (i >= n) break;
+                        float *o = ((i & 2) ? sww : swr) + 6 * (i >> 2) + 3 * (i & 1);
+                        o[0] = __uint_as_float((uint32_t)lo[g]);
+                        o[1] = __uint_as_float((uint32_t)(lo[g] >> 32));
+                        o[2] = __uint_as_float((uint32_t)hi[g]);
+                    }
+                }
+            }
+            __syncthreads();  // the new state
+            const int nst = s_cg.state;
+            going = nst != CG_CONVERGED && nst != CG_FAILED && !s_stop;
+            if (COARSE && going && nst != CG_VERIFY) {
+                // the coarse correction of the next u: h = P^T w + beta h,
+                // g = P^T r - alpha h (P^T r of the next residual; after a
+                // restart P^T r itself), c = X g for the CTA's segment
+                const bool restart = first_coarse || nst == CG_RESTART;
+                float *h = dyn<float>(gb.o_h);
+                const float *xr = dyn<float>(gb.o_xrow);
+                const float al = s_cg.alpha_f, be = s_cg.beta_f;
+                float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 2
+                for (int j = tid; j < cn; j += NT) {
+                    const float pr_j = swr[j];
+                    const float hn = restart ? 0.f : sww[j] + be * h[j];
+                    h[j] = hn;
+                    const float g = restart ? pr_j : pr_j - al * hn;
+#pragma unroll
+                    for (int l = 0; l < 6; l++) v[l] = fmaf(xr[l * cn + j], g, v[l]);
+                }
+                int idx;
+                const float t = warp_sum_multi<8>(v, idx);
+                if ((lane & 3) == 0 && idx < 6) s_red6[idx * 32 + warp] = t;
+                __syncthreads();
+#pragma unroll 1
+                for (int l = warp; l < 6; l += nw) {
+                    const float c = warp_sum<float>(lane < nw ? s_red6[l * 32 + lane] : 0.f);
+                    if (lane == 0) s_cvec[l] = c;
+                }
+                __syncthreads();  // s_cvec
+            }
+            if (!first_coarse) loops++;
+            fresh = first_coarse || nst == CG_RESTART;
+            first_coarse = false;
+            parity ^= 1;
+        }
+        maxseq = max(maxseq, seq);
+        maxloops = max(maxloops, loops);
+        // x of the own rows, and the step's Euler update (Blob::euler_integrate,
+        // src/Blob.cpp:3937-3969) for a blob that had not failed before the
+        // solve and whose solve converged
+        const bool err = run && s_stop;
+        const bool move = d.cg_euler && !err && s_cg.state == CG_CONVERGED && __ldcg(&d.status[b]) == 0;
+        const double dt = s_bp.dt;
+        if (run && in) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) static_cast<T *>(d.x)[3 * (size_t)row + k] = state_of(0, k);
+        }
+        if (move && in && row - s_bp.node_off < s_bp.node_cnt) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const size_t kk = 3 * (size_t)row + k;
+                const double xi = run ? (double)state_of(0, k) : (double)static_cast<const T *>(d.x)[kk];
+                double pn;
+                if (nomass) {
+                    d.vel[kk] = xi;
+                    pn = d.pos[kk] + xi * dt;
+                } else {
+                    const double v = d.vel[kk] + xi * dt;
+                    d.vel[kk] = v;
+                    pn = d.pos[kk] + v * dt;
+                }
+                d.pos[kk] = pn;
+                if (d.pos_df) d.pos_df[kk] = split_pos(pn);
+            }
+        }
+        if (leader && tid == 0) {
+            if (run) {
+                d.cg[b] = s_cg;
+                record_sums(d, b, s_last);  // (FP64 conversions: once per solve, off the iteration)
+            }
+            // the blob's own stream moves on by one step's draws unless the
+            // blob failed (a shared stream: below)
+            if (d.cg_euler && !err && d.num_streams == d.num_blobs && __ldcg(&d.status[b]) == 0) {
+                advance_stream(d.stream_state + 6 * s_bp.stream, d.stream_step + s_bp.stream);
+            }
+        }
+        if (err) {
+            if (tid == 0) atomicOr(&d.status[b], BLOB_FAIL_CG | BLOB_FAIL_TIMEOUT);
+            break;  // CTA-uniform: s_stop was read after a barrier by every thread
+        }
+    }
+    if (tid == 0) {
+        if (blockIdx.x == 0 && d.cg_euler && d.num_streams != d.num_blobs && !s_stop)
+#pragma unroll 1
+            for (int sm = 0; sm < d.num_streams; sm++)
+                advance_stream(d.stream_state + 6 * sm, d.stream_step + sm);
+        // the last CTA out moves the tag base past every tag of this launch
+        // (all CTAs read it when they started) and adds the longest solve's
+        // iterations to the loop count
+        atomicMax(&d.bar[7], maxseq);
+        atomicMax(&d.bar[8], (unsigned int)max(maxloops, 0));
+        __threadfence();
+        if (atomicAdd(&d.bar[9], 1u) == gridDim.x - 1) {
+            __threadfence();
+            d.bar[6] = base + atomicExch(&d.bar[7], 0u) + 1u;
+            *d.loop_count += (unsigned long long)atomicExch(&d.bar[8], 0u);
+            d.bar[9] = 0;
+        }
+    }
+}
+
+// The variant by the rows of a CTA (the longest segment).
+template <typename T, bool COARSE>
+const void *kernel_for(int rows)
+{
+    if (rows <= 256) return reinterpret_cast<const void *>(&k_cg_group<T, COARSE, 256>);
+    if (rows <= 512) return reinterpret_cast<const void *>(&k_cg_group<T, COARSE, 512>);
+    return reinterpret_cast<const void *>(&k_cg_group<T, COARSE, 1024>);
+}
+
+const void *group_kernel(const DeviceBatch &d, const GroupBatch &g)
+{
+    if (d.precision == PREC_FP64) return kernel_for<double, false>(g.rows);
+    return d.coarse ? kernel_for<float, true>(g.rows) : kernel_for<float, false>(g.rows);
+}
+
+}  // namespace
+
+int cg_group_plan(const DeviceBatch &d, GroupBatch &g, int max_slots, int max_cols, int max_rows, int max_halo,
+                  int max_segs)
+{
+    const bool f64 = d.precision == PREC_FP64;
+    g.rows = max_rows <= 256 ? 256 : max_rows <= 512 ? 512 : 1024;  // the variant's MAXT
+    g.threads = std::max(256, (max_rows + 31) / 32 * 32);
+    int dev = 0, optin = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return -1;
+    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return -1;
+    const void *fn = group_kernel(d, g);
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) return -1;
+    const size_t R = g.rows, ts = f64 ? 8 : 4;
+    const size_t reserve = 1024;  // per-CTA system use
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = off;
+        off = (off + bytes + 15) & ~(size_t)15;
+        return (int32_t)o;
+    };
+    g.o_state = take(R <= 512 ? 0 : 12 * R * ts);
+    g.o_u = take(4 * (R + max_halo) * ts);
+    g.o_halo = take(4 * (size_t)max_halo);
+    g.o_words = take(d.coarse ? 48 * (size_t)max_segs : 0);
+    if (d.coarse) {
+        g.o_phi = take(16 * R);
+        g.o_xrow = take(24 * (size_t)d.coarse_nmax);
+        g.o_h = take(4 * (size_t)d.coarse_nmax);
+    }
+    const size_t fixed = fa.sharedSizeBytes + reserve + off + 64;
+    if ((size_t)optin < fixed) return -1;
+    size_t room = optin - fixed;
+    const size_t per_col = R * sizeof(uint16_t), per_slot = R * (d.any_nomass ? 9 : 1) * ts;
+    g.cache_cols = (int32_t)std::min<size_t>(room / per_col, (size_t)std::max(0, max_cols));
+    room -= (size_t)g.cache_cols * per_col;
+    g.cache_slots = (int32_t)std::min<size_t>(
+        room / per_slot, (size_t)std::max(0, std::min(max_slots, (int)g.cache_cols)));
+    g.o_col = take((size_t)g.cache_cols * per_col);
+    g.o_kv2 = take(d.any_nomass ? 8 * ts * R * g.cache_slots : 0);
+    g.o_kv1 = take(ts * R * g.cache_slots);
+    g.dyn_smem = (int32_t)off;
+    // the limit is a property of the kernel, shared by every handle: the
+    // device maximum, so that no handle's plan lowers another's
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes) !=
+        cudaSuccess)
+        return -1;
+    return 0;
+}
+
+int cg_group_max_grid(const DeviceBatch &d, const GroupBatch &g)
+{
+    int dev = 0, sms = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, group_kernel(d, g),
+                                                      g.threads, g.dyn_smem) != cudaSuccess)
+        return 0;
+    return sms * per_sm;
+}
+
+cudaError_t launch_cg_group(const DeviceBatch &d, cudaStream_t s)
+{
+    GroupBatch g = *d.group;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)g.grid);
+    cfg.blockDim = dim3((unsigned)g.threads);
+    cfg.dynamicSmemBytes = (size_t)g.dyn_smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    DeviceBatch arg = d;
+    void *args[] = {&arg, &g};
+    count_launches(1);
+    return cudaLaunchKernelExC(&cfg, group_kernel(d, g), args);
+}
+
+}  // namespace ffea

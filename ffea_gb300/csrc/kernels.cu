@@ -26,6 +26,7 @@
 #include <atomic>
 #include <cstdio>
 
+#include "cg_common.cuh"
 #include "kernels.h"
 
 #include <algorithm>
@@ -39,15 +40,6 @@ void count_launches(int64_t n) { g_launches.fetch_add(n, std::memory_order_relax
 #define FFEA_LAUNCHED() g_launches.fetch_add(1, std::memory_order_relaxed)
 
 namespace {
-
-// ---------------------------------------------------------------- reductions
-template <typename A>
-__device__ __forceinline__ A warp_sum(A v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 
 // Sum NV per-thread values over the CTA; the butterfly inside each warp runs
 // in W (float for the mixed path: GB300's FP64 rate is a small fraction of
@@ -82,12 +74,6 @@ __device__ __forceinline__ bool last_block(unsigned int *counter, unsigned int t
     __syncthreads();
     if (is_last) __threadfence();
     return is_last != 0;
-}
-
-// SELL-32 value index of component k (0..8 row-major 3x3) of entry `off`
-__device__ __forceinline__ size_t sell_vidx(int off, int k)
-{
-    return (size_t)(off & ~31) * 9 + (size_t)k * 32 + (off & 31);
 }
 
 // ---------------------------------------------------------------- element math
@@ -157,23 +143,6 @@ __device__ __forceinline__ void jacobian_t(const DeviceBatch &d, int4 c, T J[3][
                 J[r][k] = (q.x - a[k].x) + (q.y - a[k].y);
             }
     }
-}
-
-// Double-float accumulation (Knuth's TwoSum, error-free in FP32): sums with
-// ~48-bit precision on the FP32 pipes, which on GB300 run many times faster
-// than FP64.
-struct DF {
-    float hi, lo;
-};
-
-__device__ __forceinline__ DF df_add(DF a, DF b)
-{
-    const float s = a.hi + b.hi;
-    const float bb = s - a.hi;
-    float err = (a.hi - (s - bb)) + (b.hi - bb);
-    err += a.lo + b.lo;
-    const float hi = s + err;
-    return DF{hi, err - (hi - s)};
 }
 
 // Force sum of the node kernel: FP64 in FP64 mode; in mixed precision a
@@ -712,10 +681,12 @@ __global__ void __launch_bounds__(NODE_TILE * NODE_LANES) k_nodes(DeviceBatch d,
         const T ui = dinv[k] * ri;
         x[k] = lumped ? (T)(fi * d.lumped_inv[row]) : (T)0;
         r[k] = ri;
-        u[k] = ui;
-        p[k] = (T)0;
-        sv[k] = (T)0;
-        w[k] = (T)0;
+        if (!d.group) {  // k_cg_group starts from r and D^-1 alone
+            u[k] = ui;
+            p[k] = (T)0;
+            sv[k] = (T)0;
+            w[k] = (T)0;
+        }
         gam = (double)ri * (double)ui;
         ff = fi * fi;
     }
@@ -771,8 +742,6 @@ __global__ void __launch_bounds__(NODE_TILE * NODE_LANES) k_nodes(DeviceBatch d,
 }
 
 // ---------------------------------------------------------------- persistent CG
-constexpr unsigned int kSpinLimit = 1u << 24;  // ~1 s of 64 ns sleeps, then give up
-constexpr int kMaxRestarts = 4;
 
 // Grid-wide barrier on a counter that only grows during a solve: each CTA
 // adds one and waits until the count reaches `target` (the number of CTAs
@@ -859,15 +828,6 @@ __device__ __forceinline__ void sell_row(const DeviceBatch &d, int row, bool nom
     out[2] = a2;
 }
 
-// Vector of 4 T: the published copy of u in the CG kernel (x, y, z, 0), one
-// 16-byte (FP32) load per neighbour instead of three 4-byte loads that each
-// touch the same sectors.
-struct alignas(16) Dbl4 {
-    double x, y, z, w;
-};
-template <typename T> struct Vec4T;
-template <> struct Vec4T<float> { using type = float4; };
-template <> struct Vec4T<double> { using type = Dbl4; };
 
 __device__ __forceinline__ float4 ldcg4(const float4 *p) { return __ldcg(p); }
 
@@ -905,51 +865,23 @@ __device__ __forceinline__ Dbl4 ldcg4(const Dbl4 *p)
     return Dbl4{a.x, a.y, b.x, b.y};
 }
 
-// On-chip copy of a CTA's matrix rows for one solve (register-resident CG
-// variant): the column indices of slots j < JC (col[j * CG_THREADS + t] for
-// thread t) and the 9 values of slots j < J as four pairs and a single
-// (kv2[(4 j + m) * CG_THREADS + t], kv1[j * CG_THREADS + t]).  The matrix is
-// constant during a solve; each slot held on chip saves its L2 reads in every
-// iteration, and cached column indices take the index -> neighbour dependency
-// off the critical path of the gathers.
+// q = A u for one row of the CG kernel (sell_row's arithmetic) in groups of
+// two slots: the column indices of the next group are loaded together with
+// this group's values and neighbours, so a group costs one memory round trip
+// instead of two (index, then neighbour).
 template <typename T>
-struct CgCache {
-    using T2 = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
-    const int *col = nullptr;
-    const T2 *kv2 = nullptr;
-    const T *kv1 = nullptr;
-    int J = 0, JC = 0;
-};
-
-// One 3x3 block times a difference vector, added with explicit FMAs so that
-// every code path gives the same bits.
-template <typename T>
-__device__ __forceinline__ void block_fma(const T K[9], T d0, T d1, T d2, T &a0, T &a1, T &a2)
-{
-    a0 = fma(K[2], d2, fma(K[1], d1, fma(K[0], d0, a0)));
-    a1 = fma(K[5], d2, fma(K[4], d1, fma(K[3], d0, a1)));
-    a2 = fma(K[8], d2, fma(K[7], d1, fma(K[6], d0, a2)));
-}
-
-// q = A u for one row of the CG kernel (sell_row's arithmetic): slots with
-// values on chip in groups of 4 (only the neighbour loads go to L2), then the
-// rest in groups of 2 (values and neighbours from L2, issued together).
-template <typename T, bool MEM = false>
 __device__ __forceinline__ void sell_row_cg(const DeviceBatch &d, int row, bool nomass, T diag,
-                                            const typename Vec4T<T>::type *u4, T out[3], const CgCache<T> &cc)
+                                            const typename Vec4T<T>::type *u4, T out[3])
 {
-    const int sl = row >> 5, lane = row & 31, t = threadIdx.x;
+    const int sl = row >> 5, lane = row & 31;
     const int L = __ldg(&d.slice_len[sl]);
     const int base = __ldg(&d.slice_ptr[sl]);
     const auto me = ldcg4(&u4[row]);
     T a0 = diag * me.x, a1 = diag * me.y, a2 = diag * me.z;
-    auto col_of = [&](int j) {
-        return j < cc.JC ? cc.col[j * CG_THREADS + t] : __ldg(&d.sell_col[base + 32 * j + lane]);
-    };
     if (!nomass) {
         const T *mv = static_cast<const T *>(d.sell_mval);
         for (int j = 0; j < L; j++) {
-            const auto y = ldcg4(&u4[col_of(j)]);
+            const auto y = ldcg4(&u4[__ldg(&d.sell_col[base + 32 * j + lane])]);
             const T m = __ldg(&mv[base + 32 * j + lane]);
             a0 = fma(m, y.x, a0);
             a1 = fma(m, y.y, a1);
@@ -960,79 +892,31 @@ __device__ __forceinline__ void sell_row_cg(const DeviceBatch &d, int row, bool 
         out[2] = a2;
         return;
     }
-    if constexpr (MEM) {
-        // memory-resident kernel (no on-chip copy): the column indices of the
-        // next group are loaded together with this group's values and
-        // neighbours, so a group costs one memory round trip instead of two
-        // (index, then neighbour).  Same slots, same FMA order: same bits.
-        const T *val = static_cast<const T *>(d.sell_val);
-        const uint64_t pol = l2_evict_first();
-        constexpr int G2 = 2;
-        int cn[G2];
-#pragma unroll
-        for (int g = 0; g < G2; g++) cn[g] = g < L ? ld_stream(&d.sell_col[base + 32 * g + lane], pol) : row;
-        for (int j0 = 0; j0 < L; j0 += G2) {
-            typename Vec4T<T>::type y[G2];
-            T K[G2][9];
-            int nx[G2];
-#pragma unroll
-            for (int g = 0; g < G2; g++) {
-                const int j = j0 + g;
-                y[g] = ldcg4(&u4[cn[g]]);
-                const size_t vb = (size_t)(base + 32 * j) * 9 + lane;
-#pragma unroll
-                for (int k = 0; k < 9; k++) K[g][k] = j < L ? ld_stream(&val[vb + 32 * k], pol) : (T)0;
-                const int jn = j + G2;
-                nx[g] = jn < L ? ld_stream(&d.sell_col[base + 32 * jn + lane], pol) : row;
-            }
-#pragma unroll
-            for (int g = 0; g < G2; g++)
-                if (j0 + g < L) block_fma(K[g], y[g].x - me.x, y[g].y - me.y, y[g].z - me.z, a0, a1, a2);
-#pragma unroll
-            for (int g = 0; g < G2; g++) cn[g] = nx[g];
-        }
-        out[0] = a0;
-        out[1] = a1;
-        out[2] = a2;
-        return;
-    }
-    const int Jk = min(cc.J, L);
-    constexpr int G1 = 4;
-    for (int j0 = 0; j0 < Jk; j0 += G1) {
-        typename Vec4T<T>::type y[G1];
-#pragma unroll
-        for (int g = 0; g < G1; g++) y[g] = ldcg4(&u4[j0 + g < Jk ? col_of(j0 + g) : row]);
-#pragma unroll
-        for (int g = 0; g < G1; g++) {
-            const int j = j0 + g;
-            if (j >= Jk) break;
-            T K[9];
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-                const auto kp = cc.kv2[(4 * j + m) * CG_THREADS + t];
-                K[2 * m] = kp.x;
-                K[2 * m + 1] = kp.y;
-            }
-            K[8] = cc.kv1[j * CG_THREADS + t];
-            block_fma(K, y[g].x - me.x, y[g].y - me.y, y[g].z - me.z, a0, a1, a2);
-        }
-    }
     const T *val = static_cast<const T *>(d.sell_val);
+    const uint64_t pol = l2_evict_first();
     constexpr int G2 = 2;
-    for (int j0 = Jk; j0 < L; j0 += G2) {
+    int cn[G2];
+#pragma unroll
+    for (int g = 0; g < G2; g++) cn[g] = g < L ? ld_stream(&d.sell_col[base + 32 * g + lane], pol) : row;
+    for (int j0 = 0; j0 < L; j0 += G2) {
         typename Vec4T<T>::type y[G2];
         T K[G2][9];
+        int nx[G2];
 #pragma unroll
         for (int g = 0; g < G2; g++) {
             const int j = j0 + g;
-            y[g] = ldcg4(&u4[j < L ? col_of(j) : row]);
+            y[g] = ldcg4(&u4[cn[g]]);
             const size_t vb = (size_t)(base + 32 * j) * 9 + lane;
 #pragma unroll
-            for (int k = 0; k < 9; k++) K[g][k] = j < L ? __ldg(&val[vb + 32 * k]) : (T)0;
+            for (int k = 0; k < 9; k++) K[g][k] = j < L ? ld_stream(&val[vb + 32 * k], pol) : (T)0;
+            const int jn = j + G2;
+            nx[g] = jn < L ? ld_stream(&d.sell_col[base + 32 * jn + lane], pol) : row;
         }
 #pragma unroll
         for (int g = 0; g < G2; g++)
             if (j0 + g < L) block_fma(K[g], y[g].x - me.x, y[g].y - me.y, y[g].z - me.z, a0, a1, a2);
+#pragma unroll
+        for (int g = 0; g < G2; g++) cn[g] = nx[g];
     }
     out[0] = a0;
     out[1] = a1;
@@ -1172,76 +1056,6 @@ __device__ __forceinline__ void store_fields(const DeviceBatch &d, int row, cons
         if (m & RF_S) static_cast<T *>(d.s)[o + c] = S.s[c];
         if (m & RF_P) static_cast<T *>(d.p)[o + c] = S.p[c];
     }
-}
-
-template <typename T>
-__device__ __forceinline__ void load_row(const DeviceBatch &d, int row, RowState<T> &S)
-{
-    const size_t o = 3 * (size_t)row;
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        S.x[c] = static_cast<const T *>(d.x)[o + c];
-        S.r[c] = static_cast<const T *>(d.r)[o + c];
-        S.u[c] = static_cast<const T *>(d.u)[o + c];
-        S.w[c] = static_cast<const T *>(d.w)[o + c];
-        S.s[c] = static_cast<const T *>(d.s)[o + c];
-        S.p[c] = static_cast<const T *>(d.p)[o + c];
-        S.dinv[c] = static_cast<const T *>(d.dinv)[o + c];
-    }
-}
-
-template <typename T>
-__device__ __forceinline__ void store_row(const DeviceBatch &d, int row, const RowState<T> &S)
-{
-    const size_t o = 3 * (size_t)row;
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        static_cast<T *>(d.x)[o + c] = S.x[c];
-        static_cast<T *>(d.r)[o + c] = S.r[c];
-        static_cast<T *>(d.u)[o + c] = S.u[c];
-        static_cast<T *>(d.w)[o + c] = S.w[c];
-        static_cast<T *>(d.s)[o + c] = S.s[c];
-        static_cast<T *>(d.p)[o + c] = S.p[c];
-    }
-}
-
-__device__ __forceinline__ DF df_warp_sum(DF v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        DF w{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
-        v = df_add(v, w);
-    }
-    return v;
-}
-
-// Sum of N values per lane over a warp (N a power of two, 2..32) by a
-// transposed butterfly: at offsets 16, 8, ... each lane keeps half of its
-// values and adds its partner's copy of that half (N/2 + N/4 + ... shuffles),
-// then the remaining offsets add whole values.  Returns this lane's total of
-// value index idx; every lane holding the same idx holds the same bits.
-template <int N>
-__device__ __forceinline__ float warp_sum_multi(float (&v)[N], int &idx)
-{
-    static_assert(N >= 2 && N <= 32 && (N & (N - 1)) == 0, "N must be a power of two in [2, 32]");
-    const int lane = threadIdx.x & 31;
-    idx = 0;
-    int o = 16;
-#pragma unroll
-    for (int h = N / 2; h >= 1; h /= 2, o /= 2) {
-        const bool upper = (lane & o) != 0;
-#pragma unroll
-        for (int k = 0; k < h; k++) {
-            const float send = upper ? v[k] : v[k + h];
-            const float keep = upper ? v[k + h] : v[k];
-            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-        if (upper) idx += h;
-    }
-    float x = v[0];
-#pragma unroll
-    for (; o > 0; o /= 2) x += __shfl_xor_sync(0xffffffffu, x, o);
-    return x;
 }
 
 // Partial sums of a CG segment, written to its slot P of the partials
@@ -1445,151 +1259,6 @@ __device__ __forceinline__ void block_blob_sums(const DeviceBatch &d, const doub
     }
 }
 
-// One CG transition of a blob from its three sums:
-//   ACTIVE   sums r.u, w.u, r.r: stop test, then alpha / beta of the next update
-//   VERIFY   sums r.u, -, |b - A x|^2: converged, or restart from that residual
-//   RESTART  sums r.u, w.u, -: alpha of the first restarted update, beta = 0
-// Returns true when the blob stops (cg.state is then CONVERGED or FAILED) and
-// sets *fail_bits to the failure bits (0 if none).
-//
-// FP64 precision runs the recurrence in FP64: alpha = r.u / (w.u - beta r.u /
-// alpha_prev), beta = r.u / r.u_prev, stop when r.r / f.f < eps^2.  Mixed
-// precision (`fast`) applies alpha and beta in FP32 anyway and runs it in
-// FP32 as alpha = r.u / p.Ap with p.Ap = w.u - beta^2 (p.Ap)_prev (the same
-// recurrence), stop when r.r < eps^2 f.f: FP64 arithmetic and conversions run
-// at 1/64 of the FP32 rate and would sit on the critical path of every
-// iteration.  VERIFY (once per solve) stays in FP64.
-__device__ __forceinline__ bool transition_core(CgScalars &cg, const BlobParams &bp, const DF sums[3],
-                                                int *fail_bits, bool fast)
-{
-    const int limit = bp.solver == SOLVER_MASS ? bp.max_iter - 1 : bp.max_iter;
-    int finish = 0, bits = 0;
-    if (cg.state == CG_ACTIVE) {
-        bool conv, nan, breakdown = false, at_floor = false;
-        if (fast) {
-            const float g = sums[0].hi + sums[0].lo, dl = sums[1].hi + sums[1].lo, rr = sums[2].hi + sums[2].lo;
-            conv = rr < cg.stop_f;
-            nan = !(rr == rr) || !(g == g) || !(dl == dl);
-            if (!(cg.iters > 0 && conv) && !nan && cg.iters < limit) {
-                const float beta = cg.iters == 0 ? 0.f : g / cg.gamma_f;
-                const float pap = cg.iters == 0 ? dl : fmaf(-beta * beta, cg.pap_f, dl);
-                if (!(pap > 0.f) || !(g > 0.f)) {
-                    // the FP32 recurrence broke down (p.Ap or r.u not
-                    // positive, so alpha would not be finite).  Below the
-                    // floor this is the precision limit of FP32 vectors
-                    // (an epsilon tighter than FP32 can reach): stop there;
-                    // above it, it is a failure.
-                    breakdown = true;
-                    at_floor = rr < cg.floor_f;
-                } else {
-                    cg.beta_f = beta;
-                    cg.pap_f = pap;
-                    cg.alpha_f = g / pap;
-                    cg.gamma_f = g;
-                }
-            }
-        } else {
-            const double g = (double)sums[0].hi + (double)sums[0].lo, dl = (double)sums[1].hi + (double)sums[1].lo;
-            const double rr = (double)sums[2].hi + (double)sums[2].lo;
-            cg.rr = rr;
-            const double res = (cg.ff == 0.0) ? 0.0 : rr / cg.ff;
-            conv = res < bp.epsilon2;
-            nan = !(res == res) || !(g == g) || !(dl == dl);
-            if (!(cg.iters > 0 && conv) && !nan && cg.iters < limit) {
-                if (cg.iters == 0) {
-                    cg.beta = 0.0;
-                    cg.alpha = g / dl;
-                } else {
-                    const double beta = g / cg.gamma;
-                    cg.alpha = g / (dl - beta * g / cg.alpha);
-                    cg.beta = beta;
-                }
-                cg.gamma = g;
-            }
-        }
-        if ((cg.iters > 0 && conv) || (breakdown && at_floor)) {
-            // with the true-residual check on, the FP64 b - A x decides
-            // (converged, or a restart from it)
-            if (bp.true_residual) cg.state = CG_VERIFY;
-            else finish = CG_CONVERGED;
-        } else if (breakdown) {
-            finish = CG_FAILED;
-            bits = BLOB_FAIL_CG;
-        } else if (nan) {
-            finish = CG_FAILED;
-            bits = BLOB_FAIL_CG | BLOB_FAIL_NAN;
-        } else if (cg.iters >= limit) {
-            finish = CG_FAILED;
-            bits = BLOB_FAIL_CG;
-        } else {
-            cg.iters += 1;
-        }
-    } else if (cg.state == CG_VERIFY) {
-        const double tr = (double)sums[2].hi + (double)sums[2].lo;
-        cg.true_relres2 = (cg.ff == 0.0) ? 0.0 : tr / cg.ff;
-        if (cg.true_relres2 < bp.epsilon2) {
-            finish = CG_CONVERGED;
-        } else if (cg.restarts >= kMaxRestarts || cg.iters >= limit) {
-            finish = CG_FAILED;
-            bits = BLOB_FAIL_CG;
-        } else {
-            cg.restarts += 1;
-            cg.gamma = (double)sums[0].hi + (double)sums[0].lo;
-            cg.gamma_f = sums[0].hi + sums[0].lo;
-            cg.state = CG_RESTART;
-        }
-    } else if (cg.state == CG_RESTART) {
-        // r.u of the restarted u (phase B of the restart step recomputes it,
-        // with the coarse correction where there is one)
-        cg.state = CG_ACTIVE;
-        cg.iters += 1;
-        bool nan;
-        if (fast) {
-            cg.gamma_f = sums[0].hi + sums[0].lo;
-            cg.beta_f = 0.f;
-            cg.pap_f = sums[1].hi + sums[1].lo;
-            cg.alpha_f = cg.gamma_f / cg.pap_f;
-            nan = !(cg.alpha_f == cg.alpha_f);
-        } else {
-            cg.gamma = (double)sums[0].hi + (double)sums[0].lo;
-            cg.beta = 0.0;
-            cg.alpha = cg.gamma / ((double)sums[1].hi + (double)sums[1].lo);
-            nan = !(cg.alpha == cg.alpha);
-        }
-        if (nan) {
-            finish = CG_FAILED;
-            bits = BLOB_FAIL_CG | BLOB_FAIL_NAN;
-        }
-    }
-    if (finish) cg.state = finish;
-    *fail_bits = bits;
-    return finish != 0;
-}
-
-// The coefficients of the next update in the arithmetic type of the vectors.
-template <typename T>
-__device__ __forceinline__ void cg_coefs(const CgScalars &cg, T &alpha, T &beta);
-template <>
-__device__ __forceinline__ void cg_coefs<float>(const CgScalars &cg, float &alpha, float &beta)
-{
-    alpha = cg.alpha_f;
-    beta = cg.beta_f;
-}
-template <>
-__device__ __forceinline__ void cg_coefs<double>(const CgScalars &cg, double &alpha, double &beta)
-{
-    alpha = cg.alpha;
-    beta = cg.beta;
-}
-
-// The iteration's reduced sums (r.u, w.u, r.r) as the transition received
-// them, kept per blob for inspection of the reduction's accuracy.
-__device__ __forceinline__ void record_sums(const DeviceBatch &d, int b, const DF sums[3])
-{
-#pragma unroll
-    for (int i = 0; i < 3; i++) d.last_sums[3 * (size_t)b + i] = (double)sums[i].hi + (double)sums[i].lo;
-}
-
 // The transition run by the CTA that arrived last at a reducing barrier
 // (exactly once per blob), on the blob's record in global memory.
 __device__ __forceinline__ void cg_transition(const DeviceBatch &d, int b, const DF sums[3])
@@ -1681,82 +1350,6 @@ __device__ __forceinline__ unsigned int reducing_barrier(const DeviceBatch &d, c
     return *s_pub;
 }
 
-// Reduction without a serial step: after a plain grid barrier every CTA sums
-// the partials of every busy blob itself, in the same fixed order, and runs
-// the transitions on its own copy of the blob records in shared memory, so
-// all CTAs reach bit-identical states.  CTA 0 alone records failure bits.
-// Also refreshes the CTA's view (state, alpha, beta of its nb blobs) and
-// returns the number of blobs still iterating.
-//
-// With the coarse space (coarse_n > 0; one blob per CTA) it also forms the
-// CTA's coarse correction for the next update: thread j holds coarse dof j
-// of the blob, with h_j = (P^T s)_j carried from iteration to iteration, and
-// from the segment restrictions of this iteration (slot floats 8..: P^T r_k,
-// 14..: P^T w_k) computes h = P^T w_k + beta h, g = P^T r_(k+1) = P^T r_k -
-// alpha h with the new alpha and beta (after a failed true-residual check,
-// RESTART: g = P^T r of the true residual), then c = X g over the CTA's six
-// rows of X ~ A_c^-1 in one block reduction.
-// The coarse-space region of the dynamic shared memory: per thread the rest
-// offset and smoother weight (phi), the CTA's 6 rows of X, c (8 floats),
-// 6 x 32 reduction floats, and (P^T s)_j per coarse dof j.  The addresses are
-// recomputed from kernel parameters wherever they are used, so that they
-// need no registers across the iteration.
-struct CoarseView {
-    float4 *phi;
-    float *xrow, *cvec, *red6, *h;
-};
-
-template <typename T>
-__device__ __forceinline__ CoarseView coarse_view(const DeviceBatch &d)
-{
-    using T2 = typename CgCache<T>::T2;
-    size_t off = 12 * (size_t)CG_THREADS * sizeof(T) + (size_t)d.cg_cache_cols * CG_THREADS * sizeof(int) +
-                 (size_t)d.cg_cache_slots * CG_THREADS * (4 * sizeof(T2) + sizeof(T));
-    off = (off + 15) & ~(size_t)15;
-    CoarseView v;
-    v.phi = reinterpret_cast<float4 *>(cg_dyn + off);
-    v.xrow = reinterpret_cast<float *>(v.phi + CG_THREADS);
-    v.cvec = v.xrow + 6 * (size_t)d.coarse_nmax;
-    v.red6 = v.cvec + 8;
-    v.h = v.red6 + 6 * 32;
-    return v;
-}
-
-// The on-chip matrix copy of the register-resident CG kernel (layout in
-// k_cg), recomputed from kernel parameters where it is used.
-template <typename T>
-__device__ __forceinline__ CgCache<T> cg_cache_view(const DeviceBatch &d)
-{
-    using T2 = typename CgCache<T>::T2;
-    CgCache<T> cc;
-    cc.J = d.cg_cache_slots;
-    cc.JC = d.cg_cache_cols;
-    cc.col = reinterpret_cast<const int *>(cg_dyn + 12 * (size_t)CG_THREADS * sizeof(T));
-    cc.kv2 = reinterpret_cast<const T2 *>(cc.col + (size_t)cc.JC * CG_THREADS);
-    cc.kv1 = reinterpret_cast<const T *>(cc.kv2 + 4 * (size_t)cc.J * CG_THREADS);
-    return cc;
-}
-
-// c = X g, g_j held by thread j (zero beyond n): a 6-value block reduction.
-template <typename T>
-__device__ __forceinline__ void coarse_apply(const DeviceBatch &d, int n, float g)
-{
-    const CoarseView cv = coarse_view<T>(d);
-    const int j = threadIdx.x, lane = j & 31, warp = j >> 5;
-    float v[8];
-#pragma unroll
-    for (int l = 0; l < 8; l++) v[l] = (l < 6 && j < n) ? cv.xrow[l * n + j] * g : 0.f;
-    int idx;
-    const float t = warp_sum_multi<8>(v, idx);
-    if ((lane & 3) == 0 && idx < 6) cv.red6[idx * 32 + warp] = t;
-    __syncthreads();
-    if (warp < 6) {
-        const float u = warp_sum<float>(lane < (int)(blockDim.x >> 5) ? cv.red6[warp * 32 + lane] : 0.f);
-        if (lane == 0) cv.cvec[warp] = u;
-    }
-    __syncthreads();
-}
-
 // Coarse space of the memory-resident CG kernel (several segments per CTA,
 // any number of coarse dofs per blob).  Dynamic shared memory, after the
 // deferred-partials region: c of each of the CTA's segments (8 floats),
@@ -1779,30 +1372,6 @@ __device__ __forceinline__ CoarseMemView coarse_mem_view(const DeviceBatch &d)
     v.g = reinterpret_cast<float *>(v.hoff + CG_MAX_SEGS);
     v.h = v.g + d.coarse_hmax;
     return v;
-}
-
-// Phi_p^T v = (v, d_p x v) into ex[0..5] for the rest offset f.xyz of row p
-template <typename T>
-__device__ __forceinline__ void restrict6_of(const float4 f, const T v[3], float *ex)
-{
-    const float v0 = (float)v[0], v1 = (float)v[1], v2 = (float)v[2];
-    ex[0] = v0;
-    ex[1] = v1;
-    ex[2] = v2;
-    ex[3] = f.y * v2 - f.z * v1;
-    ex[4] = f.z * v0 - f.x * v2;
-    ex[5] = f.x * v1 - f.y * v0;
-}
-
-// u = omega D^-1 r + Phi_p c for row p (f = rest offset and omega, c = its
-// segment's coarse correction)
-template <typename T>
-__device__ __forceinline__ void coarse_u_of(const float4 f, const float *c, const T dinv[3], const T r[3], T u[3])
-{
-    const float cx = c[3], cy = c[4], cz = c[5];
-    const T pc[3] = {(T)(c[0] + cy * f.z - cz * f.y), (T)(c[1] + cz * f.x - cx * f.z), (T)(c[2] + cx * f.y - cy * f.x)};
-#pragma unroll
-    for (int k = 0; k < 3; k++) u[k] = (T)f.w * dinv[k] * r[k] + pc[k];
 }
 
 // acc + sum_t h_t g_t over the eight FP16 values h of one 16-byte load
@@ -1928,35 +1497,19 @@ __device__ __forceinline__ void coarse_mem_step(const DeviceBatch &d, const floa
     }
 }
 
-// L2 load issued where it stands (volatile asm keeps it ahead of the
-// barriers that follow, so its latency overlaps the reduction's own loads)
-__device__ __forceinline__ float ld_early(const float *p)
-{
-    float v;
-    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-
+// Reduction without a serial step: after a plain grid barrier every CTA sums
+// the partials of every busy blob itself, in the same fixed order, and runs
+// the transitions on its own copy of the blob records in shared memory, so
+// all CTAs reach bit-identical states.  CTA 0 alone records failure bits.
+// Also refreshes the CTA's view (state, alpha, beta of its nb blobs) and
+// returns the number of blobs still iterating.
 template <typename T>
 __device__ __forceinline__ unsigned int local_reduce(const DeviceBatch &d, const double *part, CgScalars *s_cg,
                                                      float *sm, unsigned int *s_run, int nb, const int *s_blob,
-                                                     int *s_state, T *s_alpha, T *s_beta, int coarse_n)
+                                                     int *s_state, T *s_alpha, T *s_beta)
 {
     const int nbl = d.num_blobs, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr bool fast = sizeof(T) == 4;
-    // coarse restrictions, loaded first so that they travel with the sums
-    float ptr = 0.f, ptw = 0.f;
-    int cb = -1;
-    if (coarse_n) {
-        cb = s_blob[0];
-        const BlobParams &bp = d.bp[cb];
-        const int j = threadIdx.x;
-        if (j < bp.coarse_n) {
-            const float *slot = reinterpret_cast<const float *>(part) + (size_t)d.part_stride * (bp.seg_off + j / 6);
-            ptr = ld_early(slot + 8 + j % 6);
-            ptw = ld_early(slot + 14 + j % 6);
-        }
-    }
     if (nbl < 8) {
         // one blob after the other with the whole CTA; thread 0 (in warp 0,
         // which holds the sums) runs every transition
@@ -1999,44 +1552,29 @@ __device__ __forceinline__ unsigned int local_reduce(const DeviceBatch &d, const
         }
     }
     __syncthreads();
-    if (coarse_n) {
-        const CgScalars &cg = s_cg[cb];
-        float g = 0.f;
-        if (threadIdx.x < coarse_n) {
-            float &h = coarse_view<T>(d).h[threadIdx.x];
-            if (cg.state == CG_RESTART) {
-                h = 0.f;
-                g = ptr;
-            } else {
-                h = ptw + cg.beta_f * h;
-                g = ptr - cg.alpha_f * h;
-            }
-        }
-        coarse_apply<T>(d, coarse_n, g);
-    }
     return *s_run;
 }
 
-// The whole solve of every blob in one cooperative launch: Jacobi-PCG in the
-// Chronopoulos-Gear form (one SpMV and one group of dot products per
-// iteration), x0 = 0, stopping on residual2() = sum r^2 / sum f^2 < eps^2
-// after each update (src/NoMassCGSolver.cpp:180-189, :233-247).  Per
-// iteration: phase A updates p, s, x, r and u = D^-1 r of the own rows; a
-// grid barrier makes u visible; phase B computes w = A u; then r.u, r.r and
-// w.u are summed per blob and each blob's CG state advances.  With few
-// segments and blobs (cg_local) every CTA does that sum itself after a plain
-// barrier, from partials double-buffered by iteration parity (a fast CTA's
-// next phase A must not overwrite what a slow CTA is still summing); else a
-// reducing barrier does it once, in the last CTA to arrive.  With
+// The memory-resident solve of every blob in one cooperative launch, for
+// batches with a blob of more CG segments than CTAs (the others run in
+// k_cg_group): PCG in the Chronopoulos-Gear form (one SpMV and one group of
+// dot products per iteration), x0 = 0, stopping on residual2() = sum r^2 /
+// sum f^2 < eps^2 after each update (src/NoMassCGSolver.cpp:180-189,
+// :233-247).  Per iteration: phase A updates p, s, x, r and u = M r of the
+// own rows; a grid barrier makes u visible; phase B computes w = A u; then
+// r.u, r.r and w.u are summed per blob and each blob's CG state advances.
+// With few segments and blobs (cg_local) every CTA does that sum itself after
+// a plain barrier, from partials double-buffered by iteration parity (a fast
+// CTA's next phase A must not overwrite what a slow CTA is still summing);
+// else a reducing barrier does it once, in the last CTA to arrive.  With
 // true_residual on, a recursive convergence is confirmed by an FP64 b - A x
 // and a failed check restarts the recurrences from that residual.
 //
 // Work split: the rows of each blob are cut into segments (32-row aligned, at
 // most CG_THREADS rows); CTA c owns segments [n_segs*c/G, n_segs*(c+1)/G) and
-// thread t row t of each.  With one segment per CTA (REG) the row state stays
-// in registers for the whole solve; only u and x go to memory, for the
-// neighbours.
-template <typename T, bool REG>
+// thread t row t of each.  The row state lives in global memory and each
+// phase moves only the fields it uses.
+template <typename T>
 __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
 {
     using W = T;
@@ -2104,7 +1642,6 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
     auto slot = [&](int seg) { return reinterpret_cast<float *>(part()) + (size_t)d.part_stride * seg; };
     refresh();
     using V4 = typename Vec4T<T>::type;
-    using T2 = typename CgCache<T>::T2;
     // x and the published u in global memory: addresses from the kernel
     // parameters at each use (no registers held across the iteration)
     auto X = [&]() { return static_cast<T *>(d.x); };
@@ -2121,65 +1658,8 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
         nomass = bp.solver == SOLVER_NOMASS;
         return nomass ? (T)(bp.calc_stokes == 1 ? d.drag[row] : 0.0) : static_cast<const T *>(d.mass_diag)[row];
     };
-    // REG: r, u, w of the CTA's only segment in registers; x, D^-1, p, s and
-    // the on-chip matrix copy in dynamic shared memory (p and s are used in
-    // phase A only; in registers they would be spilled around the SpMV):
-    //   x[3 CG_THREADS] T | dinv[3 CG_THREADS] T | p[3 CG_THREADS] T |
-    //   s[3 CG_THREADS] T | col[JC CG_THREADS] int | kv2[4 J CG_THREADS] T2 |
-    //   kv1[J CG_THREADS] T | coarse region (coarse_view)
-    RowState<T> reg;
-    bool reg_valid = false, reg_nomass = true;
-    T reg_diag = 0;
-    T *sx = reinterpret_cast<T *>(cg_dyn);
-    T *sdinv = sx + 3 * CG_THREADS;
-    if (REG) {
-        const CgCache<T> cc = cg_cache_view<T>(d);
-        const int row = row_of(0, reg_valid);
-        const size_t o = 3 * (size_t)row;
-        if (tid < s_rows[0]) {
-            reg_diag = diag_of(0, row, reg_nomass);
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                reg.r[k] = static_cast<const T *>(d.r)[o + k];
-                reg.u[k] = static_cast<const T *>(d.u)[o + k];
-                reg.w[k] = static_cast<const T *>(d.w)[o + k];
-                sx[(9 + k) * CG_THREADS + tid] = static_cast<const T *>(d.s)[o + k];
-                sx[(6 + k) * CG_THREADS + tid] = static_cast<const T *>(d.p)[o + k];
-                sx[k * CG_THREADS + tid] = static_cast<const T *>(d.x)[o + k];
-                sdinv[k * CG_THREADS + tid] = static_cast<const T *>(d.dinv)[o + k];
-            }
-        }
-        // every free row (NoMass or mass) reads its column indices from the
-        // copy; only NoMass rows read values from it
-        if (reg_valid) {
-            const int sl = row >> 5, lane = row & 31;
-            const int L = d.slice_len[sl], base = d.slice_ptr[sl];
-            const T *val = static_cast<const T *>(d.sell_val);
-            int *col = const_cast<int *>(cc.col);
-            T2 *kv2 = const_cast<T2 *>(cc.kv2);
-            T *kv1 = const_cast<T *>(cc.kv1);
-            for (int j = 0; j < min(cc.JC, L); j++) col[j * CG_THREADS + tid] = d.sell_col[base + 32 * j + lane];
-            for (int j = 0; reg_nomass && j < min(cc.J, L); j++) {
-                const size_t vb = (size_t)(base + 32 * j) * 9 + lane;
-#pragma unroll
-                for (int m = 0; m < 4; m++) {
-                    T2 kp;
-                    kp.x = val[vb + 32 * (2 * m)];
-                    kp.y = val[vb + 32 * (2 * m + 1)];
-                    kv2[(4 * j + m) * CG_THREADS + tid] = kp;
-                }
-                kv1[j * CG_THREADS + tid] = val[vb + 32 * 8];
-            }
-        }
-    }
-    // two-level preconditioner (REG and local only): per row the rest offset
-    // d_p and smoother weight, the CTA's 6 rows of X ~ A_c^-1, the blob's
-    // coarse residual g and this segment's coarse correction c
-    const bool coarse = REG && local && d.coarse;
-    // the same preconditioner in the memory-resident kernel (coarse_mem_step)
-    const bool mcoarse = !REG && d.coarse;
-    // memory-resident kernel in FP32: segment partials deferred (flush_partials)
-    constexpr bool kDefer = !REG && sizeof(T) == 4;
+    const bool mcoarse = d.coarse;  // two-level preconditioner (coarse_mem_step)
+    constexpr bool kDefer = sizeof(T) == 4;  // FP32: segment partials deferred (flush_partials)
     int dcnt = 0;  // deferred segments not yet flushed (CTA-uniform)
     auto defer_flush = [&]() {
         if constexpr (kDefer) {
@@ -2189,77 +1669,16 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
             }
         }
     };
-    int coarse_n = 0;  // coarse dofs of the CTA's blob (0: no coarse space)
-    if (coarse) {
-        const CoarseView cv = coarse_view<T>(d);
-        const BlobParams &bp = d.bp[s_blob[0]];
-        coarse_n = bp.coarse_n;
-        cv.h[tid] = 0.f;
-        cv.phi[tid] = reg_valid ? d.phi[s_row0[0] + tid] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float *Xg = d.coarse_X + bp.coarse_xoff + (size_t)(6 * (s_sid[0] - bp.seg_off)) * bp.coarse_n;
-        for (int k = tid; k < 6 * bp.coarse_n; k += CG_THREADS) cv.xrow[k] = Xg[k];
-    }
-    // u = omega D^-1 r + Phi_p c of the thread's row (REG, coarse)
-    auto coarse_u = [&](RowState<T> &S) {
-        const CoarseView cv = coarse_view<T>(d);
-        const float4 f = cv.phi[tid];
-        const float *cvec = cv.cvec;
-        const float cx = cvec[3], cy = cvec[4], cz = cvec[5];
-        const T pc[3] = {(T)(cvec[0] + cy * f.z - cz * f.y), (T)(cvec[1] + cz * f.x - cx * f.z),
-                         (T)(cvec[2] + cx * f.y - cy * f.x)};
-#pragma unroll
-        for (int k = 0; k < 3; k++) S.u[k] = (T)f.w * sdinv[k * CG_THREADS + tid] * S.r[k] + pc[k];
-    };
-    // Phi_p^T v = (v, d_p x v) into ex[0..5]
-    auto restrict6 = [&](const T v[3], float *ex) {
-        const float4 f = coarse_view<T>(d).phi[tid];
-        const float v0 = (float)v[0], v1 = (float)v[1], v2 = (float)v[2];
-        ex[0] = v0;
-        ex[1] = v1;
-        ex[2] = v2;
-        ex[3] = f.y * v2 - f.z * v1;
-        ex[4] = f.z * v0 - f.x * v2;
-        ex[5] = f.x * v1 - f.y * v0;
-    };
     auto row_info = [&](int j, int &row, bool &valid, T &diag, bool &nomass) {
-        if (REG) {
-            row = s_row0[0] + tid;
-            valid = reg_valid;
-            diag = reg_diag;
-            nomass = reg_nomass;
-        } else {
-            row = row_of(j, valid);
-            if (valid) diag = diag_of(j, row, nomass);
-        }
-    };
-    // x and D^-1 of the thread's row (component k)
-    auto xref = [&](RowState<T> &S, int k) -> T & { return REG ? sx[k * CG_THREADS + tid] : S.x[k]; };
-    auto pref = [&](RowState<T> &S, int k) -> T & { return REG ? sx[(6 + k) * CG_THREADS + tid] : S.p[k]; };
-    auto sref = [&](RowState<T> &S, int k) -> T & { return REG ? sx[(9 + k) * CG_THREADS + tid] : S.s[k]; };
-    auto dinv_of = [&](const RowState<T> &S, int k) -> T { return REG ? sdinv[k * CG_THREADS + tid] : S.dinv[k]; };
-    // REG: x of the own rows to global memory (for the FP64 true residual and
-    // the Euler update; the memory-resident variant keeps it there)
-    auto publish_x = [&]() {
-        if (REG && reg_valid) {
-            const size_t o = 3 * (size_t)(s_row0[0] + tid);
-#pragma unroll
-            for (int k = 0; k < 3; k++) X()[o + k] = sx[k * CG_THREADS + tid];
-        }
+        row = row_of(j, valid);
+        if (valid) diag = diag_of(j, row, nomass);
     };
     // phase A of segment j: p = u + beta p; s = w + beta s; x += alpha p;
     // r -= alpha s; u = D^-1 r.  Partials: slot 0 r.u, slot 2 r.r.
     auto phase_a = [&](int j) {
         const int k = s_tslot[j];
-        if (coarse && s_state[k] == CG_RESTART) {
-            // restart from the true residual: u = M r, published for phase B
-            if (reg_valid) {
-                coarse_u(reg);
-                U4()[s_row0[0] + tid] = V4{reg.u[0], reg.u[1], reg.u[2], (T)0};
-            }
-            return;
-        }
         if (mcoarse && s_state[k] == CG_RESTART) {
-            // the same from the row state in memory
+            // restart from the true residual: u = M r, published for phase B
             int row;
             bool valid, nomass = true;
             T diag = 0;
@@ -2279,16 +1698,15 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
         T diag = 0;
         row_info(j, row, valid, diag, nomass);
         W pg = 0, pr = 0;
-        RowState<T> loc;
-        RowState<T> &S = REG ? reg : loc;
-        if (!REG && valid) {
+        RowState<T> S;
+        if (valid) {
             // u of the last iteration from its published copy (the plain u
             // array is not kept up to date by the memory-resident iteration)
-            load_fields<T>(d, row, loc, RF_X | RF_R | RF_W | RF_S | RF_P | RF_DINV);
+            load_fields<T>(d, row, S, RF_X | RF_R | RF_W | RF_S | RF_P | RF_DINV);
             const V4 uo = U4()[row];
-            loc.u[0] = uo.x;
-            loc.u[1] = uo.y;
-            loc.u[2] = uo.z;
+            S.u[0] = uo.x;
+            S.u[1] = uo.y;
+            S.u[2] = uo.z;
         }
         float4 fm = make_float4(0.f, 0.f, 0.f, 0.f);  // mcoarse: the row's rest offset and omega
         if (mcoarse && valid) fm = d.phi[row];
@@ -2297,16 +1715,15 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
             const bool first = b == (T)0;
 #pragma unroll
             for (int cc2 = 0; cc2 < 3; cc2++) {
-                const T pn = first ? S.u[cc2] : S.u[cc2] + b * pref(S, cc2);
-                const T sn = first ? S.w[cc2] : S.w[cc2] + b * sref(S, cc2);
-                pref(S, cc2) = pn;
-                sref(S, cc2) = sn;
-                xref(S, cc2) += a * pn;
+                const T pn = first ? S.u[cc2] : S.u[cc2] + b * S.p[cc2];
+                const T sn = first ? S.w[cc2] : S.w[cc2] + b * S.s[cc2];
+                S.p[cc2] = pn;
+                S.s[cc2] = sn;
+                S.x[cc2] += a * pn;
                 S.r[cc2] -= a * sn;
-                S.u[cc2] = dinv_of(S, cc2) * S.r[cc2];
+                S.u[cc2] = S.dinv[cc2] * S.r[cc2];
             }
-            if (coarse) coarse_u(S);
-            else if (mcoarse) coarse_u_of<T>(fm, coarse_mem_view(d).cvec + 8 * j, S.dinv, S.r, S.u);
+            if (mcoarse) coarse_u_of<T>(fm, coarse_mem_view(d).cvec + 8 * j, S.dinv, S.r, S.u);
 #pragma unroll
             for (int cc2 = 0; cc2 < 3; cc2++) {
                 pg += S.r[cc2] * S.u[cc2];
@@ -2314,7 +1731,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
             }
             U4()[row] = V4{S.u[0], S.u[1], S.u[2], (T)0};
         }
-        if (!REG && valid) store_fields<T>(d, row, loc, RF_X | RF_R | RF_S | RF_P);
+        if (valid) store_fields<T>(d, row, S, RF_X | RF_R | RF_S | RF_P);
         if constexpr (kDefer) {
             const float inf[3] = {(float)pg, 0.f, (float)pr};
             if (mcoarse) {
@@ -2328,12 +1745,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
             return;
         }
         const W in[3] = {pg, (W)0, pr};
-        if (coarse) {
-            // restriction of the new r: slot floats 8..
-            float ex[6] = {0, 0, 0, 0, 0, 0};
-            if (valid) restrict6(S.r, ex);
-            seg_partials<W, 6>(slot(s_sid[j]), in, 5, ex, 8, red);
-        } else if (mcoarse) {
+        if (mcoarse) {
             float ex[6] = {0, 0, 0, 0, 0, 0};
             if (valid) restrict6_of<T>(fm, S.r, ex);
             seg_partials<W, 6>(slot(s_sid[j]), in, 5, ex, 8, red);
@@ -2353,31 +1765,29 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
         row_info(j, row, valid, diag, nomass);
         W pg = 0, pd = 0, pr = 0;
         double vr = 0.0, vg = 0.0;
-        RowState<T> loc;
-        RowState<T> &S = REG ? reg : loc;
+        RowState<T> S;
         // an ACTIVE iteration only needs w.u here (r.u and r.r came from
         // phase A); the prologue and a restart also sum r.u and r.r
         const bool need_r = prologue || state != CG_ACTIVE;
-        if (!REG && valid) {
-            if (need_r) load_fields<T>(d, row, loc, RF_R | (state == CG_VERIFY ? RF_DINV : 0));
+        if (valid) {
+            if (need_r) load_fields<T>(d, row, S, RF_R | (state == CG_VERIFY ? RF_DINV : 0));
             if (state != CG_VERIFY) {
                 const V4 uo = U4()[row];  // the u the product reads (published in phase A)
-                loc.u[0] = uo.x;
-                loc.u[1] = uo.y;
-                loc.u[2] = uo.z;
+                S.u[0] = uo.x;
+                S.u[1] = uo.y;
+                S.u[2] = uo.z;
             }
         }
         if (valid) {
             if (state != CG_VERIFY) {
                 T au[3];
-                sell_row_cg<T, !REG>(d, row, nomass, diag, static_cast<const V4 *>(d.u4), au,
-                                     REG ? cg_cache_view<T>(d) : CgCache<T>{});
+                sell_row_cg<T>(d, row, nomass, diag, static_cast<const V4 *>(d.u4), au);
 #pragma unroll
                 for (int cc2 = 0; cc2 < 3; cc2++) {
                     S.w[cc2] = au[cc2];
                     pd += au[cc2] * S.u[cc2];
                 }
-                if (REG || need_r) {
+                if (need_r) {
 #pragma unroll
                     for (int cc2 = 0; cc2 < 3; cc2++) {
                         pg += S.r[cc2] * S.u[cc2];
@@ -2390,14 +1800,14 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
 #pragma unroll
                 for (int cc2 = 0; cc2 < 3; cc2++) {
                     S.r[cc2] = (T)rt[cc2];
-                    S.u[cc2] = dinv_of(S, cc2) * S.r[cc2];
+                    S.u[cc2] = S.dinv[cc2] * S.r[cc2];
                     vr += rt[cc2] * rt[cc2];
                     vg += (double)S.r[cc2] * (double)S.u[cc2];
                 }
                 U4()[row] = V4{S.u[0], S.u[1], S.u[2], (T)0};
             }
         }
-        if (!REG && valid) store_fields<T>(d, row, loc, state == CG_VERIFY ? (RF_R | RF_U) : RF_W);
+        if (valid) store_fields<T>(d, row, S, state == CG_VERIFY ? (RF_R | RF_U) : RF_W);
         if constexpr (kDefer) {
             if (!prologue && state == CG_ACTIVE) {
                 const float inf[3] = {(float)pg, (float)pd, (float)pr};
@@ -2413,8 +1823,9 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
             }
         }
         if (mcoarse) {
-            // the restrictions of the register-resident branch below, with
-            // the rest offset from memory
+            // restrictions: ACTIVE P^T w (slot floats 14..); the prologue,
+            // RESTART and VERIFY restart the coarse recurrence: P^T r (8..)
+            // and P^T w (14.., zero for VERIFY)
             const float4 fm = valid ? d.phi[row] : make_float4(0.f, 0.f, 0.f, 0.f);
             float ex[12];
 #pragma unroll
@@ -2423,28 +1834,6 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
             if (valid) {
                 if (full) restrict6_of<T>(fm, S.r, ex);
                 if (state != CG_VERIFY) restrict6_of<T>(fm, S.w, ex + 6);
-            }
-            if (state == CG_VERIFY) {
-                const double in[3] = {vg, 0.0, vr};
-                seg_partials<double, 12>(slot(s_sid[j]), in, 5, ex, 8, red);
-            } else if (full) {
-                const W in[3] = {pg, pd, pr};
-                seg_partials<W, 12>(slot(s_sid[j]), in, 7, ex, 8, red);
-            } else {
-                const W in[3] = {pg, pd, pr};
-                seg_partials<W, 6>(slot(s_sid[j]), in, 2, ex + 6, 14, red);
-            }
-        } else if (coarse) {
-            // restrictions: ACTIVE P^T w (slot floats 14..); the prologue,
-            // RESTART and VERIFY restart the coarse recurrence: P^T r (8..)
-            // and P^T w (14.., zero for VERIFY)
-            float ex[12];
-#pragma unroll
-            for (int m = 0; m < 12; m++) ex[m] = 0.f;
-            const bool full = prologue || state != CG_ACTIVE;
-            if (valid) {
-                if (full) restrict6(S.r, ex);
-                if (state != CG_VERIFY) restrict6(S.w, ex + 6);
             }
             if (state == CG_VERIFY) {
                 const double in[3] = {vg, 0.0, vr};
@@ -2471,30 +1860,12 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
         if (!local) return reducing_barrier(d, mcoarse ? part() : d.partials, &s_err, &s_pub, s_last, sm_df);
         counting_barrier(d.bar, (++n_bar) * (unsigned int)G, &s_err);
         if (s_err) return 0u;
-        return local_reduce<T>(d, part(), s_cg, sm_df, &s_run, nb, s_blob, s_state, s_alpha, s_beta,
-                               coarse_n);
+        return local_reduce<T>(d, part(), s_cg, sm_df, &s_run, nb, s_blob, s_state, s_alpha, s_beta);
     };
-    if (coarse) {
-        // u_0 = M r_0 needs P^T r_0 of every segment of the blob: restrict
-        // into the second partials buffer, sum after a barrier, solve
-        parity = 1;
-        {
-            float ex[6] = {0, 0, 0, 0, 0, 0};
-            if (reg_valid) restrict6(reg.r, ex);
-            const W none[3] = {(W)0, (W)0, (W)0};
-            seg_partials<W, 6>(slot(s_sid[0]), none, 0, ex, 8, red);
-        }
-        counting_barrier(d.bar, (++n_bar) * (unsigned int)G, &s_err);
-        if (!s_err) {
-            const BlobParams &bp = d.bp[s_blob[0]];
-            coarse_apply<T>(d, coarse_n, tid < coarse_n ? __ldcg(slot(bp.seg_off + tid / 6) + 8 + tid % 6) : 0.f);
-            if (reg_valid) coarse_u(reg);
-        }
-        parity = 0;
-    }
     if (mcoarse) {
-        // the same with the row state in memory: P^T r_0 of every segment,
-        // then c per segment and u_0 = M r_0 stored for the publication below
+        // u_0 = M r_0 needs P^T r_0 of every segment of the blob: restrict
+        // into the second partials buffer, sum after a barrier, then c per
+        // segment and u_0 stored for the publication below
         parity = 1;
         for (int j = 0; j < nt; j++) {
             int row;
@@ -2535,12 +1906,8 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
     for (int j = 0; j < nt; j++) {
         const int row = s_row0[j] + tid;
         if (tid < s_rows[j]) {
-            if (coarse) {
-                U4()[row] = reg_valid ? V4{reg.u[0], reg.u[1], reg.u[2], (T)0} : V4{(T)0, (T)0, (T)0, (T)0};
-            } else {
-                const T *u = static_cast<const T *>(d.u) + 3 * (size_t)row;
-                U4()[row] = V4{u[0], u[1], u[2], (T)0};
-            }
+            const T *u = static_cast<const T *>(d.u) + 3 * (size_t)row;
+            U4()[row] = V4{u[0], u[1], u[2], (T)0};
         }
     }
     counting_barrier(d.bar, (++n_bar) * (unsigned int)G, &s_err);
@@ -2557,7 +1924,6 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
             coarse_mem_step<T>(d, reinterpret_cast<const float *>(part()), s_sid, nt, nb, s_blob, s_tslot, s_state,
                                s_alpha, s_beta, false);
         if (local || mcoarse) parity ^= 1;
-        if (REG && s_state[0] == CG_VERIFY) publish_x();
         for (int j = 0; j < nt; j++) phase_a(j);
         defer_flush();
         counting_barrier(d.bar, (++n_bar) * (unsigned int)G, &s_err);
@@ -2567,7 +1933,6 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
         loops++;
         running = reduce();
     }
-    publish_x();
     if (d.cg_euler && !s_err) {
         // the step's Euler update (Blob::euler_integrate, src/Blob.cpp:3937-3969)
         // of the own rows, for blobs that had not failed before the solve and
@@ -2584,7 +1949,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cg(DeviceBatch d)
 #pragma unroll
             for (int cc2 = 0; cc2 < 3; cc2++) {
                 const size_t kk = 3 * (size_t)row + cc2;
-                const double xi = REG ? (double)sx[cc2 * CG_THREADS + tid] : (double)X()[kk];
+                const double xi = (double)X()[kk];
                 double pn;
                 if (bp.solver == SOLVER_NOMASS) {
                     d.vel[kk] = xi;
@@ -2955,40 +2320,6 @@ void launch_nodes(const DeviceBatch &d, cudaStream_t s, int use_given_rhs)
     PREC_DISPATCH(d, k_nodes, d.n_tiles, NODE_TILE * NODE_LANES, s, d, use_given_rhs);
 }
 
-template <typename T>
-static int cg_smem_plan_t(int max_slots, int max_cols, size_t extra_bytes, int *J, int *JC, size_t *dyn_bytes)
-{
-    int dev = 0, optin = 0;
-    *J = *JC = 0;
-    *dyn_bytes = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return -1;
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return -1;
-    cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, k_cg<T, true>) != cudaSuccess) return -1;
-    const size_t reserve = 1024;  // per-CTA system use
-    const size_t state = 12 * (size_t)CG_THREADS * sizeof(T);  // x, D^-1, p and s
-    const size_t fixed = fa.sharedSizeBytes + reserve + state + extra_bytes;
-    if ((size_t)optin < fixed) return -1;
-    size_t room = optin - fixed;
-    const size_t per_col = (size_t)CG_THREADS * sizeof(int), per_slot = (size_t)CG_THREADS * 9 * sizeof(T);
-    *JC = (int)std::min<size_t>(room / per_col, (size_t)std::max(0, max_cols));
-    room -= (size_t)*JC * per_col;
-    *J = (int)std::min<size_t>(room / per_slot, (size_t)std::max(0, std::min(max_slots, *JC)));
-    *dyn_bytes = state + (size_t)*JC * per_col + (size_t)*J * per_slot + extra_bytes;
-    // the limit is a property of the kernel, shared by every handle: set it
-    // to the device maximum so that no handle's plan lowers another's
-    if (cudaFuncSetAttribute(k_cg<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             optin - (int)fa.sharedSizeBytes) != cudaSuccess)
-        return -1;
-    return 0;
-}
-
-int cg_smem_plan(int precision, int max_slots, int max_cols, size_t extra_bytes, int *J, int *JC, size_t *dyn_bytes)
-{
-    return precision == PREC_FP64 ? cg_smem_plan_t<double>(max_slots, max_cols, extra_bytes, J, JC, dyn_bytes)
-                                  : cg_smem_plan_t<float>(max_slots, max_cols, extra_bytes, J, JC, dyn_bytes);
-}
-
 // Dynamic shared memory of the memory-resident CG kernel with the coarse
 // space (coarse_mem_view): its size for the given coarse dimensions, and
 // whether the device allows it (the kernel's limit is raised to the device
@@ -3007,7 +2338,7 @@ int cg_mem_smem_allow(int precision, size_t dyn_bytes)
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return -1;
     cudaFuncAttributes fa;
-    const void *fn = precision == PREC_FP64 ? (const void *)k_cg<double, false> : (const void *)k_cg<float, false>;
+    const void *fn = precision == PREC_FP64 ? (const void *)k_cg<double> : (const void *)k_cg<float>;
     if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) return -1;
     const size_t reserve = 1024;
     if (fa.sharedSizeBytes + reserve + dyn_bytes > (size_t)optin) return -1;
@@ -3017,18 +2348,15 @@ int cg_mem_smem_allow(int precision, size_t dyn_bytes)
     return 0;
 }
 
-int cg_max_grid(int precision, int reg, size_t dyn_bytes)
+int cg_max_grid(int precision, size_t dyn_bytes)
 {
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    cudaError_t e;
-    if (precision == PREC_FP64)
-        e = reg ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg<double, true>, CG_THREADS, dyn_bytes)
-                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg<double, false>, CG_THREADS, dyn_bytes);
-    else
-        e = reg ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg<float, true>, CG_THREADS, dyn_bytes)
-                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg<float, false>, CG_THREADS, dyn_bytes);
+    const cudaError_t e =
+        precision == PREC_FP64
+            ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg<double>, CG_THREADS, dyn_bytes)
+            : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg<float>, CG_THREADS, dyn_bytes);
     if (e != cudaSuccess) return 0;
     return sms * per_sm;
 }
@@ -3053,6 +2381,7 @@ cudaError_t launch_cg(const DeviceBatch &dev, cudaStream_t s, bool euler)
 {
     DeviceBatch d = dev;
     d.cg_euler = euler ? 1 : 0;
+    if (d.group) return launch_cg_group(d, s);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)d.cg_grid);
     cfg.blockDim = dim3(CG_THREADS);
@@ -3064,9 +2393,8 @@ cudaError_t launch_cg(const DeviceBatch &dev, cudaStream_t s, bool euler)
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     FFEA_LAUNCHED();
-    if (d.precision == PREC_FP64)
-        return d.cg_reg ? cudaLaunchKernelEx(&cfg, k_cg<double, true>, d) : cudaLaunchKernelEx(&cfg, k_cg<double, false>, d);
-    return d.cg_reg ? cudaLaunchKernelEx(&cfg, k_cg<float, true>, d) : cudaLaunchKernelEx(&cfg, k_cg<float, false>, d);
+    if (d.precision == PREC_FP64) return cudaLaunchKernelEx(&cfg, k_cg<double>, d);
+    return cudaLaunchKernelEx(&cfg, k_cg<float>, d);
 }
 
 void launch_energies(const DeviceBatch &d, cudaStream_t s)

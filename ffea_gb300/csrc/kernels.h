@@ -20,13 +20,11 @@ struct DeviceBatch {
     int32_t precision = PREC_MIXED;
     int32_t any_mass = 0, any_nomass = 0, any_lumped = 0;
     int32_t cg_grid = 0;          // CTAs of the persistent CG kernel
-    int32_t cg_reg = 0;           // 1: one CG segment per CTA, row state kept in registers
+    const struct GroupBatch *group = nullptr;  // (host memory) every blob fits on chip: k_cg_group, else k_cg
     int32_t cg_local = 0;         // 1: every CTA reduces the dot products itself (few segments and blobs)
     int32_t cg_euler = 0;         // 1 (per launch): the CG kernel ends with the Euler update of the step
-    int32_t cg_cache_slots = 0;   // REG: matrix slots per row whose values are copied to shared memory
-    int32_t cg_cache_cols = 0;    // REG: matrix slots per row whose column indices are copied
     int32_t part_stride = 8;      // floats per segment slot of the CG partials (32 with the coarse space)
-    // two-level preconditioner (REG and local reduction, NoMass, mixed precision)
+    // two-level preconditioner (NoMass, mixed precision)
     int32_t coarse = 0;           // 1: u = diag(omega) D^-1 r + P A_c^-1 P^T r
     int32_t coarse_nmax = 0;      // largest coarse dimension of a blob
     int32_t coarse_hmax = 0;      // memory-resident CG kernel: most coarse dofs of the blobs one CTA touches
@@ -41,7 +39,7 @@ struct DeviceBatch {
     float *coarse_T = nullptr, *coarse_Xn = nullptr;      // Newton-Schulz scratch (coarse_nmax^2)
     float *coarse_part = nullptr;                         // split-K partial products of the Newton-Schulz GEMMs
     float *coarse_asm = nullptr;                          // partial A_c blocks: 36 floats x CG_SEG_MAX_ROWS / 256 per neighbour entry
-    int32_t cg_dyn_smem = 0;      // REG: dynamic shared memory bytes of that copy
+    int32_t cg_dyn_smem = 0;      // dynamic shared memory of the CG kernel, bytes
     // blobs
     BlobParams *bp = nullptr;
     Material *mats = nullptr;
@@ -99,12 +97,38 @@ struct DeviceBatch {
     CgScalars *cg = nullptr;        // per blob
     double *last_sums = nullptr;    // per blob: r.u, w.u, r.r of the last reduction (written by CTA 0)
     unsigned int *counters = nullptr;  // one per reduction site
-    unsigned int *bar = nullptr;    // grid barrier: arrival count, generation
+    // CG kernels: [0, 1] reducing barrier (arrivals, generation), [2, 3]
+    // running blobs, [4] time-out flag, [5] counting-barrier arrivals;
+    // k_cg_group: [6] base of the exchange tags, [7] tags used and [8]
+    // iterations of the launch's longest solve, [9] CTAs that have finished
+    unsigned int *bar = nullptr;
     int32_t *status = nullptr;      // per blob failure bits
     int32_t *inverted = nullptr;    // per blob inverted-element count of the last step
     double *energy = nullptr;       // per blob: strain, kinetic
     double *epartials = nullptr;    // 2 per element tile
     unsigned long long *loop_count = nullptr;  // CG iterations executed by the persistent kernel (max over blobs)
+};
+
+// What k_cg_group needs beside the batch.  CTA c solves segments
+// task[ptr[c]] .. task[ptr[c + 1] - 1].
+struct GroupBatch {
+    int32_t grid = 0, threads = 0;  // launch shape
+    int32_t rows = 0;               // rows a CTA has room for
+    int32_t dyn_smem = 0;
+    int32_t cache_slots = 0;  // matrix slots per row whose values are copied to shared memory
+    int32_t cache_cols = 0;   // matrix slots per row whose column places are copied
+    int32_t *ptr = nullptr, *task = nullptr;
+    // per segment its halo, the rows of other segments it couples to, and per
+    // matrix entry its column as a place in the CTA's copy of u: the local
+    // row, or `rows` + its place in the halo
+    int32_t *hptr = nullptr, *halo = nullptr;
+    uint16_t *lcol = nullptr;
+    // exchange: GRP_WORDS words of sums per segment and exchange parity; the
+    // published u per row
+    uint4 *words = nullptr, *pub = nullptr;
+    // byte offsets into the dynamic shared memory
+    int32_t o_state = 0, o_u = 0, o_halo = 0, o_words = 0, o_phi = 0, o_xrow = 0, o_h = 0, o_col = 0, o_kv2 = 0,
+            o_kv1 = 0;
 };
 
 // A position as a double-float pair (DeviceBatch::pos_df): hi = (float)p,
@@ -144,6 +168,7 @@ enum ElemMode { ELEM_STEP = 0, ELEM_MATRIX_ONLY = 1 };
 
 constexpr int CG_THREADS = CG_SEG_MAX_ROWS;  // threads per CTA of the CG kernel = maximum rows of a segment
 constexpr int CG_MAX_SEGS = 64;         // segments per CTA of the persistent kernel
+constexpr int GRP_WORDS = 6;            // k_cg_group: 16-byte words of sums per segment (2 of dot terms, 4 of the coarse space)
 constexpr int CG_LOCAL_MAX_BLOBS = 64;  // local reduction: blob records kept in shared memory
 constexpr int CG_LOCAL_MAX_SEGS = 2048; // local reduction: partial sums every CTA reads per iteration
 // memory-resident CG kernel (FP32): segment partials deferred in shared memory
@@ -176,12 +201,16 @@ void launch_apply(const DeviceBatch &d, cudaStream_t s, const double *in, double
 void launch_spmv_variant(const DeviceBatch &d, cudaStream_t s, int variant);
 void launch_rng_draws(const mrg::JumpMat *table, const uint32_t *state, uint64_t offset, int64_t count, double *out,
                       cudaStream_t s);
-// Shared-memory plan of the register-resident CG kernel on the current
-// device: column indices of JC slots per row (at most max_cols) and values of
-// J slots (at most max_slots), plus x and D^-1 and extra_bytes (the coarse
-// space); dyn_bytes is the dynamic shared memory that takes (also set as the
-// kernel's limit).  -1 on error.
-int cg_smem_plan(int precision, int max_slots, int max_cols, size_t extra_bytes, int *J, int *JC, size_t *dyn_bytes);
+cudaError_t launch_cg_group(const DeviceBatch &d, cudaStream_t s);
+// Launch shape and shared-memory plan of k_cg_group on the current device:
+// column places of at most max_cols slots per row and values of at most
+// max_slots, for segments of max_rows rows with max_halo halo rows in groups
+// of max_segs; sets g's threads, rows, cache_*, dyn_smem and o_* (and raises
+// the kernel's limit).  -1 on error.
+int cg_group_plan(const DeviceBatch &d, GroupBatch &g, int max_slots, int max_cols, int max_rows, int max_halo,
+                  int max_segs);
+// CTAs of k_cg_group with that plan that fit co-resident, 0 on error
+int cg_group_max_grid(const DeviceBatch &d, const GroupBatch &g);
 // Learned smoother weights (learned.cu): a 3-layer mesh message-passing
 // network, hidden width 32, 8 input features per node.
 constexpr int MPNN_FEATURES = 8;
@@ -221,10 +250,9 @@ void sgemm_batched(const float *A, const float *B, const float *D, float *C, int
 int sgemm_splits(int n, int batch);
 // floats of split-K scratch the coarse refresh of these blobs needs (0: none)
 size_t coarse_part_floats(const std::vector<BlobParams> &bps);
-// CTAs of the persistent CG kernel (register-resident variant with dyn_bytes
-// of dynamic shared memory, or not) that fit co-resident on the current
-// device, 0 on error
-int cg_max_grid(int precision, int reg, size_t dyn_bytes);
+// CTAs of the memory-resident CG kernel with dyn_bytes of dynamic shared
+// memory that fit co-resident on the current device, 0 on error
+int cg_max_grid(int precision, size_t dyn_bytes);
 size_t cg_mem_defer_bytes(int precision);
 size_t cg_mem_coarse_bytes(int coarse_hmax);
 int cg_mem_smem_allow(int precision, size_t dyn_bytes);
