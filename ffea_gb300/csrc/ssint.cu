@@ -79,6 +79,8 @@ struct ffea_gpu_ssint {
     int *d_blob = nullptr;
     int *d_type = nullptr;
     double *d_geo = nullptr;    // 16 doubles: corners (9), unit normal (3), area, fourth node (3)
+    double *d_gp = nullptr;     // 16 doubles: Gauss points (9), unit normal (3), area, centroid (3)
+    float4 *d_nb = nullptr;     // the normal in FP32 and the blob (its bits)
     int *d_cell = nullptr;      // -1: outside the box
     double *d_fforce = nullptr; // 12 doubles: force on each corner and on the fourth node
     double *d_corr = nullptr;   // periodic blob corrections (num_blobs^2 x 3), when set
@@ -137,7 +139,8 @@ __device__ __forceinline__ int wrap(int x, int n)
 }
 
 __global__ void k_face_geom(const double *__restrict__ pos, const int *__restrict__ corner, int nf, double h,
-                            int nx, int ny, int nz, double *__restrict__ geo, int *__restrict__ cell,
+                            int nx, int ny, int nz, const int *__restrict__ fblob, double *__restrict__ geo,
+                            double *__restrict__ gp, float4 *__restrict__ nb, int *__restrict__ cell,
                             int *__restrict__ count, unsigned long long *stats)
 {
     int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -170,13 +173,26 @@ __global__ void k_face_geom(const double *__restrict__ pos, const int *__restric
     g[12] = .5 * mag;
 #pragma unroll
     for (int d = 0; d < 3; d++) g[13 + d] = apex >= 0 ? pos[3 * (long long)apex + d] : 0.0;
+    // what the pair kernel reads of a face, formed once here instead of once
+    // per pair
+    double *q = gp + 16 * (long long)f;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) q[3 * k + d] = eta(k, 0) * v[0][d] + eta(k, 1) * v[1][d] + eta(k, 2) * v[2][d];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        q[9 + d] = g[9 + d];
+        q[13 + d] = (1.0 / 3.0) * (v[0][d] + v[1][d] + v[2][d]);
+    }
+    q[12] = g[12];
+    nb[f] = make_float4((float)g[9], (float)g[10], (float)g[11], __int_as_float(fblob[f]));
     int c[3];
     const int dims[3] = {nx, ny, nz};
     bool inside = true;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        const double cen = (1.0 / 3.0) * (v[0][d] + v[1][d] + v[2][d]);
-        const double fl = floor(cen / h);
+        const double fl = floor(q[13 + d] / h);
         // cells beyond int range (or a NaN centroid) are outside the box as well
         int x = (fl >= -2147483647.0 && fl <= 2147483647.0) ? (int)fl : -2147483647;
         x = (x < -dims[d] || x >= 2 * dims[d]) ? -1 : wrap(x, dims[d]);
@@ -348,88 +364,80 @@ __global__ void __launch_bounds__(256) k_sort_large(long long ncell, int nblocks
     }
 }
 
-// The integrated point-pair potentials of one face pair, for f1 = A, f2 = B:
+// The integrated point-pair potentials of one face pair (FFEA's f1 the face
+// with the lower index):
 //   POT_LJ    do_lj_interaction (src/VdW_solver.cpp:237-330) with
 //             calc_lj_force_pair_matrix / calc_lj_factors (:664-699, :736-752);
 //   POT_SOFT  do_gensoft_interaction (:488-563) with
 //             calc_gensoft_force_pair_matrix / calc_gensoft_factors (:701-734, :754-771).
-// Adds force1 (A_SIDE) or force2 (!A_SIDE) to out[0..2] and returns the pair
-// energy.  k0: the soft potential's k0 (unused by POT_LJ).
+// own, oth: the Gauss points of the face whose force is summed and of its
+// partner; lower: own is f1.  FFEA's matrix of point forces is symmetric by
+// construction (the entry of points k < l of f1 and f2 stands for (l, k) too),
+// so both faces' forces are weighted sums of its column sums
+// S_l = sum_k fpm[k][l] (force1_j = sum_l W^2 eta_l[j] S_l, force2 = -force1),
+// and with d = own - oth the own face's S has the same form on either side.
+// Adds area product * S to S (the weights follow once per face) and returns
+// the pair energy.  k0: the soft potential's k0 (unused by POT_LJ).
+//
+// FP64-bound: an FP64 instruction takes 64 issue slots on GB300, so the point
+// forces are written with the fewest of them: fm (p - q) / r =
+// 12 emin f6 (f6 - 1) / r^2 (p - q) needs one reciprocal and no square root,
+// and products are fused (explicitly: the file is compiled without
+// contraction).  About 200 instructions a pair and side, from about 600.
 constexpr int POT_LJ = 0, POT_SOFT = 1;
 
-template <int POT, bool A_SIDE>
-__device__ __forceinline__ double pot_pair(const double *A, const double *B, double emin, double rmin, double k0,
-                                           double out[4][3])
+template <int POT>
+__device__ __forceinline__ double pot_pair(const double (&own)[9], const double (&oth)[9], double apaq, bool lower,
+                                           double emin, double rmin, double k0, double (&S)[3][3])
 {
-    double p[3][3], q[3][3];
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            p[k][d] = eta(k, 0) * A[d] + eta(k, 1) * A[3 + d] + eta(k, 2) * A[6 + d];
-            q[k][d] = eta(k, 0) * B[d] + eta(k, 1) * B[3 + d] + eta(k, 2) * B[6 + d];
-        }
-    const double r2 = rmin * rmin;
-    const double r4 = r2 * r2;
-    const double r6 = r4 * r2;
-    double fpm[3][3][3];
+    double T[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    const double r2m = rmin * rmin;
+    const double r6 = r2m * r2m * r2m;
+    const double c12 = 12 * emin;
+    // soft potential: t = fm / r = s1 r^2 + s2 r + k0, e = e4 r^4 + e3 r^3 + k0/2 r^2 - emin
+    double s1 = 0, s2 = 0, e4 = 0, e3 = 0;
+    if constexpr (POT == POT_SOFT) {
+        const double irm = 1. / rmin, irm2 = irm * irm, k0rm = k0 * rmin, k0rm2 = k0rm * rmin, eps = emin * irm;
+        s1 = 2 * (k0rm - 6 * eps) * irm2 * irm;
+        s2 = 3 * (4 * eps - k0rm) * irm2;
+        e4 = (0.5 * k0rm2 - 3 * emin) * irm2 * irm2;
+        e3 = (4 * emin - k0rm2) * irm2 * irm;
+    }
     double energy = 0.0;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
 #pragma unroll
         for (int l = k; l < 3; l++) {
-            const double dx = p[k][0] - q[l][0], dy = p[k][1] - q[l][1], dz = p[k][2] - q[l][2];
-            const double mag_r = sqrt(dx * dx + dy * dy + dz * dz);
-            const double ri = 1. / mag_r;
-            double fm, e;
+            // points k of f1 and l of f2
+            double v[3];
+#pragma unroll
+            for (int d = 0; d < 3; d++)
+                v[d] = (lower ? own[3 * k + d] : own[3 * l + d]) - (lower ? oth[3 * l + d] : oth[3 * k + d]);
+            const double r2 = fma(v[0], v[0], fma(v[1], v[1], v[2] * v[2]));
+            double t, e;
             if constexpr (POT == POT_LJ) {
-                const double ri2 = ri * ri;
-                const double ri4 = ri2 * ri2;
-                const double ri6 = ri4 * ri2;
-                const double ri7 = ri6 * ri;
-                const double f6 = r6 * ri6;
-                fm = 12 * ri7 * r6 * emin * (f6 - 1);
-                e = kW * kW * emin * f6 * (f6 - 2);
+                const double ri2 = __drcp_rn(r2);
+                const double f6 = r6 * (ri2 * ri2 * ri2);
+                t = c12 * f6 * (f6 - 1) * ri2;
+                e = f6 * (f6 - 2);
             } else {
-                const double mag_r_2 = mag_r * mag_r;
-                const double gf2 = mag_r_2 / r2;
-                const double gf3 = gf2 * mag_r / rmin;
-                const double k0rm = k0 * rmin;
-                const double k0rm2 = k0rm * rmin;
-                const double epsonrm = emin / rmin;
-                fm = 2 * (k0rm - 6 * epsonrm) * gf3 + 3 * (4 * epsonrm - k0rm) * gf2 + k0 * mag_r;
-                e = kW * kW *
-                    ((0.5 * k0rm2 - 3 * emin) * gf2 * gf2 + (4 * emin - k0rm2) * gf3 + 0.5 * k0 * mag_r_2 - emin);
+                const double r = sqrt(r2);
+                t = fma(s1, r2, fma(s2, r, k0));
+                e = fma(r2, fma(e4, r2, fma(e3, r, 0.5 * k0)), -emin);
             }
-            energy += (l == k) ? e : 2 * e;
+            energy = l == k ? energy + e : fma(2.0, e, energy);
 #pragma unroll
             for (int d = 0; d < 3; d++) {
-                fpm[k][l][d] = fm * ((p[k][d] - q[l][d]) * ri);  // FFEA divides by mag_r: within 1 ulp
-                fpm[l][k][d] = fpm[k][l][d];
+                T[l][d] = fma(t, v[d], T[l][d]);
+                if (l != k) T[k][d] = fma(t, v[d], T[k][d]);
             }
         }
     }
-    const double apaq = A[12] * B[12];
-    // FFEA sums W^2 eta * fpm over all nine (k, l) for each corner j.  The
-    // matrix is symmetric, so both sides need only the column sums
-    // S_l = sum_k fpm[k][l]: force1_j = sum_l W^2 eta_l[j] S_l and
-    // force2_j = -sum_k W^2 eta_k[j] S_k.  Same terms, regrouped (27 products
-    // per pair instead of 243; the sums round differently, within 1e-15).
-    double S[3][3];
 #pragma unroll
     for (int l = 0; l < 3; l++)
 #pragma unroll
-        for (int d = 0; d < 3; d++) S[l][d] = fpm[0][l][d] + fpm[1][l][d] + fpm[2][l][d];
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            const double f = (kW * kW * eta(0, j)) * S[0][d] + (kW * kW * eta(1, j)) * S[1][d] +
-                             (kW * kW * eta(2, j)) * S[2][d];
-            out[j][d] += (A_SIDE ? f : -f) * apaq;
-        }
-    }
-    return energy * apaq;
+        for (int d = 0; d < 3; d++) S[l][d] = fma(apaq, T[l][d], S[l][d]);
+    return (POT == POT_LJ ? kW * kW * emin : kW * kW) * energy * apaq;
 }
 
 // ---- steric: the overlap of two tetrahedra -------------------------------
@@ -639,21 +647,18 @@ __device__ double st_overlap(const double (*A)[3], const double (*B)[3], double 
     return vol;
 }
 
-// One steric pair, f1 = A, f2 = B (the tetrahedra of the faces' elements):
+// The forces of one steric pair, f1 = A, f2 = B (the tetrahedra of the faces'
+// elements), from its overlap volumes:
 // Face::getTetraIntersectionVolumeTotalGradientAndShapeFunctions
 // (src/Face.cpp:473-514) and do_steric_interaction's scaling
-// (src/VdW_solver.cpp:470-483).  false when they do not overlap; else adds
-// the A side's (phi1 k dV/dr) or the B side's (-phi2 k dV/dr) node forces to
-// out and sets vol = k V.
-__device__ bool steric_pair(const double (*A)[3], const double (*B)[3], double dr, double k, bool a_side,
-                            double out[4][3], double &vol)
+// (src/VdW_solver.cpp:470-483).  V > 0 and centre cm of A and B; vb[dir] with
+// B moved by dr along dir, va[dir] with A moved.  Adds the node forces of the
+// side with tetrahedron T, the A side's (phi1 k dV/dr) or the B side's
+// (-phi2 k dV/dr), to out.
+__device__ void steric_forces(const double (*T)[3], double V, const double *cm, const double *vb, const double *va,
+                              double dr, double k, bool a_side, double out[4][3])
 {
-    double cm[3];
-    const double V = st_overlap(A, B, cm);
-    if (V == 0) return false;
-    // getLocalCoordinatesForLinTet (src/mat_vec_fns_II.cpp:725-734) of the
-    // side's own tetrahedron
-    const double (*T)[3] = a_side ? A : B;
+    // getLocalCoordinatesForLinTet (src/mat_vec_fns_II.cpp:725-734)
     double phi[4];
     phi[0] = st_tet_volume(cm, T[1], T[2], T[3]);
     phi[1] = -st_tet_volume(cm, T[0], T[2], T[3]);
@@ -663,21 +668,12 @@ __device__ bool steric_pair(const double (*A)[3], const double (*B)[3], double d
     for (int i = 0; i < 4; i++) phi[i] /= tv;
     double g[3];
     for (int dir = 0; dir < 3; dir++) {
-        double S[4][3];
-        for (int i = 0; i < 4; i++)
-            for (int j = 0; j < 3; j++) S[i][j] = B[i][j] + (j == dir ? dr : 0.0);
-        const double vb = st_overlap(A, S, nullptr);
-        g[dir] = (vb - V) / dr;
-        for (int i = 0; i < 4; i++)
-            for (int j = 0; j < 3; j++) S[i][j] = A[i][j] + (j == dir ? dr : 0.0);
-        const double va = st_overlap(B, S, nullptr);
-        g[dir] -= (va - V) / dr;
+        g[dir] = (vb[dir] - V) / dr;
+        g[dir] -= (va[dir] - V) / dr;
+        g[dir] *= k;
     }
-    vol = V * k;
-    for (int d = 0; d < 3; d++) g[d] *= k;
     for (int i = 0; i < 4; i++)
         for (int d = 0; d < 3; d++) out[i][d] += a_side ? phi[i] * g[d] : -1.0 * phi[i] * g[d];
-    return true;
 }
 
 __constant__ int c_adj[27][3] = {{-1, -1, -1}, {-1, -1, 0}, {-1, -1, 1}, {-1, 0, -1}, {-1, 0, 0}, {-1, 0, 1},
@@ -735,13 +731,14 @@ __device__ __forceinline__ int warp_candidate(int k, const int *s_beg, const int
 // With periodic corrections, cs = blob_corr[blob of A][blob of G] enters the
 // separation (c_G - c_A - cs; FFEA's c2 - c1 - blob_corr[b1][b2] with its
 // faces in either order, blob_corr being antisymmetric).
+// A, G: face records of d_gp.
 __device__ __forceinline__ bool steric_type_ok(const double *A, const double *G, bool same_blob, int inc_self,
                                                const int *ni, const int *nj, const double *cs)
 {
     double sa = 0.0, sb = 0.0;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        double sep = (1.0 / 3.0) * (G[d] + G[3 + d] + G[6 + d]) - (1.0 / 3.0) * (A[d] + A[3 + d] + A[6 + d]);
+        double sep = G[13 + d] - A[13 + d];
         if (cs) sep -= cs[d];
         sa += sep * A[9 + d];
         sb += sep * G[9 + d];
@@ -770,33 +767,59 @@ __device__ __forceinline__ void face_tet(const double *__restrict__ geo, int f, 
     for (int d = 0; d < 3; d++) T[3][d] = g[13 + d];
 }
 
-constexpr int kStericWarps = 4;  // warps (faces) per CTA of k_steric
+// Whether face i (normal and blob in ni) admits face j: another face, another
+// blob unless self-interaction is on, and normals that do not agree,
+// n_i . n_j <= 0 in FP64.  The FP32 product is within 1e-6 of it and decides
+// all but the nearly perpendicular pairs, which take the FP64 records.
+__device__ __forceinline__ bool admits(int i, int j, float4 ni, const float4 *__restrict__ nb,
+                                       const double *__restrict__ gp, int inc_self)
+{
+    const float4 nj = nb[j];
+    if (j == i || (!inc_self && __float_as_int(ni.w) == __float_as_int(nj.w))) return false;
+    const float c = ni.x * nj.x + ni.y * nj.y + ni.z * nj.z;
+    if (fabsf(c) > 1e-6f) return c < 0.f;  // (a NaN goes on to the FP64 test)
+    const double *A = gp + 16 * (long long)i, *G = gp + 16 * (long long)j;
+    return !(A[9] * G[9] + A[10] * G[10] + A[11] * G[11] > 0.0);
+}
 
-// The steric part of the steric types, one warp per face i in cell order:
-// every partner j of the 27 cells that consider_interaction admits and whose
-// element tetrahedron's bounding box meets i's is queued; the queue is
-// evaluated a lane per pair, each pair as (lower index, higher index) = FFEA's
-// (f1, f2), so both sides compute the same overlap.  Face i's side of the
-// forces goes to fforce (12 values, written here: this kernel runs first), the
-// partners that overlapped to i's steric list (k_pairs skips them), the energy
+constexpr int kStericWarps = 4;  // warps per CTA (face) of k_steric
+
+// The steric part of the steric types, one CTA per face i in cell order: every
+// partner j of the 27 cells that consider_interaction admits and whose element
+// tetrahedron's bounding box meets i's is queued, warp w taking every
+// kStericWarps-th group of 32 candidates.  A pair needs seven overlap volumes
+// (its own and six with one tetrahedron moved, for the forward differences):
+// eight lanes take a pair, one volume each, so four pairs of a warp's queue go
+// at once.  The clipping is a long serial FP64 chain (64 issue slots an
+// instruction) with few pairs in contact, so its length decides: with a lane
+// per pair running the seven in turn, two 8 nm spheres in contact took 1.97
+// ms.  Each pair is computed as (lower index, higher index) = FFEA's (f1, f2),
+// so both sides compute the same overlap.  Face i's side of the forces goes
+// to fforce (12 values, written here: this kernel runs first), the partners
+// that overlapped to i's steric list (a set: k_pairs skips them), the energy
 // and the pair count from the side with the lower index.
 __global__ void __launch_bounds__(32 * kStericWarps) k_steric(
-    const double *__restrict__ geo, const int *__restrict__ sorted, const int *__restrict__ cell,
-    const int *__restrict__ start, const int *__restrict__ block, long long ncell, int nblocks, int nx, int ny,
-    int nz, const int *__restrict__ fblob, const int *__restrict__ corner, int num_blobs, int inc_self,
+    const double *__restrict__ geo, const double *__restrict__ gp, const float4 *__restrict__ nb,
+    const int *__restrict__ sorted, const int *__restrict__ cell, const int *__restrict__ start,
+    const int *__restrict__ block, long long ncell, int nblocks, int nx, int ny, int nz,
+    const int *__restrict__ fblob, const int *__restrict__ corner, int num_blobs, int inc_self,
     double steric_factor, double steric_dr, const double *__restrict__ corr, double *__restrict__ fforce,
     int *__restrict__ stlist, int *__restrict__ stcnt, double *__restrict__ energy, unsigned long long *stats)
 {
     __shared__ int s_pre[kStericWarps][28];
     __shared__ int s_beg[kStericWarps][27];
     __shared__ int s_q[kStericWarps][64];
+    __shared__ int s_listed;
+    __shared__ double s_out[kStericWarps][12];
     const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long w = (long long)blockIdx.x * kStericWarps + wi;
-    if (w >= block[nblocks]) return;  // warp-uniform
+    const long long w = blockIdx.x;
+    if (w >= block[nblocks]) return;  // CTA-uniform
     if (stats[3]) return;             // the call fails (a cell too full to sort)
     const int i = sorted[w];
+    if (threadIdx.x == 0) s_listed = 0;
+    __syncthreads();
     const int total = warp_cells(cell[i], nx, ny, nz, start, block, ncell, nblocks, lane, s_beg[wi], s_pre[wi]);
-    const double *A = geo + 16 * (long long)i;
+    const float4 nbi = nb[i];
     const int bi = fblob[i];
     int ni[4];
 #pragma unroll
@@ -814,48 +837,58 @@ __global__ void __launch_bounds__(32 * kStericWarps) k_steric(
     for (int u = 0; u < 4; u++)
 #pragma unroll
         for (int d = 0; d < 3; d++) out[u][d] = 0.0;
-    int listed = 0;
     unsigned long long npairs = 0;
-    auto evaluate = [&](bool have, int j) {
-        bool hit = false;
-        if (have) {
-            double Tj[4][3], vol;
-            face_tet(geo, j, Tj);
-            if (i < j) {
+    // the first n partners of the warp's queue
+    auto evaluate = [&](int n) {
+        const int g = lane & ~7, v = lane & 7;  // the pair's first lane, and the volume this lane takes
+        for (int q0 = 0; q0 < n; q0 += 4) {
+            const int q = q0 + (lane >> 3);
+            const int j = q < n ? s_q[wi][q] : -1;
+            const bool lower = i < j;
+            double A[4][3], B[4][3], cm[3] = {0.0, 0.0, 0.0}, vol = 0.0;
+            if (j >= 0 && v < 7) {
+                face_tet(geo, j, lower ? B : A);
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+#pragma unroll
+                    for (int d = 0; d < 3; d++) (lower ? A : B)[u][d] = Ti[u][d];
                 // periodic: f2's tetrahedron minus blob_corr[b1][b2]
                 // (Face::getTetraIntersectionVolumeTotalGradientAndShapeFunctions,
                 // src/Face.cpp:517-531)
                 if (corr) {
-                    const double *c = corr + 3 * ((long long)bi * num_blobs + fblob[j]);
-#pragma unroll
+                    const int b1 = lower ? bi : fblob[j], b2 = lower ? fblob[j] : bi;
+                    const double *c = corr + 3 * ((long long)b1 * num_blobs + b2);
                     for (int u = 0; u < 4; u++)
-#pragma unroll
-                        for (int d = 0; d < 3; d++) Tj[u][d] -= c[d];
+                        for (int d = 0; d < 3; d++) B[u][d] -= c[d];
                 }
-                hit = steric_pair(Ti, Tj, steric_dr, steric_factor, true, out, vol);
-            } else {
-                double Tb[4][3];
-                const double *c = corr ? corr + 3 * ((long long)fblob[j] * num_blobs + bi) : nullptr;
-#pragma unroll
+                // lane 0: A and B; 1..3: B moved; 4..6: A moved, clipped out of B
+                const bool swap = v > 3;
+                double M[4][3];
                 for (int u = 0; u < 4; u++)
+                    for (int d = 0; d < 3; d++)
+                        M[u][d] = (swap ? A : B)[u][d] + (v > 0 && d == (v - 1) % 3 ? steric_dr : 0.0);
+                vol = st_overlap(swap ? B : A, M, v == 0 ? cm : nullptr);
+            }
+            double va[3], vb[3];
 #pragma unroll
-                    for (int d = 0; d < 3; d++) Tb[u][d] = c ? Ti[u][d] - c[d] : Ti[u][d];
-                hit = steric_pair(Tj, Tb, steric_dr, steric_factor, false, out, vol);
+            for (int d = 0; d < 3; d++) {
+                vb[d] = __shfl_sync(0xffffffffu, vol, g + 1 + d);
+                va[d] = __shfl_sync(0xffffffffu, vol, g + 4 + d);
             }
-            if (hit && i < j) {
-                atomicAdd(&energy[bi * num_blobs + fblob[j]], vol);
-                npairs++;
+            if (j >= 0 && v == 0 && vol != 0) {
+                steric_forces(lower ? A : B, vol, cm, vb, va, steric_dr, steric_factor, lower, out);
+                const int slot = atomicAdd(&s_listed, 1);
+                if (slot < FFEA_GPU_SSINT_MAX_STERIC_PARTNERS)
+                    stlist[FFEA_GPU_SSINT_MAX_STERIC_PARTNERS * i + slot] = j;
+                if (lower) {
+                    atomicAdd(&energy[bi * num_blobs + fblob[j]], vol * steric_factor);
+                    npairs++;
+                }
             }
         }
-        const unsigned m = __ballot_sync(0xffffffffu, hit);
-        if (hit) {
-            const int slot = listed + __popc(m & ((1u << lane) - 1u));
-            if (slot < FFEA_GPU_SSINT_MAX_STERIC_PARTNERS) stlist[FFEA_GPU_SSINT_MAX_STERIC_PARTNERS * i + slot] = j;
-        }
-        listed += __popc(m);
     };
     int qn = 0;  // warp-uniform queue length, < 64
-    for (int base = 0; base < total; base += 32) {
+    for (int base = 32 * wi; base < total; base += 32 * kStericWarps) {
         const int k = base + lane;
         bool ok = false;
         int j = -1;
@@ -863,7 +896,7 @@ __global__ void __launch_bounds__(32 * kStericWarps) k_steric(
             j = warp_candidate(k, s_beg[wi], s_pre[wi], sorted);
             const double *G = geo + 16 * (long long)j;
             const bool same = bi == fblob[j];
-            ok = j != i && (inc_self || !same) && !(A[9] * G[9] + A[10] * G[10] + A[11] * G[11] > 0.0);
+            ok = admits(i, j, nbi, nb, gp, inc_self);
             // periodic: the partner as seen from face i, shifted by
             // -blob_corr[bi][bj]
             const double *cs = corr ? corr + 3 * ((long long)bi * num_blobs + fblob[j]) : nullptr;
@@ -871,7 +904,7 @@ __global__ void __launch_bounds__(32 * kStericWarps) k_steric(
                 int nj[4];
 #pragma unroll
                 for (int u = 0; u < 4; u++) nj[u] = corner[4 * j + u];
-                ok = steric_type_ok(A, G, same, inc_self, ni, nj, cs);
+                ok = steric_type_ok(gp + 16 * (long long)i, gp + 16 * (long long)j, same, inc_self, ni, nj, cs);
             }
             if (ok) {  // bounding boxes of the two tetrahedra
 #pragma unroll
@@ -888,7 +921,7 @@ __global__ void __launch_bounds__(32 * kStericWarps) k_steric(
         qn += __popc(m);
         __syncwarp();
         if (qn >= 32) {
-            evaluate(true, s_q[wi][lane]);
+            evaluate(32);
             const int rest = qn - 32;
             const int moved = lane < rest ? s_q[wi][32 + lane] : 0;
             __syncwarp();
@@ -897,22 +930,30 @@ __global__ void __launch_bounds__(32 * kStericWarps) k_steric(
             __syncwarp();
         }
     }
-    if (qn > 0) evaluate(lane < qn, lane < qn ? s_q[wi][lane] : -1);
+    evaluate(qn);
 #pragma unroll
     for (int u = 0; u < 4; u++)
 #pragma unroll
-        for (int d = 0; d < 3; d++) out[u][d] = warp_sum_d(out[u][d]);
+        for (int d = 0; d < 3; d++) {
+            // (only lanes 0, 8, 16 and 24 hold a sum)
+            double t = out[u][d];
+            t += __shfl_xor_sync(0xffffffffu, t, 16);
+            t += __shfl_xor_sync(0xffffffffu, t, 8);
+            if (lane == 0) s_out[wi][3 * u + d] = t;
+        }
     unsigned long long np = npairs;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) np += __shfl_xor_sync(0xffffffffu, np, o);
-    if (lane == 0) {
-        if (np) atomicAdd(&stats[0], np);
-        stcnt[i] = min(listed, FFEA_GPU_SSINT_MAX_STERIC_PARTNERS);
-        if (listed > FFEA_GPU_SSINT_MAX_STERIC_PARTNERS) atomicAdd(&stats[4], 1ull);
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-#pragma unroll
-            for (int d = 0; d < 3; d++) fforce[12 * (long long)i + 3 * u + d] = out[u][d];
+    if (lane == 0 && np) atomicAdd(&stats[0], np);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        stcnt[i] = min(s_listed, FFEA_GPU_SSINT_MAX_STERIC_PARTNERS);
+        if (s_listed > FFEA_GPU_SSINT_MAX_STERIC_PARTNERS) atomicAdd(&stats[4], 1ull);
+    }
+    if (threadIdx.x < 12) {
+        double t = 0.0;
+        for (int k = 0; k < kStericWarps; k++) t += s_out[k][threadIdx.x];
+        fforce[12 * (long long)i + threadIdx.x] = t;
     }
 }
 
@@ -926,9 +967,10 @@ __global__ void __launch_bounds__(32 * kStericWarps) k_steric(
 // forces add to what k_steric wrote.
 template <int POT, bool STERIC>
 __global__ void __launch_bounds__(32 * kPairWarps) k_pairs(
-    const double *__restrict__ geo, const int *__restrict__ cell, const int *__restrict__ sorted,
-    const int *__restrict__ start, const int *__restrict__ block, long long ncell, int nblocks, int nx, int ny,
-    int nz, const int *__restrict__ fblob, const int *__restrict__ ftype, const double *__restrict__ emin,
+    const double *__restrict__ gp, const float4 *__restrict__ nb, const int *__restrict__ cell,
+    const int *__restrict__ sorted, const int *__restrict__ start, const int *__restrict__ block, long long ncell,
+    int nblocks, int nx, int ny, int nz, const int *__restrict__ fblob, const int *__restrict__ ftype,
+    const double *__restrict__ emin,
     const double *__restrict__ rmin, const double *__restrict__ k0, const int *__restrict__ corner,
     const int *__restrict__ stlist, const int *__restrict__ stcnt, int num_types, int num_blobs, int inc_self,
     const double *__restrict__ corr, double *__restrict__ fforce, double *__restrict__ energy,
@@ -953,35 +995,46 @@ __global__ void __launch_bounds__(32 * kPairWarps) k_pairs(
         for (int u = 0; u < 4; u++) ni[u] = corner[4 * i + u];
         __syncwarp();
     }
-    double A[13];
+    const double *A = gp + 16 * (long long)i;
+    const float4 nbi = nb[i];
+    double own[9];
 #pragma unroll
-    for (int k = 0; k < 13; k++) A[k] = geo[16 * (long long)i + k];
+    for (int k = 0; k < 9; k++) own[k] = A[k];
+    const double area = A[12];
     const int bi = fblob[i], ti = ftype[i];
-    double out[4][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    double S[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};  // the lane's sum of area products * column sums
     double e_acc = 0.0;
     int e_key = -1;
     unsigned long long npairs = 0;
     // one partner j: face i's side of the pair, FFEA's f1 being the lower index
     auto pair = [&](int j) {
-        const double *G = geo + 16 * (long long)j;
-        double B[13];
+        const double2 *G = reinterpret_cast<const double2 *>(gp + 16 * (long long)j);
+        double oth[10];
 #pragma unroll
-        for (int q = 0; q < 13; q++) B[q] = G[q];
-        if (i < j) {
-            const int tt = ti * num_types + ftype[j];
-            double en;
-            if (corr) {
-                // periodic: f1's corners minus blob_corr[b2][b1]
-                // (Face::barycentric_calc_point_f2, src/Face.cpp:271-277)
-                const double *c = corr + 3 * ((long long)fblob[j] * num_blobs + bi);
-                double As[13];
+        for (int q = 0; q < 5; q++) {
+            const double2 g2 = __ldg(G + q);
+            oth[2 * q] = g2.x;
+            oth[2 * q + 1] = g2.y;
+        }
+        const double apaq = area * __ldg(gp + 16 * (long long)j + 12);
+        const int bj = fblob[j];
+        double q[9];
 #pragma unroll
-                for (int q = 0; q < 13; q++) As[q] = q < 9 ? A[q] - c[q % 3] : A[q];
-                en = pot_pair<POT, true>(As, B, emin[tt], rmin[tt], k0 ? k0[tt] : 0.0, out);
-            } else {
-                en = pot_pair<POT, true>(A, B, emin[tt], rmin[tt], k0 ? k0[tt] : 0.0, out);
-            }
-            const int key = bi * num_blobs + fblob[j];
+        for (int c = 0; c < 9; c++) q[c] = oth[c];
+        if (corr) {
+            // periodic: f1's points minus blob_corr[b2][b1]
+            // (Face::barycentric_calc_point_f2, src/Face.cpp:271-277), the
+            // same as the partner's minus blob_corr[bi][bj] on either side
+            // (blob_corr is antisymmetric)
+            const double *c = corr + 3 * ((long long)bi * num_blobs + bj);
+#pragma unroll
+            for (int k = 0; k < 9; k++) q[k] -= c[k % 3];
+        }
+        const bool lower = i < j;
+        const int tt = lower ? ti * num_types + ftype[j] : ftype[j] * num_types + ti;
+        const double en = pot_pair<POT>(own, q, apaq, lower, emin[tt], rmin[tt], k0 ? k0[tt] : 0.0, S);
+        if (lower) {
+            const int key = bi * num_blobs + bj;
             if (key != e_key) {
                 if (e_key >= 0) atomicAdd(&energy[e_key], e_acc);
                 e_key = key;
@@ -989,14 +1042,6 @@ __global__ void __launch_bounds__(32 * kPairWarps) k_pairs(
             }
             e_acc += en;
             npairs++;
-        } else {
-            const int tt = ftype[j] * num_types + ti;
-            if (corr) {
-                const double *c = corr + 3 * ((long long)bi * num_blobs + fblob[j]);
-#pragma unroll
-                for (int q = 0; q < 9; q++) B[q] -= c[q % 3];
-            }
-            pot_pair<POT, false>(B, A, emin[tt], rmin[tt], k0 ? k0[tt] : 0.0, out);
         }
     };
     // The cheap tests (same face, same blob, normals facing the same way) run
@@ -1010,14 +1055,13 @@ __global__ void __launch_bounds__(32 * kPairWarps) k_pairs(
         int j = -1;
         if (k < total) {
             j = warp_candidate(k, s_beg[wi], s_pre[wi], sorted);
-            const double *G = geo + 16 * (long long)j;
-            ok = j != i && (inc_self || bi != fblob[j]) && !(A[9] * G[9] + A[10] * G[10] + A[11] * G[11] > 0.0);
+            ok = admits(i, j, nbi, nb, gp, inc_self);
             if constexpr (STERIC) {
                 if (ok) {
                     int nj[4];
 #pragma unroll
                     for (int u = 0; u < 4; u++) nj[u] = corner[4 * j + u];
-                    ok = steric_type_ok(A, G, bi == fblob[j], inc_self, ni, nj,
+                    ok = steric_type_ok(A, gp + 16 * (long long)j, bi == fblob[j], inc_self, ni, nj,
                                         corr ? corr + 3 * ((long long)bi * num_blobs + fblob[j]) : nullptr);
                 }
                 for (int t = 0; ok && t < nst; t++)
@@ -1048,22 +1092,27 @@ __global__ void __launch_bounds__(32 * kPairWarps) k_pairs(
         if (lane == 0) atomicAdd(&energy[lk], part);
         if (e_key == lk) e_key = -1;
     }
+    // the lanes' sums, then the corner weights: lane 3 j + d < 9 writes force
+    // component d of corner j (the fourth node has none from these)
 #pragma unroll
     for (int k = 0; k < 3; k++)
 #pragma unroll
-        for (int d = 0; d < 3; d++) out[k][d] = warp_sum_d(out[k][d]);
+        for (int d = 0; d < 3; d++) S[k][d] = warp_sum_d(S[k][d]);
     unsigned long long np = npairs;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) np += __shfl_xor_sync(0xffffffffu, np, o);
-    if (lane == 0) {
-        if (np) atomicAdd(&stats[0], np);
+    if (lane == 0 && np) atomicAdd(&stats[0], np);
+    if (lane < 12) {
+        const int c = lane / 3, d = lane % 3;
+        double f = 0.0;
+        if (c < 3)
 #pragma unroll
-        for (int k = 0; k < 4; k++)
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-                double *f = &fforce[12 * (long long)i + 3 * k + d];
-                *f = STERIC ? *f + out[k][d] : out[k][d];
+            for (int l = 0; l < 3; l++) {
+                const double sl = d == 0 ? S[l][0] : d == 1 ? S[l][1] : S[l][2];
+                f = fma(kW * kW * (l == c ? eta(0, 0) : eta(0, 1)), sl, f);
             }
+        double *o = &fforce[12 * (long long)i + lane];
+        *o = STERIC ? *o + f : f;
     }
 }
 
@@ -1204,7 +1253,7 @@ extern "C" int ffea_gpu_ssint_create(const ffea_gpu_ssint_desc *d, ffea_gpu_ssin
         // cudaMemcpy returns
         SSINT_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamDefault));
         if (dalloc(&s->d_corner, 4 * (size_t)na) || dalloc(&s->d_blob, na) || dalloc(&s->d_type, na) ||
-            dalloc(&s->d_geo, 16 * (size_t)na) || dalloc(&s->d_cell, na) || dalloc(&s->d_fforce, 12 * (size_t)na) ||
+            dalloc(&s->d_geo, 16 * (size_t)na) || dalloc(&s->d_gp, 16 * (size_t)na) || dalloc(&s->d_nb, na) || dalloc(&s->d_cell, na) || dalloc(&s->d_fforce, 12 * (size_t)na) ||
             dalloc(&s->d_count, ncell) || dalloc(&s->d_start, ncell) || dalloc(&s->d_block, s->nblocks + 1) ||
             dalloc(&s->d_sorted, na) || dalloc(&s->d_node_ptr, d->num_nodes + 1) ||
             dalloc(&s->d_node_ent, ent.size()) || dalloc(&s->d_emin, T2) || dalloc(&s->d_rmin, T2) ||
@@ -1242,7 +1291,7 @@ extern "C" void ffea_gpu_ssint_destroy(ffea_gpu_ssint_t *s)
 {
     if (!s) return;
     if (s->stream) cudaStreamSynchronize(s->stream);
-    void *bufs[] = {s->d_corner, s->d_blob, s->d_type, s->d_geo, s->d_cell, s->d_fforce, s->d_count,
+    void *bufs[] = {s->d_corner, s->d_blob, s->d_type, s->d_geo, s->d_gp, s->d_nb, s->d_cell, s->d_fforce, s->d_count,
                     s->d_start, s->d_block, s->d_sorted, s->d_node_ptr, s->d_node_ent, s->d_emin, s->d_rmin,
                     s->d_pos, s->d_force, s->d_energy, s->d_stats, s->d_large, s->d_stlist, s->d_stcnt, s->d_k0,
                     s->d_corr};
@@ -1267,8 +1316,8 @@ extern "C" int ffea_gpu_ssint_forces_device(ffea_gpu_ssint_t *s, const double *p
     }
     SSINT_CUDA(cudaMemsetAsync(s->d_count, 0, sizeof(int) * s->ncell, st));
     const int fb = (na + 127) / 128;
-    k_face_geom<<<fb, 128, 0, st>>>(pos, s->d_corner, na, s->h, s->nx, s->ny, s->nz, s->d_geo, s->d_cell,
-                                    s->d_count, s->d_stats);
+    k_face_geom<<<fb, 128, 0, st>>>(pos, s->d_corner, na, s->h, s->nx, s->ny, s->nz, s->d_blob, s->d_geo,
+                                    s->d_gp, s->d_nb, s->d_cell, s->d_count, s->d_stats);
     k_scan_local<<<s->nblocks, kScanBlock, 0, st>>>(s->d_count, s->ncell, s->d_start, s->d_block);
     k_scan_blocks<<<1, kScanBlock, 0, st>>>(s->d_block, s->nblocks);
     k_scatter<<<fb, 128, 0, st>>>(s->d_cell, na, s->d_start, s->d_block, s->d_count, s->d_sorted);
@@ -1280,13 +1329,13 @@ extern "C" int ffea_gpu_ssint_forces_device(ffea_gpu_ssint_t *s, const double *p
                                                  s->d_large, s->d_stats);
     const int pw = (na + kPairWarps - 1) / kPairWarps;
     if (s->type != FFEA_GPU_SSINT_LJ)
-        k_steric<<<(na + kStericWarps - 1) / kStericWarps, 32 * kStericWarps, 0, st>>>(
-            s->d_geo, s->d_sorted, s->d_cell, s->d_start, s->d_block, s->ncell, s->nblocks, s->nx, s->ny, s->nz,
+        k_steric<<<na, 32 * kStericWarps, 0, st>>>(
+            s->d_geo, s->d_gp, s->d_nb, s->d_sorted, s->d_cell, s->d_start, s->d_block, s->ncell, s->nblocks, s->nx, s->ny, s->nz,
             s->d_blob, s->d_corner, s->num_blobs, s->inc_self, s->steric_factor, s->steric_dr,
             s->has_corr ? s->d_corr : nullptr, s->d_fforce, s->d_stlist, s->d_stcnt, energy, s->d_stats);
 #define SSINT_PAIRS(POT, STERIC)                                                                                   \
     k_pairs<POT, STERIC><<<pw, 32 * kPairWarps, 0, st>>>(                                                           \
-        s->d_geo, s->d_cell, s->d_sorted, s->d_start, s->d_block, s->ncell, s->nblocks, s->nx, s->ny, s->nz,        \
+        s->d_gp, s->d_nb, s->d_cell, s->d_sorted, s->d_start, s->d_block, s->ncell, s->nblocks, s->nx, s->ny, s->nz, \
         s->d_blob, s->d_type, s->d_emin, s->d_rmin, s->d_k0, s->d_corner, s->d_stlist, s->d_stcnt, s->num_types,     \
         s->num_blobs, s->inc_self, s->has_corr ? s->d_corr : nullptr, s->d_fforce, energy, s->d_stats)
     if (s->type == FFEA_GPU_SSINT_LJ) SSINT_PAIRS(POT_LJ, false);
