@@ -91,7 +91,8 @@ struct ffea_gpu_ssint {
     int *d_count = nullptr;     // ncell
     int *d_start = nullptr;     // ncell, block-local exclusive prefix
     int *d_block = nullptr;     // nblocks, global prefix of each block
-    int *d_sorted = nullptr;    // num_active faces in cell order
+    int *d_binned = nullptr;    // num_active faces by cell, in no order within a cell
+    int *d_sorted = nullptr;    // num_active faces in cell order, each cell in face order
     // nodes
     int *d_node_ptr = nullptr;  // num_nodes + 1
     int *d_node_ent = nullptr;  // face * 4 + corner (3: the fourth node), face order
@@ -289,41 +290,39 @@ __global__ void k_scatter(const int *__restrict__ cell, int nf, const int *__res
     sorted[slot] = f;
 }
 
-// Each cell's faces sorted by face index.  A cell of at most kSortSmall
-// faces is insertion-sorted by its thread; a larger one, up to kSortMax
-// faces, is listed for k_sort_large (one CTA per cell); a cell above that is
-// counted in stats[3] and makes the call an error, so that a grid far too
-// coarse for the mesh fails at once instead of one thread sorting many
-// thousands of faces.
+// Each cell's faces sorted by face index: a thread per face counts the faces
+// of its cell with a lower index, which is its place (cells of at most
+// kSortSmall faces; a thread per cell sorting by insertion took 43-54 us where
+// this takes a few).  A larger cell, up to kSortMax faces, is copied and listed
+// for k_sort_large (one CTA per cell); a cell above that is counted in stats[3]
+// and makes the call an error, so that a grid far too coarse for the mesh
+// fails at once.
 constexpr int kSortSmall = 64;
 constexpr int kSortMax = 4096;
 constexpr int kSortLargeCtas = 256;
 
 __global__ void k_sort_cells(long long ncell, int nblocks, const int *__restrict__ start,
-                             const int *__restrict__ block, int *__restrict__ sorted, int *__restrict__ large,
+                             const int *__restrict__ block, const int *__restrict__ cell,
+                             const int *__restrict__ binned, int *__restrict__ sorted, int *__restrict__ large,
                              unsigned long long *stats)
 {
-    long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncell) return;
+    const int w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w >= block[nblocks]) return;
+    const int f = binned[w];
+    const long long c = cell[f];
     const int b = cell_begin(start, block, c);
     const int e = cell_end(start, block, c, ncell, nblocks);
-    if (e - b > kSortMax) {
-        atomicAdd(&stats[3], 1ull);
-        return;
-    }
     if (e - b > kSortSmall) {
-        large[atomicAdd(&stats[2], 1ull)] = (int)c;
+        sorted[w] = f;
+        if (w == b) {  // once per cell
+            if (e - b > kSortMax) atomicAdd(&stats[3], 1ull);
+            else large[atomicAdd(&stats[2], 1ull)] = (int)c;
+        }
         return;
     }
-    for (int i = b + 1; i < e; i++) {
-        const int v = sorted[i];
-        int j = i - 1;
-        while (j >= b && sorted[j] > v) {
-            sorted[j + 1] = sorted[j];
-            j--;
-        }
-        sorted[j + 1] = v;
-    }
+    int place = b;
+    for (int k = b; k < e; k++) place += binned[k] < f;
+    sorted[place] = f;
 }
 
 // The listed large cells, one CTA each (grid-stride over the list): a
@@ -468,58 +467,87 @@ __device__ __forceinline__ double st_tet_volume(const double *a, const double *b
     return (u0 * x0 + u1 * x1 + u2 * x2) / 6.0;
 }
 
-__device__ __forceinline__ void st_add_unique(double (*pts)[3], int &n, int cap, const double *x, double tol2)
+// x joins the n distinct points pts unless one is within sqrt(tol2) of it.
+// org and far decide most comparisons in FP32: points whose FP32 offsets from
+// org differ by more than far in a component are distinct (far is 1e-5 of the
+// extent, a hundred FP32 roundings of an offset; the tolerance is 1e-9 of it).
+__device__ __forceinline__ void st_add_unique(double (*pts)[3], float (*off)[3], int &n, int cap, const double *x,
+                                              const double *org, float far, double tol2)
 {
+    const float f[3] = {(float)(x[0] - org[0]), (float)(x[1] - org[1]), (float)(x[2] - org[2])};
     for (int u = 0; u < n; u++) {
+        const float g = fmaxf(fmaxf(fabsf(f[0] - off[u][0]), fabsf(f[1] - off[u][1])), fabsf(f[2] - off[u][2]));
+        if (g > far) continue;
         const double e0 = x[0] - pts[u][0], e1 = x[1] - pts[u][1], e2 = x[2] - pts[u][2];
         if (e0 * e0 + e1 * e1 + e2 * e2 <= tol2) return;
     }
     if (n < cap) {
-        pts[n][0] = x[0];
-        pts[n][1] = x[1];
-        pts[n][2] = x[2];
+        for (int c = 0; c < 3; c++) {
+            pts[n][c] = x[c];
+            off[n][c] = f[c];
+        }
         n++;
     }
 }
 
+// the sign of a double from its bits (-1, 0, 1), off the FP64 pipe
+__device__ __forceinline__ int st_sign(double x)
+{
+    const int hi = __double2hiint(x);
+    return ((hi & 0x7fffffff) | __double2loint(x)) == 0 ? 0 : hi < 0 ? -1 : 1;
+}
+
+// increasing with atan2(y, x) over (-pi, pi], without its cost
+__device__ __forceinline__ double st_angle(double y, double x)
+{
+    const double t = y / (fabs(x) + fabs(y));
+    return __double2hiint(x) >= 0 ? t : copysign(2.0, y) - t;
+}
+
 __constant__ int c_tri[4][3] = {{1, 2, 3}, {0, 2, 3}, {0, 1, 3}, {0, 1, 2}};
 
-// clip P by n . x <= off; false when nothing is left
-__device__ bool st_clip(StPolyh &P, const double *nrm, double off, double tol2)
+// clip P by n . x <= off; false when nothing is left.  A vertex's distance is
+// formed once and kept, and its sign read from its bits: comparisons run on
+// the FP64 pipe too.
+__device__ bool st_clip(StPolyh &P, const double *nrm, double off, const double *org, float far, double tol2)
 {
-    double smin = 0.0, smax = 0.0;
-    bool first = true;
+    double sd[kStF][kStV];
+    bool neg = false, pos = false;
     for (int f = 0; f < P.nf; f++)
         for (int k = 0; k < P.n[f]; k++) {
             const double sv = st_dot(nrm, P.v[f][k]) - off;
-            if (first || sv < smin) smin = sv;
-            if (first || sv > smax) smax = sv;
-            first = false;
+            const int g = st_sign(sv);
+            sd[f][k] = sv;
+            neg |= g < 0;
+            pos |= g > 0;
         }
-    if (first || smin >= 0) {
+    if (!neg) {
         P.nf = 0;
         return false;
     }
-    if (smax <= 0) return true;
+    if (!pos) return true;
     double cap[kStC][3];
+    float capf[kStC][3];
     int nc = 0, nf = 0;
     for (int f = 0; f < P.nf; f++) {
         double out[kStV][3];
         int no = 0;
         const int m = P.n[f];
         for (int k = 0; k < m; k++) {
-            const double *a = P.v[f][k], *b = P.v[f][k + 1 < m ? k + 1 : 0];
-            const double sa = st_dot(nrm, a) - off, sb = st_dot(nrm, b) - off;
-            if (sa <= 0) {
+            const int kn = k + 1 < m ? k + 1 : 0;
+            const double *a = P.v[f][k], *b = P.v[f][kn];
+            const double sa = sd[f][k], sb = sd[f][kn];
+            const int ga = st_sign(sa), gb = st_sign(sb);
+            if (ga <= 0) {
                 if (no < kStV) {
                     out[no][0] = a[0];
                     out[no][1] = a[1];
                     out[no][2] = a[2];
                     no++;
                 }
-                if (sa == 0) st_add_unique(cap, nc, kStC, a, tol2);
+                if (ga == 0) st_add_unique(cap, capf, nc, kStC, a, org, far, tol2);
             }
-            if ((sa < 0 && sb > 0) || (sa > 0 && sb < 0)) {
+            if (ga * gb < 0) {
                 const double t = sa / (sa - sb);
                 double x[3];
                 for (int c = 0; c < 3; c++) x[c] = a[c] + t * (b[c] - a[c]);
@@ -529,7 +557,7 @@ __device__ bool st_clip(StPolyh &P, const double *nrm, double off, double tol2)
                     out[no][2] = x[2];
                     no++;
                 }
-                st_add_unique(cap, nc, kStC, x, tol2);
+                st_add_unique(cap, capf, nc, kStC, x, org, far, tol2);
             }
         }
         if (no >= 3) {
@@ -562,7 +590,7 @@ __device__ bool st_clip(StPolyh &P, const double *nrm, double off, double tol2)
             double ang[kStC];
             for (int k = 0; k < nc; k++) {
                 const double e[3] = {cap[k][0] - ctr[0], cap[k][1] - ctr[1], cap[k][2] - ctr[2]};
-                ang[k] = atan2(st_dot(e, w), st_dot(e, u));
+                ang[k] = st_angle(st_dot(e, w), st_dot(e, u));
             }
             for (int i = 1; i < nc; i++) {  // insertion sort by angle
                 const double a = ang[i], v0 = cap[i][0], v1 = cap[i][1], v2 = cap[i][2];
@@ -598,6 +626,8 @@ __device__ double st_overlap(const double (*A)[3], const double (*B)[3], double 
             ext = fmax(ext, fabs(B[i][d] - A[0][d]));
         }
     const double tol2 = (1e-9 * ext) * (1e-9 * ext);
+    const double *org = A[0];
+    const float far = 1e-5f * (float)ext;
     StPolyh P;
     P.nf = 4;
     for (int f = 0; f < 4; f++) {
@@ -618,7 +648,7 @@ __device__ double st_overlap(const double (*A)[3], const double (*B)[3], double 
             nrm[2] = -nrm[2];
             off = -off;
         }
-        if (!st_clip(P, nrm, off, tol2)) {
+        if (!st_clip(P, nrm, off, org, far, tol2)) {
             if (cm) cm[0] = cm[1] = cm[2] = 0.0;
             return 0.0;
         }
@@ -631,14 +661,29 @@ __device__ double st_overlap(const double (*A)[3], const double (*B)[3], double 
             nv++;
         }
     for (int d = 0; d < 3; d++) o[d] /= nv;
-    double vol = 0.0;
-    for (int f = 0; f < P.nf; f++)
-        for (int k = 1; k + 1 < P.n[f]; k++) vol += fabs(st_tet_volume(o, P.v[f][0], P.v[f][k], P.v[f][k + 1]));
+    // six times the volume: a fan of tetrahedra per face, with the vertices'
+    // offsets from o
+    double vol6 = 0.0;
+    for (int f = 0; f < P.nf; f++) {
+        double u[3], v[3], w[3];
+        for (int d = 0; d < 3; d++) {
+            u[d] = P.v[f][0][d] - o[d];
+            v[d] = P.v[f][1][d] - o[d];
+        }
+        for (int k = 2; k < P.n[f]; k++) {
+            for (int d = 0; d < 3; d++) w[d] = P.v[f][k][d] - o[d];
+            vol6 += fabs(u[0] * (v[1] * w[2] - v[2] * w[1]) + u[1] * (v[2] * w[0] - v[0] * w[2]) +
+                         u[2] * (v[0] * w[1] - v[1] * w[0]));
+            for (int d = 0; d < 3; d++) v[d] = w[d];
+        }
+    }
+    const double vol = vol6 / 6.0;
     if (cm) {
         double uniq[kStU][3];
+        float uniqf[kStU][3];
         int nu = 0;
         for (int f = 0; f < P.nf; f++)
-            for (int k = 0; k < P.n[f]; k++) st_add_unique(uniq, nu, kStU, P.v[f][k], tol2);
+            for (int k = 0; k < P.n[f]; k++) st_add_unique(uniq, uniqf, nu, kStU, P.v[f][k], org, far, tol2);
         cm[0] = cm[1] = cm[2] = 0.0;
         for (int u = 0; u < nu; u++)
             for (int d = 0; d < 3; d++) cm[d] += uniq[u][d];
@@ -682,7 +727,9 @@ __constant__ int c_adj[27][3] = {{-1, -1, -1}, {-1, -1, 0}, {-1, -1, 1}, {-1, 0,
                                  {1, -1, -1},  {1, -1, 0},  {1, -1, 1},  {1, 0, -1},  {1, 0, 0},  {1, 0, 1},
                                  {1, 1, -1},   {1, 1, 0},   {1, 1, 1}};
 
-constexpr int kPairWarps = 8;  // warps (faces) per CTA of k_pairs
+// warps (faces) per CTA of k_pairs, and CTAs per SM (128 registers a thread):
+// sixteen warps keep the FP64 pipes busy while others test candidates
+constexpr int kPairWarps = 4, kPairCtas = 4;
 
 __device__ __forceinline__ double warp_sum_d(double v)
 {
@@ -782,23 +829,22 @@ __device__ __forceinline__ bool admits(int i, int j, float4 ni, const float4 *__
     return !(A[9] * G[9] + A[10] * G[10] + A[11] * G[11] > 0.0);
 }
 
-constexpr int kStericWarps = 4;  // warps per CTA (face) of k_steric
+constexpr int kStericWarps = 8;  // warps per CTA (face) of k_steric
 
 // The steric part of the steric types, one CTA per face i in cell order: every
 // partner j of the 27 cells that consider_interaction admits and whose element
-// tetrahedron's bounding box meets i's is queued, warp w taking every
-// kStericWarps-th group of 32 candidates.  A pair needs seven overlap volumes
-// (its own and six with one tetrahedron moved, for the forward differences):
-// eight lanes take a pair, one volume each, so four pairs of a warp's queue go
-// at once.  The clipping is a long serial FP64 chain (64 issue slots an
-// instruction) with few pairs in contact, so its length decides: with a lane
-// per pair running the seven in turn, two 8 nm spheres in contact took 1.97
-// ms.  Each pair is computed as (lower index, higher index) = FFEA's (f1, f2),
+// tetrahedron's bounding box meets i's is queued in candidate order.  A pair
+// needs seven overlap volumes (its own and six with one tetrahedron moved, for
+// the forward differences): eight lanes take a pair, one volume each, and the
+// queue is dealt over the warps.  The clipping is a long serial FP64 chain (64
+// issue slots an instruction) with few pairs in contact, so its length and
+// the lanes that diverge in it decide: with a lane per pair running the seven
+// in turn, two 8 nm spheres in contact took 1.97 ms.  Each pair is computed as (lower index, higher index) = FFEA's (f1, f2),
 // so both sides compute the same overlap.  Face i's side of the forces goes
 // to fforce (12 values, written here: this kernel runs first), the partners
 // that overlapped to i's steric list (a set: k_pairs skips them), the energy
 // and the pair count from the side with the lower index.
-__global__ void __launch_bounds__(32 * kStericWarps) k_steric(
+__global__ void __launch_bounds__(32 * kStericWarps, 1) k_steric(
     const double *__restrict__ geo, const double *__restrict__ gp, const float4 *__restrict__ nb,
     const int *__restrict__ sorted, const int *__restrict__ cell, const int *__restrict__ start,
     const int *__restrict__ block, long long ncell, int nblocks, int nx, int ny, int nz,
@@ -808,7 +854,8 @@ __global__ void __launch_bounds__(32 * kStericWarps) k_steric(
 {
     __shared__ int s_pre[kStericWarps][28];
     __shared__ int s_beg[kStericWarps][27];
-    __shared__ int s_q[kStericWarps][64];
+    __shared__ int s_q[64 * kStericWarps];
+    __shared__ int s_cnt[kStericWarps];
     __shared__ int s_listed;
     __shared__ double s_out[kStericWarps][12];
     const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -838,12 +885,13 @@ __global__ void __launch_bounds__(32 * kStericWarps) k_steric(
 #pragma unroll
         for (int d = 0; d < 3; d++) out[u][d] = 0.0;
     unsigned long long npairs = 0;
-    // the first n partners of the warp's queue
+    // the first n partners of the queue, dealt over the warps first and over
+    // a warp's four groups of lanes then
     auto evaluate = [&](int n) {
         const int g = lane & ~7, v = lane & 7;  // the pair's first lane, and the volume this lane takes
-        for (int q0 = 0; q0 < n; q0 += 4) {
-            const int q = q0 + (lane >> 3);
-            const int j = q < n ? s_q[wi][q] : -1;
+        for (int q0 = wi; q0 < n; q0 += 4 * kStericWarps) {
+            const int q = q0 + kStericWarps * (lane >> 3);
+            const int j = q < n ? s_q[q] : -1;
             const bool lower = i < j;
             double A[4][3], B[4][3], cm[3] = {0.0, 0.0, 0.0}, vol = 0.0;
             if (j >= 0 && v < 7) {
@@ -887,9 +935,9 @@ __global__ void __launch_bounds__(32 * kStericWarps) k_steric(
             }
         }
     };
-    int qn = 0;  // warp-uniform queue length, < 64
-    for (int base = 32 * wi; base < total; base += 32 * kStericWarps) {
-        const int k = base + lane;
+    int qn = 0;  // CTA-uniform queue length
+    for (int base = 0; base < total; base += 32 * kStericWarps) {
+        const int k = base + threadIdx.x;
         bool ok = false;
         int j = -1;
         if (k < total) {
@@ -917,20 +965,21 @@ __global__ void __launch_bounds__(32 * kStericWarps) k_steric(
             }
         }
         const unsigned m = __ballot_sync(0xffffffffu, ok);
-        if (ok) s_q[wi][qn + __popc(m & ((1u << lane) - 1u))] = j;
-        qn += __popc(m);
-        __syncwarp();
-        if (qn >= 32) {
-            evaluate(32);
-            const int rest = qn - 32;
-            const int moved = lane < rest ? s_q[wi][32 + lane] : 0;
-            __syncwarp();
-            if (lane < rest) s_q[wi][lane] = moved;
-            qn = rest;
-            __syncwarp();
+        if (lane == 0) s_cnt[wi] = __popc(m);
+        __syncthreads();
+        int at = qn;
+        for (int k2 = 0; k2 < kStericWarps; k2++) {
+            if (k2 == wi && ok) s_q[at + __popc(m & ((1u << lane) - 1u))] = j;
+            at += s_cnt[k2];
+        }
+        qn = at;
+        __syncthreads();  // the queue, and s_cnt free
+        if (qn > 32 * kStericWarps || base + 32 * kStericWarps >= total) {
+            evaluate(qn);
+            qn = 0;
+            __syncthreads();
         }
     }
-    evaluate(qn);
 #pragma unroll
     for (int u = 0; u < 4; u++)
 #pragma unroll
@@ -966,7 +1015,7 @@ __global__ void __launch_bounds__(32 * kStericWarps) k_steric(
 // steric list are skipped (k_steric gave them the steric force) and the
 // forces add to what k_steric wrote.
 template <int POT, bool STERIC>
-__global__ void __launch_bounds__(32 * kPairWarps) k_pairs(
+__global__ void __launch_bounds__(32 * kPairWarps, kPairCtas) k_pairs(
     const double *__restrict__ gp, const float4 *__restrict__ nb, const int *__restrict__ cell,
     const int *__restrict__ sorted, const int *__restrict__ start, const int *__restrict__ block, long long ncell,
     int nblocks, int nx, int ny, int nz, const int *__restrict__ fblob, const int *__restrict__ ftype,
@@ -1092,12 +1141,27 @@ __global__ void __launch_bounds__(32 * kPairWarps) k_pairs(
         if (lane == 0) atomicAdd(&energy[lk], part);
         if (e_key == lk) e_key = -1;
     }
-    // the lanes' sums, then the corner weights: lane 3 j + d < 9 writes force
-    // component d of corner j (the fourth node has none from these)
+    // the lanes' sums: nine values by a transposed butterfly (at offsets 16,
+    // 8, 4 and 2 a lane keeps half of its values: 16 additions, not 45); the
+    // total of value v ends in lanes 2 v and 2 v + 1
+    {
+        double v[16];
 #pragma unroll
-    for (int k = 0; k < 3; k++)
+        for (int k = 0; k < 16; k++) v[k] = k < 9 ? S[k / 3][k % 3] : 0.0;
 #pragma unroll
-        for (int d = 0; d < 3; d++) S[k][d] = warp_sum_d(S[k][d]);
+        for (int h = 8, o = 16; h >= 1; h >>= 1, o >>= 1) {
+            const bool upper = (lane & o) != 0;
+#pragma unroll
+            for (int k = 0; k < h; k++) {
+                const double send = upper ? v[k] : v[k + h], keep = upper ? v[k + h] : v[k];
+                // (values 9..15 are zeros: nothing to add where both halves are)
+                if (k + h < 9 || k < 9) v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        }
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+#pragma unroll
+        for (int k = 0; k < 9; k++) S[k / 3][k % 3] = __shfl_sync(0xffffffffu, v[0], 2 * k);
+    }
     unsigned long long np = npairs;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) np += __shfl_xor_sync(0xffffffffu, np, o);
@@ -1255,7 +1319,7 @@ extern "C" int ffea_gpu_ssint_create(const ffea_gpu_ssint_desc *d, ffea_gpu_ssin
         if (dalloc(&s->d_corner, 4 * (size_t)na) || dalloc(&s->d_blob, na) || dalloc(&s->d_type, na) ||
             dalloc(&s->d_geo, 16 * (size_t)na) || dalloc(&s->d_gp, 16 * (size_t)na) || dalloc(&s->d_nb, na) || dalloc(&s->d_cell, na) || dalloc(&s->d_fforce, 12 * (size_t)na) ||
             dalloc(&s->d_count, ncell) || dalloc(&s->d_start, ncell) || dalloc(&s->d_block, s->nblocks + 1) ||
-            dalloc(&s->d_sorted, na) || dalloc(&s->d_node_ptr, d->num_nodes + 1) ||
+            dalloc(&s->d_binned, na) || dalloc(&s->d_sorted, na) || dalloc(&s->d_node_ptr, d->num_nodes + 1) ||
             dalloc(&s->d_node_ent, ent.size()) || dalloc(&s->d_emin, T2) || dalloc(&s->d_rmin, T2) ||
             dalloc(&s->d_pos, 3 * (size_t)d->num_nodes) || dalloc(&s->d_force, 3 * (size_t)d->num_nodes) ||
             dalloc(&s->d_energy, (size_t)d->num_blobs * d->num_blobs) || dalloc(&s->d_stats, 5) ||
@@ -1292,7 +1356,7 @@ extern "C" void ffea_gpu_ssint_destroy(ffea_gpu_ssint_t *s)
     if (!s) return;
     if (s->stream) cudaStreamSynchronize(s->stream);
     void *bufs[] = {s->d_corner, s->d_blob, s->d_type, s->d_geo, s->d_gp, s->d_nb, s->d_cell, s->d_fforce, s->d_count,
-                    s->d_start, s->d_block, s->d_sorted, s->d_node_ptr, s->d_node_ent, s->d_emin, s->d_rmin,
+                    s->d_start, s->d_block, s->d_binned, s->d_sorted, s->d_node_ptr, s->d_node_ent, s->d_emin, s->d_rmin,
                     s->d_pos, s->d_force, s->d_energy, s->d_stats, s->d_large, s->d_stlist, s->d_stcnt, s->d_k0,
                     s->d_corr};
     for (void *p : bufs)
@@ -1320,11 +1384,11 @@ extern "C" int ffea_gpu_ssint_forces_device(ffea_gpu_ssint_t *s, const double *p
                                     s->d_gp, s->d_nb, s->d_cell, s->d_count, s->d_stats);
     k_scan_local<<<s->nblocks, kScanBlock, 0, st>>>(s->d_count, s->ncell, s->d_start, s->d_block);
     k_scan_blocks<<<1, kScanBlock, 0, st>>>(s->d_block, s->nblocks);
-    k_scatter<<<fb, 128, 0, st>>>(s->d_cell, na, s->d_start, s->d_block, s->d_count, s->d_sorted);
+    k_scatter<<<fb, 128, 0, st>>>(s->d_cell, na, s->d_start, s->d_block, s->d_count, s->d_binned);
     // faces outside the box are left out of the grid (and make the call an
     // error); the kernels below bound every segment by the scan's total
-    k_sort_cells<<<(int)((s->ncell + 255) / 256), 256, 0, st>>>(s->ncell, s->nblocks, s->d_start, s->d_block,
-                                                                s->d_sorted, s->d_large, s->d_stats);
+    k_sort_cells<<<fb, 128, 0, st>>>(s->ncell, s->nblocks, s->d_start, s->d_block, s->d_cell, s->d_binned,
+                                     s->d_sorted, s->d_large, s->d_stats);
     k_sort_large<<<kSortLargeCtas, 256, 0, st>>>(s->ncell, s->nblocks, s->d_start, s->d_block, s->d_sorted,
                                                  s->d_large, s->d_stats);
     const int pw = (na + kPairWarps - 1) / kPairWarps;
