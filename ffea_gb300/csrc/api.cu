@@ -881,11 +881,10 @@ int mpnn_alloc(ffea_gpu *h)
     CK(A.alloc(B.e, n));
     CK(A.alloc(B.gw, n));
     CK(A.alloc(B.gvec, (size_t)coarse_total));
-    CK(A.alloc(B.cvec, (size_t)coarse_total));
-    CK(A.alloc(B.cta_sums, 3 * ((n + 127) / 128)));
+    CK(A.alloc(B.cta_sums, 3 * ((n + MPNN_LOSS_ROWS - 1) / MPNN_LOSS_ROWS)));
     CK(A.alloc(B.scal, 3));
-    for (float **p : {&B.dh, &B.dh2, &B.dself, &B.tbuf}) CK(A.alloc(*p, n * MPNN_HIDDEN));
-    CK(A.alloc(B.partial, ((n + 63) / 64) * (size_t)MPNN_NUM_PARAMS));
+    for (float **p : {&B.dself[0], &B.dself[1], &B.tbuf[0], &B.tbuf[1]}) CK(A.alloc(*p, n * MPNN_HIDDEN));
+    CK(A.alloc(B.partial, ((n + MPNN_BWD_ROWS - 1) / MPNN_BWD_ROWS) * (size_t)MPNN_NUM_PARAMS));
     CK(A.alloc(B.theta, (size_t)MPNN_NUM_PARAMS));
     CK(A.alloc(B.grad, (size_t)MPNN_NUM_PARAMS));
     h->mpnn_ready = true;

@@ -217,16 +217,17 @@ constexpr int MPNN_FEATURES = 8;
 constexpr int MPNN_HIDDEN = 32;
 constexpr int MPNN_NUM_PARAMS = 2 * MPNN_HIDDEN * MPNN_FEATURES + MPNN_HIDDEN +
                                 2 * (2 * MPNN_HIDDEN * MPNN_HIDDEN + MPNN_HIDDEN) + MPNN_HIDDEN + 1;
+constexpr int MPNN_LOSS_ROWS = 128, MPNN_BWD_ROWS = 64;  // rows per CTA whose partial sums are kept
 struct MpnnBuffers {
     float *x0 = nullptr;                    // features, 8 per padded row
     __nv_bfloat16 *h[3] = {nullptr, nullptr, nullptr};  // activations, 32 per padded row
     float *omega = nullptr;                 // per padded row
     float4 *v = nullptr, *e = nullptr;      // D^-1 f and z = M f
     float2 *gw = nullptr;                   // per row (Az.v, f.v): dL/d omega = k1 x - k2 y
-    float *gvec = nullptr, *cvec = nullptr; // coarse P^T f and X P^T f
-    double *cta_sums = nullptr, *scal = nullptr;   // 3 per forward CTA; loss, k1, k2
-    float *dh = nullptr, *dh2 = nullptr, *dself = nullptr, *tbuf = nullptr;  // 32 per padded row
-    float *partial = nullptr;               // per backward CTA: MPNN_NUM_PARAMS
+    float *gvec = nullptr;                  // coarse P^T f
+    double *cta_sums = nullptr, *scal = nullptr;   // 3 per MPNN_LOSS_ROWS rows; loss, k1, k2
+    float *dself[2] = {nullptr, nullptr}, *tbuf[2] = {nullptr, nullptr};  // 32 per padded row, of layers 2 and 1
+    float *partial = nullptr;               // MPNN_NUM_PARAMS per MPNN_BWD_ROWS rows
     float *theta = nullptr, *grad = nullptr;
 };
 // forward pass (omega; write_phi: also the smoother weights of the solve),

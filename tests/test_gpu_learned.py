@@ -168,3 +168,48 @@ def test_committed_weights_take_effect_in_a_batch(gpulib, monkeypatch, memory_st
     for i in range(len(specs)):
         assert np.array_equal(vels["learned"][i], vels["learned-again"][i]), i
         assert not np.array_equal(vels["learned"][i], vels["two-level"][i]), i
+
+
+@pytest.mark.parametrize("blob", [0, 1, 2])
+def test_network_on_each_blob_of_a_batch_matches_cpu_oracle(gpulib, blob):
+    """Rows of several blobs in one launch, with row lengths on both sides of
+    the eight neighbours that are in flight together: omega and the gradient
+    for one blob's rows, at the tolerances of the single-blob test."""
+    from ffea_gb300 import learned
+    from oracle import mpnn
+    specs = [spec(radius_nm=r, seed=i, rng_seed=30 + i, precision=P.PRECISION_MIXED, epsilon=1e-6)
+             for i, r in enumerate((4.0, 9.0, 5.5))]
+    s, theta = specs[blob], _theta(5)
+    n, nl = s.mesh.num_nodes, s.mesh.num_linear
+    with _world(specs, preconditioner=LEARNED) as w:
+        w.run(1)
+        domega = np.zeros(n, np.float32)
+        domega[:nl] = np.random.default_rng(6 + blob).normal(size=nl)
+        feats, om, grad = learned.probe(w, blob, theta, domega)
+    ptr, idx = mpnn.edge_neighbours(s.mesh.topology, n)
+    om_ref, cache = mpnn.forward(theta, feats.astype(np.float64), ptr, idx)
+    assert np.max(np.abs(om[:nl] - om_ref[:nl])) < 5e-3
+    g_ref = mpnn.backward(theta, cache, om_ref, domega.astype(np.float64), ptr, idx)
+    assert np.linalg.norm(grad - g_ref) < 2e-2 * np.linalg.norm(g_ref)
+
+
+def test_loss_gradient_of_a_batch_matches_central_differences(gpulib):
+    """The coarse product, a segment a CTA, over blobs of different sizes: as
+    the single-blob test, omega uniform, against central differences."""
+    from ffea_gb300 import learned
+    specs = [spec(radius_nm=r, seed=i, rng_seed=50 + i, precision=P.PRECISION_MIXED, epsilon=1e-6)
+             for i, r in enumerate((6.0, 5.0, 10.0))]
+    lay, _ = learned.layout()
+    bo = lay["bo"][0]
+    with _world(specs, preconditioner=LEARNED) as w:
+        w.run(2)
+        for b0 in (-0.5, 0.7):
+            theta = np.zeros(learned.NUM_PARAMS, np.float32)
+            theta[bo] = b0
+            g = learned.loss_grad(w, theta)[1]
+            h = 1e-2
+            tp, tm = theta.copy(), theta.copy()
+            tp[bo] += h
+            tm[bo] -= h
+            fd = (learned.loss_grad(w, tp, with_grad=False)[0] - learned.loss_grad(w, tm, with_grad=False)[0]) / (2 * h)
+            assert abs(fd - g[bo]) <= 2e-2 * abs(fd) + 1e-6, (b0, fd, g[bo])
