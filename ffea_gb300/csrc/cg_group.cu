@@ -294,13 +294,83 @@ template <> struct SlotDepth<float, 1024> { static constexpr int kOn = 2, kOff =
 template <> struct SlotDepth<double, 512> { static constexpr int kOn = 2, kOff = 2; };
 template <> struct SlotDepth<double, 1024> { static constexpr int kOn = 1, kOff = 1; };
 
+// ---------------------------------------------------------------- tensor memory
+// Matrix values in the SM's tensor memory, 256 KB beside shared memory: a
+// thread's lane of it is private to it, so its row's blocks are stored and
+// read back with no address arithmetic and no bank conflicts.  W: 32-bit
+// words of a block, at `addr` (lane in bits 16 up, column below).  A warp
+// reaches the 32 lanes of its number modulo 4.
+constexpr int kTmemCols = 512;
+
+__device__ __forceinline__ void tmem_alloc(uint32_t *slot)
+{
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(slot);
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(a), "n"(kTmemCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_free(uint32_t addr)
+{
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "n"(kTmemCols) : "memory");
+}
+__device__ __forceinline__ void tmem_put(uint32_t addr, const uint32_t (&v)[9])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%2, %3, %4, %5, %6, %7, %8, %9};\n\t"
+                 "tcgen05.st.sync.aligned.32x32b.x1.b32 [%1], {%10};" ::"r"(addr), "r"(addr + 8), "r"(v[0]), "r"(v[1]),
+                 "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_put(uint32_t addr, const uint32_t (&v)[18])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                 "%14, %15, %16, %17};\n\t"
+                 "tcgen05.st.sync.aligned.32x32b.x2.b32 [%1], {%18, %19};" ::"r"(addr), "r"(addr + 16), "r"(v[0]),
+                 "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+                 "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_put_done() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// (the wait is part of the read: nothing can use the registers before it)
+__device__ __forceinline__ void tmem_get(uint32_t addr, uint32_t (&v)[9])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%9];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x1.b32 {%8}, [%10];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                   "=r"(v[8])
+                 : "r"(addr), "r"(addr + 8)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_get(uint32_t addr, uint32_t (&v)[18])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                 "%14, %15}, [%18];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x2.b32 {%16, %17}, [%19];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+                   "=r"(v[16]), "=r"(v[17])
+                 : "r"(addr), "r"(addr + 16)
+                 : "memory");
+}
+template <typename T>
+__device__ __forceinline__ T word_at(const uint32_t *v, int k)
+{
+    if constexpr (sizeof(T) == 4) return __uint_as_float(v[k]);
+    else return __hiloint2double((int)v[2 * k + 1], (int)v[2 * k]);
+}
+
 // ---------------------------------------------------------------- the kernel
 // T: arithmetic type of the vectors and the matrix.  COARSE: the two-level
 // preconditioner (FP32).  MAXT: threads per CTA at most, which sets the
 // registers a thread may use and the strides of the shared-memory arrays.
 //
 // A thread has one row.  The values of a row's first cache_slots matrix
-// slots are in shared memory, the others come from L2.
+// slots are in shared memory, those of the next tmem_slots in tensor memory
+// (not MAXT = 256, where shared memory has room for nearly all), the others
+// come from L2.  With 965 rows to a CTA (a 40 nm sphere, 14 slots a row) the
+// product was bound by L2, 469 KB a CTA at 34 bytes a clock: seven slots in
+// tensor memory take 229 KB off that, 12.6 to 10.1 thousand clocks a product,
+// 1,174 to 1,080 us a solve.
 template <typename T, bool COARSE, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch gb)
 {
@@ -318,6 +388,9 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
     __shared__ DF s_last[3];                 // the sums of the last transition
     __shared__ BlobParams s_bp;
     __shared__ int s_err, s_stop;
+    __shared__ uint32_t s_tmem;
+    constexpr bool kTmem = MAXT > 256;
+    constexpr int kBlockWords = 9 * (int)sizeof(T) / 4;
     const int tid = threadIdx.x, NT = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = NT >> 5;
     const uint32_t base = __ldcg(&d.bar[6]);  // the tags of this launch start above it
     T *const sx = dyn<T>(gb.o_state);         // x | D^-1 | p | s, 3 MAXT each (unless kRegs)
@@ -326,6 +399,15 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
     uint32_t maxseq = 0;
     int maxloops = 0;
     if (tid == 0) s_err = s_stop = 0;
+    uint32_t tmem = 0;  // the warp's part: its lanes, and its share of their columns
+    if constexpr (kTmem) {
+        if (gb.tmem_slots > 0) {
+            __syncwarp();
+            if (warp == 0) tmem_alloc(&s_tmem);
+            __syncthreads();
+            tmem = s_tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)((warp >> 2) * gb.tmem_slots * kBlockWords);
+        }
+    }
 
 #pragma unroll 1
     for (int ti = gb.ptr[blockIdx.x]; ti < gb.ptr[blockIdx.x + 1]; ti++) {
@@ -402,6 +484,35 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
                 } else {
                     kv1[i * MAXT] = static_cast<const T *>(d.sell_mval)[e];
                 }
+            }
+        }
+        int T0 = 0, T1 = 0;  // the slots in tensor memory, the same for the warp
+        if constexpr (kTmem) {
+            if (run && nomass && warp < nsl) {
+                const int Lw = d.slice_len[(row0 >> 5) + warp];
+                // every other warp of a scheduler keeps its last slots there,
+                // so that half of the warps read L2 while the others do not
+                T0 = min(gb.cache_slots, Lw);
+                if (warp & 4) T0 = max(T0, min(gb.cache_cols, Lw) - gb.tmem_slots);
+                T1 = min(T0 + gb.tmem_slots, min(gb.cache_cols, Lw));
+                __syncwarp();
+#pragma unroll 1
+                for (int j = T0; j < T1; j++) {
+                    const T *val = static_cast<const T *>(d.sell_val) + sell_vidx(ebase + 32 * j, 0);
+                    uint32_t v[kBlockWords];
+#pragma unroll
+                    for (int k = 0; k < 9; k++) {
+                        const T x = valid ? val[32 * k] : (T)0;
+                        if constexpr (fast) {
+                            v[k] = __float_as_uint(x);
+                        } else {
+                            v[2 * k] = (uint32_t)__double2loint(x);
+                            v[2 * k + 1] = (uint32_t)__double2hiint(x);
+                        }
+                    }
+                    tmem_put(tmem + (j - T0) * kBlockWords, v);
+                }
+                tmem_put_done();
             }
         }
         if (COARSE && run && in)
@@ -567,22 +678,63 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
                             block_fma(Kj, y[g][0] - u[0], y[g][1] - u[1], y[g][2] - u[2], acc[0], acc[1], acc[2]);
                         }
                     }
-                    const T *vp = static_cast<const T *>(d.sell_val) + sell_vidx(ebase + 32 * J1, 0);
+                    // values from L2, slots ja .. jb - 1
+                    auto from_l2 = [&](int ja, int jb) {
+                        const T *vp = static_cast<const T *>(d.sell_val) + sell_vidx(ebase + 32 * ja, 0);
 #pragma unroll 1
-                    for (int j0 = J1; j0 < L; j0 += G2, vp += 288 * G2) {
-                        T Kj[G2][9];
+                        for (int j0 = ja; j0 < jb; j0 += G2, vp += 288 * G2) {
+                            T Kj[G2][9];
 #pragma unroll
-                        for (int g = 0; g < G2; g++)
+                            for (int g = 0; g < G2; g++)
 #pragma unroll
-                            for (int k = 0; k < 9; k++)
-                                Kj[g][k] = j0 + g < L ? __ldg(vp + 288 * g + 32 * k) : (T)0;
+                                for (int k = 0; k < 9; k++)
+                                    Kj[g][k] = j0 + g < jb ? __ldg(vp + 288 * g + 32 * k) : (T)0;
 #pragma unroll
-                        for (int g = 0; g < G2; g++) {
-                            const int j = j0 + g;
-                            T y[3];
-                            load3(j >= L ? tid : j < JC ? col[j * MAXT] : __ldg(&gb.lcol[ebase + 32 * j]), y);
-                            block_fma(Kj[g], y[0] - u[0], y[1] - u[1], y[2] - u[2], acc[0], acc[1], acc[2]);
+                            for (int g = 0; g < G2; g++) {
+                                const int j = j0 + g;
+                                T y[3];
+                                load3(j >= jb ? tid : j < JC ? col[j * MAXT] : __ldg(&gb.lcol[ebase + 32 * j]), y);
+                                block_fma(Kj[g], y[0] - u[0], y[1] - u[1], y[2] - u[2], acc[0], acc[1], acc[2]);
+                            }
                         }
+                    };
+                    if constexpr (kTmem) {
+                        constexpr int GT = sizeof(T) == 4 ? 2 : 1;
+                        constexpr int W = GT * kBlockWords;
+#pragma unroll 1
+                        for (int pass = 0; pass < 2; pass++) {
+                            from_l2(pass == 0 ? J1 : max(J1, min(T1, L)), pass == 0 ? min(T0, L) : L);
+                            if (pass > 0) break;
+                            __syncwarp();
+                            int j = T0;
+#pragma unroll 1
+                            for (; j + GT <= T1; j += GT) {
+                                uint32_t v[W];
+                                T y[GT][3];
+#pragma unroll
+                                for (int g = 0; g < GT; g++) load3(j + g < L ? col[(j + g) * MAXT] : tid, y[g]);
+                                tmem_get(tmem + (j - T0) * kBlockWords, v);
+#pragma unroll
+                                for (int g = 0; g < GT; g++) {
+                                    T Kj[9];
+#pragma unroll
+                                    for (int k = 0; k < 9; k++) Kj[k] = word_at<T>(v + g * kBlockWords, k);
+                                    block_fma(Kj, y[g][0] - u[0], y[g][1] - u[1], y[g][2] - u[2], acc[0], acc[1],
+                                              acc[2]);
+                                }
+                            }
+                            if (GT > 1 && j < T1) {
+                                uint32_t v[kBlockWords];
+                                T y[3], Kj[9];
+                                load3(j < L ? col[j * MAXT] : tid, y);
+                                tmem_get(tmem + (j - T0) * kBlockWords, v);
+#pragma unroll
+                                for (int k = 0; k < 9; k++) Kj[k] = word_at<T>(v, k);
+                                block_fma(Kj, y[0] - u[0], y[1] - u[1], y[2] - u[2], acc[0], acc[1], acc[2]);
+                            }
+                        }
+                    } else {
+                        from_l2(J1, L);
                     }
                 } else {
                     const T *mv = static_cast<const T *>(d.sell_mval);
@@ -875,6 +1027,12 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
             break;  // CTA-uniform: s_stop was read after a barrier by every thread
         }
     }
+    if constexpr (kTmem) {
+        if (gb.tmem_slots > 0) {
+            __syncthreads();
+            if (warp == 0) tmem_free(s_tmem);
+        }
+    }
     if (tid == 0) {
         if (blockIdx.x == 0 && d.cg_euler && d.num_streams != d.num_blobs && !s_stop)
 #pragma unroll 1
@@ -952,6 +1110,16 @@ int cg_group_plan(const DeviceBatch &d, GroupBatch &g, int max_slots, int max_co
     g.o_col = take((size_t)g.cache_cols * per_col);
     g.o_kv2 = take(d.any_nomass ? 8 * ts * R * g.cache_slots : 0);
     g.o_kv1 = take(ts * R * g.cache_slots);
+    g.tmem_slots = 0;
+    if (g.rows > 256 && d.any_nomass) {
+        // the warps of a quarter of the lanes share its columns.  The places
+        // of a block in tensor memory are read from shared memory
+        const int warps = (g.threads / 32 + 3) / 4;
+        g.tmem_slots = std::min(kTmemCols / warps / (int)(9 * ts / 4),
+                                std::min(max_slots, (int)g.cache_cols) - (int)g.cache_slots);
+        // a CTA takes all of its SM's tensor memory: no second one beside it
+        if (g.tmem_slots > 0) off = std::max<size_t>(off, (size_t)optin / 2 + 1024);
+    }
     g.dyn_smem = (int32_t)off;
     // the limit is a property of the kernel, shared by every handle: the
     // device maximum, so that no handle's plan lowers another's

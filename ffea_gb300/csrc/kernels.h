@@ -116,6 +116,7 @@ struct GroupBatch {
     int32_t rows = 0;               // rows a CTA has room for
     int32_t dyn_smem = 0;
     int32_t cache_slots = 0;  // matrix slots per row whose values are copied to shared memory
+    int32_t tmem_slots = 0;   // matrix slots per row, after those, whose values are copied to tensor memory
     int32_t cache_cols = 0;   // matrix slots per row whose column places are copied
     int32_t *ptr = nullptr, *task = nullptr;
     // per segment its halo, the rows of other segments it couples to, and per

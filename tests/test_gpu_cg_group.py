@@ -70,3 +70,20 @@ def test_fp64_matches_oracle(gpulib, oracle, monkeypatch, radii, max_ctas, solve
         pos, vel, _ = ref.nodes()
         assert np.linalg.norm(on[i][1] - vel) <= 1e-9 * np.linalg.norm(vel), i
         assert np.abs(on[i][0] - pos).max() < 1e-10, i
+
+
+@pytest.mark.parametrize("slots", [1, 8, 11])
+@pytest.mark.parametrize("radii,max_ctas", [((5.0,), 1), ((8.0,), 2)])
+def test_matrix_slots_in_each_memory(gpulib, monkeypatch, radii, max_ctas, slots):
+    """The variants of more than 256 rows keep a row's first matrix slots in
+    shared memory, more in tensor memory (an odd or an even number of them,
+    the first or the last of a row's) and read the rest from L2; the
+    environment variable caps the slots on chip."""
+    monkeypatch.setenv("FFEA_GPU_CG_SMEM_SLOTS", str(slots))
+    specs = [_mixed(r, i + 1, pinned=[0, 7]) for i, r in enumerate(radii)]
+    on, s_on, _ = _run(monkeypatch, specs, max_ctas, False)
+    mem, s_mem, _ = _run(monkeypatch, specs, max_ctas, True)
+    for i in range(len(specs)):
+        for a, b in zip(on[i], mem[i]):
+            assert np.array_equal(a, b), i
+        assert s_on[i]["fail_bits"] == 0 and s_on[i]["cg_iters"] == s_mem[i]["cg_iters"]
