@@ -354,11 +354,70 @@ struct GroupPlan {
     int max_rows = 0, max_halo = 0, max_segs = 0;
 };
 
+// Each blob, in the given order, on the CTAs that are free first; returns
+// the time at which the last one ends.
+double schedule_groups(const HostBatch &H, const std::vector<int32_t> &blobs, const std::vector<double> &cost, int G,
+                       std::vector<std::vector<int32_t>> &per)
+{
+    std::vector<double> busy(G, 0.0);
+    std::vector<int> order(G);
+    per.assign(G, {});
+    double last = 0.0;
+    for (int b : blobs) {
+        const BlobParams &bp = H.bp[b];
+        for (int c = 0; c < G; c++) order[c] = c;
+        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return busy[x] < busy[y]; });
+        const double end = busy[order[bp.seg_cnt - 1]] + cost[b];
+        last = std::max(last, end);
+        // segments to CTAs in CTA order: neighbours in the blob on neighbouring CTAs
+        std::sort(order.begin(), order.begin() + bp.seg_cnt);
+        for (int k = 0; k < bp.seg_cnt; k++) {
+            per[order[k]].push_back(bp.seg_off + k);
+            busy[order[k]] = end;
+        }
+    }
+    return last;
+}
+
+// The blobs in rounds of at most G segments: the longest solve left, beside
+// it the others that fill most of the round's CTAs (0/1 knapsack over the
+// segment counts, a segment worth its blob's time).  Thirty-two equal blobs
+// of 9 or 10 segments on 152 CTAs take two rounds so (16 blobs, 152 segments
+// each), three when the 10s come first (the solves of 32 spheres of 15 nm 2.30 ms
+// then, 1.60 so).
+std::vector<int32_t> fill_rounds(const HostBatch &H, std::vector<int32_t> blobs, const std::vector<double> &cost, int G)
+{
+    std::vector<int32_t> out;
+    while (!blobs.empty()) {
+        const int n = (int)blobs.size(), room = G - H.bp[blobs[0]].seg_cnt;
+        std::vector<double> best(room + 1, 0.0);
+        std::vector<std::vector<char>> with(n, std::vector<char>(room + 1, 0));
+        for (int i = 1; i < n; i++) {
+            const int k = H.bp[blobs[i]].seg_cnt;
+            for (int w = room; w >= k; w--)
+                if (best[w - k] + k * cost[blobs[i]] > best[w]) {
+                    best[w] = best[w - k] + k * cost[blobs[i]];
+                    with[i][w] = 1;
+                }
+        }
+        std::vector<char> take(n, 0);
+        take[0] = 1;
+        for (int i = n - 1, w = room; i > 0; i--)
+            if (with[i][w]) {
+                take[i] = 1;
+                w -= H.bp[blobs[i]].seg_cnt;
+            }
+        std::vector<int32_t> rest;
+        for (int i = 0; i < n; i++) (take[i] ? out : rest).push_back(blobs[i]);
+        blobs.swap(rest);
+    }
+    return out;
+}
+
 // One CTA per segment; false when a blob has more segments than CTAs.
 // Longest solve first (iterations grow with the radius, an iteration with
-// the rows of a CTA), each blob on the CTAs that are free first.  Every CTA
-// runs its segments in this order, so waiting for a group's CTAs cannot form
-// a cycle.  Sets g.grid.
+// the rows of a CTA), or in rounds.  Every CTA runs its segments in one order
+// of the blobs, so waiting for a group's CTAs cannot form a cycle.  Sets g.grid.
 bool plan_groups(const HostBatch &H, int ctas, GroupBatch &g, GroupPlan &plan)
 {
     const int nb = H.num_blobs, ns = (int)H.seg_row0.size();
@@ -394,25 +453,16 @@ bool plan_groups(const HostBatch &H, int ctas, GroupBatch &g, GroupPlan &plan)
         plan.max_halo = std::max(plan.max_halo, (int)(plan.halo.size() - h0));
     }
     if (plan.max_halo > 32768) return false;  // (16-bit places)
-    // the schedule
+    // the schedule: longest first, or by rounds where that leaves CTAs idle
+    // and gains
     g.grid = std::min(ctas, ns);
     std::stable_sort(blobs.begin(), blobs.end(), [&](int a, int b) { return cost[a] > cost[b]; });
-    const int G = g.grid;
-    std::vector<double> busy(G, 0.0);
-    std::vector<int> order(G);
-    std::vector<std::vector<int32_t>> per(G);
-    for (int b : blobs) {
-        const BlobParams &bp = H.bp[b];
-        for (int c = 0; c < G; c++) order[c] = c;
-        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return busy[x] < busy[y]; });
-        const double end = busy[order[bp.seg_cnt - 1]] + cost[b];
-        // segments to CTAs in CTA order: neighbours in the blob on neighbouring CTAs
-        std::sort(order.begin(), order.begin() + bp.seg_cnt);
-        for (int k = 0; k < bp.seg_cnt; k++) {
-            per[order[k]].push_back(bp.seg_off + k);
-            busy[order[k]] = end;
-        }
-    }
+    std::vector<std::vector<int32_t>> per, per2;
+    const double end = schedule_groups(H, blobs, cost, g.grid, per);
+    double area = 0.0;
+    for (int b = 0; b < nb; b++) area += H.bp[b].seg_cnt * cost[b];
+    if (nb <= 2048 && end > 1.02 * area / g.grid &&
+        schedule_groups(H, fill_rounds(H, blobs, cost, g.grid), cost, g.grid, per2) < end) per.swap(per2);
     plan.ptr.assign(1, 0);
     for (const auto &v : per) {
         plan.task.insert(plan.task.end(), v.begin(), v.end());

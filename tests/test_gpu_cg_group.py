@@ -87,3 +87,17 @@ def test_matrix_slots_in_each_memory(gpulib, monkeypatch, radii, max_ctas, slots
         for a, b in zip(on[i], mem[i]):
             assert np.array_equal(a, b), i
         assert s_on[i]["fail_bits"] == 0 and s_on[i]["cg_iters"] == s_mem[i]["cg_iters"]
+
+
+@pytest.mark.parametrize("radii,max_ctas", [((8.0, 7.9, 8.0, 10.0, 10.0, 10.0), 5), ((8.0, 3.0, 10.0, 3.5, 8.0), 4)])
+def test_blobs_scheduled_in_rounds(gpulib, monkeypatch, radii, max_ctas):
+    """Groups of two and three CTAs on five (two rounds' worth when a two and a
+    three share each, more when the threes come first), and of one to three on four."""
+    specs = [_mixed(r, i + 1) for i, r in enumerate(radii)]
+    on, s_on, g_on = _run(monkeypatch, specs, max_ctas, False)
+    mem, s_mem, g_mem = _run(monkeypatch, specs, max_ctas, True)
+    for i in range(len(specs)):
+        for a, b in zip(on[i], mem[i]):
+            assert np.array_equal(a, b), i
+        assert np.array_equal(g_on[i], g_mem[i])
+        assert s_on[i]["fail_bits"] == 0 and s_on[i]["cg_iters"] == s_mem[i]["cg_iters"]
