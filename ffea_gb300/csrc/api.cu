@@ -350,29 +350,36 @@ std::vector<int32_t> deal_segments(const HostBatch &H, int G)
 // and the rows of other segments each segment couples to.
 struct GroupPlan {
     std::vector<int32_t> ptr, task;   // per CTA: its segments
-    std::vector<int32_t> hptr, halo;  // per segment: its halo rows, ascending
+    std::vector<int32_t> hptr, halo;  // per segment that starts a task: the task's halo rows, ascending
     int max_rows = 0, max_halo = 0, max_segs = 0;
 };
 
-// Each blob, in the given order, on the CTAs that are free first; returns
-// the time at which the last one ends.
-double schedule_groups(const HostBatch &H, const std::vector<int32_t> &blobs, const std::vector<double> &cost, int G,
-                       std::vector<std::vector<int32_t>> &per)
+// One past the last segment of the task that segment s starts, s where it
+// starts none.
+int task_end(const HostBatch &H, int width, int s)
+{
+    const BlobParams &bp = H.bp[H.seg_blob[s]];
+    return (s - bp.seg_off) % width ? s : std::min(s + width, bp.seg_off + bp.seg_cnt);
+}
+
+// Each blob, in the given order, on the CTAs that are free first (size[b] of
+// them, `width` segments each); returns the time at which the last one ends.
+double schedule_groups(const HostBatch &H, const std::vector<int32_t> &blobs, const std::vector<int> &size,
+                       const std::vector<double> &cost, int width, int G, std::vector<std::vector<int32_t>> &per)
 {
     std::vector<double> busy(G, 0.0);
     std::vector<int> order(G);
     per.assign(G, {});
     double last = 0.0;
     for (int b : blobs) {
-        const BlobParams &bp = H.bp[b];
         for (int c = 0; c < G; c++) order[c] = c;
         std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return busy[x] < busy[y]; });
-        const double end = busy[order[bp.seg_cnt - 1]] + cost[b];
+        const double end = busy[order[size[b] - 1]] + cost[b];
         last = std::max(last, end);
         // segments to CTAs in CTA order: neighbours in the blob on neighbouring CTAs
-        std::sort(order.begin(), order.begin() + bp.seg_cnt);
-        for (int k = 0; k < bp.seg_cnt; k++) {
-            per[order[k]].push_back(bp.seg_off + k);
+        std::sort(order.begin(), order.begin() + size[b]);
+        for (int k = 0; k < size[b]; k++) {
+            per[order[k]].push_back(H.bp[b].seg_off + width * k);
             busy[order[k]] = end;
         }
     }
@@ -385,15 +392,16 @@ double schedule_groups(const HostBatch &H, const std::vector<int32_t> &blobs, co
 // of 9 or 10 segments on 152 CTAs take two rounds so (16 blobs, 152 segments
 // each), three when the 10s come first (the solves of 32 spheres of 15 nm 2.30 ms
 // then, 1.60 so).
-std::vector<int32_t> fill_rounds(const HostBatch &H, std::vector<int32_t> blobs, const std::vector<double> &cost, int G)
+std::vector<int32_t> fill_rounds(std::vector<int32_t> blobs, const std::vector<int> &size,
+                                 const std::vector<double> &cost, int G)
 {
     std::vector<int32_t> out;
     while (!blobs.empty()) {
-        const int n = (int)blobs.size(), room = G - H.bp[blobs[0]].seg_cnt;
+        const int n = (int)blobs.size(), room = G - size[blobs[0]];
         std::vector<double> best(room + 1, 0.0);
         std::vector<std::vector<char>> with(n, std::vector<char>(room + 1, 0));
         for (int i = 1; i < n; i++) {
-            const int k = H.bp[blobs[i]].seg_cnt;
+            const int k = size[blobs[i]];
             for (int w = room; w >= k; w--)
                 if (best[w - k] + k * cost[blobs[i]] > best[w]) {
                     best[w] = best[w - k] + k * cost[blobs[i]];
@@ -405,7 +413,7 @@ std::vector<int32_t> fill_rounds(const HostBatch &H, std::vector<int32_t> blobs,
         for (int i = n - 1, w = room; i > 0; i--)
             if (with[i][w]) {
                 take[i] = 1;
-                w -= H.bp[blobs[i]].seg_cnt;
+                w -= size[blobs[i]];
             }
         std::vector<int32_t> rest;
         for (int i = 0; i < n; i++) (take[i] ? out : rest).push_back(blobs[i]);
@@ -414,18 +422,24 @@ std::vector<int32_t> fill_rounds(const HostBatch &H, std::vector<int32_t> blobs,
     return out;
 }
 
-// One CTA per segment; false when a blob has more segments than CTAs.
+// A CTA per segment, or per two neighbouring ones where a blob has more
+// segments than there are CTAs (every blob's then); false where that is not
+// enough.
 // Longest solve first (iterations grow with the radius, an iteration with
 // the rows of a CTA), or in rounds.  Every CTA runs its segments in one order
-// of the blobs, so waiting for a group's CTAs cannot form a cycle.  Sets g.grid.
+// of the blobs, so waiting for a group's CTAs cannot form a cycle.  Sets
+// g.grid and g.per.
 bool plan_groups(const HostBatch &H, int ctas, GroupBatch &g, GroupPlan &plan)
 {
     const int nb = H.num_blobs, ns = (int)H.seg_row0.size();
     std::vector<int32_t> blobs(nb);
     std::vector<double> cost(nb);
+    std::vector<int> size(nb);  // CTAs
+    g.per = 1;
+    int tasks = 0;
     for (int b = 0; b < nb; b++) {
         const BlobParams &bp = H.bp[b];
-        if (bp.seg_cnt > ctas) return false;
+        if (bp.seg_cnt > ctas) g.per = 2;
         blobs[b] = b;
         int rows = 0;
         for (int s = bp.seg_off; s < bp.seg_off + bp.seg_cnt; s++) rows = std::max(rows, H.seg_rows[s]);
@@ -434,35 +448,43 @@ bool plan_groups(const HostBatch &H, int ctas, GroupBatch &g, GroupPlan &plan)
         cost[b] = std::cbrt((double)bp.node_cnt) * (500.0 + rows);
     }
     if (plan.max_rows > CG_SEG_MAX_ROWS) return false;
+    for (int b = 0; b < nb; b++) {
+        size[b] = (H.bp[b].seg_cnt + g.per - 1) / g.per;
+        tasks += size[b];
+        if (size[b] > ctas) return false;
+    }
     // halos
     std::vector<int32_t> seen(H.nl_pad, -1);
     plan.hptr.assign(1, 0);
     for (int s = 0; s < ns; s++) {
-        const int r0 = H.seg_row0[s], r1 = r0 + H.seg_rows[s];
         const size_t h0 = plan.halo.size();
-        for (int r = r0; r < r1; r++)
-            for (int j = 0; j < H.slice_len[r >> 5]; j++) {
-                const int q = H.sell_col[H.slice_ptr[r >> 5] + 32 * j + (r & 31)];
-                if ((q < r0 || q >= r1) && seen[q] != s) {
-                    seen[q] = s;
-                    plan.halo.push_back(q);
+        const int e = task_end(H, g.per, s);
+        for (int t = s; t < e; t++)
+            for (int r = H.seg_row0[t]; r < H.seg_row0[t] + H.seg_rows[t]; r++) seen[r] = s;
+        for (int t = s; t < e; t++)
+            for (int r = H.seg_row0[t]; r < H.seg_row0[t] + H.seg_rows[t]; r++)
+                for (int j = 0; j < H.slice_len[r >> 5]; j++) {
+                    const int q = H.sell_col[H.slice_ptr[r >> 5] + 32 * j + (r & 31)];
+                    if (seen[q] != s) {
+                        seen[q] = s;
+                        plan.halo.push_back(q);
+                    }
                 }
-            }
         std::sort(plan.halo.begin() + h0, plan.halo.end());
         plan.hptr.push_back((int32_t)plan.halo.size());
         plan.max_halo = std::max(plan.max_halo, (int)(plan.halo.size() - h0));
     }
-    if (plan.max_halo > 32768) return false;  // (16-bit places)
+    if (plan.max_halo > 32768) return false;  // (16-bit places, beside 2,048 rows)
     // the schedule: longest first, or by rounds where that leaves CTAs idle
     // and gains
-    g.grid = std::min(ctas, ns);
+    g.grid = std::min(ctas, tasks);
     std::stable_sort(blobs.begin(), blobs.end(), [&](int a, int b) { return cost[a] > cost[b]; });
     std::vector<std::vector<int32_t>> per, per2;
-    const double end = schedule_groups(H, blobs, cost, g.grid, per);
+    const double end = schedule_groups(H, blobs, size, cost, g.per, g.grid, per);
     double area = 0.0;
-    for (int b = 0; b < nb; b++) area += H.bp[b].seg_cnt * cost[b];
+    for (int b = 0; b < nb; b++) area += size[b] * cost[b];
     if (nb <= 2048 && end > 1.02 * area / g.grid &&
-        schedule_groups(H, fill_rounds(H, blobs, cost, g.grid), cost, g.grid, per2) < end) per.swap(per2);
+        schedule_groups(H, fill_rounds(blobs, size, cost, g.grid), size, cost, g.per, g.grid, per2) < end) per.swap(per2);
     plan.ptr.assign(1, 0);
     for (const auto &v : per) {
         plan.task.insert(plan.task.end(), v.begin(), v.end());
@@ -471,21 +493,23 @@ bool plan_groups(const HostBatch &H, int ctas, GroupBatch &g, GroupPlan &plan)
     return true;
 }
 
-// Per matrix entry its column's place in the CTA's copy of u: the local row,
-// or `rows` + its place in the segment's halo.
-std::vector<uint16_t> group_columns(const HostBatch &H, const GroupPlan &plan, int rows)
+// Per matrix entry its column's place in the CTA's copy of u (GroupBatch::lcol).
+std::vector<uint16_t> group_columns(const HostBatch &H, const GroupPlan &plan, const GroupBatch &g)
 {
     std::vector<uint16_t> out(H.sell_col.size(), 0);
     std::vector<int32_t> place(H.nl_pad, 0);
-    for (size_t s = 0; s + 1 < plan.hptr.size(); s++) {
-        const int r0 = H.seg_row0[s], r1 = r0 + H.seg_rows[s];
-        for (int k = plan.hptr[s]; k < plan.hptr[s + 1]; k++) place[plan.halo[k]] = rows + (k - plan.hptr[s]);
-        for (int r = r0; r < r1; r++)
-            for (int j = 0; j < H.slice_len[r >> 5]; j++) {
-                const size_t e = (size_t)H.slice_ptr[r >> 5] + 32 * j + (r & 31);
-                const int q = H.sell_col[e];
-                out[e] = (uint16_t)(q >= r0 && q < r1 ? q - r0 : place[q]);
-            }
+    for (int s = 0; s + 1 < (int)plan.hptr.size(); s++) {
+        const int e = task_end(H, g.per, s);
+        for (int t = s; t < e; t++)
+            for (int r = 0; r < H.seg_rows[t]; r++) place[H.seg_row0[t] + r] = g.rows * (t - s) + r;
+        for (int k = plan.hptr[s]; k < plan.hptr[s + 1]; k++)
+            place[plan.halo[k]] = g.rows * g.per + (k - plan.hptr[s]);
+        for (int t = s; t < e; t++)
+            for (int r = H.seg_row0[t]; r < H.seg_row0[t] + H.seg_rows[t]; r++)
+                for (int j = 0; j < H.slice_len[r >> 5]; j++) {
+                    const size_t i = (size_t)H.slice_ptr[r >> 5] + 32 * j + (r & 31);
+                    out[i] = (uint16_t)place[H.sell_col[i]];
+                }
     }
     return out;
 }
@@ -617,7 +641,7 @@ int ffea_gpu_create_batch(int32_t num_blobs, const ffea_gpu_mesh *meshes, const 
         CK(upload(A, g.task, groups.task));
         CK(upload(A, g.hptr, groups.hptr));
         CK(upload(A, g.halo, groups.halo));
-        CK(upload(A, g.lcol, group_columns(H, groups, g.rows)));
+        CK(upload(A, g.lcol, group_columns(H, groups, g)));
         CK(A.alloc(g.words, 2 * (size_t)GRP_WORDS * n_segs));
         CK(A.alloc(g.pub, (size_t)(H.precision == PREC_FP64 ? 3 : 1) * H.nl_pad));
     } else {

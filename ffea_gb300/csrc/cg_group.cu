@@ -116,6 +116,25 @@ template <> struct PubRow<double> {
     __device__ __forceinline__ bool is(uint32_t t) const { return tag == t && tag1 == t && tag2 == t; }
 };
 
+// A read of a matrix that is larger than L2, which an iteration reads once:
+// evicted first, but for a tenth of it, so that it does not displace what
+// else the iteration reads (50 nm sphere, 138 MB of matrix: 47.1 us an
+// iteration with plain reads, 36.1 with all of it evicted first, 35.7 with a
+// tenth kept, 37.4 with three tenths).
+__device__ __forceinline__ uint64_t stream_policy()
+{
+    uint64_t pol;
+    asm volatile("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, %1;" : "=l"(pol) : "f"(0.1f));
+    return pol;
+}
+__device__ __forceinline__ float ld_stream(const float *p, uint64_t pol)
+{
+    float v;
+    asm volatile("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+    return v;
+}
+__device__ __forceinline__ double ld_stream(const double *p, uint64_t) { return __ldg(p); }
+
 constexpr unsigned int kGroupSpins = 1u << 22;  // reads of one word, a few seconds, then give up
 
 // Whether a wait goes on: bounded, and given up when another wait of the CTA
@@ -305,7 +324,8 @@ constexpr int kTmemCols = 512;
 __device__ __forceinline__ void tmem_alloc(uint32_t *slot)
 {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(slot);
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(a), "n"(kTmemCols) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(a), "n"(kTmemCols)
+                 : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_free(uint32_t addr)
@@ -352,6 +372,22 @@ __device__ __forceinline__ void tmem_get(uint32_t addr, uint32_t (&v)[18])
                  : "r"(addr), "r"(addr + 16)
                  : "memory");
 }
+// row q of the CTA's copy of u
+template <bool VEC, typename T>
+__device__ __forceinline__ void put_u(T *su, int q, T x, T y, T z)
+{
+    T *o = su + 4 * (size_t)q;
+    if constexpr (!VEC) {
+        o[0] = x;
+        o[1] = y;
+        o[2] = z;
+    } else if constexpr (sizeof(T) == 4) {
+        *reinterpret_cast<float4 *>(o) = make_float4(x, y, z, 0.f);
+    } else {
+        *reinterpret_cast<double2 *>(o) = make_double2(x, y);
+        o[2] = z;
+    }
+}
 template <typename T>
 __device__ __forceinline__ T word_at(const uint32_t *v, int k)
 {
@@ -364,26 +400,31 @@ __device__ __forceinline__ T word_at(const uint32_t *v, int k)
 // preconditioner (FP32).  MAXT: threads per CTA at most, which sets the
 // registers a thread may use and the strides of the shared-memory arrays.
 //
-// A thread has one row.  The values of a row's first cache_slots matrix
+// R: segments of a CTA, two where a blob has more of them than there are CTAs
+// (a 50 nm sphere: 304 of 931 rows; 59.1 us an iteration in the
+// memory-resident solve, 35.1 here, 16 of them the matrix from HBM).  A
+// thread has one row of each.  The values of a row's first cache_slots matrix
 // slots are in shared memory, those of the next tmem_slots in tensor memory
 // (not MAXT = 256, where shared memory has room for nearly all), the others
 // come from L2.  With 965 rows to a CTA (a 40 nm sphere, 14 slots a row) the
 // product was bound by L2, 469 KB a CTA at 34 bytes a clock: seven slots in
 // tensor memory take 229 KB off that, 12.6 to 10.1 thousand clocks a product,
 // 1,174 to 1,080 us a solve.
-template <typename T, bool COARSE, int MAXT>
+template <typename T, bool COARSE, int MAXT, int R>
 __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch gb)
 {
     constexpr bool fast = sizeof(T) == 4;
     constexpr bool kRegs = MAXT <= 512;      // x, D^-1, p and s in registers, else in shared memory
+    constexpr bool kWide = R > 1;            // u of the own rows from su, phi and X from L2: no room elsewhere
+    constexpr bool kVec = MAXT > 512;        // (16-byte stores of u: 1 % slower in the small variants)
     using Row = PubRow<T>;
     using T2 = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
-    __shared__ double s_dot[3 * 32];         // per slice: r.u, w.u, r.r (T, or FP64 for the true residual)
-    __shared__ float s_res[12 * 32];         // per slice: P^T r, P^T w
-    __shared__ float s_red6[6 * 32];
-    __shared__ float s_cvec[8];
+    __shared__ double s_dots[R][3 * 32];     // per slice: r.u, w.u, r.r (T, or FP64 for the true residual)
+    __shared__ float s_ress[R][12 * 32];     // per slice: P^T r, P^T w
+    __shared__ float s_red6[R][6 * 32];
+    __shared__ float s_cvec[R][8];
     __shared__ CgScalars s_cg;
-    __shared__ float s_out[18];              // the segment's sums: r.u, w.u, r.r (hi, lo), P^T r, P^T w
+    __shared__ float s_outs[R][18];          // a segment's sums: r.u, w.u, r.r (hi, lo), P^T r, P^T w
     __shared__ DF s_part[3 * 32];            // the dot terms summed over 32 segments of the group each
     __shared__ DF s_last[3];                 // the sums of the last transition
     __shared__ BlobParams s_bp;
@@ -393,10 +434,11 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
     constexpr int kBlockWords = 9 * (int)sizeof(T) / 4;
     const int tid = threadIdx.x, NT = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = NT >> 5;
     const uint32_t base = __ldcg(&d.bar[6]);  // the tags of this launch start above it
-    T *const sx = dyn<T>(gb.o_state);         // x | D^-1 | p | s, 3 MAXT each (unless kRegs)
+    T *const sx = dyn<T>(gb.o_state);         // per segment x | D^-1 | p | s, 3 MAXT each (unless kRegs)
     T *const su = dyn<T>(gb.o_u);             // u of the CTA's rows, then of its halo, (x, y, z, 0) each
     uint4 *const pub = gb.pub;
     uint32_t maxseq = 0;
+    const uint64_t pol = kWide ? stream_policy() : 0;
     int maxloops = 0;
     if (tid == 0) s_err = s_stop = 0;
     uint32_t tmem = 0;  // the warp's part: its lanes, and its share of their columns
@@ -405,7 +447,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
             __syncwarp();
             if (warp == 0) tmem_alloc(&s_tmem);
             __syncthreads();
-            tmem = s_tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)((warp >> 2) * gb.tmem_slots * kBlockWords);
+            tmem = s_tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)((warp >> 2) * R * gb.tmem_slots * kBlockWords);
         }
     }
 
@@ -419,120 +461,146 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
 #pragma unroll 1
         for (int k = tid; k < (int)(sizeof(CgScalars) / 4); k += NT)
             reinterpret_cast<int *>(&s_cg)[k] = __ldcg(reinterpret_cast<const int *>(d.cg + b) + k);
-        const int row0 = d.seg_row0[seg], nrows = d.seg_rows[seg], nsl = (nrows + 31) >> 5;
         __syncthreads();
         const int cnt = s_bp.seg_cnt;          // segments of the group
         const bool solo = cnt == 1;
+        int row0[R], nsl[R];
+        bool in[R], valid[R];  // a row of the segment, a free one
+#pragma unroll
+        for (int q = 0; q < R; q++) {
+            const bool has = q == 0 || seg + q < s_bp.seg_off + cnt;
+            row0[q] = has ? d.seg_row0[seg + q] : 0;
+            const int nrows = has ? d.seg_rows[seg + q] : 0;
+            nsl[q] = (nrows + 31) >> 5;
+            in[q] = tid < nrows;
+            valid[q] = in[q] && !(d.flags[row0[q] + tid] & NODE_PINNED);
+        }
         const bool leader = seg == s_bp.seg_off;
         const bool nomass = s_bp.solver == SOLVER_NOMASS;
         const int cn = COARSE ? s_bp.coarse_n : 0;
         const int limit = s_bp.solver == SOLVER_MASS ? s_bp.max_iter - 1 : s_bp.max_iter;
         const bool run = s_cg.state == CG_ACTIVE;
         const int h0 = gb.hptr[seg], nh = gb.hptr[seg + 1] - h0;  // halo rows
-        const int row = row0 + tid;
-        const bool in = tid < nrows;
-        const bool valid = in && !(d.flags[row] & NODE_PINNED);  // a free row of the segment
-        T diag = (T)0;
-        int L = 0, ebase = 0;  // slots of the row, its first entry
-        T r[3] = {0, 0, 0}, u[3] = {0, 0, 0}, w[3] = {0, 0, 0};
+        T diag[R];
+        int L[R], ebase[R];  // slots of the row, its first entry
+        T r[R][3], u[kWide ? 1 : R][3], w[R][3];
         T st[4][kRegs ? 3 : 1];  // x, D^-1, p, s
-        auto state_of = [&](int f, int k) -> T & {
+        auto state_of = [&](int q, int f, int k) -> T & {
             if constexpr (kRegs) return st[f][k];
-            else return sx[(3 * f + k) * MAXT + tid];
+            else return sx[((4 * q + f) * 3 + k) * MAXT + tid];
+        };
+        auto phi_of = [&](int q) -> float4 {
+            if constexpr (kWide) return __ldg(&d.phi[row0[q] + tid]);
+            else return dyn<float4>(gb.o_phi)[tid];
         };
 #pragma unroll
-        for (int f = 0; f < 4; f++)
+        for (int q = 0; q < R; q++) {
+            const int row = row0[q] + tid;
+            diag[q] = (T)0;
+            L[q] = ebase[q] = 0;
 #pragma unroll
-            for (int k = 0; k < 3; k++) state_of(f, k) = (T)0;
-        if (run) {
-            if (in) {
+            for (int k = 0; k < 3; k++) {
+                r[q][k] = w[q][k] = (T)0;
+                if (!kWide) u[q][k] = (T)0;
+#pragma unroll
+                for (int f = 0; f < 4; f++) state_of(q, f, k) = (T)0;
+            }
+            if (kWide) put_u<kVec>(su, q * MAXT + tid, (T)0, (T)0, (T)0);
+            if (run && in[q]) {
                 const size_t o = 3 * (size_t)row;
 #pragma unroll
                 for (int k = 0; k < 3; k++) {
-                    r[k] = static_cast<const T *>(d.r)[o + k];
-                    state_of(1, k) = static_cast<const T *>(d.dinv)[o + k];
+                    r[q][k] = static_cast<const T *>(d.r)[o + k];
+                    state_of(q, 1, k) = static_cast<const T *>(d.dinv)[o + k];
                 }
             }
-            if (valid) {
-                diag = nomass ? (T)(s_bp.calc_stokes == 1 ? d.drag[row] : 0.0)
-                                  : static_cast<const T *>(d.mass_diag)[row];
-                L = d.slice_len[row >> 5];
-                ebase = d.slice_ptr[row >> 5] + (row & 31);
+            if (run && valid[q]) {
+                diag[q] = nomass ? (T)(s_bp.calc_stokes == 1 ? d.drag[row] : 0.0)
+                                 : static_cast<const T *>(d.mass_diag)[row];
+                L[q] = d.slice_len[row >> 5];
+                ebase[q] = d.slice_ptr[row >> 5] + (row & 31);
             }
         }
         // the row's neighbours (places in su) and matrix values on chip:
         // constant during the solve
-        if (run && valid) {
-            uint16_t *col = dyn<uint16_t>(gb.o_col) + tid;
-#pragma unroll 1
-            for (int j = 0; j < min(gb.cache_cols, L); j++) col[j * MAXT] = gb.lcol[ebase + 32 * j];
-            T *kv1 = dyn<T>(gb.o_kv1) + tid;
-            T2 *kv2 = dyn<T2>(gb.o_kv2) + tid;
-#pragma unroll 1
-            for (int i = 0; i < min(gb.cache_slots, L); i++) {
-                const int e = ebase + 32 * i;
-                if (nomass) {
-                    const T *val = static_cast<const T *>(d.sell_val) + sell_vidx(e, 0);
+        int T0[R], T1[R];  // the slots in tensor memory, the same for the warp
 #pragma unroll
-                    for (int m = 0; m < 4; m++) {
-                        T2 kp;
-                        kp.x = val[32 * (2 * m)];
-                        kp.y = val[32 * (2 * m + 1)];
-                        kv2[(4 * i + m) * MAXT] = kp;
-                    }
-                    kv1[i * MAXT] = val[32 * 8];
-                } else {
-                    kv1[i * MAXT] = static_cast<const T *>(d.sell_mval)[e];
-                }
-            }
-        }
-        int T0 = 0, T1 = 0;  // the slots in tensor memory, the same for the warp
-        if constexpr (kTmem) {
-            if (run && nomass && warp < nsl) {
-                const int Lw = d.slice_len[(row0 >> 5) + warp];
-                // every other warp of a scheduler keeps its last slots there,
-                // so that half of the warps read L2 while the others do not
-                T0 = min(gb.cache_slots, Lw);
-                if (warp & 4) T0 = max(T0, min(gb.cache_cols, Lw) - gb.tmem_slots);
-                T1 = min(T0 + gb.tmem_slots, min(gb.cache_cols, Lw));
-                __syncwarp();
+        for (int q = 0; q < R; q++) {
+            if (run && valid[q]) {
+                uint16_t *col = dyn<uint16_t>(gb.o_col) + q * gb.cache_cols * MAXT + tid;
 #pragma unroll 1
-                for (int j = T0; j < T1; j++) {
-                    const T *val = static_cast<const T *>(d.sell_val) + sell_vidx(ebase + 32 * j, 0);
-                    uint32_t v[kBlockWords];
+                for (int j = 0; j < min(gb.cache_cols, L[q]); j++) col[j * MAXT] = gb.lcol[ebase[q] + 32 * j];
+                T *kv1 = dyn<T>(gb.o_kv1) + q * gb.cache_slots * MAXT + tid;
+                T2 *kv2 = dyn<T2>(gb.o_kv2) + q * 4 * gb.cache_slots * MAXT + tid;
+#pragma unroll 1
+                for (int i = 0; i < min(gb.cache_slots, L[q]); i++) {
+                    const int e = ebase[q] + 32 * i;
+                    if (nomass) {
+                        const T *val = static_cast<const T *>(d.sell_val) + sell_vidx(e, 0);
 #pragma unroll
-                    for (int k = 0; k < 9; k++) {
-                        const T x = valid ? val[32 * k] : (T)0;
-                        if constexpr (fast) {
-                            v[k] = __float_as_uint(x);
-                        } else {
-                            v[2 * k] = (uint32_t)__double2loint(x);
-                            v[2 * k + 1] = (uint32_t)__double2hiint(x);
+                        for (int m = 0; m < 4; m++) {
+                            T2 kp;
+                            kp.x = val[32 * (2 * m)];
+                            kp.y = val[32 * (2 * m + 1)];
+                            kv2[(4 * i + m) * MAXT] = kp;
                         }
+                        kv1[i * MAXT] = val[32 * 8];
+                    } else {
+                        kv1[i * MAXT] = static_cast<const T *>(d.sell_mval)[e];
                     }
-                    tmem_put(tmem + (j - T0) * kBlockWords, v);
                 }
-                tmem_put_done();
             }
+            T0[q] = T1[q] = 0;
+            if constexpr (kTmem) {
+                if (run && nomass && warp < nsl[q]) {
+                    const int Lw = d.slice_len[(row0[q] >> 5) + warp];
+                    // every other warp of a scheduler keeps its last slots there,
+                    // so that half of the warps read L2 while the others do not
+                    T0[q] = min(gb.cache_slots, Lw);
+                    if (warp & 4) T0[q] = max(T0[q], min(gb.cache_cols, Lw) - gb.tmem_slots);
+                    T1[q] = min(T0[q] + gb.tmem_slots, min(gb.cache_cols, Lw));
+                    __syncwarp();
+#pragma unroll 1
+                    for (int j = T0[q]; j < T1[q]; j++) {
+                        const T *val = static_cast<const T *>(d.sell_val) + sell_vidx(ebase[q] + 32 * j, 0);
+                        uint32_t v[kBlockWords];
+#pragma unroll
+                        for (int k = 0; k < 9; k++) {
+                            const T x = valid[q] ? val[32 * k] : (T)0;
+                            if constexpr (fast) {
+                                v[k] = __float_as_uint(x);
+                            } else {
+                                v[2 * k] = (uint32_t)__double2loint(x);
+                                v[2 * k + 1] = (uint32_t)__double2hiint(x);
+                            }
+                        }
+                        tmem_put(tmem + (q * gb.tmem_slots + j - T0[q]) * kBlockWords, v);
+                    }
+                    tmem_put_done();
+                }
+            }
+            if (COARSE && !kWide && run && in[q])
+                dyn<float4>(gb.o_phi)[tid] = valid[q] ? d.phi[row0[q] + tid] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        if (COARSE && run && in)
-            dyn<float4>(gb.o_phi)[tid] = valid ? d.phi[row] : make_float4(0.f, 0.f, 0.f, 0.f);
         if (run) {
             int *halo = dyn<int>(gb.o_halo);
 #pragma unroll 1
             for (int k = tid; k < nh; k += NT) halo[k] = gb.halo[h0 + k];
             if (COARSE) {
-                const float *Xg = d.coarse_X + s_bp.coarse_xoff + (size_t)(6 * (seg - s_bp.seg_off)) * cn;
-                float *xr = dyn<float>(gb.o_xrow), *h = dyn<float>(gb.o_h);
+                float *h = dyn<float>(gb.o_h);
+                if (!kWide) {
+                    const float *Xg = d.coarse_X + s_bp.coarse_xoff + (size_t)(6 * (seg - s_bp.seg_off)) * cn;
+                    float *xr = dyn<float>(gb.o_xrow);
 #pragma unroll 1
-                for (int k = tid; k < 6 * cn; k += NT) xr[k] = Xg[k];
+                    for (int k = tid; k < 6 * cn; k += NT) xr[k] = Xg[k];
+                }
 #pragma unroll 1
                 for (int k = tid; k < cn; k += NT) h[k] = 0.f;
             }
 #pragma unroll 1
-            for (int k = tid; k < 3 * 32; k += NT) s_dot[k] = 0.0;
+            for (int k = tid; k < R * 3 * 32; k += NT) s_dots[0][k] = 0.0;
 #pragma unroll 1
-            for (int k = tid; k < 12 * 32; k += NT) s_res[k] = 0.f;
+            for (int k = tid; k < R * 12 * 32; k += NT) s_ress[0][k] = 0.f;
         }
         __syncthreads();
 
@@ -548,74 +616,87 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
             const uint32_t tag = base + ++seq;
             const bool verify = state == CG_VERIFY;
             const bool product = !verify && !first_coarse;
-            if (product) {
-                // phase A: p = u + beta p; s = w + beta s; x += alpha p;
-                // r -= alpha s; u = M r; publish u
-                T a, be;
-                cg_coefs<T>(s_cg, a, be);
-                if (valid) {
-                    if (!fresh) {
-                        const bool first = be == (T)0;
-#pragma unroll
-                        for (int k = 0; k < 3; k++) {
-                            T &p = state_of(2, k), &s = state_of(3, k);
-                            const T pn = first ? u[k] : u[k] + be * p;
-                            const T sn = first ? w[k] : w[k] + be * s;
-                            p = pn;
-                            s = sn;
-                            state_of(0, k) += a * pn;
-                            r[k] -= a * sn;
-                        }
-                    }
-                    T dinv[3];
-#pragma unroll
-                    for (int k = 0; k < 3; k++) dinv[k] = state_of(1, k);
-                    if (COARSE) {
-                        coarse_u_of<T>(dyn<float4>(gb.o_phi)[tid], s_cvec, dinv, r, u);
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < 3; k++) u[k] = dinv[k] * r[k];
-                    }
-                }
-                if (in) {
-                    if (!solo) Row::put(pub, d.nl_pad, row, u, tag);
-#pragma unroll
-                    for (int k = 0; k < 3; k++) su[4 * tid + k] = u[k];
-                }
-            } else if (verify) {
-                // publish x for the true residual
-                if (in) {
-                    const T xv[3] = {state_of(0, 0), state_of(0, 1), state_of(0, 2)};
-                    if (!solo) Row::put(pub, d.nl_pad, row, xv, tag);
-#pragma unroll
-                    for (int k = 0; k < 3; k++) su[4 * tid + k] = xv[k];
-                }
-            }
             // the row's terms of r.u and r.r and its restriction of r, and
             // their slice sums (a slice is a warp)
-            T pg = (T)0, pr = (T)0;
-            float ex[6] = {0, 0, 0, 0, 0, 0};
-            if (valid && product)
+            T pg[R], pr[R];
+            float ex[R][6];
 #pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    pg += r[k] * u[k];
-                    pr += r[k] * r[k];
-                }
-            if (COARSE && valid && !verify) restrict6_of<T>(dyn<float4>(gb.o_phi)[tid], r, ex);
-            if constexpr (fast) {
+            for (int q = 0; q < R; q++) {
+                double *s_dot = s_dots[q];
+                float *s_res = s_ress[q];
+                const int me = q * MAXT + tid;  // the row's place in su
+                T uq[3];
+#pragma unroll
+                for (int k = 0; k < 3; k++) uq[k] = kWide ? su[4 * me + k] : u[kWide ? 0 : q][k];
                 if (product) {
-                    constexpr int NV = COARSE ? 8 : 2;
-                    float v[NV];
-                    v[0] = (float)pg;
-                    v[1] = (float)pr;
-                    if (COARSE)
+                    // phase A: p = u + beta p; s = w + beta s; x += alpha p;
+                    // r -= alpha s; u = M r; publish u
+                    T a, be;
+                    cg_coefs<T>(s_cg, a, be);
+                    if (valid[q]) {
+                        if (!fresh) {
+                            const bool first = be == (T)0;
 #pragma unroll
-                        for (int k = 0; k < 6; k++) v[2 + k] = ex[k];
-                    int idx;
-                    const float t = warp_sum_multi<NV>(v, idx);
-                                        if ((lane & (32 / NV - 1)) == 0) {
-                        if (idx < 2) reinterpret_cast<float *>(s_dot)[(idx == 0 ? 0 : 2) * 32 + warp] = t;
-                        else s_res[(idx - 2) * 32 + warp] = t;
+                            for (int k = 0; k < 3; k++) {
+                                T &p = state_of(q, 2, k), &s = state_of(q, 3, k);
+                                const T pn = first ? uq[k] : uq[k] + be * p;
+                                const T sn = first ? w[q][k] : w[q][k] + be * s;
+                                p = pn;
+                                s = sn;
+                                state_of(q, 0, k) += a * pn;
+                                r[q][k] -= a * sn;
+                            }
+                        }
+                        T dinv[3];
+#pragma unroll
+                        for (int k = 0; k < 3; k++) dinv[k] = state_of(q, 1, k);
+                        if (COARSE) {
+                            coarse_u_of<T>(phi_of(q), s_cvec[q], dinv, r[q], uq);
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < 3; k++) uq[k] = dinv[k] * r[q][k];
+                        }
+                    }
+                    if (in[q]) {
+                        if (!solo) Row::put(pub, d.nl_pad, row0[q] + tid, uq, tag);
+                        put_u<kVec>(su, me, uq[0], uq[1], uq[2]);
+                    }
+                    if (!kWide)
+#pragma unroll
+                        for (int k = 0; k < 3; k++) u[kWide ? 0 : q][k] = uq[k];
+                } else if (verify) {
+                    // publish x for the true residual
+                    if (in[q]) {
+                        const T xv[3] = {state_of(q, 0, 0), state_of(q, 0, 1), state_of(q, 0, 2)};
+                        if (!solo) Row::put(pub, d.nl_pad, row0[q] + tid, xv, tag);
+                        put_u<kVec>(su, me, xv[0], xv[1], xv[2]);
+                    }
+                }
+                pg[q] = pr[q] = (T)0;
+#pragma unroll
+                for (int k = 0; k < 6; k++) ex[q][k] = 0.f;
+                if (valid[q] && product)
+#pragma unroll
+                    for (int k = 0; k < 3; k++) {
+                        pg[q] += r[q][k] * uq[k];
+                        pr[q] += r[q][k] * r[q][k];
+                    }
+                if (COARSE && valid[q] && !verify) restrict6_of<T>(phi_of(q), r[q], ex[q]);
+                if constexpr (fast) {
+                    if (product) {
+                        constexpr int NV = COARSE ? 8 : 2;
+                        float v[NV];
+                        v[0] = (float)pg[q];
+                        v[1] = (float)pr[q];
+                        if (COARSE)
+#pragma unroll
+                            for (int k = 0; k < 6; k++) v[2 + k] = ex[q][k];
+                        int idx;
+                        const float t = warp_sum_multi<NV>(v, idx);
+                        if ((lane & (32 / NV - 1)) == 0) {
+                            if (idx < 2) reinterpret_cast<float *>(s_dot)[(idx == 0 ? 0 : 2) * 32 + warp] = t;
+                            else s_res[(idx - 2) * 32 + warp] = t;
+                        }
                     }
                 }
             }
@@ -627,10 +708,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
                     Row y;
                     y.get(pub, d.nl_pad, q);
                     if (!y.is(tag)) y = wait_row<T>(pub, d.nl_pad, q, tag, &s_err, d.bar);
-                    T *o = su + 4 * (size_t)(MAXT + k);
-                    o[0] = y.x;
-                    o[1] = y.y;
-                    o[2] = y.z;
+                    put_u<kVec>(su, R * MAXT + k, y.x, y.y, y.z);
                 }
             __syncthreads();  // su
             auto load3 = [&](int q, T y[3]) {
@@ -647,233 +725,267 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
                     y[2] = s[2];
                 }
             };
-            if (product) {
-                // phase B: w = A u
-                T acc[3] = {diag * u[0], diag * u[1], diag * u[2]};
-                // slots on chip, then the others.  Past the last of them a
-                // step takes the row itself with zero values
-                const int JC = gb.cache_cols, J1 = min(gb.cache_slots, L);
-                const uint16_t *col = dyn<uint16_t>(gb.o_col) + tid;
-                const T *kv1 = dyn<T>(gb.o_kv1) + tid;
-                if (nomass) {
-                    const T2 *kv2 = dyn<T2>(gb.o_kv2) + tid;
-                    constexpr int G1 = SlotDepth<T, MAXT>::kOn, G2 = SlotDepth<T, MAXT>::kOff;
-#pragma unroll 1
-                    for (int j0 = 0; j0 < J1; j0 += G1) {
-                        T y[G1][3];
 #pragma unroll
-                        for (int g = 0; g < G1; g++) load3(j0 + g < J1 ? col[(j0 + g) * MAXT] : tid, y[g]);
+            for (int q = 0; q < R; q++) {
+                double *s_dot = s_dots[q];
+                float *s_res = s_ress[q];
+                const int me = q * MAXT + tid;
+                if (product) {
+                    // phase B: w = A u
+                    T uq[3];
+                    if (kWide) {
+                        load3(me, uq);  // (zeros past the segment's rows)
+                    } else {
 #pragma unroll
-                        for (int g = 0; g < G1; g++) {
-                            const int j = j0 + g < J1 ? j0 + g : j0;
-                            T Kj[9];
-#pragma unroll
-                            for (int m = 0; m < 4; m++) {
-                                const T2 kp = kv2[(4 * j + m) * MAXT];
-                                Kj[2 * m] = kp.x;
-                                Kj[2 * m + 1] = kp.y;
-                            }
-                            Kj[8] = kv1[j * MAXT];
-                            // (past the last slot y is u: the products are zeros)
-                            block_fma(Kj, y[g][0] - u[0], y[g][1] - u[1], y[g][2] - u[2], acc[0], acc[1], acc[2]);
-                        }
+                        for (int k = 0; k < 3; k++) uq[k] = u[kWide ? 0 : q][k];
                     }
-                    // values from L2, slots ja .. jb - 1
-                    auto from_l2 = [&](int ja, int jb) {
-                        const T *vp = static_cast<const T *>(d.sell_val) + sell_vidx(ebase + 32 * ja, 0);
+                    T acc[3] = {diag[q] * uq[0], diag[q] * uq[1], diag[q] * uq[2]};
+                    // slots on chip, then the others.  Past the last of them a
+                    // step takes the row itself with zero values
+                    const int JC = gb.cache_cols, J1 = min(gb.cache_slots, L[q]);
+                    const uint16_t *col = dyn<uint16_t>(gb.o_col) + q * gb.cache_cols * MAXT + tid;
+                    const T *kv1 = dyn<T>(gb.o_kv1) + q * gb.cache_slots * MAXT + tid;
+                    if (nomass) {
+                        const T2 *kv2 = dyn<T2>(gb.o_kv2) + q * 4 * gb.cache_slots * MAXT + tid;
+                        constexpr int G1 = SlotDepth<T, MAXT>::kOn, G2 = SlotDepth<T, MAXT>::kOff;
 #pragma unroll 1
-                        for (int j0 = ja; j0 < jb; j0 += G2, vp += 288 * G2) {
-                            T Kj[G2][9];
+                        for (int j0 = 0; j0 < J1; j0 += G1) {
+                            T y[G1][3];
 #pragma unroll
-                            for (int g = 0; g < G2; g++)
+                            for (int g = 0; g < G1; g++) load3(j0 + g < J1 ? col[(j0 + g) * MAXT] : me, y[g]);
 #pragma unroll
-                                for (int k = 0; k < 9; k++)
-                                    Kj[g][k] = j0 + g < jb ? __ldg(vp + 288 * g + 32 * k) : (T)0;
+                            for (int g = 0; g < G1; g++) {
+                                const int j = j0 + g < J1 ? j0 + g : j0;
+                                T Kj[9];
 #pragma unroll
-                            for (int g = 0; g < G2; g++) {
-                                const int j = j0 + g;
-                                T y[3];
-                                load3(j >= jb ? tid : j < JC ? col[j * MAXT] : __ldg(&gb.lcol[ebase + 32 * j]), y);
-                                block_fma(Kj[g], y[0] - u[0], y[1] - u[1], y[2] - u[2], acc[0], acc[1], acc[2]);
+                                for (int m = 0; m < 4; m++) {
+                                    const T2 kp = kv2[(4 * j + m) * MAXT];
+                                    Kj[2 * m] = kp.x;
+                                    Kj[2 * m + 1] = kp.y;
+                                }
+                                Kj[8] = kv1[j * MAXT];
+                                // (past the last slot y is u: the products are zeros)
+                                block_fma(Kj, y[g][0] - uq[0], y[g][1] - uq[1], y[g][2] - uq[2], acc[0], acc[1],
+                                          acc[2]);
                             }
                         }
-                    };
-                    if constexpr (kTmem) {
-                        constexpr int GT = sizeof(T) == 4 ? 2 : 1;
-                        constexpr int W = GT * kBlockWords;
+                        // values from L2, slots ja .. jb - 1
+                        auto from_l2 = [&](int ja, int jb) {
+                            const T *vp = static_cast<const T *>(d.sell_val) + sell_vidx(ebase[q] + 32 * ja, 0);
 #pragma unroll 1
-                        for (int pass = 0; pass < 2; pass++) {
-                            from_l2(pass == 0 ? J1 : max(J1, min(T1, L)), pass == 0 ? min(T0, L) : L);
-                            if (pass > 0) break;
-                            __syncwarp();
-                            int j = T0;
-#pragma unroll 1
-                            for (; j + GT <= T1; j += GT) {
-                                uint32_t v[W];
-                                T y[GT][3];
+                            for (int j0 = ja; j0 < jb; j0 += G2, vp += 288 * G2) {
+                                T Kj[G2][9];
 #pragma unroll
-                                for (int g = 0; g < GT; g++) load3(j + g < L ? col[(j + g) * MAXT] : tid, y[g]);
-                                tmem_get(tmem + (j - T0) * kBlockWords, v);
+                                for (int g = 0; g < G2; g++)
 #pragma unroll
-                                for (int g = 0; g < GT; g++) {
-                                    T Kj[9];
+                                    for (int k = 0; k < 9; k++)
+                                        Kj[g][k] = j0 + g >= jb ? (T)0
+                                                   : kWide      ? ld_stream(vp + 288 * g + 32 * k, pol)
+                                                                : __ldg(vp + 288 * g + 32 * k);
 #pragma unroll
-                                    for (int k = 0; k < 9; k++) Kj[k] = word_at<T>(v + g * kBlockWords, k);
-                                    block_fma(Kj, y[g][0] - u[0], y[g][1] - u[1], y[g][2] - u[2], acc[0], acc[1],
-                                              acc[2]);
+                                for (int g = 0; g < G2; g++) {
+                                    const int j = j0 + g;
+                                    T y[3];
+                                    load3(j >= jb  ? me
+                                          : j < JC ? col[j * MAXT]
+                                                   : __ldg(&gb.lcol[ebase[q] + 32 * j]),
+                                          y);
+                                    block_fma(Kj[g], y[0] - uq[0], y[1] - uq[1], y[2] - uq[2], acc[0], acc[1], acc[2]);
                                 }
                             }
-                            if (GT > 1 && j < T1) {
-                                uint32_t v[kBlockWords];
-                                T y[3], Kj[9];
-                                load3(j < L ? col[j * MAXT] : tid, y);
-                                tmem_get(tmem + (j - T0) * kBlockWords, v);
+                        };
+                        if constexpr (kTmem) {
+                            constexpr int GT = sizeof(T) == 4 ? 2 : 1;
+                            constexpr int W = GT * kBlockWords;
+#pragma unroll 1
+                            for (int pass = 0; pass < 2; pass++) {
+                                const int ja = pass == 0 ? J1 : max(J1, min(T1[q], L[q]));
+                                from_l2(ja, pass == 0 ? min(T0[q], L[q]) : L[q]);
+                                if (pass > 0) break;
+                                __syncwarp();
+                                int j = T0[q];
+#pragma unroll 1
+                                for (; j + GT <= T1[q]; j += GT) {
+                                    uint32_t v[W];
+                                    T y[GT][3];
 #pragma unroll
-                                for (int k = 0; k < 9; k++) Kj[k] = word_at<T>(v, k);
-                                block_fma(Kj, y[0] - u[0], y[1] - u[1], y[2] - u[2], acc[0], acc[1], acc[2]);
+                                    for (int g = 0; g < GT; g++) load3(j + g < L[q] ? col[(j + g) * MAXT] : me, y[g]);
+                                    tmem_get(tmem + (q * gb.tmem_slots + j - T0[q]) * kBlockWords, v);
+#pragma unroll
+                                    for (int g = 0; g < GT; g++) {
+                                        T Kj[9];
+#pragma unroll
+                                        for (int k = 0; k < 9; k++) Kj[k] = word_at<T>(v + g * kBlockWords, k);
+                                        block_fma(Kj, y[g][0] - uq[0], y[g][1] - uq[1], y[g][2] - uq[2], acc[0], acc[1],
+                                                  acc[2]);
+                                    }
+                                }
+                                if (GT > 1 && j < T1[q]) {
+                                    uint32_t v[kBlockWords];
+                                    T y[3], Kj[9];
+                                    load3(j < L[q] ? col[j * MAXT] : me, y);
+                                    tmem_get(tmem + (q * gb.tmem_slots + j - T0[q]) * kBlockWords, v);
+#pragma unroll
+                                    for (int k = 0; k < 9; k++) Kj[k] = word_at<T>(v, k);
+                                    block_fma(Kj, y[0] - uq[0], y[1] - uq[1], y[2] - uq[2], acc[0], acc[1], acc[2]);
+                                }
                             }
+                        } else {
+                            from_l2(J1, L[q]);
                         }
                     } else {
-                        from_l2(J1, L);
-                    }
-                } else {
-                    const T *mv = static_cast<const T *>(d.sell_mval);
+                        const T *mv = static_cast<const T *>(d.sell_mval);
 #pragma unroll 2
-                    for (int j = 0; j < L; j++) {
-                        T y[3];
-                        load3(j < JC ? col[j * MAXT] : __ldg(&gb.lcol[ebase + 32 * j]), y);
-                        const T m = j < J1 ? kv1[j * MAXT] : __ldg(&mv[ebase + 32 * j]);
+                        for (int j = 0; j < L[q]; j++) {
+                            T y[3];
+                            load3(j < JC ? col[j * MAXT] : __ldg(&gb.lcol[ebase[q] + 32 * j]), y);
+                            const T m = j < J1 ? kv1[j * MAXT] : __ldg(&mv[ebase[q] + 32 * j]);
 #pragma unroll
-                        for (int k = 0; k < 3; k++) acc[k] = fma(m, y[k], acc[k]);
+                            for (int k = 0; k < 3; k++) acc[k] = fma(m, y[k], acc[k]);
+                        }
                     }
-                }
-                T pd = (T)0;
-                if (valid)
-#pragma unroll
-                    for (int k = 0; k < 3; k++) {
-                        w[k] = acc[k];
-                        pd += w[k] * u[k];
-                    }
-                                if constexpr (fast) {
-                    float ew[6] = {0, 0, 0, 0, 0, 0};
-                    if (COARSE && valid) restrict6_of<T>(dyn<float4>(gb.o_phi)[tid], w, ew);
-                    constexpr int NV = COARSE ? 8 : 2;
-                    float v[NV];
-                    v[0] = (float)pd;
-                    v[1] = 0.f;
-                    if (COARSE)
-#pragma unroll
-                        for (int k = 0; k < 6; k++) v[2 + k] = ew[k];
-                    int idx;
-                    const float t = warp_sum_multi<NV>(v, idx);
-                    if ((lane & (32 / NV - 1)) == 0) {
-                        if (idx == 0) reinterpret_cast<float *>(s_dot)[1 * 32 + warp] = t;
-                        else if (idx >= 2) s_res[(6 + idx - 2) * 32 + warp] = t;
-                    }
-                } else {
-                    T v[4] = {pg, pd, pr, (T)0}, t = (T)0;
-                    int idx = lane >> 3;
-                    if (warp < nsl) t = warp_sum_multi<4>(v, idx);
-                    if ((lane & 7) == 0 && idx < 3) reinterpret_cast<T *>(s_dot)[idx * 32 + warp] = t;
-                }
-            } else {
-                // the FP64 true residual b - A x of the published x becomes r
-                // (VERIFY), or the restriction of r_0 alone.
-                double vr = 0.0, vg = 0.0;
-                if (verify) {
-                    double a[3] = {0.0, 0.0, 0.0};
-                    if (valid) {
-                        const T *xr = su + 4 * (size_t)tid;
-#pragma unroll
-                        for (int k = 0; k < 3; k++) a[k] = (double)diag * (double)xr[k];
-                        add_residual_slots(a, static_cast<const T *>(nomass ? d.sell_val : d.sell_mval), gb.lcol,
-                                              su, xr, ebase, 0, L, nomass);
-                    }
-                    if (valid) {
-                        const size_t o = 3 * (size_t)(row);
+                    T pd = (T)0;
+                    if (valid[q])
 #pragma unroll
                         for (int k = 0; k < 3; k++) {
-                            const double rt = d.rhs[o + k] - a[k];
-                            r[k] = (T)rt;
-                            const T uk = state_of(1, k) * r[k];
-                            vr += rt * rt;
-                            vg += (double)r[k] * (double)uk;
+                            w[q][k] = acc[k];
+                            pd += w[q][k] * uq[k];
                         }
-                        if (COARSE) restrict6_of<T>(dyn<float4>(gb.o_phi)[tid], r, ex);
-                    }
-                    vg = warp_sum<double>(vg);
-                    vr = warp_sum<double>(vr);
-                }
-                                if (lane == 0) {
-                    s_dot[0 * 32 + warp] = vg;
-                    s_dot[1 * 32 + warp] = 0.0;
-                    s_dot[2 * 32 + warp] = vr;
-                }
-                if (COARSE) {
+                    if constexpr (fast) {
+                        float ew[6] = {0, 0, 0, 0, 0, 0};
+                        if (COARSE && valid[q]) restrict6_of<T>(phi_of(q), w[q], ew);
+                        constexpr int NV = COARSE ? 8 : 2;
+                        float v[NV];
+                        v[0] = (float)pd;
+                        v[1] = 0.f;
+                        if (COARSE)
 #pragma unroll
-                    for (int k = 0; k < 6; k++) {
-                        const float t = warp_sum<float>(ex[k]);
-                        if (lane == 0) {
-                            s_res[k * 32 + warp] = t;
-                            s_res[(6 + k) * 32 + warp] = 0.f;
+                            for (int k = 0; k < 6; k++) v[2 + k] = ew[k];
+                        int idx;
+                        const float t = warp_sum_multi<NV>(v, idx);
+                        if ((lane & (32 / NV - 1)) == 0) {
+                            if (idx == 0) reinterpret_cast<float *>(s_dot)[1 * 32 + warp] = t;
+                            else if (idx >= 2) s_res[(6 + idx - 2) * 32 + warp] = t;
+                        }
+                    } else {
+                        T v[4] = {pg[q], pd, pr[q], (T)0}, t = (T)0;
+                        int idx = lane >> 3;
+                        if (warp < nsl[q]) t = warp_sum_multi<4>(v, idx);
+                        if ((lane & 7) == 0 && idx < 3) reinterpret_cast<T *>(s_dot)[idx * 32 + warp] = t;
+                    }
+                } else {
+                    // the FP64 true residual b - A x of the published x becomes r
+                    // (VERIFY), or the restriction of r_0 alone.
+                    double vr = 0.0, vg = 0.0;
+                    if (verify) {
+                        double a[3] = {0.0, 0.0, 0.0};
+                        if (valid[q]) {
+                            const T *xr = su + 4 * (size_t)me;
+#pragma unroll
+                            for (int k = 0; k < 3; k++) a[k] = (double)diag[q] * (double)xr[k];
+                            add_residual_slots(a, static_cast<const T *>(nomass ? d.sell_val : d.sell_mval), gb.lcol,
+                                                  su, xr, ebase[q], 0, L[q], nomass);
+                        }
+                        if (valid[q]) {
+                            const size_t o = 3 * (size_t)(row0[q] + tid);
+#pragma unroll
+                            for (int k = 0; k < 3; k++) {
+                                const double rt = d.rhs[o + k] - a[k];
+                                r[q][k] = (T)rt;
+                                const T uk = state_of(q, 1, k) * r[q][k];
+                                vr += rt * rt;
+                                vg += (double)r[q][k] * (double)uk;
+                            }
+                            if (COARSE) restrict6_of<T>(phi_of(q), r[q], ex[q]);
+                        }
+                        vg = warp_sum<double>(vg);
+                        vr = warp_sum<double>(vr);
+                    }
+                    if (lane == 0) {
+                        s_dot[0 * 32 + warp] = vg;
+                        s_dot[1 * 32 + warp] = 0.0;
+                        s_dot[2 * 32 + warp] = vr;
+                    }
+                    if (COARSE) {
+#pragma unroll
+                        for (int k = 0; k < 6; k++) {
+                            const float t = warp_sum<float>(ex[q][k]);
+                            if (lane == 0) {
+                                s_res[k * 32 + warp] = t;
+                                s_res[(6 + k) * 32 + warp] = 0.f;
+                            }
                         }
                     }
                 }
             }
             __syncthreads();  // the slices' sums
             // butterflies as wide as the slices need
-            const int half = nsl > 1 ? 1 << (31 - __clz(nsl - 1)) : 0;
-            // The segment's sums over its slices into s_out: warp q < 3 dot
-            // term q (hi, lo), warps 3..6 three values each of P^T r, P^T w
-            if (warp < 3) {
-                float hi, lo;
-                if (sizeof(T) == 8 || !product) {
-                    double a = lane < nsl ? s_dot[warp * 32 + lane] : 0.0;
+            const int most = max(nsl[0], nsl[R - 1]);
+            const int half = most > 1 ? 1 << (31 - __clz(most - 1)) : 0;
+            // A segment's sums over its slices into s_outs: warps 0..2 a dot
+            // term each (hi, lo), warps 3..6 three values each of P^T r, P^T w
+            auto combine = [&](int q, int l) {
+                const int n = R == 1 || q == 0 ? nsl[0] : nsl[R - 1];
+                float *s_out = s_outs[q];
+                if (l < 3) {
+                    float hi, lo;
+                    if (sizeof(T) == 8 || !product) {
+                        double a = lane < n ? s_dots[q][l * 32 + lane] : 0.0;
 #pragma unroll
-                    for (int k = 16; k > 0; k >>= 1)
-                        if (k <= half) a += __shfl_xor_sync(0xffffffffu, a, k);
-                    hi = (float)a;
-                    lo = (float)(a - (double)hi);
-                } else {
-                    DF v{lane < nsl ? reinterpret_cast<const float *>(s_dot)[warp * 32 + lane] : 0.f, 0.f};
+                        for (int k = 16; k > 0; k >>= 1)
+                            if (k <= half) a += __shfl_xor_sync(0xffffffffu, a, k);
+                        hi = (float)a;
+                        lo = (float)(a - (double)hi);
+                    } else {
+                        DF v{lane < n ? reinterpret_cast<const float *>(s_dots[q])[l * 32 + lane] : 0.f, 0.f};
+#pragma unroll
+                        for (int k = 16; k > 0; k >>= 1)
+                            if (k <= half)
+                                v = df_add(v, DF{__shfl_xor_sync(0xffffffffu, v.hi, k),
+                                                 __shfl_xor_sync(0xffffffffu, v.lo, k)});
+                        hi = v.hi;
+                        lo = v.lo;
+                    }
+                    if (lane == 0) {
+                        s_out[2 * l] = hi;
+                        s_out[2 * l + 1] = lo;
+                    }
+                } else if (COARSE) {
+                    const int k0 = 3 * (l - 3);
+                    float v[3];
+#pragma unroll
+                    for (int c = 0; c < 3; c++) v[c] = lane < n ? s_ress[q][(k0 + c) * 32 + lane] : 0.f;
 #pragma unroll
                     for (int k = 16; k > 0; k >>= 1)
                         if (k <= half)
-                            v = df_add(v, DF{__shfl_xor_sync(0xffffffffu, v.hi, k), __shfl_xor_sync(0xffffffffu, v.lo, k)});
-                    hi = v.hi;
-                    lo = v.lo;
+#pragma unroll
+                            for (int c = 0; c < 3; c++) v[c] += __shfl_xor_sync(0xffffffffu, v[c], k);
+                    if (lane == 0)
+#pragma unroll
+                        for (int c = 0; c < 3; c++) s_out[6 + k0 + c] = v[c];
                 }
-                if (lane == 0) {
-                    s_out[2 * warp] = hi;
-                    s_out[2 * warp + 1] = lo;
-                }
-            } else if (COARSE && warp < 7) {
-                const int k0 = 3 * (warp - 3);
-                float v[3];
-#pragma unroll
-                for (int q = 0; q < 3; q++) v[q] = lane < nsl ? s_res[(k0 + q) * 32 + lane] : 0.f;
-#pragma unroll
-                for (int k = 16; k > 0; k >>= 1)
-                    if (k <= half)
-#pragma unroll
-                        for (int q = 0; q < 3; q++) v[q] += __shfl_xor_sync(0xffffffffu, v[q], k);
-                if (lane == 0)
-#pragma unroll
-                    for (int q = 0; q < 3; q++) s_out[6 + k0 + q] = v[q];
+            };
+            if constexpr (R == 1) {
+                if (warp < 7) combine(0, warp);
+            } else {
+#pragma unroll 1
+                for (int k = warp; k < 7 * R; k += nw) combine(k / 7, k % 7);
             }
-            __syncthreads();  // s_out
+            __syncthreads();  // s_outs
             // published in whole 32-byte sectors by one store: words 0, 1 the
             // dot terms, 2..5 P^T r and P^T w, three values each
             uint4 *const dots = gb.words + (size_t)parity * 2 * d.n_segs;
             uint4 *const rest = gb.words + (size_t)4 * d.n_segs + (size_t)parity * 4 * d.n_segs;
             float *const swr = dyn<float>(gb.o_words), *const sww = swr + 6 * cnt;  // the group's P^T r and P^T w
-            if (warp == 0 && lane < (COARSE ? 6 : 2)) {
-                const float a = s_out[3 * lane], b2 = s_out[3 * lane + 1], c = s_out[3 * lane + 2];
+            const int pq = R == 1 ? 0 : lane >> 3, l = R == 1 ? lane : lane & 7;
+            if (warp == 0 && l < (COARSE ? 6 : 2) && (pq == 0 || (pq < R && nsl[R - 1] > 0))) {
+                const int q = R == 1 ? 0 : pq;
+                const float a = s_outs[q][3 * l], b2 = s_outs[q][3 * l + 1], c = s_outs[q][3 * l + 2];
                 if (!solo) {
-                    uint4 *o = lane < 2 ? dots + 2 * (size_t)seg + lane : rest + 4 * (size_t)seg + lane - 2;
+                    uint4 *o = l < 2 ? dots + 2 * (size_t)(seg + q) + l : rest + 4 * (size_t)(seg + q) + l - 2;
                     st_b128(o, pack2(__float_as_uint(a), __float_as_uint(b2)), pack2(__float_as_uint(c), tag));
-                } else if (lane >= 2) {
-                    float *o = swr + 3 * (lane - 2);  // (sww follows: one segment)
+                } else if (l >= 2) {
+                    float *o = swr + 3 * (l - 2);  // (sww follows: one segment)
                     o[0] = a;
                     o[1] = b2;
                     o[2] = c;
@@ -887,7 +999,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
                 if (solo) {
                     if (lane == 0)
 #pragma unroll
-                        for (int q = 0; q < 3; q++) sum[q] = DF{s_out[2 * q], s_out[2 * q + 1]};
+                        for (int q = 0; q < 3; q++) sum[q] = DF{s_outs[0][2 * q], s_outs[0][2 * q + 1]};
                 } else if (sg < cnt) {
                     uint64_t lo[2], hi[2];
                     wait_words<2>(dots + 2 * (size_t)(s_bp.seg_off + sg), 1, 2, tag, lo, hi, &s_err, d.bar);
@@ -909,15 +1021,20 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
             }
             __syncthreads();  // sw
             if (warp == 0) {
+                // a lane for each sum over the parts
+                DF sum{0.f, 0.f};
+                if (lane < 3) {
+                    sum = s_part[lane];
+                    for (int k = 1; 32 * k < cnt; k++) sum = df_add(sum, s_part[3 * k + lane]);
+                }
+                DF sums[3];
+#pragma unroll
+                for (int q = 0; q < 3; q++)
+                    sums[q] = DF{__shfl_sync(0xffffffffu, sum.hi, q), __shfl_sync(0xffffffffu, sum.lo, q)};
                 if (lane == 0) {
                     if (!first_coarse) {
-                        DF sums[3];
 #pragma unroll
-                        for (int q = 0; q < 3; q++) {
-                            sums[q] = s_part[q];
-                            for (int k = 1; 32 * k < cnt; k++) sums[q] = df_add(sums[q], s_part[3 * k + q]);
-                            s_last[q] = sums[q];
-                        }
+                        for (int q = 0; q < 3; q++) s_last[q] = sums[q];
                         int bits;
                         if (!(fast && transition_on(s_cg, limit, sums)) &&
                             transition_any(&s_cg, &s_bp, s_last, &bits, fast) && bits && leader)
@@ -953,26 +1070,36 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
                 // restart P^T r itself), c = X g for the CTA's segment
                 const bool restart = first_coarse || nst == CG_RESTART;
                 float *h = dyn<float>(gb.o_h);
-                const float *xr = dyn<float>(gb.o_xrow);
                 const float al = s_cg.alpha_f, be = s_cg.beta_f;
-                float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll 2
-                for (int j = tid; j < cn; j += NT) {
-                    const float pr_j = swr[j];
-                    const float hn = restart ? 0.f : sww[j] + be * h[j];
-                    h[j] = hn;
-                    const float g = restart ? pr_j : pr_j - al * hn;
 #pragma unroll
-                    for (int l = 0; l < 6; l++) v[l] = fmaf(xr[l * cn + j], g, v[l]);
+                for (int q = 0; q < R; q++) {
+                    const float *xr = dyn<float>(gb.o_xrow);
+                    if (kWide)
+                        xr = d.coarse_X + s_bp.coarse_xoff +
+                             (size_t)(6 * (seg - s_bp.seg_off + (nsl[q] > 0 ? q : 0))) * cn;
+                    float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 2
+                    for (int j = tid; j < cn; j += NT) {
+                        const float pr_j = swr[j];
+                        float hn = h[j];
+                        if (q == 0) {
+                            hn = restart ? 0.f : sww[j] + be * hn;
+                            h[j] = hn;
+                        }
+                        const float g = restart ? pr_j : pr_j - al * hn;
+#pragma unroll
+                        for (int l = 0; l < 6; l++) v[l] = fmaf(xr[l * cn + j], g, v[l]);
+                    }
+                    int idx;
+                    const float t = warp_sum_multi<8>(v, idx);
+                    if ((lane & 3) == 0 && idx < 6) s_red6[q][idx * 32 + warp] = t;
                 }
-                int idx;
-                const float t = warp_sum_multi<8>(v, idx);
-                if ((lane & 3) == 0 && idx < 6) s_red6[idx * 32 + warp] = t;
                 __syncthreads();
 #pragma unroll 1
-                for (int l = warp; l < 6; l += nw) {
-                    const float c = warp_sum<float>(lane < nw ? s_red6[l * 32 + lane] : 0.f);
-                    if (lane == 0) s_cvec[l] = c;
+                for (int l = warp; l < 6 * R; l += nw) {
+                    const int q = R == 1 ? 0 : l / 6, k = l - 6 * q;
+                    const float c = warp_sum<float>(lane < nw ? s_red6[q][k * 32 + lane] : 0.f);
+                    if (lane == 0) s_cvec[q][k] = c;
                 }
                 __syncthreads();  // s_cvec
             }
@@ -989,15 +1116,19 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
         const bool err = run && s_stop;
         const bool move = d.cg_euler && !err && s_cg.state == CG_CONVERGED && __ldcg(&d.status[b]) == 0;
         const double dt = s_bp.dt;
-        if (run && in) {
 #pragma unroll
-            for (int k = 0; k < 3; k++) static_cast<T *>(d.x)[3 * (size_t)row + k] = state_of(0, k);
-        }
-        if (move && in && row - s_bp.node_off < s_bp.node_cnt) {
+        for (int q = 0; q < R; q++) {
+            if (!in[q]) continue;
+            const int row = row0[q] + tid;
+            if (run) {
+#pragma unroll
+                for (int k = 0; k < 3; k++) static_cast<T *>(d.x)[3 * (size_t)row + k] = state_of(q, 0, k);
+            }
+            if (!move || row - s_bp.node_off >= s_bp.node_cnt) continue;
 #pragma unroll
             for (int k = 0; k < 3; k++) {
                 const size_t kk = 3 * (size_t)row + k;
-                const double xi = run ? (double)state_of(0, k) : (double)static_cast<const T *>(d.x)[kk];
+                const double xi = run ? (double)state_of(q, 0, k) : (double)static_cast<const T *>(d.x)[kk];
                 double pn;
                 if (nomass) {
                     d.vel[kk] = xi;
@@ -1053,19 +1184,21 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
     }
 }
 
-// The variant by the rows of a CTA (the longest segment).
+// The variant by the rows of a segment (the longest) and the segments of a CTA.
 template <typename T, bool COARSE>
-const void *kernel_for(int rows)
+const void *kernel_for(const GroupBatch &g)
 {
-    if (rows <= 256) return reinterpret_cast<const void *>(&k_cg_group<T, COARSE, 256>);
-    if (rows <= 512) return reinterpret_cast<const void *>(&k_cg_group<T, COARSE, 512>);
-    return reinterpret_cast<const void *>(&k_cg_group<T, COARSE, 1024>);
+    if constexpr (sizeof(T) == 4)
+        if (g.per > 1) return reinterpret_cast<const void *>(&k_cg_group<T, COARSE, 1024, 2>);
+    if (g.rows <= 256) return reinterpret_cast<const void *>(&k_cg_group<T, COARSE, 256, 1>);
+    if (g.rows <= 512) return reinterpret_cast<const void *>(&k_cg_group<T, COARSE, 512, 1>);
+    return reinterpret_cast<const void *>(&k_cg_group<T, COARSE, 1024, 1>);
 }
 
 const void *group_kernel(const DeviceBatch &d, const GroupBatch &g)
 {
-    if (d.precision == PREC_FP64) return kernel_for<double, false>(g.rows);
-    return d.coarse ? kernel_for<float, true>(g.rows) : kernel_for<float, false>(g.rows);
+    if (d.precision == PREC_FP64) return kernel_for<double, false>(g);
+    return d.coarse ? kernel_for<float, true>(g) : kernel_for<float, false>(g);
 }
 
 }  // namespace
@@ -1074,15 +1207,19 @@ int cg_group_plan(const DeviceBatch &d, GroupBatch &g, int max_slots, int max_co
                   int max_segs)
 {
     const bool f64 = d.precision == PREC_FP64;
-    g.rows = max_rows <= 256 ? 256 : max_rows <= 512 ? 512 : 1024;  // the variant's MAXT
-    g.threads = std::max(256, (max_rows + 31) / 32 * 32);
+    if (g.per > 1 && f64) return -1;
+    g.rows = g.per > 1 || max_rows > 512 ? 1024 : max_rows > 256 ? 512 : 256;  // the variant's MAXT
+    // (a lane for each segment whose sums are waited for)
+    g.threads = std::max({256, (max_rows + 31) / 32 * 32, (max_segs + 31) / 32 * 32});
+    if (g.threads > g.rows) return -1;
     int dev = 0, optin = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return -1;
     const void *fn = group_kernel(d, g);
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, fn) != cudaSuccess) return -1;
-    const size_t R = g.rows, ts = f64 ? 8 : 4;
+    const size_t R = (size_t)g.per * g.rows, ts = f64 ? 8 : 4;
+    const bool wide = g.per > 1;
     const size_t reserve = 1024;  // per-CTA system use
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -1090,13 +1227,13 @@ int cg_group_plan(const DeviceBatch &d, GroupBatch &g, int max_slots, int max_co
         off = (off + bytes + 15) & ~(size_t)15;
         return (int32_t)o;
     };
-    g.o_state = take(R <= 512 ? 0 : 12 * R * ts);
+    g.o_state = take(g.rows <= 512 ? 0 : 12 * R * ts);
     g.o_u = take(4 * (R + max_halo) * ts);
     g.o_halo = take(4 * (size_t)max_halo);
     g.o_words = take(d.coarse ? 48 * (size_t)max_segs : 0);
     if (d.coarse) {
-        g.o_phi = take(16 * R);
-        g.o_xrow = take(24 * (size_t)d.coarse_nmax);
+        g.o_phi = take(wide ? 0 : 16 * R);
+        g.o_xrow = take(wide ? 0 : 24 * (size_t)d.coarse_nmax);
         g.o_h = take(4 * (size_t)d.coarse_nmax);
     }
     const size_t fixed = fa.sharedSizeBytes + reserve + off + 64;
@@ -1115,7 +1252,7 @@ int cg_group_plan(const DeviceBatch &d, GroupBatch &g, int max_slots, int max_co
         // the warps of a quarter of the lanes share its columns.  The places
         // of a block in tensor memory are read from shared memory
         const int warps = (g.threads / 32 + 3) / 4;
-        g.tmem_slots = std::min(kTmemCols / warps / (int)(9 * ts / 4),
+        g.tmem_slots = std::min(kTmemCols / warps / g.per / (int)(9 * ts / 4),
                                 std::min(max_slots, (int)g.cache_cols) - (int)g.cache_slots);
         // a CTA takes all of its SM's tensor memory: no second one beside it
         if (g.tmem_slots > 0) off = std::max<size_t>(off, (size_t)optin / 2 + 1024);

@@ -113,7 +113,8 @@ struct DeviceBatch {
 // task[ptr[c]] .. task[ptr[c + 1] - 1].
 struct GroupBatch {
     int32_t grid = 0, threads = 0;  // launch shape
-    int32_t rows = 0;               // rows a CTA has room for
+    int32_t per = 1;                // segments per CTA (at most)
+    int32_t rows = 0;               // rows of each a CTA has room for
     int32_t dyn_smem = 0;
     int32_t cache_slots = 0;  // matrix slots per row whose values are copied to shared memory
     int32_t tmem_slots = 0;   // matrix slots per row, after those, whose values are copied to tensor memory
@@ -121,7 +122,7 @@ struct GroupBatch {
     int32_t *ptr = nullptr, *task = nullptr;
     // per segment its halo, the rows of other segments it couples to, and per
     // matrix entry its column as a place in the CTA's copy of u: the local
-    // row, or `rows` + its place in the halo
+    // row (the second segment's from `rows` on), or per x rows + its place in the halo
     int32_t *hptr = nullptr, *halo = nullptr;
     uint16_t *lcol = nullptr;
     // exchange: GRP_WORDS words of sums per segment and exchange parity; the

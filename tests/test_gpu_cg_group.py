@@ -101,3 +101,32 @@ def test_blobs_scheduled_in_rounds(gpulib, monkeypatch, radii, max_ctas):
             assert np.array_equal(a, b), i
         assert np.array_equal(g_on[i], g_mem[i])
         assert s_on[i]["fail_bits"] == 0 and s_on[i]["cg_iters"] == s_mem[i]["cg_iters"]
+
+
+# two segments to a CTA: (radii, CTA cap) one CTA with both; four on two CTAs; three (one CTA has a single one)
+# beside a blob of one
+WIDE = [((8.0,), 1), ((10.0,), 2), ((10.0, 3.0), 2)]
+
+
+@pytest.mark.parametrize("radii,max_ctas", WIDE)
+@pytest.mark.parametrize("solver", [P.SOLVER_NOMASS, P.SOLVER_MASS])
+def test_two_segments_to_a_cta_same_bits(gpulib, monkeypatch, radii, max_ctas, solver):
+    specs = [_mixed(r, i + 1, solver=solver, pinned=[0, 7] if i % 2 == 0 else None) for i, r in enumerate(radii)]
+    on, s_on, g_on = _run(monkeypatch, specs, max_ctas, False, true_residual=True)
+    mem, s_mem, g_mem = _run(monkeypatch, specs, max_ctas, True, true_residual=True)
+    for i in range(len(specs)):
+        for a, b in zip(on[i], mem[i]):
+            assert np.array_equal(a, b), i
+        assert np.array_equal(g_on[i], g_mem[i])
+        assert s_on[i]["fail_bits"] == 0 and s_on[i]["cg_iters"] == s_mem[i]["cg_iters"]
+        assert s_on[i]["true_relres"] == pytest.approx(s_mem[i]["true_relres"], rel=1e-12)
+
+
+@pytest.mark.parametrize("radii,max_ctas", WIDE)
+def test_two_segments_to_a_cta_two_level(gpulib, monkeypatch, radii, max_ctas):
+    specs = [_mixed(r, i + 1) for i, r in enumerate(radii)]
+    _, st, _ = _run(monkeypatch, specs, max_ctas, False, true_residual=True, preconditioner=1)
+    _, s_mem, _ = _run(monkeypatch, specs, max_ctas, True, true_residual=True, preconditioner=1)
+    for s, m in zip(st, s_mem):
+        assert s["fail_bits"] == 0 and s["true_relres"] < 1e-6, s
+        assert abs(s["cg_iters"] - m["cg_iters"]) <= 1
