@@ -721,7 +721,7 @@ int ffea_gpu_create_batch(int32_t num_blobs, const ffea_gpu_mesh *meshes, const 
     CK(A.alloc_bytes(d.sell_mval, H.any_mass ? (size_t)d.n_entries * ts : 16));
     CK(A.alloc_bytes(d.mass_diag, H.any_mass ? (size_t)H.nl_pad * ts : 16));
     if (H.any_lumped) CK(A.alloc(d.lumped_inv, (size_t)H.nl_pad));
-    CK(A.alloc(d.partials, std::max(4 * (size_t)H.n_tiles, (size_t)d.part_stride * n_segs)));
+    CK(A.alloc(d.partials, std::max(2 * (size_t)NODE_PARTS * H.n_tiles, (size_t)d.part_stride * n_segs)));
     if (d.coarse) {
         CK(upload(A, d.seg_of_row, H.seg_of_row));
         CK(upload(A, d.seg_nbr_ptr, H.seg_nbr_ptr));

@@ -572,21 +572,46 @@ __global__ void k_lumped_mass(DeviceBatch d)
     d.lumped_inv[i] = 1.0 / s;
 }
 
+// Sums of two FP64 values over a warp: the lower half of the lanes ends with
+// the sum of a, the upper half with that of b (five additions, not ten: an
+// FP64 instruction takes 64 issue slots on GB300 however few lanes it has).
+__device__ __forceinline__ double warp_sum_pair(double a, double b)
+{
+    const bool up = threadIdx.x & 16;
+    double v = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 // Node kernel: rhs and the CG start (for a lumped-mass blob the solve
 // itself, x = M_lumped^-1 f, MassLumpedSolver::solve src/MassLumpedSolver.cpp:81-89).
+//
+// Bound by latency (three chains of dependent loads: a row's element forces,
+// its folded noise, its diagonal) and by the FP64 pipe.  With 256 rows to a
+// CTA a 437-node blob ran on two SMs, 32 warps of FP64 work on each, and the
+// chains went one load at a time: 20 us; 64 rows to a CTA and the loads of
+// kNodeBatch entries in flight together take 13, and 61 where a
+// 40 nm sphere (146,737 nodes) took 67.
+constexpr int kNodeRows = 64;     // rows per CTA
+constexpr int kNodeBatch = 8;     // entries whose loads are in flight together
+constexpr int kNodeBlobs = 64;    // blobs whose sums the last CTA finishes at a time
+static_assert(NODE_TILE % kNodeRows == 0 && NODE_TILE / kNodeRows == NODE_PARTS, "partial sums of a tile");
+
 template <typename T>
-__global__ void __launch_bounds__(NODE_TILE * NODE_LANES) k_nodes(DeviceBatch d, int use_given_rhs)
+__global__ void __launch_bounds__(kNodeRows * NODE_LANES) k_nodes(DeviceBatch d, int use_given_rhs)
 {
     // NODE_LANES lanes per row: the lanes split the row's gather list
     // (entries q, q + NODE_LANES, ...), combine their partial sums in a fixed
     // order, then lanes 0..2 each finish one component.
     static_assert(NODE_LANES == 4, "the combine below is a two-step butterfly");
-    __shared__ double red[2 * 32];
-    const int tile = blockIdx.x;
-    const int b = d.tile_blob[tile];
+    constexpr int NW = kNodeRows * NODE_LANES / 32;
+    __shared__ double red[2][NW];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int b = d.tile_blob[blockIdx.x / NODE_PARTS];
     const BlobParams &bp = d.bp[b];
-    const int q = threadIdx.x & (NODE_LANES - 1);
-    const int row = tile * NODE_TILE + threadIdx.x / NODE_LANES;
+    const int q = tid & (NODE_LANES - 1);
+    const int row = blockIdx.x * kNodeRows + tid / NODE_LANES;
     const int local = row - bp.node_off;
     const bool failed = d.status[b] != 0;
     const bool valid = local < bp.node_cnt && !(d.flags[row] & NODE_PINNED) && !failed;
@@ -601,24 +626,34 @@ __global__ void __launch_bounds__(NODE_TILE * NODE_LANES) k_nodes(DeviceBatch d,
             for (int i = 0; i < 3; i++) fs[i].add_d(d.ext[3 * (size_t)row + i]);
         }
         const T *ef = static_cast<const T *>(d.efrc);
-#pragma unroll 2
-        for (int k = d.gather_ptr[row] + q; k < d.gather_ptr[row + 1]; k += NODE_LANES) {
-            const int gi = d.gather_idx[k];  // (element << 2) | corner: the corner's 4-vector
-            T f[3];
-            if (sizeof(T) == 4) {
-                const float4 v = __ldg(reinterpret_cast<const float4 *>(ef) + gi);
-                f[0] = (T)v.x;
-                f[1] = (T)v.y;
-                f[2] = (T)v.z;
-            } else {
-                const double2 v0 = __ldg(reinterpret_cast<const double2 *>(ef) + 2 * (size_t)gi);
-                const double2 v1 = __ldg(reinterpret_cast<const double2 *>(ef) + 2 * (size_t)gi + 1);
-                f[0] = (T)v0.x;
-                f[1] = (T)v0.y;
-                f[2] = (T)v1.x;
+        const int end = d.gather_ptr[row + 1];
+        for (int k0 = d.gather_ptr[row] + q; k0 < end; k0 += kNodeBatch * NODE_LANES) {
+            int gi[kNodeBatch];  // (element << 2) | corner: the corner's 4-vector
+            T f[kNodeBatch][3];
+#pragma unroll
+            for (int u = 0; u < kNodeBatch; u++)
+                gi[u] = k0 + u * NODE_LANES < end ? d.gather_idx[k0 + u * NODE_LANES] : -1;
+#pragma unroll
+            for (int u = 0; u < kNodeBatch; u++) {
+                if (gi[u] < 0) continue;
+                if (sizeof(T) == 4) {
+                    const float4 v = __ldg(reinterpret_cast<const float4 *>(ef) + gi[u]);
+                    f[u][0] = (T)v.x;
+                    f[u][1] = (T)v.y;
+                    f[u][2] = (T)v.z;
+                } else {
+                    const double2 v0 = __ldg(reinterpret_cast<const double2 *>(ef) + 2 * (size_t)gi[u]);
+                    const double2 v1 = __ldg(reinterpret_cast<const double2 *>(ef) + 2 * (size_t)gi[u] + 1);
+                    f[u][0] = (T)v0.x;
+                    f[u][1] = (T)v0.y;
+                    f[u][2] = (T)v1.x;
+                }
             }
 #pragma unroll
-            for (int i = 0; i < 3; i++) fs[i].add(f[i]);
+            for (int u = 0; u < kNodeBatch; u++)
+                if (gi[u] >= 0)
+#pragma unroll
+                    for (int i = 0; i < 3; i++) fs[i].add(f[u][i]);
         }
     }
     // (lane 0 + lane 1) + (lane 2 + lane 3), the lower lane's partial first,
@@ -645,28 +680,55 @@ __global__ void __launch_bounds__(NODE_TILE * NODE_LANES) k_nodes(DeviceBatch d,
             // draws from k_noise, amplitudes sqrt((24 kT drag) / dt) set up once
             const T *nz = static_cast<const T *>(d.node_noise) + 3 * (size_t)bp.noise_node_off;
             const T *na = static_cast<const T *>(d.node_amp), *fa = static_cast<const T *>(d.fold_amp);
-            if (drag != 0.0) fc.add(-(nz[3 * (size_t)d.orig[row] + c] * na[row]));
+            if (__double_as_longlong(drag) << 1 != 0) fc.add(-(nz[3 * (size_t)d.orig[row] + c] * na[row]));
             // secondary nodes with a drag: half of their force lands here
-            for (int k = d.fold_ptr[row]; k < d.fold_ptr[row + 1]; k++)
-                fc.add((T)0.5 * (-(nz[3 * (size_t)d.fold_sec[k] + c] * fa[k])));
+            const int end = d.fold_ptr[row + 1];
+            for (int k0 = d.fold_ptr[row]; k0 < end; k0 += kNodeBatch) {
+                int sec[kNodeBatch];
+                T z[kNodeBatch], amp[kNodeBatch];
+#pragma unroll
+                for (int u = 0; u < kNodeBatch; u++) {
+                    sec[u] = k0 + u < end ? d.fold_sec[k0 + u] : -1;
+                    if (k0 + u < end) amp[u] = fa[k0 + u];
+                }
+#pragma unroll
+                for (int u = 0; u < kNodeBatch; u++)
+                    if (sec[u] >= 0) z[u] = nz[3 * (size_t)sec[u] + c];
+#pragma unroll
+                for (int u = 0; u < kNodeBatch; u++)
+                    if (sec[u] >= 0) fc.add((T)0.5 * (-(z[u] * amp[u])));
+            }
         }
     }
     double f = fc.value();
     if (use_given_rhs && valid) f = d.rhs[3 * (size_t)row + c];
     const bool store = q < 3;
     T *dinv = static_cast<T *>(d.dinv);
-    if (nomass && store) {
+    T Dinv = (T)1;
+    if (nomass) {
         // Jacobi diagonal of component c: zeta_p - sum_q K_pq[c][c] over the
         // row's assembled blocks (padding slots hold zeros).  The viscosity
         // diagonal block is minus the sum of the row's off-diagonal blocks,
         // as the gradients of a linear element's shape functions sum to zero.
-        T Dc = (T)0;
-        if (valid) {
-            const int sl = row >> 5, L = d.slice_len[sl], base = d.slice_ptr[sl] + (row & 31);
-            const T *val = static_cast<const T *>(d.sell_val);
-            for (int j = 0; j < L; j++) Dc -= val[sell_vidx(base + 32 * j, 4 * c)];
+        if (store) {
+            T Dc = (T)0;
+            if (valid) {
+                const int sl = row >> 5, L = d.slice_len[sl], base = d.slice_ptr[sl] + (row & 31);
+                const T *val = static_cast<const T *>(d.sell_val);
+                for (int j0 = 0; j0 < L; j0 += kNodeBatch) {
+                    T v[kNodeBatch];
+#pragma unroll
+                    for (int u = 0; u < kNodeBatch; u++)
+                        v[u] = j0 + u < L ? val[sell_vidx(base + 32 * (j0 + u), 4 * c)] : (T)0;
+#pragma unroll
+                    for (int u = 0; u < kNodeBatch; u++) Dc -= v[u];
+                }
+            }
+            Dinv = valid ? (T)1 / (Dc + (T)drag) : (T)1;
+            dinv[3 * (size_t)row + c] = Dinv;
         }
-        dinv[3 * (size_t)row + c] = valid ? (T)1 / (Dc + (T)drag) : (T)1;
+    } else {
+        Dinv = dinv[3 * (size_t)row + c];
     }
     // CG start: x = 0, r = f, u = D^-1 r, w = s = p = 0
     T *x = static_cast<T *>(d.x), *r = static_cast<T *>(d.r), *u = static_cast<T *>(d.u);
@@ -678,7 +740,7 @@ __global__ void __launch_bounds__(NODE_TILE * NODE_LANES) k_nodes(DeviceBatch d,
         const double fi = valid ? f : 0.0;
         if (!use_given_rhs) d.rhs[k] = fi;
         const T ri = (T)fi;
-        const T ui = dinv[k] * ri;
+        const T ui = Dinv * ri;
         x[k] = lumped ? (T)(fi * d.lumped_inv[row]) : (T)0;
         r[k] = ri;
         if (!d.group) {  // k_cg_group starts from r and D^-1 alone
@@ -690,28 +752,43 @@ __global__ void __launch_bounds__(NODE_TILE * NODE_LANES) k_nodes(DeviceBatch d,
         gam = (double)ri * (double)ui;
         ff = fi * fi;
     }
-    const double in[2] = {gam, ff};
-    double sums[2];
-    block_sum<2, double>(in, sums, red);
-    if (threadIdx.x == 0) {
-        d.partials[4 * (size_t)tile] = sums[0];
-        d.partials[4 * (size_t)tile + 1] = sums[1];
+    const double sum = warp_sum_pair(gam, ff);
+    if ((lane & 15) == 0) red[lane >> 4][warp] = sum;
+    __syncthreads();
+    if (warp == 0) {
+        double v = lane < 2 * NW ? red[lane / NW][lane % NW] : 0.0;
+#pragma unroll
+        for (int o = NW / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane % NW == 0 && lane < 2 * NW) d.partials[2 * (size_t)blockIdx.x + lane / NW] = v;
     }
     if (last_block(&d.counters[CNT_NODES], gridDim.x)) {
+        // the blobs' sums: all warps on each of a few blobs, or a warp per blob
         __shared__ unsigned int running;
-        if (threadIdx.x == 0) running = 0;
-        __syncthreads();
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        for (int bb = warp; bb < d.num_blobs; bb += nw) {
-            const int t0 = d.bp[bb].tile_off, tc = d.bp[bb].tile_cnt;
-            double s0 = 0.0, s1 = 0.0;
-            for (int t = lane; t < tc; t += 32) {
-                s0 += __ldcg(&d.partials[4 * (size_t)(t0 + t)]);
-                s1 += __ldcg(&d.partials[4 * (size_t)(t0 + t) + 1]);
+        __shared__ double tot[2][kNodeBlobs][NW];
+        if (tid == 0) running = 0;
+        const int nb = d.num_blobs;
+        const int share = nb >= NW ? 1 : nb > NW / 2 ? 1 : nb > NW / 4 ? 2 : nb > 1 ? 4 : NW;  // warps per blob
+        for (int b0 = 0; b0 < nb; b0 += kNodeBlobs) {
+            const int n = min(kNodeBlobs, nb - b0), part = warp % share;
+            for (int i = warp / share; i < n; i += NW / share) {
+                const int t0 = NODE_PARTS * d.bp[b0 + i].tile_off, tc = NODE_PARTS * d.bp[b0 + i].tile_cnt;
+                double s0 = 0.0, s1 = 0.0;
+                for (int t = 32 * part + lane; t < tc; t += 32 * share) {
+                    const double2 v = __ldcg(reinterpret_cast<const double2 *>(d.partials) + t0 + t);
+                    s0 += v.x;
+                    s1 += v.y;
+                }
+                const double s = warp_sum_pair(s0, s1);
+                if ((lane & 15) == 0) tot[lane >> 4][i][part] = s;
             }
-            s0 = warp_sum<double>(s0);
-            s1 = warp_sum<double>(s1);
-            if (lane == 0) {
+            __syncthreads();
+            if (tid < n) {
+                const int bb = b0 + tid;
+                double s0 = tot[0][tid][0], s1 = tot[1][tid][0];
+                for (int k = 1; k < share; k++) {
+                    s0 += tot[0][tid][k];
+                    s1 += tot[1][tid][k];
+                }
                 CgScalars &cg = d.cg[bb];
                 cg.gamma = s0;
                 cg.ff = s1;
@@ -728,9 +805,9 @@ __global__ void __launch_bounds__(NODE_TILE * NODE_LANES) k_nodes(DeviceBatch d,
                 cg.state = done ? CG_CONVERGED : CG_ACTIVE;
                 if (!done) atomicAdd(&running, 1u);
             }
+            __syncthreads();
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
+        if (tid == 0) {
             d.bar[0] = 0;          // arrival count
             d.bar[2] = running;    // blobs still iterating
             d.bar[3] = running;
@@ -2317,7 +2394,7 @@ void launch_noise(const DeviceBatch &d, cudaStream_t s)
 
 void launch_nodes(const DeviceBatch &d, cudaStream_t s, int use_given_rhs)
 {
-    PREC_DISPATCH(d, k_nodes, d.n_tiles, NODE_TILE * NODE_LANES, s, d, use_given_rhs);
+    PREC_DISPATCH(d, k_nodes, NODE_PARTS * d.n_tiles, kNodeRows * NODE_LANES, s, d, use_given_rhs);
 }
 
 // Dynamic shared memory of the memory-resident CG kernel with the coarse

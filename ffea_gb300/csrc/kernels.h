@@ -93,7 +93,7 @@ struct DeviceBatch {
     void *sell_mval = nullptr;    // mass matrix: 1 T per entry
     void *mass_diag = nullptr;    // T per node
     // reductions / status
-    double *partials = nullptr;     // 4 per node tile (node kernel); CG: two buffers of part_stride floats per segment
+    double *partials = nullptr;     // 2 per CTA of the node kernel; CG: two buffers of part_stride floats per segment
     CgScalars *cg = nullptr;        // per blob
     double *last_sums = nullptr;    // per blob: r.u, w.u, r.r of the last reduction (written by CTA 0)
     unsigned int *counters = nullptr;  // one per reduction site

@@ -130,3 +130,21 @@ def test_two_segments_to_a_cta_two_level(gpulib, monkeypatch, radii, max_ctas):
     for s, m in zip(st, s_mem):
         assert s["fail_bits"] == 0 and s["true_relres"] < 1e-6, s
         assert abs(s["cg_iters"] - m["cg_iters"]) <= 1
+
+
+@pytest.mark.parametrize("blobs", [2, 3, 5, 9, 65])
+def test_start_sums_of_batches(gpulib, oracle, blobs):
+    """r.u and f.f of every blob come from the last CTA of k_nodes: all its
+    warps on one blob, four or two warps a blob, a warp per blob, and more
+    blobs than it finishes at a time; FP64 steps against the oracle."""
+    from ffea_gb300.world import World
+    specs = [spec(radius_nm=3.0 + 0.25 * (i % 5), seed=i + 1, rng_seed=40 + i) for i in range(blobs)]
+    with World(specs) as w:
+        w.run(2)
+        for i in sorted({0, 1, blobs // 2, blobs - 2, blobs - 1}):
+            ref = oracle.blob_from_spec(specs[i])
+            assert ref.step(2) == 0 and w.blob(i).status()["fail_bits"] == 0
+            pos, vel, _ = ref.nodes()
+            on = w.blob(i).get_nodes()
+            assert np.linalg.norm(on[1] - vel) <= 1e-9 * np.linalg.norm(vel), i
+            assert np.abs(on[0] - pos).max() < 1e-10, i
