@@ -306,6 +306,33 @@ __device__ __forceinline__ bool transition_on(CgScalars &cg, int limit, const DF
     return true;
 }
 
+// The same in FP64, run by a warp (lane q < 3 with sum q): the conversions of
+// the sums on a lane each and two of the four divisions on two lanes at once
+// (a division takes nine times an instruction's 64 issue slots).
+__device__ __forceinline__ bool transition_on64(CgScalars &cg, const BlobParams &bp, int limit, DF mine)
+{
+    const int lane = threadIdx.x & 31;
+    const double v = (double)mine.hi + (double)mine.lo;
+    const double g = __shfl_sync(0xffffffffu, v, 0), dl = __shfl_sync(0xffffffffu, v, 1),
+                 rr = __shfl_sync(0xffffffffu, v, 2);
+    const int iters = cg.iters;
+    const double ff = cg.ff, gamma = cg.gamma, alpha = cg.alpha;
+    if (cg.state != CG_ACTIVE || iters == 0 || iters >= limit || ff == 0.0) return false;
+    const double t = (lane == 0 ? rr : g) / (lane == 0 ? ff : gamma);
+    const double res = __shfl_sync(0xffffffffu, t, 0), beta = __shfl_sync(0xffffffffu, t, 1);
+    if (!(res >= bp.epsilon2) || !(g == g) || !(dl == dl)) return false;  // (a NaN res too)
+    const double an = g / (dl - beta * g / alpha);
+    __syncwarp();
+    if (lane == 0) {
+        cg.rr = rr;
+        cg.alpha = an;
+        cg.beta = beta;
+        cg.gamma = g;
+        cg.iters = iters + 1;
+    }
+    return true;
+}
+
 // Matrix slots per step of the product: values on chip, and values from L2 (9
 // registers in flight each).
 template <typename T, int MAXT> struct SlotDepth { static constexpr int kOn = 4, kOff = 4; };
@@ -432,6 +459,14 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
     __shared__ uint32_t s_tmem;
     constexpr bool kTmem = MAXT > 256;
     constexpr int kBlockWords = 9 * (int)sizeof(T) / 4;
+    // FP64 products run in quarters of a slice, dealt over the CTA's warps,
+    // where whole slices would leave some of the four schedulers idle: an FP64
+    // instruction takes 64 issue slots, so the 160 of a row's product took a
+    // warp 17 thousand clocks (two slices a CTA), its quarters 9 on eight warps
+    constexpr bool kSplit = sizeof(T) == 8 && MAXT == 256;
+    constexpr int kSplitRows = kSplit ? 192 : 1;
+    __shared__ T s_acc[kSplit ? 3 : 1][3][kSplitRows];
+    __shared__ int s_rowL[kSplitRows], s_rowE[kSplitRows];  // slots and first entry of a row
     const int tid = threadIdx.x, NT = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = NT >> 5;
     const uint32_t base = __ldcg(&d.bar[6]);  // the tags of this launch start above it
     T *const sx = dyn<T>(gb.o_state);         // per segment x | D^-1 | p | s, 3 MAXT each (unless kRegs)
@@ -523,6 +558,10 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
         }
         // the row's neighbours (places in su) and matrix values on chip:
         // constant during the solve
+        if (kSplit && tid < kSplitRows) {
+            s_rowL[kSplit ? tid : 0] = L[0];
+            s_rowE[kSplit ? tid : 0] = ebase[0];
+        }
         int T0[R], T1[R];  // the slots in tensor memory, the same for the warp
 #pragma unroll
         for (int q = 0; q < R; q++) {
@@ -740,108 +779,166 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
                         for (int k = 0; k < 3; k++) uq[k] = u[kWide ? 0 : q][k];
                     }
                     T acc[3] = {diag[q] * uq[0], diag[q] * uq[1], diag[q] * uq[2]};
-                    // slots on chip, then the others.  Past the last of them a
-                    // step takes the row itself with zero values
-                    const int JC = gb.cache_cols, J1 = min(gb.cache_slots, L[q]);
-                    const uint16_t *col = dyn<uint16_t>(gb.o_col) + q * gb.cache_cols * MAXT + tid;
-                    const T *kv1 = dyn<T>(gb.o_kv1) + q * gb.cache_slots * MAXT + tid;
-                    if (nomass) {
-                        const T2 *kv2 = dyn<T2>(gb.o_kv2) + q * 4 * gb.cache_slots * MAXT + tid;
-                        constexpr int G1 = SlotDepth<T, MAXT>::kOn, G2 = SlotDepth<T, MAXT>::kOff;
+                    bool split = false;
+                    if constexpr (kSplit) split = (nsl[0] & 3) != 0 && 32 * nsl[0] <= kSplitRows;
+                    if (kSplit && split) {
 #pragma unroll 1
-                        for (int j0 = 0; j0 < J1; j0 += G1) {
-                            T y[G1][3];
+                        for (int item = warp; item < 4 * nsl[0]; item += nw) {
+                            const int part = item / nsl[0], hr = 32 * (item % nsl[0]) + lane;
+                            const int Lr = s_rowL[kSplit ? hr : 0], er = s_rowE[kSplit ? hr : 0];
+                            const uint16_t *col = dyn<uint16_t>(gb.o_col) + hr;
+                            const T *kv1 = dyn<T>(gb.o_kv1) + hr;
+                            const T2 *kv2 = dyn<T2>(gb.o_kv2) + hr;
+                            T uh[3], sum[3] = {0, 0, 0};
+                            load3(hr, uh);
+#pragma unroll 2
+                            for (int j = part; j < Lr; j += 4) {
+                                const int e = er + 32 * j;
+                                const bool on = j < gb.cache_slots;
+                                T y[3];
+                                load3(j < gb.cache_cols ? col[j * MAXT] : __ldg(&gb.lcol[e]), y);
+                                if (nomass) {
+                                    T Kj[9];
+                                    if (on) {
 #pragma unroll
-                            for (int g = 0; g < G1; g++) load3(j0 + g < J1 ? col[(j0 + g) * MAXT] : me, y[g]);
+                                        for (int m = 0; m < 4; m++) {
+                                            const T2 kp = kv2[(4 * j + m) * MAXT];
+                                            Kj[2 * m] = kp.x;
+                                            Kj[2 * m + 1] = kp.y;
+                                        }
+                                        Kj[8] = kv1[j * MAXT];
+                                    } else {
+                                        const T *vp = static_cast<const T *>(d.sell_val) + sell_vidx(e, 0);
 #pragma unroll
-                            for (int g = 0; g < G1; g++) {
-                                const int j = j0 + g < J1 ? j0 + g : j0;
-                                T Kj[9];
+                                        for (int k = 0; k < 9; k++) Kj[k] = __ldg(vp + 32 * k);
+                                    }
+                                    block_fma(Kj, y[0] - uh[0], y[1] - uh[1], y[2] - uh[2], sum[0], sum[1], sum[2]);
+                                } else {
+                                    const T m = on ? kv1[j * MAXT] : __ldg(static_cast<const T *>(d.sell_mval) + e);
 #pragma unroll
-                                for (int m = 0; m < 4; m++) {
-                                    const T2 kp = kv2[(4 * j + m) * MAXT];
-                                    Kj[2 * m] = kp.x;
-                                    Kj[2 * m + 1] = kp.y;
+                                    for (int k = 0; k < 3; k++) sum[k] = fma(m, y[k], sum[k]);
                                 }
-                                Kj[8] = kv1[j * MAXT];
-                                // (past the last slot y is u: the products are zeros)
-                                block_fma(Kj, y[g][0] - uq[0], y[g][1] - uq[1], y[g][2] - uq[2], acc[0], acc[1],
-                                          acc[2]);
+                            }
+                            // (the first quarter of a slice is its own warp's)
+#pragma unroll
+                            for (int k = 0; k < 3; k++) {
+                                if (part > 0) s_acc[kSplit ? part - 1 : 0][k][kSplit ? hr : 0] = sum[k];
+                                else acc[k] += sum[k];
                             }
                         }
-                        // values from L2, slots ja .. jb - 1
-                        auto from_l2 = [&](int ja, int jb) {
-                            const T *vp = static_cast<const T *>(d.sell_val) + sell_vidx(ebase[q] + 32 * ja, 0);
+                        __syncthreads();  // s_acc
+                        if (valid[q])
+#pragma unroll
+                            for (int k = 0; k < 3; k++)
+                                acc[k] = (acc[k] + s_acc[0][k][kSplit ? tid : 0]) +
+                                         (s_acc[kSplit ? 1 : 0][k][kSplit ? tid : 0] +
+                                          s_acc[kSplit ? 2 : 0][k][kSplit ? tid : 0]);
+                    } else {
+                        // slots on chip, then the others.  Past the last of them a
+                        // step takes the row itself with zero values
+                        const int JC = gb.cache_cols, J1 = min(gb.cache_slots, L[q]);
+                        const uint16_t *col = dyn<uint16_t>(gb.o_col) + q * gb.cache_cols * MAXT + tid;
+                        const T *kv1 = dyn<T>(gb.o_kv1) + q * gb.cache_slots * MAXT + tid;
+                        if (nomass) {
+                            const T2 *kv2 = dyn<T2>(gb.o_kv2) + q * 4 * gb.cache_slots * MAXT + tid;
+                            constexpr int G1 = SlotDepth<T, MAXT>::kOn, G2 = SlotDepth<T, MAXT>::kOff;
 #pragma unroll 1
-                            for (int j0 = ja; j0 < jb; j0 += G2, vp += 288 * G2) {
-                                T Kj[G2][9];
+                            for (int j0 = 0; j0 < J1; j0 += G1) {
+                                T y[G1][3];
 #pragma unroll
-                                for (int g = 0; g < G2; g++)
+                                for (int g = 0; g < G1; g++) load3(j0 + g < J1 ? col[(j0 + g) * MAXT] : me, y[g]);
 #pragma unroll
-                                    for (int k = 0; k < 9; k++)
-                                        Kj[g][k] = j0 + g >= jb ? (T)0
-                                                   : kWide      ? ld_stream(vp + 288 * g + 32 * k, pol)
-                                                                : __ldg(vp + 288 * g + 32 * k);
+                                for (int g = 0; g < G1; g++) {
+                                    const int j = j0 + g < J1 ? j0 + g : j0;
+                                    T Kj[9];
 #pragma unroll
-                                for (int g = 0; g < G2; g++) {
-                                    const int j = j0 + g;
-                                    T y[3];
-                                    load3(j >= jb  ? me
-                                          : j < JC ? col[j * MAXT]
-                                                   : __ldg(&gb.lcol[ebase[q] + 32 * j]),
-                                          y);
-                                    block_fma(Kj[g], y[0] - uq[0], y[1] - uq[1], y[2] - uq[2], acc[0], acc[1], acc[2]);
+                                    for (int m = 0; m < 4; m++) {
+                                        const T2 kp = kv2[(4 * j + m) * MAXT];
+                                        Kj[2 * m] = kp.x;
+                                        Kj[2 * m + 1] = kp.y;
+                                    }
+                                    Kj[8] = kv1[j * MAXT];
+                                    // (past the last slot y is u: the products are zeros)
+                                    block_fma(Kj, y[g][0] - uq[0], y[g][1] - uq[1], y[g][2] - uq[2], acc[0], acc[1],
+                                              acc[2]);
                                 }
                             }
-                        };
-                        if constexpr (kTmem) {
-                            constexpr int GT = sizeof(T) == 4 ? 2 : 1;
-                            constexpr int W = GT * kBlockWords;
+                            // values from L2, slots ja .. jb - 1
+                            auto from_l2 = [&](int ja, int jb) {
+                                const T *vp = static_cast<const T *>(d.sell_val) + sell_vidx(ebase[q] + 32 * ja, 0);
 #pragma unroll 1
-                            for (int pass = 0; pass < 2; pass++) {
-                                const int ja = pass == 0 ? J1 : max(J1, min(T1[q], L[q]));
-                                from_l2(ja, pass == 0 ? min(T0[q], L[q]) : L[q]);
-                                if (pass > 0) break;
-                                __syncwarp();
-                                int j = T0[q];
-#pragma unroll 1
-                                for (; j + GT <= T1[q]; j += GT) {
-                                    uint32_t v[W];
-                                    T y[GT][3];
+                                for (int j0 = ja; j0 < jb; j0 += G2, vp += 288 * G2) {
+                                    T Kj[G2][9];
 #pragma unroll
-                                    for (int g = 0; g < GT; g++) load3(j + g < L[q] ? col[(j + g) * MAXT] : me, y[g]);
-                                    tmem_get(tmem + (q * gb.tmem_slots + j - T0[q]) * kBlockWords, v);
+                                    for (int g = 0; g < G2; g++)
 #pragma unroll
-                                    for (int g = 0; g < GT; g++) {
-                                        T Kj[9];
+                                        for (int k = 0; k < 9; k++)
+                                            Kj[g][k] = j0 + g >= jb ? (T)0
+                                                       : kWide      ? ld_stream(vp + 288 * g + 32 * k, pol)
+                                                                    : __ldg(vp + 288 * g + 32 * k);
 #pragma unroll
-                                        for (int k = 0; k < 9; k++) Kj[k] = word_at<T>(v + g * kBlockWords, k);
-                                        block_fma(Kj, y[g][0] - uq[0], y[g][1] - uq[1], y[g][2] - uq[2], acc[0], acc[1],
+                                    for (int g = 0; g < G2; g++) {
+                                        const int j = j0 + g;
+                                        T y[3];
+                                        load3(j >= jb  ? me
+                                              : j < JC ? col[j * MAXT]
+                                                       : __ldg(&gb.lcol[ebase[q] + 32 * j]),
+                                              y);
+                                        block_fma(Kj[g], y[0] - uq[0], y[1] - uq[1], y[2] - uq[2], acc[0], acc[1],
                                                   acc[2]);
                                     }
                                 }
-                                if (GT > 1 && j < T1[q]) {
-                                    uint32_t v[kBlockWords];
-                                    T y[3], Kj[9];
-                                    load3(j < L[q] ? col[j * MAXT] : me, y);
-                                    tmem_get(tmem + (q * gb.tmem_slots + j - T0[q]) * kBlockWords, v);
+                            };
+                            if constexpr (kTmem) {
+                                constexpr int GT = sizeof(T) == 4 ? 2 : 1;
+                                constexpr int W = GT * kBlockWords;
+#pragma unroll 1
+                                for (int pass = 0; pass < 2; pass++) {
+                                    const int ja = pass == 0 ? J1 : max(J1, min(T1[q], L[q]));
+                                    from_l2(ja, pass == 0 ? min(T0[q], L[q]) : L[q]);
+                                    if (pass > 0) break;
+                                    __syncwarp();
+                                    int j = T0[q];
+#pragma unroll 1
+                                    for (; j + GT <= T1[q]; j += GT) {
+                                        uint32_t v[W];
+                                        T y[GT][3];
 #pragma unroll
-                                    for (int k = 0; k < 9; k++) Kj[k] = word_at<T>(v, k);
-                                    block_fma(Kj, y[0] - uq[0], y[1] - uq[1], y[2] - uq[2], acc[0], acc[1], acc[2]);
+                                        for (int g = 0; g < GT; g++)
+                                            load3(j + g < L[q] ? col[(j + g) * MAXT] : me, y[g]);
+                                        tmem_get(tmem + (q * gb.tmem_slots + j - T0[q]) * kBlockWords, v);
+#pragma unroll
+                                        for (int g = 0; g < GT; g++) {
+                                            T Kj[9];
+#pragma unroll
+                                            for (int k = 0; k < 9; k++) Kj[k] = word_at<T>(v + g * kBlockWords, k);
+                                            block_fma(Kj, y[g][0] - uq[0], y[g][1] - uq[1], y[g][2] - uq[2], acc[0],
+                                                      acc[1], acc[2]);
+                                        }
+                                    }
+                                    if (GT > 1 && j < T1[q]) {
+                                        uint32_t v[kBlockWords];
+                                        T y[3], Kj[9];
+                                        load3(j < L[q] ? col[j * MAXT] : me, y);
+                                        tmem_get(tmem + (q * gb.tmem_slots + j - T0[q]) * kBlockWords, v);
+#pragma unroll
+                                        for (int k = 0; k < 9; k++) Kj[k] = word_at<T>(v, k);
+                                        block_fma(Kj, y[0] - uq[0], y[1] - uq[1], y[2] - uq[2], acc[0], acc[1], acc[2]);
+                                    }
                                 }
+                            } else {
+                                from_l2(J1, L[q]);
                             }
                         } else {
-                            from_l2(J1, L[q]);
-                        }
-                    } else {
-                        const T *mv = static_cast<const T *>(d.sell_mval);
+                            const T *mv = static_cast<const T *>(d.sell_mval);
 #pragma unroll 2
-                        for (int j = 0; j < L[q]; j++) {
-                            T y[3];
-                            load3(j < JC ? col[j * MAXT] : __ldg(&gb.lcol[ebase[q] + 32 * j]), y);
-                            const T m = j < J1 ? kv1[j * MAXT] : __ldg(&mv[ebase[q] + 32 * j]);
+                            for (int j = 0; j < L[q]; j++) {
+                                T y[3];
+                                load3(j < JC ? col[j * MAXT] : __ldg(&gb.lcol[ebase[q] + 32 * j]), y);
+                                const T m = j < J1 ? kv1[j * MAXT] : __ldg(&mv[ebase[q] + 32 * j]);
 #pragma unroll
-                            for (int k = 0; k < 3; k++) acc[k] = fma(m, y[k], acc[k]);
+                                for (int k = 0; k < 3; k++) acc[k] = fma(m, y[k], acc[k]);
+                            }
                         }
                     }
                     T pd = (T)0;
@@ -1031,12 +1128,14 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
 #pragma unroll
                 for (int q = 0; q < 3; q++)
                     sums[q] = DF{__shfl_sync(0xffffffffu, sum.hi, q), __shfl_sync(0xffffffffu, sum.lo, q)};
+                bool on = false;
+                if constexpr (!fast) on = transition_on64(s_cg, s_bp, limit, sum);
                 if (lane == 0) {
                     if (!first_coarse) {
 #pragma unroll
                         for (int q = 0; q < 3; q++) s_last[q] = sums[q];
                         int bits;
-                        if (!(fast && transition_on(s_cg, limit, sums)) &&
+                        if (!(fast ? transition_on(s_cg, limit, sums) : on) &&
                             transition_any(&s_cg, &s_bp, s_last, &bits, fast) && bits && leader)
                             atomicOr(&d.status[b], bits);
                     }

@@ -148,3 +148,18 @@ def test_start_sums_of_batches(gpulib, oracle, blobs):
             on = w.blob(i).get_nodes()
             assert np.linalg.norm(on[1] - vel) <= 1e-9 * np.linalg.norm(vel), i
             assert np.abs(on[0] - pos).max() < 1e-10, i
+
+
+@pytest.mark.parametrize("radius,max_ctas", [(1.9, 1), (3.0, 2), (3.0, 1), (3.4, 1)])
+@pytest.mark.parametrize("solver", [P.SOLVER_NOMASS, P.SOLVER_MASS])
+def test_fp64_products_in_quarters(gpulib, oracle, monkeypatch, radius, max_ctas, solver):
+    """FP64 segments of one to six slices, whose products run in quarters of a
+    slice over the CTA's warps (not those of four slices), at the tolerances
+    of the test above; the true residual is checked too."""
+    s = spec(radius_nm=radius, seed=3, rng_seed=91, solver=solver, pinned=[1])
+    on, st, _ = _run(monkeypatch, [s], max_ctas, False, true_residual=True)
+    ref = oracle.blob_from_spec(s)
+    assert ref.step(3) == 0 and st[0]["fail_bits"] == 0 and st[0]["true_relres"] < 1e-12
+    pos, vel, _ = ref.nodes()
+    assert np.linalg.norm(on[0][1] - vel) <= 1e-9 * np.linalg.norm(vel)
+    assert np.abs(on[0][0] - pos).max() < 1e-10
