@@ -611,6 +611,26 @@ bool build_batch(int32_t num_blobs, const ffea_gpu_mesh *meshes, const ffea_gpu_
                 else H.edge_pos_qp[e] = off;
             }
         }
+        // edges in the order of their entries in the rows p: k_assemble's
+        // stores of a warp to those rows fill lines
+        std::vector<int32_t> at(H.sell_col.size(), -1), order;
+        for (int32_t e = 0; e < H.n_edges; e++) at[H.edge_pos_pq[e]] = e;
+        order.reserve(H.n_edges);
+        for (int32_t e : at)
+            if (e >= 0) order.push_back(e);
+        std::vector<int32_t> cptr(1, 0), cidx;
+        cidx.reserve(H.edge_cidx.size());
+        for (int32_t e : order) {
+            cidx.insert(cidx.end(), H.edge_cidx.begin() + H.edge_cptr[e], H.edge_cidx.begin() + H.edge_cptr[e + 1]);
+            cptr.push_back((int32_t)cidx.size());
+        }
+        H.edge_cptr.swap(cptr);
+        H.edge_cidx.swap(cidx);
+        for (std::vector<int32_t> *v : {&H.edge_p, &H.edge_q, &H.edge_pos_pq, &H.edge_pos_qp}) {
+            std::vector<int32_t> o(H.n_edges);
+            for (int32_t e = 0; e < H.n_edges; e++) o[e] = (*v)[order[e]];
+            v->swap(o);
+        }
     }
 
     // ---- RNG streams ----------------------------------------------------------------

@@ -38,7 +38,7 @@ struct HostBatch {
     std::vector<int32_t> fold_ptr, fold_sec;              // node -> secondary nodes folded onto it
     std::vector<double> fold_amp;                         // noise amplitude of each folded secondary node
     std::vector<double> node_amp;                         // per padded node: amplitude of its own noise
-    std::vector<int32_t> edge_p, edge_q;                  // edges (p < q), sorted by (p, q)
+    std::vector<int32_t> edge_p, edge_q;                  // edges (p < q), in the order of edge_pos_pq
     std::vector<int32_t> edge_cptr, edge_cidx;            // edge -> (elem*16 + a*4 + b), element order
     // SELL-32 layout of the node-node matrix: slices of 32 consecutive rows,
     // slot j of row r at entry slice_ptr[r/32] + 32*j + r%32, columns ascending
