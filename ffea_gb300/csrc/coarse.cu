@@ -33,7 +33,7 @@ namespace ffea {
 namespace {
 
 constexpr int kAsmThreads = 256;
-constexpr int kAsmParts = CG_SEG_MAX_ROWS / kAsmThreads;  // CTAs per segment, one row per thread
+constexpr int kAsmParts = CG_SEG_MAX_ROWS / kAsmThreads;  // row blocks per segment, one row per thread
 
 // C (6 x 6, row-major) += Phi_p^T K Phi_q for rest offsets dp, dq.
 __device__ __forceinline__ void add_block(float C[36], const float dp[3], const float K[9], const float dq[3])
@@ -103,10 +103,15 @@ __device__ __forceinline__ float warp_sum32_transposed(float (&v)[36])
 // Partial coarse blocks: CTA (s, part) of a NoMass blob's segment s takes
 // rows part * 256 .. part * 256 + 255 of the segment, one row per thread.  A
 // row's slots are sorted by column and segments are contiguous row ranges,
-// so the slots of each coupled segment t form one run: a cursor per row walks
-// them once over the targets.  Each (s, t) block of the CTA's rows is a
-// fixed-order block reduction, written to part slot (k, part) of the
-// segment's neighbour entry k; k_coarse_sum adds the parts in order.
+// so the slots of each coupled segment t form one run.  Each (s, t) block of
+// the CTA's rows is a fixed-order block reduction, written to part slot
+// (k, part) of the segment's neighbour entry k; k_coarse_sum adds the parts
+// in order.
+// Bound by latency (column, then block and neighbour, then the reduction,
+// target after target): the targets are spread over gridDim.z CTAs, each row
+// finds its run by comparing its columns (in L1 after the first target) with
+// the target's row range, and warps and parts without rows only store zeros.
+// Four 20 nm spheres (152 segments of 100 rows): 81 -> 48 us a launch.
 template <typename T>
 __global__ void __launch_bounds__(kAsmThreads) k_coarse_assemble(DeviceBatch d)
 {
@@ -132,9 +137,16 @@ __global__ void __launch_bounds__(kAsmThreads) k_coarse_assemble(DeviceBatch d)
         L = d.slice_len[p >> 5];
         base = d.slice_ptr[p >> 5];
     }
-    int j = 0;
-    for (int k = d.seg_nbr_ptr[s]; k < d.seg_nbr_ptr[s + 1]; k++) {
+    const bool warp_active = __any_sync(0xffffffffu, active);
+    const int kend = d.seg_nbr_ptr[s + 1];
+    if (part * kAsmThreads >= nrows) {  // CTA-uniform
+        for (int k = d.seg_nbr_ptr[s] + blockIdx.z; k < kend; k += gridDim.z)
+            if (threadIdx.x < 36) d.coarse_asm[((size_t)k * kAsmParts + part) * 36 + threadIdx.x] = 0.f;
+        return;
+    }
+    for (int k = d.seg_nbr_ptr[s] + blockIdx.z; k < kend; k += gridDim.z) {
         const int t = d.seg_nbr[k];
+        const int t0 = d.seg_row0[t], t1 = t0 + d.seg_rows[t];
         float C[36];
 #pragma unroll
         for (int i = 0; i < 36; i++) C[i] = 0.f;
@@ -145,6 +157,7 @@ __global__ void __launch_bounds__(kAsmThreads) k_coarse_assemble(DeviceBatch d)
                 float S[9];
 #pragma unroll
                 for (int m = 0; m < 9; m++) S[m] = 0.f;
+#pragma unroll 4
                 for (int jj = 0; jj < L; jj++) {
                     load_K<T>(d, base, jj, lane, K);
 #pragma unroll
@@ -156,31 +169,41 @@ __global__ void __launch_bounds__(kAsmThreads) k_coarse_assemble(DeviceBatch d)
                 S[8] += z;
                 add_block(C, dp, S, dp);
             }
-            while (j < L) {
+            // the run of t among the row's slots (padding slots hold the row itself)
+            int j0 = 0, j1 = 0;
+#pragma unroll 8
+            for (int j = 0; j < L; j++) {
                 const int q = d.sell_col[base + 32 * j + lane];
-                const int tq = d.seg_of_row[q];
-                if (tq > t) break;
-                if (tq == t && q != p && !(d.flags[q] & NODE_PINNED)) {
-                    load_K<T>(d, base, j, lane, K);
-                    const float4 fq = d.phi[q];
-                    const float dq[3] = {fq.x, fq.y, fq.z};
-                    add_block(C, dp, K, dq);
-                }
-                j++;
+                j0 += q != p && q < t0;
+                j1 += q != p && q < t1;
+            }
+#pragma unroll 2
+            for (int j = j0; j < j1; j++) {
+                const int q = d.sell_col[base + 32 * j + lane];
+                if (d.flags[q] & NODE_PINNED) continue;
+                load_K<T>(d, base, j, lane, K);
+                const float4 fq = d.phi[q];
+                const float dq[3] = {fq.x, fq.y, fq.z};
+                add_block(C, dp, K, dq);
             }
         }
         // fixed-order block reduction of the 36 entries: 32 by the transposed
         // butterfly, 4 by plain butterflies, then the warps in order
-        float tail[4];
+        if (warp_active) {
+            float tail[4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            float v = C[32 + i];
+            for (int i = 0; i < 4; i++) {
+                float v = C[32 + i];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            tail[i] = v;
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                tail[i] = v;
+            }
+            red[lane32][warp] = warp_sum32_transposed(C);
+            if (lane32 < 4) red[32 + lane32][warp] = tail[lane32];
+        } else {
+            red[lane32][warp] = 0.f;
+            if (lane32 < 4) red[32 + lane32][warp] = 0.f;
         }
-        red[lane32][warp] = warp_sum32_transposed(C);
-        if (lane32 < 4) red[32 + lane32][warp] = tail[lane32];
         __syncthreads();
         if (threadIdx.x < 36) {
             float v = 0.f;
@@ -477,7 +500,12 @@ void sgemm_batched(const float *A, const float *B, const float *D, float *C, int
 void launch_coarse_assemble(const DeviceBatch &d, cudaStream_t s)
 {
     if (!d.coarse || d.n_segs == 0) return;
-    const dim3 grid(d.n_segs, kAsmParts);
+    // up to eight CTAs to a row block's targets while that makes about eight
+    // CTAs to an SM (152 blocks: 81 us a launch -> 48; 1,106 blocks: 8 CTAs
+    // took 16 us more than one)
+    const int blocks = std::max(d.n_segs, d.nl_pad / kAsmThreads);
+    const int split = std::min(8, std::max(1, 8 * sgemm_sms() / blocks));
+    const dim3 grid(d.n_segs, kAsmParts, split);
     if (d.precision == PREC_FP64)
         k_coarse_assemble<double><<<grid, kAsmThreads, 0, s>>>(d);
     else
