@@ -839,9 +839,11 @@ constexpr int kStericWarps = 8;  // warps per CTA (face) of k_steric
 // queue is dealt over the warps.  The clipping is a long serial FP64 chain (64
 // issue slots an instruction) with few pairs in contact, so its length and
 // the lanes that diverge in it decide: with a lane per pair running the seven
-// in turn, two 8 nm spheres in contact took 1.97 ms.  Each pair is computed as (lower index, higher index) = FFEA's (f1, f2),
-// so both sides compute the same overlap.  Face i's side of the forces goes
-// to fforce (12 values, written here: this kernel runs first), the partners
+// in turn, a solve of two 8 nm spheres in contact took 1.97 ms, with eight
+// lanes a pair on one warp a face 0.78, now 0.42.  Each pair is computed as
+// (lower index, higher index) = FFEA's (f1, f2), so both sides compute the
+// same overlap.  Face i's side of the forces goes to fforce (12 values,
+// written here: this kernel runs first), the partners
 // that overlapped to i's steric list (a set: k_pairs skips them), the energy
 // and the pair count from the side with the lower index.
 __global__ void __launch_bounds__(32 * kStericWarps, 1) k_steric(

@@ -321,3 +321,27 @@ def test_sticky_wall_matches_oracle(ssint_type):
     kw["grid"] = (6, 1, 6)
     with pytest.raises(FfeaGpuError, match="two rows"):
         _solver(**kw)
+
+
+@pytest.mark.parametrize("ssint_type", [1, 2])
+@pytest.mark.parametrize("coarser", [1.5, 4.0])
+def test_steric_queue_in_several_batches_and_ranked_cells(ssint_type, coarser):
+    """Coarser cells: more candidates a face than one batch of the steric
+    queue (eight warps of 32) takes, and cells on both sides of the 64 faces
+    that are ordered by rank; at the tolerances of the test above."""
+    from tests.test_steric_oracle import overlapping_spheres
+    pos, faces, apex, blob, h, _ = overlapping_spheres()
+    h *= coarser
+    grid = tuple(int(v) for v in 2 * np.ceil((pos.max(0) - pos.min(0)) / h))
+    pos = pos - 0.5 * (pos.max(0) + pos.min(0)) + 0.5 * h * np.array(grid)
+    ftype = np.zeros(len(faces), np.int32)
+    emin, rmin = np.ones((1, 1)), np.full((1, 1), nm(1.0))
+    s = _solver(num_nodes=len(pos), faces=faces, face_blob=blob, face_type=ftype, emin=emin, rmin=rmin, num_blobs=2,
+                cell_size=h, grid=grid, inc_self=1, ssint_type=ssint_type, face_apex=apex, steric_factor=50.0,
+                steric_dr=5e-3)
+    f_gpu, e_gpu, p_gpu = s.forces(pos)
+    s.close()
+    f_ref, e_ref, p_ref = oracle.ssint(pos, faces, blob, ftype, emin, rmin, 2, h, grid, 1, ssint_type, apex, 50.0, 5e-3)
+    assert p_gpu == p_ref and p_ref > 0
+    np.testing.assert_allclose(f_gpu, f_ref, rtol=0, atol=1e-9 * np.abs(f_ref).max())
+    np.testing.assert_allclose(e_gpu, e_ref, rtol=1e-9, atol=1e-9 * np.abs(e_ref).max())
