@@ -2,9 +2,9 @@
 
 The library reads these knobs when a handle is created:
 
-  FFEA_GPU_CG_SMEM_SLOTS   matrix slots per row whose values the register-
-                           resident solve keeps in shared memory (the rest
-                           stream from L2); column indices are kept for all
+  FFEA_GPU_CG_SMEM_SLOTS   matrix slots per row whose values the solve
+                           on chip keeps in shared and tensor memory (the
+                           rest stream from L2)
   FFEA_GPU_CG_MAX_CTAS     cap on the persistent grid, hence on the number of
                            CG segments (one per CTA): fewer, longer segments
                            trade SM count for fewer coarse dofs and partials

@@ -14,7 +14,9 @@
 //                diagonal, and the CG start (Blob.cpp:3826-3928,
 //                NoMassCGSolver.cpp:205-230)
 //   k_cg         the whole Jacobi-PCG solve in one persistent cooperative
-//                launch (NoMassCGSolver.cpp:165-197, ConjugateGradientSolver.cpp:206-232),
+//                launch (NoMassCGSolver.cpp:165-197, ConjugateGradientSolver.cpp:206-232)
+//                with the state in memory; blobs that fit on chip take
+//                k_cg_group (cg_group.cu) instead; either way
 //                ending with the velocity / position update and the RNG
 //                stream advance (Blob.cpp:3937-3969)
 // Reductions are deterministic: fixed butterflies inside warps and CTAs, one
@@ -2405,7 +2407,7 @@ void launch_nodes(const DeviceBatch &d, cudaStream_t s, int use_given_rhs)
 // Dynamic shared memory of the memory-resident CG kernel with the coarse
 // space (coarse_mem_view): its size for the given coarse dimensions, and
 // whether the device allows it (the kernel's limit is raised to the device
-// maximum, as for the register-resident kernel).
+// maximum, as for k_cg_group).
 size_t cg_mem_defer_bytes(int precision) { return precision == PREC_FP64 ? 0 : kDeferBytes; }
 
 size_t cg_mem_coarse_bytes(int coarse_hmax)

@@ -52,9 +52,8 @@ extern "C" {
  * P A_c^-1 P^T r over six rigid modes per CG segment (a compact block of
  * about a thousand nodes), LEARNED also weights the Jacobi term per node by
  * ffea_gpu_set_smoother_weights.  Both stop on the same residual test; they
- * apply to NoMass blobs in mixed precision on the register-resident solve
- * path and fall back to JACOBI elsewhere (ffea_gpu_preconditioner reports
- * which). */
+ * apply to NoMass blobs in mixed precision and fall back to JACOBI elsewhere
+ * (ffea_gpu_preconditioner reports which). */
 #define FFEA_GPU_PRECOND_JACOBI 0
 #define FFEA_GPU_PRECOND_TWO_LEVEL 1
 #define FFEA_GPU_PRECOND_LEARNED 2
@@ -398,7 +397,7 @@ int ffea_gpu_diag_coarse(ffea_gpu_t *h, int32_t blob, int32_t *n, float *coarse_
  * binary16 bit patterns), n rows of *row_len halves (n rounded up to 8, the
  * padding zero), copied to host arrays (either may be NULL; query n and
  * *row_len first with both NULL).  n = 0 when the handle keeps no such copy
- * (no coarse space, or the register-resident kernel).  No reference
+ * (no coarse space, or the solve runs on chip).  No reference
  * counterpart. */
 int ffea_gpu_diag_coarse_half(ffea_gpu_t *h, int32_t blob, int32_t *n, int32_t *row_len, uint16_t *half_inverse,
                               float *scale);
