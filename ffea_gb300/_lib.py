@@ -130,6 +130,7 @@ SIGNATURES = {
                                            ctypes.c_void_p]),
     "ffea_gpu_preconditioner": (ctypes.c_int, [ctypes.c_void_p]),
     "ffea_gpu_selftest_barrier_timeout": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32, _ip]),
+    "ffea_gpu_selftest_solve_timeout": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32]),
     "ffea_gpu_set_smoother_weights": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32,
                                                      ctypes.POINTER(ctypes.c_float)]),
     "ffea_gpu_mpnn_num_params": (ctypes.c_int, []),

@@ -915,6 +915,36 @@ int ffea_gpu_selftest_barrier_timeout(int32_t ctas, int32_t spin_limit, int32_t 
     return FFEA_GPU_OK;
 }
 
+int ffea_gpu_selftest_solve_timeout(ffea_gpu_t *h, int32_t spin_limit, int32_t blob, int32_t segment)
+{
+    if (!h) return fail("null handle");
+    if (spin_limit < 64 || spin_limit > (1 << 22)) return fail("selftest: spin_limit must be in [64, 2^22]");
+    if (!h->dev.group) return fail("selftest: this handle does not solve on chip");
+    GroupBatch &g = h->group;
+    CK(cudaStreamSynchronize(h->stream));
+    if (blob >= 0) {
+        if (check_blob(h, blob)) return FFEA_GPU_ERROR;
+        std::vector<int32_t> ptr(g.grid + 1);
+        CK(cudaMemcpy(ptr.data(), g.ptr, ptr.size() * sizeof(int32_t), cudaMemcpyDeviceToHost));
+        std::vector<int32_t> task(ptr.back());
+        CK(cudaMemcpy(task.data(), g.task, task.size() * sizeof(int32_t), cudaMemcpyDeviceToHost));
+        const auto it = std::find(task.begin(), task.end(), h->host.bp[blob].seg_off + segment);
+        if (segment < 0 || segment >= h->host.bp[blob].seg_cnt || it == task.end())
+            return fail("selftest: no task starts at segment %d of blob %d", segment, blob);
+        const int32_t at = (int32_t)(it - task.begin());
+        task.erase(it);
+        for (int32_t &p : ptr) p -= p > at;
+        CK(cudaMemcpy(g.task, task.data(), task.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(g.ptr, ptr.data(), ptr.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    }
+    g.spin_limit = (uint32_t)spin_limit;
+    // the step graphs hold the plan by value: capture them again
+    if (h->step_exec) cudaGraphExecDestroy(h->step_exec);
+    if (h->step_exec_coarse) cudaGraphExecDestroy(h->step_exec_coarse);
+    h->step_exec = h->step_exec_coarse = nullptr;
+    return FFEA_GPU_OK;
+}
+
 int ffea_gpu_set_smoother_weights(ffea_gpu_t *h, int32_t blob, const float *omega)
 {
     if (check_blob(h, blob)) return FFEA_GPU_ERROR;

@@ -135,13 +135,13 @@ __device__ __forceinline__ float ld_stream(const float *p, uint64_t pol)
 }
 __device__ __forceinline__ double ld_stream(const double *p, uint64_t) { return __ldg(p); }
 
-constexpr unsigned int kGroupSpins = 1u << 22;  // reads of one word, a few seconds, then give up
-
-// Whether a wait goes on: bounded, and given up when another wait of the CTA
-// or of the grid has run out (bar[4]).  A wait that runs out raises both.
-__device__ __noinline__ bool keep_waiting(unsigned int &spins, volatile int *s_err, unsigned int *bar)
+// Whether a wait goes on: for GroupBatch::spin_limit reads, and given up when
+// another wait of the CTA or of the grid has run out (bar[4]).  A wait that
+// runs out raises both.
+__device__ __noinline__ bool keep_waiting(unsigned int &spins, unsigned int limit, volatile int *s_err,
+                                          unsigned int *bar)
 {
-    if ((++spins & 63u) == 0 && (spins > kGroupSpins || *s_err || ((volatile unsigned int *)bar)[4])) {
+    if ((++spins & 63u) == 0 && (spins > limit || *s_err || ((volatile unsigned int *)bar)[4])) {
         *s_err = 1;
         atomicExch(&bar[4], 1u);
         return false;
@@ -157,7 +157,8 @@ constexpr int kBulk = 3;
 // however many are late.
 template <int N>
 __device__ __forceinline__ void wait_words(const uint4 *p, int stride, int n, uint32_t tag, uint64_t (&lo)[N],
-                                           uint64_t (&hi)[N], volatile int *s_err, unsigned int *bar)
+                                           uint64_t (&hi)[N], unsigned int limit, volatile int *s_err,
+                                           unsigned int *bar)
 {
     unsigned int spins = 0;
     bool missing[N], any;
@@ -173,18 +174,18 @@ __device__ __forceinline__ void wait_words(const uint4 *p, int stride, int n, ui
             if (missing[g]) missing[g] = (uint32_t)(hi[g] >> 32) != tag;
             any |= missing[g];
         }
-    } while (any && keep_waiting(spins, s_err, bar));
+    } while (any && keep_waiting(spins, limit, s_err, bar));
 }
 
 // The row again until it carries the tag (the slow path of a neighbour read).
 template <typename T>
-__device__ __noinline__ PubRow<T> wait_row(const uint4 *base, int n, int row, uint32_t tag, volatile int *s_err,
-                                           unsigned int *bar)
+__device__ __noinline__ PubRow<T> wait_row(const uint4 *base, int n, int row, uint32_t tag, unsigned int limit,
+                                           volatile int *s_err, unsigned int *bar)
 {
     PubRow<T> y;
     unsigned int spins = 0;
     do y.get(base, n, row);
-    while (!y.is(tag) && keep_waiting(spins, s_err, bar));
+    while (!y.is(tag) && keep_waiting(spins, limit, s_err, bar));
     return y;
 }
 
@@ -763,7 +764,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
                     const int q = dyn<int>(gb.o_halo)[k];
                     Row y;
                     y.get(pub, d.nl_pad, q);
-                    if (!y.is(tag)) y = wait_row<T>(pub, d.nl_pad, q, tag, &s_err, d.bar);
+                    if (!y.is(tag)) y = wait_row<T>(pub, d.nl_pad, q, tag, gb.spin_limit, &s_err, d.bar);
                     put_u<kVec>(su, R * MAXT + k, y.x, y.y, y.z);
                 }
             __syncthreads();  // su
@@ -1116,7 +1117,8 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
                         for (int q = 0; q < 3; q++) sum[q] = DF{s_outs[0][2 * q], s_outs[0][2 * q + 1]};
                 } else if (sg < cnt) {
                     uint64_t lo[2], hi[2];
-                    wait_words<2>(dots + 2 * (size_t)(s_bp.seg_off + sg), 1, 2, tag, lo, hi, &s_err, d.bar);
+                    wait_words<2>(dots + 2 * (size_t)(s_bp.seg_off + sg), 1, 2, tag, lo, hi, gb.spin_limit, &s_err,
+                                  d.bar);
                     sum[0] = DF{__uint_as_float((uint32_t)lo[0]), __uint_as_float((uint32_t)(lo[0] >> 32))};
                     sum[1] = DF{__uint_as_float((uint32_t)hi[0]), __uint_as_float((uint32_t)lo[1])};
                     sum[2] = DF{__uint_as_float((uint32_t)(lo[1] >> 32)), __uint_as_float((uint32_t)hi[1])};
@@ -1165,7 +1167,8 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
 #pragma unroll 1
                 for (int i0 = tid - 32; i0 < n; i0 += kBulk * step) {
                     uint64_t lo[kBulk], hi[kBulk];
-                    wait_words<kBulk>(gr + i0, step, (n - i0 + step - 1) / step, tag, lo, hi, &s_err, d.bar);
+                    wait_words<kBulk>(gr + i0, step, (n - i0 + step - 1) / step, tag, lo, hi, gb.spin_limit, &s_err,
+                                      d.bar);
 #pragma unroll
                     for (int g = 0; g < kBulk; g++) {
                         const int i = i0 + g * step;
@@ -1270,7 +1273,11 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
             }
         }
         if (err) {
-            if (tid == 0) atomicOr(&d.status[b], BLOB_FAIL_CG | BLOB_FAIL_TIMEOUT);
+            // the blobs of the tasks that are given up with this one have not
+            // been solved either: all of them fail here
+#pragma unroll 1
+            for (int k = ti + tid; k < gb.ptr[blockIdx.x + 1]; k += NT)
+                atomicOr(&d.status[d.seg_blob[gb.task[k]]], BLOB_FAIL_CG | BLOB_FAIL_TIMEOUT);
             break;  // CTA-uniform: s_stop was read after a barrier by every thread
         }
     }

@@ -438,6 +438,15 @@ int ffea_gpu_preconditioner(ffea_gpu_t *h);
  * reported it (ctas when the time-out works).  No reference counterpart. */
 int ffea_gpu_selftest_barrier_timeout(int32_t ctas, int32_t spin_limit, int32_t *timed_out);
 
+/* Failure-detection self-test of the solve on chip, for a handle that uses it
+ * (an error otherwise): from now on a wait of the handle's solves gives up
+ * after spin_limit reads (64 to 2^22, the default), and with blob >= 0 the
+ * CTA that has the given segment of that blob leaves it out, so that the
+ * blob's other CTAs wait for values that nobody publishes.  The step then
+ * ends with FFEA_GPU_FAIL_TIMEOUT for that blob and for those still queued
+ * behind it.  No reference counterpart. */
+int ffea_gpu_selftest_solve_timeout(ffea_gpu_t *h, int32_t spin_limit, int32_t blob, int32_t segment);
+
 /* Per-node weights of the Jacobi term of the LEARNED preconditioner for one
  * blob: omega[num_nodes] in the blob's node order (secondary nodes ignored),
  * each in (0, 2].  Takes effect from the next solve.  No reference
