@@ -1288,7 +1288,9 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
         }
     }
     if (tid == 0) {
-        if (blockIdx.x == 0 && d.cg_euler && d.num_streams != d.num_blobs && !s_stop)
+        // a shared stream moves on whichever blobs failed (after a time-out
+        // too: the draws of the blobs that were solved are used up)
+        if (blockIdx.x == 0 && d.cg_euler && d.num_streams != d.num_blobs)
 #pragma unroll 1
             for (int sm = 0; sm < d.num_streams; sm++)
                 advance_stream(d.stream_state + 6 * sm, d.stream_step + sm);

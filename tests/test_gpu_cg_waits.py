@@ -32,7 +32,7 @@ def _same(a, b):
 # behind it, two to each: the left-out segment starts the second CTA's task
 @pytest.mark.parametrize("radii,segment", [((8.0, 3.0, 3.2, 3.4, 3.6), 1), ((5.0, 3.0, 3.0, 3.0, 3.0), 1),
                                            ((10.0, 3.0, 3.2, 3.4, 3.6), 2)])
-@pytest.mark.parametrize("rng_mode,preconditioner", [(0, 0), (0, 1)])
+@pytest.mark.parametrize("rng_mode,preconditioner", [(0, 0), (0, 1), (1, 0)])
 def test_a_time_out_fails_every_blob_queued_behind_it(gpulib, monkeypatch, radii, segment, rng_mode, preconditioner):
     from ffea_gb300._lib import FfeaGpuError, check
     kw = dict(rng_mode=rng_mode, preconditioner=preconditioner)
