@@ -135,18 +135,52 @@ __device__ __forceinline__ float ld_stream(const float *p, uint64_t pol)
 }
 __device__ __forceinline__ double ld_stream(const double *p, uint64_t) { return __ldg(p); }
 
-// Whether a wait goes on: for GroupBatch::spin_limit reads, and given up when
-// another wait of the CTA or of the grid has run out (bar[4]).  A wait that
-// runs out raises both.
-__device__ __noinline__ bool keep_waiting(unsigned int &spins, unsigned int limit, volatile int *s_err,
-                                          unsigned int *bar)
+// The bounds of a wait: the published sums of all n segments, the reads after
+// which they are looked at, and the flags of a wait that ran out.
+struct WaitBound {
+    const uint4 *words;
+    int n;
+    unsigned int limit;
+    volatile int *s_err;
+    unsigned int *bar;
+};
+
+// Whether a wait goes on.  It is given up when another wait of the CTA or of
+// the grid has run out (bar[4]), or when no solve of the grid has got on in
+// GroupBatch::spin_limit reads; a wait that runs out raises both flags.  The
+// CTAs waited for may still be solving the blobs before this one, for as long
+// as those take: the tags of the dot terms, which every exchange of every
+// segment moves up, tell whether anything does.
+constexpr unsigned int kGaveUp = ~0u;
+__device__ __noinline__ uint64_t check_wait(unsigned int spins, unsigned int seen, const WaitBound &w)
 {
-    if ((++spins & 63u) == 0 && (spins > limit || *s_err || ((volatile unsigned int *)bar)[4])) {
-        *s_err = 1;
-        atomicExch(&bar[4], 1u);
-        return false;
+    bool out = *w.s_err || ((volatile unsigned int *)w.bar)[4];
+    if (!out && spins > w.limit) {
+        unsigned int sum = 0;
+#pragma unroll 4
+        for (int k = 0; k < 2 * w.n; k++) {  // (two words of dot terms a segment, two buffers)
+            uint64_t lo, hi;
+            ld_b128(w.words + 2 * (size_t)k, lo, hi);
+            sum += (unsigned int)(hi >> 32);
+        }
+        out = sum == seen;
+        seen = sum;
+        spins = 0;
     }
-    return true;
+    if (out) {
+        *w.s_err = 1;
+        atomicExch(&w.bar[4], 1u);
+        spins = kGaveUp;
+    }
+    return pack2(spins, seen);
+}
+__device__ __forceinline__ bool keep_waiting(unsigned int &spins, unsigned int &seen, const WaitBound &w)
+{
+    if ((++spins & 63u) != 0) return true;
+    const uint64_t s = check_wait(spins, seen, w);
+    spins = (unsigned int)s;
+    seen = (unsigned int)(s >> 32);
+    return spins != kGaveUp;
 }
 
 // Words a thread waits for at once when it reads the restrictions.
@@ -157,10 +191,9 @@ constexpr int kBulk = 3;
 // however many are late.
 template <int N>
 __device__ __forceinline__ void wait_words(const uint4 *p, int stride, int n, uint32_t tag, uint64_t (&lo)[N],
-                                           uint64_t (&hi)[N], unsigned int limit, volatile int *s_err,
-                                           unsigned int *bar)
+                                           uint64_t (&hi)[N], const WaitBound &w)
 {
-    unsigned int spins = 0;
+    unsigned int spins = 0, seen = ~0u;
     bool missing[N], any;
 #pragma unroll
     for (int g = 0; g < N; g++) missing[g] = g < n;
@@ -174,18 +207,17 @@ __device__ __forceinline__ void wait_words(const uint4 *p, int stride, int n, ui
             if (missing[g]) missing[g] = (uint32_t)(hi[g] >> 32) != tag;
             any |= missing[g];
         }
-    } while (any && keep_waiting(spins, limit, s_err, bar));
+    } while (any && keep_waiting(spins, seen, w));
 }
 
 // The row again until it carries the tag (the slow path of a neighbour read).
 template <typename T>
-__device__ __noinline__ PubRow<T> wait_row(const uint4 *base, int n, int row, uint32_t tag, unsigned int limit,
-                                           volatile int *s_err, unsigned int *bar)
+__device__ __noinline__ PubRow<T> wait_row(const uint4 *base, int n, int row, uint32_t tag, const WaitBound &w)
 {
     PubRow<T> y;
-    unsigned int spins = 0;
+    unsigned int spins = 0, seen = ~0u;
     do y.get(base, n, row);
-    while (!y.is(tag) && keep_waiting(spins, limit, s_err, bar));
+    while (!y.is(tag) && keep_waiting(spins, seen, w));
     return y;
 }
 
@@ -457,6 +489,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
     __shared__ DF s_last[3];                 // the sums of the last transition
     __shared__ BlobParams s_bp;
     __shared__ int s_err, s_stop;
+    __shared__ WaitBound s_bound;
     __shared__ uint32_t s_tmem;
     constexpr bool kTmem = MAXT > 256;
     constexpr int kBlockWords = 9 * (int)sizeof(T) / 4;
@@ -476,7 +509,10 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
     uint32_t maxseq = 0;
     const uint64_t pol = kWide ? stream_policy() : 0;
     int maxloops = 0;
-    if (tid == 0) s_err = s_stop = 0;
+    if (tid == 0) {
+        s_err = s_stop = 0;
+        s_bound = {gb.words, d.n_segs, gb.spin_limit, &s_err, d.bar};
+    }
     uint32_t tmem = 0;  // the warp's part: its lanes, and its share of their columns
     if constexpr (kTmem) {
         if (gb.tmem_slots > 0) {
@@ -764,7 +800,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
                     const int q = dyn<int>(gb.o_halo)[k];
                     Row y;
                     y.get(pub, d.nl_pad, q);
-                    if (!y.is(tag)) y = wait_row<T>(pub, d.nl_pad, q, tag, gb.spin_limit, &s_err, d.bar);
+                    if (!y.is(tag)) y = wait_row<T>(pub, d.nl_pad, q, tag, s_bound);
                     put_u<kVec>(su, R * MAXT + k, y.x, y.y, y.z);
                 }
             __syncthreads();  // su
@@ -1096,10 +1132,11 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
             if (warp == 0 && l < (COARSE ? 6 : 2) && (pq == 0 || (pq < R && nsl[R - 1] > 0))) {
                 const int q = R == 1 ? 0 : pq;
                 const float a = s_outs[q][3 * l], b2 = s_outs[q][3 * l + 1], c = s_outs[q][3 * l + 2];
-                if (!solo) {
+                // (a blob of one segment publishes its dot terms for the waits' sake alone)
+                if (!solo || l < 2) {
                     uint4 *o = l < 2 ? dots + 2 * (size_t)(seg + q) + l : rest + 4 * (size_t)(seg + q) + l - 2;
                     st_b128(o, pack2(__float_as_uint(a), __float_as_uint(b2)), pack2(__float_as_uint(c), tag));
-                } else if (l >= 2) {
+                } else {
                     float *o = swr + 3 * (l - 2);  // (sww follows: one segment)
                     o[0] = a;
                     o[1] = b2;
@@ -1117,8 +1154,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
                         for (int q = 0; q < 3; q++) sum[q] = DF{s_outs[0][2 * q], s_outs[0][2 * q + 1]};
                 } else if (sg < cnt) {
                     uint64_t lo[2], hi[2];
-                    wait_words<2>(dots + 2 * (size_t)(s_bp.seg_off + sg), 1, 2, tag, lo, hi, gb.spin_limit, &s_err,
-                                  d.bar);
+                    wait_words<2>(dots + 2 * (size_t)(s_bp.seg_off + sg), 1, 2, tag, lo, hi, s_bound);
                     sum[0] = DF{__uint_as_float((uint32_t)lo[0]), __uint_as_float((uint32_t)(lo[0] >> 32))};
                     sum[1] = DF{__uint_as_float((uint32_t)hi[0]), __uint_as_float((uint32_t)lo[1])};
                     sum[2] = DF{__uint_as_float((uint32_t)(lo[1] >> 32)), __uint_as_float((uint32_t)hi[1])};
@@ -1167,8 +1203,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_cg_group(DeviceBatch d, GroupBatch 
 #pragma unroll 1
                 for (int i0 = tid - 32; i0 < n; i0 += kBulk * step) {
                     uint64_t lo[kBulk], hi[kBulk];
-                    wait_words<kBulk>(gr + i0, step, (n - i0 + step - 1) / step, tag, lo, hi, gb.spin_limit, &s_err,
-                                      d.bar);
+                    wait_words<kBulk>(gr + i0, step, (n - i0 + step - 1) / step, tag, lo, hi, s_bound);
 #pragma unroll
                     for (int g = 0; g < kBulk; g++) {
                         const int i = i0 + g * step;

@@ -128,7 +128,7 @@ struct GroupBatch {
     // exchange: GRP_WORDS words of sums per segment and exchange parity; the
     // published u per row
     uint4 *words = nullptr, *pub = nullptr;
-    uint32_t spin_limit = 1u << 22;  // reads of a word (about 0.7 s), then a wait gives up
+    uint32_t spin_limit = 1u << 22;  // reads of a word (about 0.7 s) without progress anywhere, then a wait gives up
     // byte offsets into the dynamic shared memory
     int32_t o_state = 0, o_u = 0, o_halo = 0, o_words = 0, o_phi = 0, o_xrow = 0, o_h = 0, o_col = 0, o_kv2 = 0,
             o_kv1 = 0;

@@ -440,7 +440,8 @@ int ffea_gpu_selftest_barrier_timeout(int32_t ctas, int32_t spin_limit, int32_t 
 
 /* Failure-detection self-test of the solve on chip, for a handle that uses it
  * (an error otherwise): from now on a wait of the handle's solves gives up
- * after spin_limit reads (64 to 2^22, the default), and with blob >= 0 the
+ * after spin_limit reads (64 to 2^22, the default) in which no blob's solve
+ * has got on, and with blob >= 0 the
  * CTA that has the given segment of that blob leaves it out, so that the
  * blob's other CTAs wait for values that nobody publishes.  The step then
  * ends with FFEA_GPU_FAIL_TIMEOUT for that blob and for those still queued

@@ -12,10 +12,11 @@ pytestmark = pytest.mark.gpu
 FAIL_TIMEOUT = 8
 
 
-def _world(monkeypatch, radii, max_ctas, **kw):
+def _world(monkeypatch, radii, max_ctas, epsilon=None, **kw):
     from ffea_gb300.world import World
     monkeypatch.setenv("FFEA_GPU_CG_MAX_CTAS", str(max_ctas))
-    specs = [spec(radius_nm=r, seed=i + 1, rng_seed=60 + i, precision=P.PRECISION_MIXED, epsilon=1e-6)
+    specs = [spec(radius_nm=r, seed=i + 1, rng_seed=60 + i, precision=P.PRECISION_MIXED,
+                  epsilon=epsilon[i] if epsilon else 1e-6)
              for i, r in enumerate(radii)]
     return World(specs, **kw)
 
@@ -55,3 +56,21 @@ def test_a_time_out_fails_every_blob_queued_behind_it(gpulib, monkeypatch, radii
                 else:  # as without the time-out, its draws and its stream's state too
                     assert _same(now[i], ref[i]), (step, i)
             assert bits[0] and any(bits[1:]) and not all(bits[1:]), bits
+
+
+# a CTA that is free early waits for its next blob's other CTA through the whole solve of the blob before: three and two
+# CTAs of two segments each on four CTAs; a blob of two segments behind one solve that is long and one that is short
+@pytest.mark.parametrize("radii,epsilon,max_ctas", [((10.0, 8.0), (1e-6, 1e-6), 4),
+                                                    ((6.4, 6.4, 7.0), (1e-6, 0.5, 1e-6), 2)])
+def test_a_wait_lasts_through_another_blobs_solve(gpulib, monkeypatch, radii, epsilon, max_ctas):
+    """The limit, 256 reads (about 50 us), is many iterations long and shorter
+    than a solve: a blob that waits longer than that for CTAs that get on with
+    another solve is solved as with the default limit."""
+    from ffea_gb300._lib import check
+    with _world(monkeypatch, radii, max_ctas, epsilon) as w, _world(monkeypatch, radii, max_ctas, epsilon) as free:
+        check(gpulib.ffea_gpu_selftest_solve_timeout(w.handle, 256, -1, 0))
+        for step in range(3):
+            free.run(1)
+            w.run(1)
+            for i, (a, b) in enumerate(zip(_state(w), _state(free))):
+                assert w.blob(i).status()["fail_bits"] == 0 and _same(a, b), (step, i)
