@@ -1069,19 +1069,18 @@ __global__ void __launch_bounds__(32 * kPairWarps, kPairCtas) k_pairs(
         }
         const double apaq = area * __ldg(gp + 16 * (long long)j + 12);
         const int bj = fblob[j];
+        const bool lower = i < j;
         double q[9];
 #pragma unroll
         for (int c = 0; c < 9; c++) q[c] = oth[c];
         if (corr) {
             // periodic: f1's points minus blob_corr[b2][b1]
-            // (Face::barycentric_calc_point_f2, src/Face.cpp:271-277), the
-            // same as the partner's minus blob_corr[bi][bj] on either side
-            // (blob_corr is antisymmetric)
-            const double *c = corr + 3 * ((long long)bi * num_blobs + bj);
+            // (Face::barycentric_calc_point_f2, src/Face.cpp:271-277), as a
+            // shift of the partner's points seen from either side
+            const double *c = corr + 3 * (lower ? (long long)bj * num_blobs + bi : (long long)bi * num_blobs + bj);
 #pragma unroll
-            for (int k = 0; k < 9; k++) q[k] -= c[k % 3];
+            for (int k = 0; k < 9; k++) q[k] += lower ? c[k % 3] : -c[k % 3];
         }
-        const bool lower = i < j;
         const int tt = lower ? ti * num_types + ftype[j] : ftype[j] * num_types + ti;
         const double en = pot_pair<POT>(own, q, apaq, lower, emin[tt], rmin[tt], k0 ? k0[tt] : 0.0, S);
         if (lower) {
