@@ -490,11 +490,15 @@ __device__ __forceinline__ void st_add_unique(double (*pts)[3], float (*off)[3],
     }
 }
 
-// the sign of a double from its bits (-1, 0, 1), off the FP64 pipe
+// the sign of a double from its bits (-1, 0, 1), off the FP64 pipe; a NaN,
+// which compares with nothing, has none of them
+constexpr int kStNan = 2;
 __device__ __forceinline__ int st_sign(double x)
 {
-    const int hi = __double2hiint(x);
-    return ((hi & 0x7fffffff) | __double2loint(x)) == 0 ? 0 : hi < 0 ? -1 : 1;
+    const int hi = __double2hiint(x), lo = __double2loint(x), mag = hi & 0x7fffffff;
+    if ((mag | lo) == 0) return 0;
+    if (mag > 0x7ff00000 || (mag == 0x7ff00000 && lo != 0)) return kStNan;
+    return hi < 0 ? -1 : 1;
 }
 
 // increasing with atan2(y, x) over (-pi, pi], without its cost
@@ -508,24 +512,27 @@ __constant__ int c_tri[4][3] = {{1, 2, 3}, {0, 2, 3}, {0, 1, 3}, {0, 1, 2}};
 
 // clip P by n . x <= off; false when nothing is left.  A vertex's distance is
 // formed once and kept, and its sign read from its bits: comparisons run on
-// the FP64 pipe too.
+// the FP64 pipe too.  What a NaN decides is what it decides in comparisons
+// (a distance from a node at infinity): it is not inside, starts no crossing,
+// and as the first of the distances it leaves their range open.
 __device__ bool st_clip(StPolyh &P, const double *nrm, double off, const double *org, float far, double tol2)
 {
     double sd[kStF][kStV];
-    bool neg = false, pos = false;
+    bool neg = false, pos = false, open = false;
     for (int f = 0; f < P.nf; f++)
         for (int k = 0; k < P.n[f]; k++) {
             const double sv = st_dot(nrm, P.v[f][k]) - off;
             const int g = st_sign(sv);
             sd[f][k] = sv;
             neg |= g < 0;
-            pos |= g > 0;
+            pos |= g == 1;
+            open |= f == 0 && k == 0 && g == kStNan;
         }
-    if (!neg) {
+    if (!neg && !open) {
         P.nf = 0;
         return false;
     }
-    if (!pos) return true;
+    if (!pos && !open) return true;
     double cap[kStC][3];
     float capf[kStC][3];
     int nc = 0, nf = 0;
@@ -547,7 +554,7 @@ __device__ bool st_clip(StPolyh &P, const double *nrm, double off, const double 
                 }
                 if (ga == 0) st_add_unique(cap, capf, nc, kStC, a, org, far, tol2);
             }
-            if (ga * gb < 0) {
+            if (ga * gb == -1) {
                 const double t = sa / (sa - sb);
                 double x[3];
                 for (int c = 0; c < 3; c++) x[c] = a[c] + t * (b[c] - a[c]);

@@ -47,3 +47,26 @@ def test_corrections_of_either_order_of_the_blobs():
     got = s.forces(pos)
     s.close()
     _compare(got, _oracle(kw, pos, blob_corr=corr))
+
+
+@pytest.mark.parametrize("ssint_type", [1, 3])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, -np.nan])
+def test_fourth_nodes_that_are_not_finite(ssint_type, value):
+    """A face whose element's fourth node is at infinity (a blob that blew up)
+    has no overlap volume with the other blob's faces: those keep finite
+    forces, the same as the oracle's, and the pairs stay the same."""
+    from ffea_gb300.surface import LJSurfaceSolver
+    kw, pos = _inputs(ssint_type, 0, seed=19)
+    surface = np.unique(kw["faces"])
+    inner = np.setdiff1d(kw["face_apex"][kw["face_blob"] == 1], surface)
+    inner = inner[np.argsort(pos[inner, 0])][:12]  # those nearest the contact
+    pos = pos.copy()
+    pos[inner[::2], 0] = value
+    pos[inner[1::2]] = value
+    s = LJSurfaceSolver(**kw)
+    got = s.forces(pos)
+    s.close()
+    ref = _oracle(kw, pos)
+    own = np.arange(len(pos)) < len(pos) // 2
+    assert np.isfinite(ref[0][own]).all()
+    _compare((got[0][own], got[1], got[2]), (ref[0][own], ref[1], ref[2]))
