@@ -8,11 +8,12 @@
 // 701-771), together with the nearest-neighbour grid they walk
 // (NearestNeighbourLinkedListCube::build_nearest_neighbour_lookup,
 // src/NearestNeighbourLinkedListCube.cpp:27-76) and the aggregation of face
-// forces onto nodes (src/Blob.cpp:3841-3851).  The steric types first run
-// k_steric (overlap volume of the two element tetrahedra by convex clipping,
-// its forward-difference gradient and FFEA's barycentric weights, between
-// steps 4 and 5 below), whose force lands on the four nodes of each face's
-// element; k_pairs then skips the pairs k_steric handled.
+// forces onto nodes (src/Blob.cpp:3841-3851).  The steric types first run,
+// between steps 4 and 5 below, k_steric_find (the faces that have partners
+// whose tetrahedra may overlap theirs) and k_steric (overlap volume of the two
+// element tetrahedra by convex clipping, its forward-difference gradient and
+// FFEA's barycentric weights) on those, whose force lands on the four nodes of
+// each face's element; k_pairs then skips the pairs k_steric handled.
 //
 // GPU layout and passes (one stream, no host round trip between them):
 //   1. k_face_geom   one thread per active face: gathers its three corners,
@@ -51,6 +52,7 @@
 // by the FP64 pipe.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
 
 #include <cmath>
@@ -81,12 +83,16 @@ struct ffea_gpu_ssint {
     double *d_geo = nullptr;    // 16 doubles: corners (9), unit normal (3), area, fourth node (3)
     double *d_gp = nullptr;     // 16 doubles: Gauss points (9), unit normal (3), area, centroid (3)
     float4 *d_nb = nullptr;     // the normal in FP32 and the blob (its bits)
+    float4 *d_box = nullptr;    // steric types: two, the element tetrahedron's bounding box in FP32, rounded outwards
     int *d_cell = nullptr;      // -1: outside the box
     double *d_fforce = nullptr; // 12 doubles: force on each corner and on the fourth node
     double *d_corr = nullptr;   // periodic blob corrections (num_blobs^2 x 3), when set
     int has_corr = 0, sticky = 0;
-    int *d_stlist = nullptr;    // steric types: the partners whose tetrahedra overlap (MAX_STERIC_PARTNERS each)
+    // steric types: per face its candidates (MAX_STERIC_PARTNERS kept), then the partners whose tetrahedra overlap
+    int *d_stlist = nullptr;
     int *d_stcnt = nullptr;     // their number per face
+    int *d_stwork = nullptr;    // the faces with candidates
+    int sms = 0;
     // grid
     int *d_count = nullptr;     // ncell
     int *d_start = nullptr;     // ncell, block-local exclusive prefix
@@ -99,13 +105,14 @@ struct ffea_gpu_ssint {
     double *d_emin = nullptr, *d_rmin = nullptr, *d_k0 = nullptr;
     double *d_pos = nullptr, *d_force = nullptr, *d_energy = nullptr;  // staging of the host entry point
     unsigned long long *d_stats = nullptr;  // [0] pairs, [1] out-of-box faces, [2] large cells, [3] oversized cells,
-                                            // [4] faces with too many steric partners
+                                            // [4] faces with too many steric partners, [5] with steric candidates, [6] of those given out
     int *d_large = nullptr;                 // cells of more than kSortSmall faces (k_sort_large)
 };
 
 namespace {
 
 constexpr int kScanBlock = 1024;
+constexpr int kStats = 7;
 
 int fail(const char *fmt, ...)
 {
@@ -141,8 +148,8 @@ __device__ __forceinline__ int wrap(int x, int n)
 
 __global__ void k_face_geom(const double *__restrict__ pos, const int *__restrict__ corner, int nf, double h,
                             int nx, int ny, int nz, const int *__restrict__ fblob, double *__restrict__ geo,
-                            double *__restrict__ gp, float4 *__restrict__ nb, int *__restrict__ cell,
-                            int *__restrict__ count, unsigned long long *stats)
+                            double *__restrict__ gp, float4 *__restrict__ nb, float4 *__restrict__ box,
+                            int *__restrict__ cell, int *__restrict__ count, unsigned long long *stats)
 {
     int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= nf) return;
@@ -188,6 +195,18 @@ __global__ void k_face_geom(const double *__restrict__ pos, const int *__restric
     }
     q[12] = g[12];
     nb[f] = make_float4((float)g[9], (float)g[10], (float)g[11], __int_as_float(fblob[f]));
+    if (box) {  // steric types: the element tetrahedron's bounding box, rounded outwards
+        float b[6];
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            b[d] = fminf(fminf(__double2float_rd(v[0][d]), __double2float_rd(v[1][d])),
+                         fminf(__double2float_rd(v[2][d]), __double2float_rd(g[13 + d])));
+            b[3 + d] = fmaxf(fmaxf(__double2float_ru(v[0][d]), __double2float_ru(v[1][d])),
+                             fmaxf(__double2float_ru(v[2][d]), __double2float_ru(g[13 + d])));
+        }
+        box[2 * (long long)f] = make_float4(b[0], b[1], b[2], 0.f);
+        box[2 * (long long)f + 1] = make_float4(b[3], b[4], b[5], 0.f);
+    }
     int c[3];
     const int dims[3] = {nx, ny, nz};
     bool inside = true;
@@ -624,7 +643,7 @@ __device__ bool st_clip(StPolyh &P, const double *nrm, double off, const double 
 }
 
 // overlap volume of tetrahedra A and B (4 x 3 each); with cm, FFEA's centre
-__device__ double st_overlap(const double (*A)[3], const double (*B)[3], double *cm)
+__device__ __noinline__ double st_overlap(const double (*A)[3], const double (*B)[3], double *cm)
 {
     double ext = 0.0;
     for (int i = 0; i < 4; i++)
@@ -836,183 +855,422 @@ __device__ __forceinline__ bool admits(int i, int j, float4 ni, const float4 *__
     return !(A[9] * G[9] + A[10] * G[10] + A[11] * G[11] > 0.0);
 }
 
-constexpr int kStericWarps = 8;  // warps per CTA (face) of k_steric
-
-// The steric part of the steric types, one CTA per face i in cell order: every
-// partner j of the 27 cells that consider_interaction admits and whose element
-// tetrahedron's bounding box meets i's is queued in candidate order.  A pair
-// needs seven overlap volumes (its own and six with one tetrahedron moved, for
-// the forward differences): eight lanes take a pair, one volume each, and the
-// queue is dealt over the warps.  The clipping is a long serial FP64 chain (64
-// issue slots an instruction) with few pairs in contact, so its length and
-// the lanes that diverge in it decide: with a lane per pair running the seven
-// in turn, a solve of two 8 nm spheres in contact took 1.97 ms, with eight
-// lanes a pair on one warp a face 0.78, now 0.42.  Each pair is computed as
-// (lower index, higher index) = FFEA's (f1, f2), so both sides compute the
-// same overlap.  Face i's side of the forces goes to fforce (12 values,
-// written here: this kernel runs first), the partners
-// that overlapped to i's steric list (a set: k_pairs skips them), the energy
-// and the pair count from the side with the lower index.
-__global__ void __launch_bounds__(32 * kStericWarps, 1) k_steric(
-    const double *__restrict__ geo, const double *__restrict__ gp, const float4 *__restrict__ nb,
-    const int *__restrict__ sorted, const int *__restrict__ cell, const int *__restrict__ start,
-    const int *__restrict__ block, long long ncell, int nblocks, int nx, int ny, int nz,
-    const int *__restrict__ fblob, const int *__restrict__ corner, int num_blobs, int inc_self,
-    double steric_factor, double steric_dr, const double *__restrict__ corr, double *__restrict__ fforce,
-    int *__restrict__ stlist, int *__restrict__ stcnt, double *__restrict__ energy, unsigned long long *stats)
+// Whether a face j that `admits` has let pass is a steric partner of face i as
+// far as is known without their overlap: consider_interaction takes the pair,
+// and the bounding boxes of the two element tetrahedra (lo, hi: face i's) meet.
+__device__ __forceinline__ bool steric_candidate(int i, int j, int bi, const int (&ni)[4],
+                                                 const double (&lo)[3], const double (&hi)[3],
+                                                 const double *__restrict__ geo, const double *__restrict__ gp,
+                                                 const int *__restrict__ fblob, const int *__restrict__ corner,
+                                                 int num_blobs, int inc_self, const double *__restrict__ corr)
 {
-    __shared__ int s_pre[kStericWarps][28];
-    __shared__ int s_beg[kStericWarps][27];
-    __shared__ int s_q[64 * kStericWarps];
-    __shared__ int s_cnt[kStericWarps];
-    __shared__ int s_listed;
-    __shared__ double s_out[kStericWarps][12];
-    const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long w = blockIdx.x;
-    if (w >= block[nblocks]) return;  // CTA-uniform
-    if (stats[3]) return;             // the call fails (a cell too full to sort)
-    const int i = sorted[w];
-    if (threadIdx.x == 0) s_listed = 0;
-    __syncthreads();
-    const int total = warp_cells(cell[i], nx, ny, nz, start, block, ncell, nblocks, lane, s_beg[wi], s_pre[wi]);
-    const float4 nbi = nb[i];
-    const int bi = fblob[i];
-    int ni[4];
+    const int bj = fblob[j];
+    // periodic: the partner as seen from face i, shifted by -blob_corr[bi][bj]
+    const double *cs = corr ? corr + 3 * ((long long)bi * num_blobs + bj) : nullptr;
+    int nj[4];
 #pragma unroll
-    for (int u = 0; u < 4; u++) ni[u] = corner[4 * i + u];
-    double Ti[4][3];
-    face_tet(geo, i, Ti);
-    double lo_i[3], hi_i[3];
+    for (int u = 0; u < 4; u++) nj[u] = corner[4 * j + u];
+    if (!steric_type_ok(gp + 16 * (long long)i, gp + 16 * (long long)j, bi == bj, inc_self, ni, nj, cs)) return false;
+    const double *G = geo + 16 * (long long)j;
+    bool ok = true;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        lo_i[d] = fmin(fmin(Ti[0][d], Ti[1][d]), fmin(Ti[2][d], Ti[3][d]));
-        hi_i[d] = fmax(fmax(Ti[0][d], Ti[1][d]), fmax(Ti[2][d], Ti[3][d]));
+        const double sh = cs ? cs[d] : 0.0;
+        const double a0 = G[d] - sh, a1 = G[3 + d] - sh, a2 = G[6 + d] - sh, a3 = G[13 + d] - sh;
+        const double l = fmin(fmin(a0, a1), fmin(a2, a3)), h = fmax(fmax(a0, a1), fmax(a2, a3));
+        if (h < lo[d] || l > hi[d]) ok = false;
     }
-    double out[4][3];
+    return ok;
+}
+
+// the bounding box of face i's element tetrahedron
+__device__ __forceinline__ void tet_box(const double *__restrict__ geo, int i, double (&lo)[3], double (&hi)[3])
+{
+    double T[4][3];
+    face_tet(geo, i, T);
 #pragma unroll
-    for (int u = 0; u < 4; u++)
+    for (int d = 0; d < 3; d++) {
+        lo[d] = fmin(fmin(T[0][d], T[1][d]), fmin(T[2][d], T[3][d]));
+        hi[d] = fmax(fmax(T[0][d], T[1][d]), fmax(T[2][d], T[3][d]));
+    }
+}
+
+// Whether the boxes of faces i (lo, hi) and j may meet: false only where the
+// FP64 boxes, which lie within, do not.  cs: the periodic shift of j, or null.
+__device__ __forceinline__ bool boxes_meet(float4 lo, float4 hi, const float4 *__restrict__ box, int j, const double *cs)
+{
+    float4 l = box[2 * (long long)j], h = box[2 * (long long)j + 1];
+    if (cs) {
+        l.x = __fsub_rd(l.x, __double2float_ru(cs[0]));
+        l.y = __fsub_rd(l.y, __double2float_ru(cs[1]));
+        l.z = __fsub_rd(l.z, __double2float_ru(cs[2]));
+        h.x = __fsub_ru(h.x, __double2float_rd(cs[0]));
+        h.y = __fsub_ru(h.y, __double2float_rd(cs[1]));
+        h.z = __fsub_ru(h.z, __double2float_rd(cs[2]));
+    }
+    return !(h.x < lo.x || l.x > hi.x || h.y < lo.y || l.y > hi.y || h.z < lo.z || l.z > hi.z);
+}
+
+// The faces that have steric candidates, one warp per face in cell order:
+// their number goes to stcnt, the first of them to the face's steric list,
+// the face to `work` (stats[5] of them, in no order).  A face without any is
+// done here: no partners, no steric force.  Most faces of most surfaces have
+// none, and k_steric's registers leave room for eight warps an SM: with the
+// candidates tested there, by a CTA a face, a solve of two 30 nm spheres apart
+// took 1.95 ms, 0.18 so.  The faces of the 27 cells first pass the tests in
+// FP32, which leave few of them, and those are queued for the ones in FP64
+// (64 issue slots an instruction however few lanes it has): 21 us for two 4 nm
+// spheres in contact and 93 for two 30 nm ones apart, 32 and 124 with every
+// test in FP64.
+constexpr int kFindWarps = 8;
+__global__ void __launch_bounds__(32 * kFindWarps) k_steric_find(
+    const double *__restrict__ geo, const double *__restrict__ gp, const float4 *__restrict__ nb,
+    const float4 *__restrict__ box, const int *__restrict__ sorted, const int *__restrict__ cell,
+    const int *__restrict__ start, const int *__restrict__ block, long long ncell, int nblocks, int nx, int ny, int nz,
+    const int *__restrict__ fblob, const int *__restrict__ corner, int num_blobs, int inc_self,
+    const double *__restrict__ corr, double *__restrict__ fforce, int *__restrict__ stlist, int *__restrict__ stcnt,
+    int *__restrict__ work, unsigned long long *stats)
+{
+    __shared__ int s_pre[kFindWarps][28];
+    __shared__ int s_beg[kFindWarps][27];
+    __shared__ int s_q[kFindWarps][64];
+    const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long w = (long long)blockIdx.x * kFindWarps + wi;
+    if (w >= block[nblocks]) return;  // warp-uniform
+    if (stats[3]) return;             // the call fails (a cell too full to sort)
+    const int i = sorted[w];
+    const int total = warp_cells(cell[i], nx, ny, nz, start, block, ncell, nblocks, lane, s_beg[wi], s_pre[wi]);
+    const float4 nbi = nb[i], lo32 = box[2 * (long long)i], hi32 = box[2 * (long long)i + 1];
+    const int bi = fblob[i];
+    int n = 0, qn = 0;  // candidates found, queue length (< 64): warp-uniform
+    // the tests in FP64 of the first (at most 32) of the queue
+    auto test = [&] {
+        int ni[4];
 #pragma unroll
-        for (int d = 0; d < 3; d++) out[u][d] = 0.0;
-    unsigned long long npairs = 0;
-    // the first n partners of the queue, dealt over the warps first and over
-    // a warp's four groups of lanes then
-    auto evaluate = [&](int n) {
-        const int g = lane & ~7, v = lane & 7;  // the pair's first lane, and the volume this lane takes
-        for (int q0 = wi; q0 < n; q0 += 4 * kStericWarps) {
-            const int q = q0 + kStericWarps * (lane >> 3);
-            const int j = q < n ? s_q[q] : -1;
-            const bool lower = i < j;
-            double A[4][3], B[4][3], cm[3] = {0.0, 0.0, 0.0}, vol = 0.0;
-            if (j >= 0 && v < 7) {
-                face_tet(geo, j, lower ? B : A);
-#pragma unroll
-                for (int u = 0; u < 4; u++)
-#pragma unroll
-                    for (int d = 0; d < 3; d++) (lower ? A : B)[u][d] = Ti[u][d];
-                // periodic: f2's tetrahedron minus blob_corr[b1][b2]
-                // (Face::getTetraIntersectionVolumeTotalGradientAndShapeFunctions,
-                // src/Face.cpp:517-531)
-                if (corr) {
-                    const int b1 = lower ? bi : fblob[j], b2 = lower ? fblob[j] : bi;
-                    const double *c = corr + 3 * ((long long)b1 * num_blobs + b2);
-                    for (int u = 0; u < 4; u++)
-                        for (int d = 0; d < 3; d++) B[u][d] -= c[d];
-                }
-                // lane 0: A and B; 1..3: B moved; 4..6: A moved, clipped out of B
-                const bool swap = v > 3;
-                double M[4][3];
-                for (int u = 0; u < 4; u++)
-                    for (int d = 0; d < 3; d++)
-                        M[u][d] = (swap ? A : B)[u][d] + (v > 0 && d == (v - 1) % 3 ? steric_dr : 0.0);
-                vol = st_overlap(swap ? B : A, M, v == 0 ? cm : nullptr);
-            }
-            double va[3], vb[3];
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-                vb[d] = __shfl_sync(0xffffffffu, vol, g + 1 + d);
-                va[d] = __shfl_sync(0xffffffffu, vol, g + 4 + d);
-            }
-            if (j >= 0 && v == 0 && vol != 0) {
-                steric_forces(lower ? A : B, vol, cm, vb, va, steric_dr, steric_factor, lower, out);
-                const int slot = atomicAdd(&s_listed, 1);
-                if (slot < FFEA_GPU_SSINT_MAX_STERIC_PARTNERS)
-                    stlist[FFEA_GPU_SSINT_MAX_STERIC_PARTNERS * i + slot] = j;
-                if (lower) {
-                    atomicAdd(&energy[bi * num_blobs + fblob[j]], vol * steric_factor);
-                    npairs++;
-                }
-            }
-        }
+        for (int u = 0; u < 4; u++) ni[u] = corner[4 * i + u];
+        double lo[3], hi[3];
+        tet_box(geo, i, lo, hi);
+        const int j = lane < qn ? s_q[wi][lane] : -1;
+        const bool ok =
+            j >= 0 && steric_candidate(i, j, bi, ni, lo, hi, geo, gp, fblob, corner, num_blobs, inc_self, corr);
+        const unsigned m = __ballot_sync(0xffffffffu, ok);
+        const int slot = n + __popc(m & ((1u << lane) - 1u));
+        if (ok && slot < FFEA_GPU_SSINT_MAX_STERIC_PARTNERS)
+            stlist[FFEA_GPU_SSINT_MAX_STERIC_PARTNERS * i + slot] = j;
+        n += __popc(m);
+        const int rest = max(qn - 32, 0);
+        const int moved = lane < rest ? s_q[wi][32 + lane] : 0;
+        __syncwarp();
+        if (lane < rest) s_q[wi][lane] = moved;
+        qn = rest;
+        __syncwarp();
     };
-    int qn = 0;  // CTA-uniform queue length
-    for (int base = 0; base < total; base += 32 * kStericWarps) {
-        const int k = base + threadIdx.x;
+    for (int base = 0; base < total; base += 32) {
+        const int k = base + lane;
         bool ok = false;
         int j = -1;
         if (k < total) {
             j = warp_candidate(k, s_beg[wi], s_pre[wi], sorted);
-            const double *G = geo + 16 * (long long)j;
-            const bool same = bi == fblob[j];
-            ok = admits(i, j, nbi, nb, gp, inc_self);
-            // periodic: the partner as seen from face i, shifted by
-            // -blob_corr[bi][bj]
-            const double *cs = corr ? corr + 3 * ((long long)bi * num_blobs + fblob[j]) : nullptr;
-            if (ok) {
-                int nj[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) nj[u] = corner[4 * j + u];
-                ok = steric_type_ok(gp + 16 * (long long)i, gp + 16 * (long long)j, same, inc_self, ni, nj, cs);
-            }
-            if (ok) {  // bounding boxes of the two tetrahedra
-#pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    const double sh = cs ? cs[d] : 0.0;
-                    const double a0 = G[d] - sh, a1 = G[3 + d] - sh, a2 = G[6 + d] - sh, a3 = G[13 + d] - sh;
-                    const double lo = fmin(fmin(a0, a1), fmin(a2, a3)), hi = fmax(fmax(a0, a1), fmax(a2, a3));
-                    if (hi < lo_i[d] || lo > hi_i[d]) ok = false;
-                }
-            }
+            ok = admits(i, j, nbi, nb, gp, inc_self) &&
+                 boxes_meet(lo32, hi32, box, j, corr ? corr + 3 * ((long long)bi * num_blobs + fblob[j]) : nullptr);
         }
         const unsigned m = __ballot_sync(0xffffffffu, ok);
-        if (lane == 0) s_cnt[wi] = __popc(m);
-        __syncthreads();
-        int at = qn;
-        for (int k2 = 0; k2 < kStericWarps; k2++) {
-            if (k2 == wi && ok) s_q[at + __popc(m & ((1u << lane) - 1u))] = j;
-            at += s_cnt[k2];
-        }
-        qn = at;
-        __syncthreads();  // the queue, and s_cnt free
-        if (qn > 32 * kStericWarps || base + 32 * kStericWarps >= total) {
-            evaluate(qn);
-            qn = 0;
-            __syncthreads();
-        }
+        if (ok) s_q[wi][qn + __popc(m & ((1u << lane) - 1u))] = j;
+        qn += __popc(m);
+        __syncwarp();
+        if (qn >= 32) test();
     }
+    if (qn > 0) test();
+    if (lane == 0) {
+        stcnt[i] = n;
+        if (n) work[atomicAdd(&stats[5], 1ull)] = i;
+    }
+    if (n == 0 && lane < 12) fforce[12 * (long long)i + lane] = 0.0;
+}
+
+// The steric part of the steric types for the faces that k_steric_find
+// listed.  A pair needs seven overlap volumes: its own and, where that is not
+// zero, six with one tetrahedron moved, for the forward differences.  Each is
+// computed as (lower index, higher index) = FFEA's (f1, f2), so both sides of
+// a pair compute the same overlap.  Face i's side of the forces goes to fforce
+// (12 values; this kernel runs before k_pairs), the partners that overlapped
+// to i's steric list (a set: k_pairs skips them), the energy and the pair
+// count from the side with the lower index.
+//
+// The clipping is a long chain of FP64 instructions, 64 issue slots each
+// however few lanes it has.  Few faces: the chain itself decides, and with
+// eight lanes a candidate, whose seven volumes take nearly the same course,
+// and the candidates over many warps it is run about once.  Many faces: the
+// FP64 pipes are busy, and the passes count; a lane per candidate for its own
+// volume and then a lane per volume for the few that overlap take fewest.
+// Lines between the ways, for a solve of two spheres in contact on 152 SMs:
+// 130 listed faces, eight warps a face 387 us, four 417; 168 faces, 452 and
+// 366; 466 faces, four warps 636 us, one 650; 903 faces, 974 and 800.  Two 8
+// nm spheres took 1.94 ms with a lane per pair running the seven volumes in
+// turn, 0.43 with eight warps a face for every face, 0.34 so; two 20 nm
+// spheres with self-interaction 3.2, 4.2 and 1.1 ms.
+constexpr int kStericWarps = 8;  // per CTA, one CTA per SM (registers)
+static_assert(FFEA_GPU_SSINT_MAX_STERIC_PARTNERS == 32, "a lane per kept candidate");
+
+struct StericArgs {
+    const double *geo, *gp;
+    const float4 *nb;
+    const int *sorted, *cell, *start, *block;
+    long long ncell;
+    int nblocks, nx, ny, nz;
+    const int *fblob, *corner;
+    int num_blobs, inc_self;
+    double factor, dr;
+    const double *corr;
+    double *fforce;
+    int *stlist, *stcnt, *work;
+    int sms;
+    double *energy;
+    unsigned long long *stats;
+};
+
+// overlap volume of the pair (i, j): v = 0 as they are, 1..3 with f2's
+// tetrahedron moved by dr along x, y or z, 4..6 with f1's (clipped out of f2)
+__device__ __forceinline__ double pair_overlap(const StericArgs &a, int i, int j, int v, double *cm)
+{
+    const int f1 = min(i, j), f2 = max(i, j);
+    double A[4][3], B[4][3];
+    face_tet(a.geo, f1, A);
+    face_tet(a.geo, f2, B);
+    // periodic: f2's tetrahedron minus blob_corr[b1][b2]
+    // (Face::getTetraIntersectionVolumeTotalGradientAndShapeFunctions,
+    // src/Face.cpp:517-531)
+    if (a.corr) {
+        const double *c = a.corr + 3 * ((long long)a.fblob[f1] * a.num_blobs + a.fblob[f2]);
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int d = 0; d < 3; d++) B[u][d] -= c[d];
+    }
+    const bool swap = v > 3;
+    double M[4][3], O[4][3];
 #pragma unroll
     for (int u = 0; u < 4; u++)
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            // (only lanes 0, 8, 16 and 24 hold a sum)
-            double t = out[u][d];
-            t += __shfl_xor_sync(0xffffffffu, t, 16);
-            t += __shfl_xor_sync(0xffffffffu, t, 8);
-            if (lane == 0) s_out[wi][3 * u + d] = t;
+            M[u][d] = (swap ? A[u][d] : B[u][d]) + (v > 0 && d == (v - 1) % 3 ? a.dr : 0.0);
+            O[u][d] = swap ? B[u][d] : A[u][d];
         }
-    unsigned long long np = npairs;
+    return st_overlap(O, M, cm);
+}
+
+// Face i's side of an overlapping pair (volume V, centre cm, volumes vb and
+// va with f2 and with f1 moved) into out, and the pair's energy; `slot`: its
+// place in the face's list
+__device__ __forceinline__ void add_steric_pair(const StericArgs &a, int i, int j, double V, const double *cm,
+                                                const double *vb, const double *va, int slot, double (&out)[4][3],
+                                                unsigned long long &npairs)
+{
+    const bool lower = i < j;
+    const int bi = a.fblob[i], bj = a.fblob[j];
+    double T[4][3];
+    face_tet(a.geo, i, T);
+    if (a.corr && !lower) {
+        const double *c = a.corr + 3 * ((long long)bj * a.num_blobs + bi);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) np += __shfl_xor_sync(0xffffffffu, np, o);
-    if (lane == 0 && np) atomicAdd(&stats[0], np);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        stcnt[i] = min(s_listed, FFEA_GPU_SSINT_MAX_STERIC_PARTNERS);
-        if (s_listed > FFEA_GPU_SSINT_MAX_STERIC_PARTNERS) atomicAdd(&stats[4], 1ull);
+        for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int d = 0; d < 3; d++) T[u][d] -= c[d];
     }
-    if (threadIdx.x < 12) {
-        double t = 0.0;
-        for (int k = 0; k < kStericWarps; k++) t += s_out[k][threadIdx.x];
-        fforce[12 * (long long)i + threadIdx.x] = t;
+    steric_forces(T, V, cm, vb, va, a.dr, a.factor, lower, out);
+    if (slot < FFEA_GPU_SSINT_MAX_STERIC_PARTNERS) a.stlist[FFEA_GPU_SSINT_MAX_STERIC_PARTNERS * i + slot] = j;
+    if (lower) {
+        atomicAdd(&a.energy[bi * a.num_blobs + bj], V * a.factor);
+        npairs++;
     }
+}
+
+// The candidates of face i by W warps (this one is number wi) into queue q,
+// evaluate(n) called for n > 0 of them at a time: the listed ones, or, where
+// there are more than the list keeps, all found again
+template <int W, typename Sync, typename Evaluate>
+__device__ __forceinline__ void steric_candidates(const StericArgs &a, int i, int wi, int lane, int *q, int *s_beg,
+                                                  int *s_pre, int *s_cnt, Sync sync, Evaluate evaluate)
+{
+    constexpr int NT = 32 * W;
+    const int t = 32 * wi + lane, cand = a.stcnt[i];
+    if (cand <= FFEA_GPU_SSINT_MAX_STERIC_PARTNERS) {
+        if (t < cand) q[t] = a.stlist[FFEA_GPU_SSINT_MAX_STERIC_PARTNERS * i + t];
+        sync();
+        evaluate(cand);
+        return;
+    }
+    if (wi == 0) {
+        const int n = warp_cells(a.cell[i], a.nx, a.ny, a.nz, a.start, a.block, a.ncell, a.nblocks, lane, s_beg, s_pre);
+        if (lane == 0) s_cnt[W] = n;
+    }
+    sync();
+    const int total = s_cnt[W], bi = a.fblob[i];
+    const float4 nbi = a.nb[i];
+    int ni[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) ni[u] = a.corner[4 * i + u];
+    double lo[3], hi[3];
+    tet_box(a.geo, i, lo, hi);
+    int qn = 0;  // queue length, the same for all warps
+#pragma unroll 1
+    for (int base = 0; base < total; base += NT) {
+        const int k = base + t;
+        const int j = k < total ? warp_candidate(k, s_beg, s_pre, a.sorted) : i;
+        const bool ok = admits(i, j, nbi, a.nb, a.gp, a.inc_self) &&
+                        steric_candidate(i, j, bi, ni, lo, hi, a.geo, a.gp, a.fblob, a.corner, a.num_blobs, a.inc_self,
+                                         a.corr);
+        const unsigned m = __ballot_sync(0xffffffffu, ok);
+        if (lane == 0) s_cnt[wi] = __popc(m);
+        sync();
+        int at = qn;
+        for (int k2 = 0; k2 < W; k2++) {
+            if (k2 == wi && ok) q[at + __popc(m & ((1u << lane) - 1u))] = j;
+            at += s_cnt[k2];
+        }
+        qn = at;
+        sync();  // the queue, and s_cnt free
+        if (qn >= 32 || base + NT >= total) {
+            if (qn > 0) evaluate(qn);
+            qn = 0;
+            sync();
+        }
+    }
+}
+
+// the sum over a warp's lanes of the twelve values of out: value v in lanes
+// 2 v and 2 v + 1 (a transposed butterfly, 16 additions)
+__device__ __forceinline__ double warp_sum12(const double (&out)[4][3], int lane)
+{
+    double v[16];
+#pragma unroll
+    for (int k = 0; k < 16; k++) v[k] = k < 12 ? out[k / 3][k % 3] : 0.0;
+#pragma unroll
+    for (int h = 8, o = 16; h >= 1; h >>= 1, o >>= 1) {
+        const bool upper = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < h; k++) {
+            const double send = upper ? v[k] : v[k + h], keep = upper ? v[k + h] : v[k];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// Shared memory of a group of W warps of k_steric
+template <int W>
+struct StericGroup {
+    int pre[28], beg[27];
+    int cnt[W + 1];
+    int q[32 * W + 32];
+    int hit[32];          // W = 1: the partners that overlap, and their six volumes
+    double vol[W == 1 ? 32 : 1][6];
+    double out[W][12];
+    int listed, next;
+};
+
+// The listed faces by groups of W warps.  W > 1: eight lanes per candidate for
+// its seven volumes, the candidates dealt over the warps first.  W = 1: a lane
+// per candidate for its volume, then a lane per volume for the six of those
+// that overlap.
+template <int W>
+__device__ __forceinline__ void steric_faces(const StericArgs &a, StericGroup<W> *groups, int nwork,
+                                             unsigned long long &npairs)
+{
+    constexpr int G = kStericWarps / W;  // groups of the CTA
+    const int lane = threadIdx.x & 31, gi = (threadIdx.x >> 5) / W, wi = (threadIdx.x >> 5) % W;
+    StericGroup<W> &s = groups[gi];
+    auto sync = [&] {
+        if constexpr (W == 1) __syncwarp();
+        else asm volatile("bar.sync %0, %1;" ::"r"(1 + gi), "n"(32 * W) : "memory");
+    };
+    int w = blockIdx.x + gridDim.x * gi;
+#pragma unroll 1
+    while (w < nwork) {
+        const int i = a.work[w];
+        double out[4][3];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int d = 0; d < 3; d++) out[u][d] = 0.0;
+        if (wi == 0 && lane == 0) {
+            s.listed = 0;
+            s.next = gridDim.x * G + (int)atomicAdd(&a.stats[6], 1ull);
+        }
+        steric_candidates<W>(a, i, wi, lane, s.q, s.beg, s.pre, s.cnt, sync, [&](int n) {
+            if constexpr (W > 1) {
+                const int g = lane & ~7, v = lane & 7;  // the pair's first lane, and the volume this lane takes
+#pragma unroll 1
+                for (int q0 = wi; q0 < n; q0 += 4 * W) {
+                    const int q = q0 + W * (lane >> 3);
+                    const int j = q < n ? s.q[q] : -1;
+                    double cm[3] = {0.0, 0.0, 0.0}, V = 0.0;
+                    if (j >= 0 && v < 7) V = pair_overlap(a, i, j, v, v == 0 ? cm : nullptr);
+                    double va[3], vb[3];
+#pragma unroll
+                    for (int d = 0; d < 3; d++) {
+                        vb[d] = __shfl_sync(0xffffffffu, V, g + 1 + d);
+                        va[d] = __shfl_sync(0xffffffffu, V, g + 4 + d);
+                    }
+                    if (v == 0 && V != 0) add_steric_pair(a, i, j, V, cm, vb, va, atomicAdd(&s.listed, 1), out, npairs);
+                }
+            } else {
+#pragma unroll 1
+                for (int q0 = 0; q0 < n; q0 += 32) {
+                    const int j = q0 + lane < n ? s.q[q0 + lane] : -1;
+                    double cm[3] = {0.0, 0.0, 0.0}, V = 0.0;
+                    if (j >= 0) V = pair_overlap(a, i, j, 0, cm);
+                    const unsigned hits = __ballot_sync(0xffffffffu, V != 0);
+                    const int m = __popc(hits), rank = __popc(hits & ((1u << lane) - 1u)), listed = s.listed;
+                    if (V != 0) s.hit[rank] = j;
+                    __syncwarp();
+#pragma unroll 1
+                    for (int t = lane; t < 6 * m; t += 32)
+                        s.vol[t / 6][t % 6] = pair_overlap(a, i, s.hit[t / 6], 1 + t % 6, nullptr);
+                    __syncwarp();
+                    if (V != 0) add_steric_pair(a, i, j, V, cm, s.vol[rank], s.vol[rank] + 3, listed + rank, out, npairs);
+                    if (lane == 0) s.listed = listed + m;
+                    __syncwarp();  // hit, vol and listed free
+                }
+            }
+        });
+        const double sum = warp_sum12(out, lane);
+        if ((lane & 1) == 0 && lane < 24) s.out[wi][lane / 2] = sum;
+        sync();
+        if (wi == 0) {
+            if (lane == 0) {
+                a.stcnt[i] = min(s.listed, FFEA_GPU_SSINT_MAX_STERIC_PARTNERS);
+                if (s.listed > FFEA_GPU_SSINT_MAX_STERIC_PARTNERS) atomicAdd(&a.stats[4], 1ull);
+            }
+            if (lane < 12) {
+                double t = 0.0;
+#pragma unroll
+                for (int k = 0; k < W; k++) t += s.out[k][lane];
+                a.fforce[12 * (long long)i + lane] = t;
+            }
+        }
+        w = s.next;
+        sync();  // the group's shared memory free
+    }
+}
+
+__global__ void __launch_bounds__(32 * kStericWarps, 1) k_steric(const __grid_constant__ StericArgs a)
+{
+    __shared__ union Shared {
+        StericGroup<8> g8[kStericWarps / 8];
+        StericGroup<4> g4[kStericWarps / 4];
+        StericGroup<1> g1[kStericWarps];
+    } s;
+    if (a.stats[3]) return;  // the call fails (a cell too full to sort)
+    const int n = (int)a.stats[5];
+    unsigned long long npairs = 0;
+    // (the lines: above)
+    if (n <= a.sms) steric_faces<8>(a, s.g8, n, npairs);
+    else if (n <= 3 * a.sms) steric_faces<4>(a, s.g4, n, npairs);
+    else steric_faces<1>(a, s.g1, n, npairs);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) npairs += __shfl_xor_sync(0xffffffffu, npairs, o);
+    if ((threadIdx.x & 31) == 0 && npairs) atomicAdd(&a.stats[0], npairs);
 }
 
 // One warp per face i (faces taken in cell order): the candidates of the 27
@@ -1324,17 +1582,20 @@ extern "C" int ffea_gpu_ssint_create(const ffea_gpu_ssint_desc *d, ffea_gpu_ssin
         // the legacy default stream and may still be in flight when
         // cudaMemcpy returns
         SSINT_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamDefault));
+        int dev = 0;
+        SSINT_CUDA(cudaGetDevice(&dev));
+        SSINT_CUDA(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, dev));
         if (dalloc(&s->d_corner, 4 * (size_t)na) || dalloc(&s->d_blob, na) || dalloc(&s->d_type, na) ||
             dalloc(&s->d_geo, 16 * (size_t)na) || dalloc(&s->d_gp, 16 * (size_t)na) || dalloc(&s->d_nb, na) || dalloc(&s->d_cell, na) || dalloc(&s->d_fforce, 12 * (size_t)na) ||
             dalloc(&s->d_count, ncell) || dalloc(&s->d_start, ncell) || dalloc(&s->d_block, s->nblocks + 1) ||
             dalloc(&s->d_binned, na) || dalloc(&s->d_sorted, na) || dalloc(&s->d_node_ptr, d->num_nodes + 1) ||
             dalloc(&s->d_node_ent, ent.size()) || dalloc(&s->d_emin, T2) || dalloc(&s->d_rmin, T2) ||
             dalloc(&s->d_pos, 3 * (size_t)d->num_nodes) || dalloc(&s->d_force, 3 * (size_t)d->num_nodes) ||
-            dalloc(&s->d_energy, (size_t)d->num_blobs * d->num_blobs) || dalloc(&s->d_stats, 5) ||
+            dalloc(&s->d_energy, (size_t)d->num_blobs * d->num_blobs) || dalloc(&s->d_stats, kStats) ||
             dalloc(&s->d_large, (size_t)na / (kSortSmall + 1) + 1))
             return FFEA_GPU_ERROR;
         if (steric && (dalloc(&s->d_stlist, (size_t)FFEA_GPU_SSINT_MAX_STERIC_PARTNERS * na) ||
-                       dalloc(&s->d_stcnt, na)))
+                       dalloc(&s->d_stcnt, na) || dalloc(&s->d_stwork, na) || dalloc(&s->d_box, 2 * (size_t)na)))
             return FFEA_GPU_ERROR;
         if (stype == FFEA_GPU_SSINT_GENSOFT && dalloc(&s->d_k0, T2)) return FFEA_GPU_ERROR;
         if (na) {
@@ -1363,9 +1624,9 @@ extern "C" void ffea_gpu_ssint_destroy(ffea_gpu_ssint_t *s)
 {
     if (!s) return;
     if (s->stream) cudaStreamSynchronize(s->stream);
-    void *bufs[] = {s->d_corner, s->d_blob, s->d_type, s->d_geo, s->d_gp, s->d_nb, s->d_cell, s->d_fforce, s->d_count,
-                    s->d_start, s->d_block, s->d_binned, s->d_sorted, s->d_node_ptr, s->d_node_ent, s->d_emin, s->d_rmin,
-                    s->d_pos, s->d_force, s->d_energy, s->d_stats, s->d_large, s->d_stlist, s->d_stcnt, s->d_k0,
+    void *bufs[] = {s->d_corner, s->d_blob, s->d_type, s->d_geo, s->d_gp, s->d_nb, s->d_box, s->d_cell, s->d_fforce,
+                    s->d_count, s->d_start, s->d_block, s->d_binned, s->d_sorted, s->d_node_ptr, s->d_node_ent, s->d_emin, s->d_rmin,
+                    s->d_pos, s->d_force, s->d_energy, s->d_stats, s->d_large, s->d_stlist, s->d_stcnt, s->d_stwork, s->d_k0,
                     s->d_corr};
     for (void *p : bufs)
         if (p) cudaFree(p);
@@ -1381,7 +1642,7 @@ extern "C" int ffea_gpu_ssint_forces_device(ffea_gpu_ssint_t *s, const double *p
     cudaStream_t st = s->stream;
     const int na = s->num_active;
     SSINT_CUDA(cudaMemsetAsync(energy, 0, sizeof(double) * s->num_blobs * s->num_blobs, st));
-    SSINT_CUDA(cudaMemsetAsync(s->d_stats, 0, sizeof(unsigned long long) * 5, st));
+    SSINT_CUDA(cudaMemsetAsync(s->d_stats, 0, sizeof(unsigned long long) * kStats, st));
     if (na == 0) {
         SSINT_CUDA(cudaMemsetAsync(force, 0, sizeof(double) * 3 * (size_t)s->num_nodes, st));
         return FFEA_GPU_OK;
@@ -1389,7 +1650,7 @@ extern "C" int ffea_gpu_ssint_forces_device(ffea_gpu_ssint_t *s, const double *p
     SSINT_CUDA(cudaMemsetAsync(s->d_count, 0, sizeof(int) * s->ncell, st));
     const int fb = (na + 127) / 128;
     k_face_geom<<<fb, 128, 0, st>>>(pos, s->d_corner, na, s->h, s->nx, s->ny, s->nz, s->d_blob, s->d_geo,
-                                    s->d_gp, s->d_nb, s->d_cell, s->d_count, s->d_stats);
+                                    s->d_gp, s->d_nb, s->d_box, s->d_cell, s->d_count, s->d_stats);
     k_scan_local<<<s->nblocks, kScanBlock, 0, st>>>(s->d_count, s->ncell, s->d_start, s->d_block);
     k_scan_blocks<<<1, kScanBlock, 0, st>>>(s->d_block, s->nblocks);
     k_scatter<<<fb, 128, 0, st>>>(s->d_cell, na, s->d_start, s->d_block, s->d_count, s->d_binned);
@@ -1400,11 +1661,20 @@ extern "C" int ffea_gpu_ssint_forces_device(ffea_gpu_ssint_t *s, const double *p
     k_sort_large<<<kSortLargeCtas, 256, 0, st>>>(s->ncell, s->nblocks, s->d_start, s->d_block, s->d_sorted,
                                                  s->d_large, s->d_stats);
     const int pw = (na + kPairWarps - 1) / kPairWarps;
-    if (s->type != FFEA_GPU_SSINT_LJ)
-        k_steric<<<na, 32 * kStericWarps, 0, st>>>(
-            s->d_geo, s->d_gp, s->d_nb, s->d_sorted, s->d_cell, s->d_start, s->d_block, s->ncell, s->nblocks, s->nx, s->ny, s->nz,
-            s->d_blob, s->d_corner, s->num_blobs, s->inc_self, s->steric_factor, s->steric_dr,
-            s->has_corr ? s->d_corr : nullptr, s->d_fforce, s->d_stlist, s->d_stcnt, energy, s->d_stats);
+    if (s->type != FFEA_GPU_SSINT_LJ) {
+        const double *corr = s->has_corr ? s->d_corr : nullptr;
+        k_steric_find<<<(na + kFindWarps - 1) / kFindWarps, 32 * kFindWarps, 0, st>>>(
+            s->d_geo, s->d_gp, s->d_nb, s->d_box, s->d_sorted, s->d_cell, s->d_start, s->d_block, s->ncell,
+            s->nblocks, s->nx, s->ny, s->nz, s->d_blob, s->d_corner, s->num_blobs, s->inc_self, corr, s->d_fforce,
+            s->d_stlist, s->d_stcnt, s->d_stwork, s->d_stats);
+        const StericArgs args{s->d_geo,    s->d_gp,  s->d_nb,      s->d_sorted, s->d_cell,        s->d_start,
+                              s->d_block,  s->ncell, s->nblocks,   s->nx,       s->ny,            s->nz,
+                              s->d_blob,   s->d_corner, s->num_blobs, s->inc_self, s->steric_factor, s->steric_dr,
+                              corr,        s->d_fforce, s->d_stlist,  s->d_stcnt,  s->d_stwork,      s->sms,
+                              energy,      s->d_stats};
+        // as many CTAs as run at a time: each takes listed faces until none is left
+        k_steric<<<std::min(na, s->sms), 32 * kStericWarps, 0, st>>>(args);
+    }
 #define SSINT_PAIRS(POT, STERIC)                                                                                   \
     k_pairs<POT, STERIC><<<pw, 32 * kPairWarps, 0, st>>>(                                                           \
         s->d_gp, s->d_nb, s->d_cell, s->d_sorted, s->d_start, s->d_block, s->ncell, s->nblocks, s->nx, s->ny, s->nz, \
@@ -1468,7 +1738,7 @@ extern "C" int ffea_gpu_ssint_blob_corr(int32_t num_blobs, const double *centroi
 extern "C" int ffea_gpu_ssint_synchronize(ffea_gpu_ssint_t *s, int64_t *pairs)
 {
     if (!s) return fail("ffea_gpu_ssint_synchronize: null handle");
-    unsigned long long st[5] = {0, 0, 0, 0, 0};
+    unsigned long long st[kStats] = {};
     SSINT_CUDA(cudaMemcpyAsync(st, s->d_stats, sizeof(st), cudaMemcpyDeviceToHost, s->stream));
     SSINT_CUDA(cudaStreamSynchronize(s->stream));
     if (pairs) *pairs = (int64_t)st[0];
