@@ -2495,7 +2495,8 @@ void launch_measurements(const DeviceBatch &d, const MeasView &m, cudaStream_t s
 template <typename T>
 static void spmv_variant_dispatch(const DeviceBatch &d, cudaStream_t s, int variant)
 {
-    const T *v = static_cast<const T *>(d.u);
+    // (the solve on chip keeps no u in memory; r holds its right-hand side)
+    const T *v = static_cast<const T *>(d.group ? d.r : d.u);
     T *o = static_cast<T *>(d.w);
     const int64_t rows = d.nl_pad;
     switch (variant) {

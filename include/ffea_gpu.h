@@ -381,8 +381,10 @@ int ffea_gpu_last_error(char *buf, size_t len);
 /* Average time (microseconds) of one standalone w = A u over every row of
  * the handle's last assembled viscosity matrix, for SpMV variant 0..3
  * (0: one thread per row with grouped loads, 1: one thread per row,
- * 2: two threads per row, 3: four threads per row).  Overwrites the solver's
- * scratch vector w. */
+ * 2: two threads per row, 3: four threads per row).  u is the start vector
+ * of the last memory-resident solve, or the right-hand side of the last solve
+ * on chip (which keeps no u in memory).  Overwrites the solver's scratch
+ * vector w. */
 int ffea_gpu_diag_spmv(ffea_gpu_t *h, int32_t variant, int32_t reps, double *us_per_spmv);
 
 /* The two-level preconditioner's dense coarse matrix A_c of one blob and
