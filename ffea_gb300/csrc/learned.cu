@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(4 * kFwdRows) k_layer(DeviceBatch d, const flo
             a[i] = fmaf(w.w, h[3], fmaf(n.w, m[3], a[i]));
         }
     }
-    __nv_bfloat162 o[O / 2];
+    alignas(16) __nv_bfloat162 o[O / 2];  // (stored as one 16-byte word)
 #pragma unroll
     for (int i = 0; i < O; i += 2) o[i / 2] = __floats2bfloat162_rn(fmaxf(a[i], 0.f), fmaxf(a[i + 1], 0.f));
     reinterpret_cast<uint4 *>(hout)[(size_t)row * 4 + (t >> 5)] = *reinterpret_cast<const uint4 *>(o);
