@@ -1420,8 +1420,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, kPairCtas) k_pairs(
 #pragma unroll
             for (int k = 0; k < h; k++) {
                 const double send = upper ? v[k] : v[k + h], keep = upper ? v[k + h] : v[k];
-                // (values 9..15 are zeros: nothing to add where both halves are)
-                if (k + h < 9 || k < 9) v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
             }
         }
         v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
