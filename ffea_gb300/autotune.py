@@ -12,18 +12,22 @@ The library reads these knobs when a handle is created:
 
 `tune` times each candidate on the batch itself (a fresh handle per
 candidate, warm-up steps, then timed steps with a device synchronisation on
-both sides) and returns the fastest; results are cached per device and batch
-signature in a JSON file, so a later run of the same batch reuses them.
+both sides) and returns the fastest; results are cached per device, batch and
+version of the kernels in a JSON file, so a later run of the same batch with
+the same kernels reuses them.
 `applied` sets a tuning for the handles created inside a `with` block.
 """
 from __future__ import annotations
 
 import contextlib
+import functools
 import hashlib
 import json
 import os
 import time
 from typing import Iterable, Sequence
+
+from .build import CSRC
 
 KNOBS = ("FFEA_GPU_CG_SMEM_SLOTS", "FFEA_GPU_CG_MAX_CTAS", "FFEA_GPU_COARSE_REFRESH")
 DEFAULT_CACHE = os.path.join(os.environ.get("XDG_CACHE_HOME", os.path.expanduser("~/.cache")), "ffea_gb300",
@@ -50,24 +54,39 @@ def applied(config: dict | None):
                 os.environ[k] = v
 
 
+@functools.lru_cache(maxsize=None)
+def kernel_version(csrc: str = CSRC) -> str:
+    """A digest of the kernels' sources: what a setting does is theirs to say
+    (the slots it caps were in shared memory alone once, then in tensor memory too)."""
+    h = hashlib.sha1()
+    for name in sorted(os.listdir(csrc)):
+        if name.endswith((".cu", ".cuh", ".cpp", ".h")):
+            h.update(name.encode())
+            with open(os.path.join(csrc, name), "rb") as fh:
+                h.update(fh.read())
+    return h.hexdigest()[:16]
+
+
 def signature(specs: Sequence, preconditioner: int) -> str:
-    """Device + batch key: GPU name and SM count, blob sizes, precision,
-    solver and preconditioner."""
+    """Device + batch + kernels key: GPU name and SM count, blob sizes,
+    precision, solver and preconditioner, and the kernels' version."""
     import torch
     p = torch.cuda.get_device_properties(torch.cuda.current_device())
     desc = {
         "gpu": p.name, "sms": p.multi_processor_count,
         "blobs": [[int(s.mesh.num_linear), int(s.mesh.num_elements), int(s.params.precision), int(s.params.solver)]
                   for s in specs],
-        "precond": int(preconditioner),
+        "precond": int(preconditioner), "kernels": kernel_version(),
     }
     return hashlib.sha1(json.dumps(desc, sort_keys=True).encode()).hexdigest()[:16]
 
 
 def candidates(sms: int) -> list[dict]:
-    """The search space: on-chip matrix slots x grid size x coarse refresh."""
+    """The search space: on-chip matrix slots x grid size x coarse refresh.
+    A CTA of about a thousand rows has room for eight slots a row, a smaller
+    one for all of them."""
     out = []
-    for slots in (0, 1, 2, 3, 64):
+    for slots in (0, 2, 4, 8, 64):
         for ctas in (sms, (3 * sms) // 4):
             for refresh in (5, 10, 25):
                 out.append({"FFEA_GPU_CG_SMEM_SLOTS": slots, "FFEA_GPU_CG_MAX_CTAS": ctas,
