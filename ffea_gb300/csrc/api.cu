@@ -707,8 +707,9 @@ int ffea_gpu_create_batch(int32_t num_blobs, const ffea_gpu_mesh *meshes, const 
     d.n_entries = (int32_t)H.sell_col.size();
     const size_t n3 = 3 * (size_t)H.nl_pad;
     CK(A.alloc(d.rhs, n3));
-    for (void **v : {&d.x, &d.r, &d.u, &d.w, &d.p, &d.s, &d.dinv})
-        CK(A.alloc_bytes(*v, n3 * ts));
+    for (void **v : {&d.x, &d.r, &d.w, &d.dinv}) CK(A.alloc_bytes(*v, n3 * ts));
+    if (!d.group)  // (the solve on chip keeps these on chip)
+        for (void **v : {&d.u, &d.p, &d.s}) CK(A.alloc_bytes(*v, n3 * ts));
     CK(A.alloc_bytes(d.u4, 4 * (size_t)H.nl_pad * ts));
     CK(A.alloc(d.det_sign, (size_t)H.ne_pad));
     CK(A.alloc_bytes(d.jinv0, 9 * (size_t)H.ne_pad * ts));
