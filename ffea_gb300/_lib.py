@@ -129,6 +129,7 @@ SIGNATURES = {
                                            ctypes.c_int32, ctypes.c_int32, ctypes.c_float, ctypes.c_float,
                                            ctypes.c_void_p]),
     "ffea_gpu_preconditioner": (ctypes.c_int, [ctypes.c_void_p]),
+    "ffea_gpu_solve_on_chip": (ctypes.c_int, [ctypes.c_void_p]),
     "ffea_gpu_selftest_barrier_timeout": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32, _ip]),
     "ffea_gpu_selftest_solve_timeout": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32]),
     "ffea_gpu_set_smoother_weights": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32,

@@ -2,9 +2,10 @@
 //
 // One persistent cooperative launch solves every blob of a batch to
 // convergence.  A blob's CG segments (at most CG_SEG_MAX_ROWS rows each) are
-// its group of CTAs, one segment per CTA.  Groups are independent: each
-// exchanges only among its own CTAs and stops when its own blob has
-// converged, and a CTA then goes on to the next segment of its list.  Every
+// its group of CTAs, a segment to each, or two in a batch with a blob of more
+// segments than CTAs.  Groups are independent: each exchanges only among its
+// own CTAs and stops when its own blob has converged, and a CTA then goes on
+// to the next task (its one or two segments of a blob) of its list.  Every
 // CTA's list follows one order of the blobs, so a group's CTAs wait for each
 // other without a cycle.
 //
@@ -35,6 +36,9 @@
 // which every CTA publishes after its last read of u; the sums alternate
 // between two buffers for the same reason.  Tags never repeat from one launch
 // to the next (the base in bar[6] grows by the tags a launch used).
+// A wait ends with its tag or, when no solve of the grid gets on any more,
+// with a time-out (check_wait): the CTA then fails the blobs of all tasks it
+// has left, and returns.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -34,7 +34,7 @@ constexpr uint8_t NODE_PINNED = 1;   // pinned or padding: identity row, zero fo
 constexpr int32_t BLOB_FAIL_INVERSION = 1;
 constexpr int32_t BLOB_FAIL_CG = 2;
 constexpr int32_t BLOB_FAIL_NAN = 4;
-constexpr int32_t BLOB_FAIL_TIMEOUT = 8;   // a grid barrier of the CG kernel gave up waiting
+constexpr int32_t BLOB_FAIL_TIMEOUT = 8;   // a wait of the CG kernel's CTAs for each other ran out
 
 struct BlobParams {
     double dt, kT, epsilon2;

@@ -24,9 +24,10 @@
 //   2. k_scan_local / k_scan_blocks   exclusive scan of the cell counts.
 //   3. k_scatter     places every face in its cell's segment.
 //   4. k_sort_cells  sorts each segment by face index (deterministic order):
-//      k_sort_large  a thread per cell of up to 64 faces, a CTA per cell of up
-//                    to 4096 (bitonic, in shared memory); a fuller cell makes
-//                    the call an error (the grid is far too coarse).
+//      k_sort_large  a thread per face ranks it among its cell's where those
+//                    are up to 64, a CTA per cell sorts up to 4096 (bitonic, in
+//                    shared memory); a fuller cell makes the call an error (the
+//                    grid is far too coarse).
 //   5. k_pairs       one warp per face, in cell order so that neighbouring
 //                    warps read the same cells: the lanes share the faces of
 //                    the 27 cells around its own and integrate the LJ force
@@ -38,18 +39,18 @@
 //                    per-blob-pair energies use FP64 atomics, so their last
 //                    bits may vary from run to run).  The pair
 //                    is always evaluated with the lower pool index as FFEA's
-//                    f1, so both sides reproduce FFEA's arithmetic.
+//                    f1, so that both sides use the same point forces.
 //   6. k_node_gather one thread per node: sums its faces' corner forces in
 //                    face order (a CSR built at creation).
 // The file is compiled with -fmad=false so that every product and sum rounds
-// as in the reference's FP64 code; cell binning and the normal test then
-// decide exactly as FFEA does.  Two deliberate differences, both in the
-// force of a pair, both changing it only at the rounding level: the unit
-// direction of each point pair is (p - q) * (1/r) where FFEA divides by r,
-// and the nine weighted terms per corner are regrouped through column sums
-// of the (symmetric) force matrix.  Together they remove three FP64 divides
-// per point pair and 216 of 243 products per pair side; the kernel is bound
-// by the FP64 pipe.
+// as in the reference's FP64 code where that decides something: cell binning,
+// and the normal test, whose FP32 form decides only what is clear of its
+// rounding.  The force of a pair differs from FFEA's at the rounding level
+// (pot_pair; bound by the FP64 pipe): Gauss points and centroids are formed
+// once a face, the point forces come from 1/r^2 with fused products (one
+// reciprocal and, for Lennard-Jones, no square root a point pair), the nine
+// weighted terms per corner are regrouped through column sums of the
+// (symmetric) force matrix, and the weights follow once per face.
 #include <cuda_runtime.h>
 
 #include <algorithm>

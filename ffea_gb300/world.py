@@ -240,6 +240,10 @@ class World:
         """The preconditioner the solves use (PRECOND_*), after fall-backs."""
         return int(L.lib().ffea_gpu_preconditioner(self._h))
 
+    def solves_on_chip(self) -> bool:
+        """Whether the solves run on chip (k_cg_group), not from memory (k_cg)."""
+        return L.lib().ffea_gpu_solve_on_chip(self._h) == 1
+
     def set_smoother_weights(self, blob: int, omega) -> None:
         """Per-node Jacobi weights of the learned preconditioner (blob node order)."""
         w = np.ascontiguousarray(omega, dtype=np.float32)

@@ -169,7 +169,7 @@ int ffea_gpu_measurements(ffea_gpu_t *h, int32_t first_blob, int32_t count, doub
 #define FFEA_GPU_FAIL_INVERSION 1  /* an element inverted (Blob::update_internal_forces' check) */
 #define FFEA_GPU_FAIL_CG 2         /* the solve did not converge in max_iterations_cg */
 #define FFEA_GPU_FAIL_NAN 4        /* non-finite values in the solve */
-#define FFEA_GPU_FAIL_TIMEOUT 8    /* a grid barrier of the solve gave up waiting */
+#define FFEA_GPU_FAIL_TIMEOUT 8    /* a wait of the solve's CTAs for each other ran out */
 int ffea_gpu_status(ffea_gpu_t *h, int32_t blob, int32_t *inverted, int32_t *cg_iters, double *true_relres,
                     int32_t *fail_bits);
 
@@ -433,6 +433,10 @@ int ffea_gpu_sizes(ffea_gpu_t *h, int64_t *linear_nodes, int64_t *elements, int6
  * fall-back rules above; -1 on a null handle.  No reference counterpart. */
 int ffea_gpu_preconditioner(ffea_gpu_t *h);
 
+/* 1 when the handle's solves run on chip (k_cg_group), 0 when they keep their
+ * state in memory (k_cg); -1 on a null handle.  No reference counterpart. */
+int ffea_gpu_solve_on_chip(ffea_gpu_t *h);
+
 /* Failure-detection self-test of the solve's grid barrier: `ctas` CTAs wait
  * for one arrival more than there are, each gives up after `spin_limit`
  * sleeps of ~32 ns and raises the barrier's time-out flag, which the solve
@@ -494,14 +498,20 @@ int ffea_gpu_phase_times(ffea_gpu_t *h, double out_ms[5]);
  * last ffea_gpu_step call): random draws (k_noise), element forces
  * (k_elements), viscosity assembly (k_assemble), coarse-space refresh (every
  * tenth step with the two-level preconditioner, else 0), node gather
- * (k_nodes), CG solve with the Euler update at its end (k_cg), and a last
- * slot, now 0, that held the separate update kernel.  No reference
- * counterpart: it exists for the per-kernel roofline. */
+ * (k_nodes), CG solve with the Euler update at its end (k_cg_group or, for
+ * batches that do not fit on chip, k_cg), and a last slot, now 0, that held
+ * the separate update kernel.  No reference counterpart: it exists for the
+ * per-kernel roofline. */
 #define FFEA_GPU_NUM_KERNEL_TIMES 7
 int ffea_gpu_kernel_times(ffea_gpu_t *h, double out_ms[FFEA_GPU_NUM_KERNEL_TIMES]);
 
 /* The handle's CUDA stream (cudaStream_t), for callers that order their own
- * work after a step. */
+ * work after a step.  While a step's solve runs, it can hold every SM it uses
+ * to itself: most of the shared memory and, with more than 256 rows to a CTA,
+ * all of the tensor memory.  Kernels of other streams wait for either until
+ * the solve ends, and a solve whose SM's tensor memory another kernel holds
+ * waits for that one (for longer than about a second, and the solve reports
+ * FFEA_GPU_FAIL_TIMEOUT). */
 void *ffea_gpu_stream(ffea_gpu_t *h);
 
 /* Execution mode: 1 = one CUDA graph per step (default); 0 = direct launches. */
